@@ -6,11 +6,13 @@
 //   mode 1 (dgrad) dx[r, :] = dy[r, :] @ W[e]^T      dy [R, N]              dx [R, K]
 //   mode 2 (wgrad) dW[e]    = x_e^T @ dy_e           contraction over the expert's rows; dW [E, K, N]
 //
-// A one-thread planner turns the device-side offsets into a tile list (expert, row block, column block); the
-// persistent CTAs (TMA producer / MMA issuer / 4 epilogue warps, TMEM double buffer: same pipeline as gemm.cu; output
-// tiles 128 x 256, or 128 x 128 when the tiled dimension is not a multiple of 256)
-// walk that list, so routing skew costs nothing but the tiles it produces.  Experts without tokens produce no
-// tiles (wgrad output is pre-zeroed by the caller).  Reference op: torch_npu.npu_grouped_matmul with group_list
+// The persistent CTAs (TMA producer / MMA issuer / 4 epilogue warps, TMEM double buffer: same pipeline as gemm.cu; output
+// tiles 128 x 256, or 128 x 128 when the tiled dimension is not a multiple of 256) number the tiles expert by expert, so
+// routing skew costs nothing but the tiles it produces.  A tile's number is turned into (expert, row block, column block)
+// where it is used: offsets are multiples of 128, so the row blocks before expert e are off[e] / 128 and a binary search
+// over the offsets finds the expert.  (A one-thread planner kernel that wrote the list down first took 210 us a call at
+// 128 experts, more than the products.)  Experts without tokens produce no rows; their wgrad tiles are written as zeros,
+// so dW needs no memset before the call.  Reference op: torch_npu.npu_grouped_matmul with group_list
 // (mindspeed_mm/fsdp/ops/moe_ops/gemm.py:16-92).
 #include "tc05.cuh"
 
@@ -35,36 +37,43 @@ struct Cfg {
 
 struct GGParams {
     const int* off;          // [E + 1] aligned row offsets (device)
-    const int* tile_e;       // planner output
-    const int* tile_m;
-    const int* tile_n;
-    const int* n_tiles;
-    int K, N;                // weight shape [E, K, N]
+    int E, K, N;             // weight shape [E, K, N]
     int* status;
 };
 
+struct Tile {
+    int e, mb, nb;           // expert, 128-row block (mode 2: block of K), column block
+};
+
 // modes 0/1: one tile per (expert row block, output column block); mode 2: per (expert, K block, N block)
-__global__ void gg_plan_kernel(const int* off, int E, int mode, int K, int N, int BN, int* tile_e, int* tile_m, int* tile_n,
-                               int* n_tiles, int max_tiles) {
-    if (threadIdx.x || blockIdx.x) return;
-    int n = 0;
-    if (mode == 2) {
-        for (int e = 0; e < E; ++e) {
-            if (off[e + 1] == off[e]) continue;
-            for (int nb = 0; nb < N / BN; ++nb)
-                for (int mb = 0; mb < K / BM && n < max_tiles; ++mb) {
-                    tile_e[n] = e; tile_m[n] = mb; tile_n[n] = nb; ++n;
-                }
-        }
-    } else {
-        const int cols = (mode == 0 ? N : K) / BN;
-        for (int e = 0; e < E; ++e)
-            for (int nb = 0; nb < cols; ++nb)
-                for (int r = off[e]; r < off[e + 1] && n < max_tiles; r += BM) {
-                    tile_e[n] = e; tile_m[n] = r / BM; tile_n[n] = nb; ++n;
-                }
+template <int MODE, int BN>
+__device__ __forceinline__ int tile_count(const GGParams& p) {
+    if (MODE == 2) return p.E * (p.K / BM) * (p.N / BN);
+    return __ldg(p.off + p.E) / BM * ((MODE == 0 ? p.N : p.K) / BN);
+}
+
+template <int MODE, int BN>
+__device__ __forceinline__ Tile tile_at(const GGParams& p, int t) {
+    Tile r;
+    if (MODE == 2) {
+        const int kb = p.K / BM, per = kb * (p.N / BN), i = t % per;
+        r.e = t / per;
+        r.nb = i / kb;
+        r.mb = i % kb;
+        return r;
     }
-    *n_tiles = n;
+    const int cols = (MODE == 0 ? p.N : p.K) / BN, row = t / cols;      // row block counted over all experts
+    int lo = 0, hi = p.E;                                               // off[lo] / BM <= row < off[hi] / BM
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(p.off + mid) / BM <= row) lo = mid;
+        else hi = mid;
+    }
+    const int first = __ldg(p.off + lo) / BM, rows = __ldg(p.off + hi) / BM - first, i = t - first * cols;
+    r.e = lo;
+    r.nb = i / rows;
+    r.mb = first + i % rows;
+    return r;
 }
 
 template <int MODE, int BN>
@@ -87,7 +96,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     volatile int* epi_stop = abort_flag + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = *p.n_tiles;
+    const int n_tiles = tile_count<MODE, BN>(p);
     auto kblocks = [&](int e) { return MODE == 2 ? (p.off[e + 1] - p.off[e]) / BK : (MODE == 0 ? p.K : p.N) / BK; };
 
     if (threadIdx.x == 0) {
@@ -120,7 +129,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             uint32_t phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                const int e = p.tile_e[t], mb = p.tile_m[t], nb = p.tile_n[t];
+                const auto [e, mb, nb] = tile_at<MODE, BN>(p, t);
                 const int kbs = kblocks(e);
                 for (int kb = 0; kb < kbs; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
@@ -162,7 +171,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             uint32_t phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++it) {
-                const int kbs = kblocks(p.tile_e[t]);
+                const int kbs = kblocks(tile_at<MODE, BN>(p, t).e);
                 const int acc = it & 1;
                 if (!mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag)) {
                     atomicExch(p.status, MM_TIMEOUT_MMA);
@@ -198,7 +207,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const bool issuer = threadIdx.x == 64;
         int it = 0, slab_count = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
-            const int e = p.tile_e[t], mb = p.tile_m[t], nb = p.tile_n[t];
+            const auto [e, mb, nb] = tile_at<MODE, BN>(p, t);
+            const bool empty_tile = MODE == 2 && kblocks(e) == 0;       // nothing was accumulated: the tile is zero
             const int acc = it & 1;
             if (!mbar_wait(&tfull[acc], (it >> 1) & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -216,6 +226,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 tmem_ld_32x32(t_row + slab * 64, r);
                 tmem_ld_32x32(t_row + slab * 64 + 32, r + 32);
                 tmem_wait_ld();
+                if (MODE == 2 && empty_tile) {
+#pragma unroll
+                    for (int j = 0; j < 64; ++j) r[j] = 0;
+                }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     uint4 v;
@@ -268,26 +282,16 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tC, 
 
 }  // namespace
 
-// Upper bound of the tile count (128-wide column blocks; the 256-wide plan has at most as many).
-MM_API int mm_grouped_gemm_max_tiles(int R, int E, int K, int N, int mode) {
-    if (mode == 2) return E * (K / BM) * (N / 128) + 1;
-    return (R / BM + E) * ((mode == 0 ? N : K) / 128) + 1;
-}
-
 // a, b, c by mode:  0: a = x [R,K], b = W [E,K,N], c = y [R,N]      1: a = dy [R,N], b = W, c = dx [R,K]
-//                   2: a = x [R,K], b = dy [R,N], c = dW [E,K,N] (zero it first)
-// off: int32 [E+1] on the device, multiples of 128, off[E] <= R.  plan: int32 scratch of 3 * max_tiles + 1.
-// K and N must be multiples of 128.
-MM_API int mm_grouped_gemm_bf16(const void* a, const void* b, void* c, const int* off, int* plan, int R, int E, int K, int N,
-                                int mode, int* status, cudaStream_t st) {
+//                   2: a = x [R,K], b = dy [R,N], c = dW [E,K,N]
+// off: int32 [E+1] on the device, multiples of 128, off[E] <= R.  K and N must be multiples of 128.  Rows from off[E] on
+// are neither read nor written.
+MM_API int mm_grouped_gemm_bf16(const void* a, const void* b, void* c, const int* off, int R, int E, int K, int N, int mode,
+                                int* status, cudaStream_t st) {
     if (K % 128 || N % 128 || R % 128 || mode < 0 || mode > 2) return -1;
-    const int max_tiles = mm_grouped_gemm_max_tiles(R, E, K, N, mode);
-    int* tile_e = plan;
-    int* tile_m = plan + max_tiles;
-    int* tile_n = plan + 2 * max_tiles;
-    int* n_tiles = plan + 3 * max_tiles;
     const int BN = ((mode == 1 ? K : N) % 256 == 0) ? 256 : 128;      // the dimension the column blocks tile
-    gg_plan_kernel<<<1, 32, 0, st>>>(off, E, mode, K, N, BN, tile_e, tile_m, tile_n, n_tiles, max_tiles);
+    const long long max_tiles = mode == 2 ? (long long)E * (K / BM) * (N / BN) : (long long)(R / BM) * ((mode == 0 ? N : K) / BN);
+    if (max_tiles > 0x7fffffffLL) return -1;
     CUtensorMap tA, tB, tC;
     int r;
     if (mode == 0) {
@@ -309,8 +313,8 @@ MM_API int mm_grouped_gemm_bf16(const void* a, const void* b, void* c, const int
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
-    GGParams p{off, tile_e, tile_m, tile_n, n_tiles, K, N, status};
-    const int grid = max_tiles - 1 < sms ? (max_tiles - 1 < 1 ? 1 : max_tiles - 1) : sms;
+    GGParams p{off, E, K, N, status};
+    const int grid = max_tiles < sms ? (max_tiles < 1 ? 1 : (int)max_tiles) : sms;
     if (BN == 256) {
         if (mode == 0) return launch<0, 256>(tA, tB, tC, p, grid, st);
         if (mode == 1) return launch<1, 256>(tA, tB, tC, p, grid, st);
@@ -340,7 +344,7 @@ __global__ void moe_permute_kernel(const bf16* __restrict__ x, const int* __rest
         reinterpret_cast<Vec8*>(out + (size_t)r * H)[c] = v;
     }
 }
-// out[t, :] = sum_s probs[t, s] * y[row_of_pair[t * k + s], :]
+// out[t, :] = sum_s probs[t, s] * y[row_of_pair[t * k + s], :]   (probs null: all ones)
 __global__ void moe_unpermute_kernel(const bf16* __restrict__ y, const int* __restrict__ row_of_pair,
                                      const bf16* __restrict__ probs, bf16* __restrict__ out, int T, int k, int H) {
     const int hv = H >> 3;
@@ -349,13 +353,136 @@ __global__ void moe_unpermute_kernel(const bf16* __restrict__ y, const int* __re
         const int t = (int)(i / hv), c = (int)(i % hv);
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int s = 0; s < k; ++s) {
-            const float w = __bfloat162float(probs[t * k + s]);
+            const float w = probs ? __bfloat162float(probs[t * k + s]) : 1.f;
             float f[8];
             unpack8(reinterpret_cast<const Vec8*>(y + (size_t)row_of_pair[t * k + s] * H)[c], f);
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] += w * f[j];
         }
         reinterpret_cast<Vec8*>(out + (size_t)t * H)[c] = pack8(acc);
+    }
+}
+
+// Backward of the weighted un-permute: dy[row of (t, s)] = probs[t, s] * g[t], dprobs[t, s] = <g[t], y[row of (t, s)]>, and
+// zeros in the pad rows (src_of_row < 0; null: there are none).  A warp owns a (token, slot) pair or a pad row, so every
+// row of y is read once and every row of dy written once; the k warps of a token sit in one block and share its row of g in L1.
+// Bound by HBM: reads y, writes dy.  4096 tokens x 8 of 2048 (49024 rows): 79 us, 4.4 TB/s; the PyTorch form
+// (repeat, multiply, index_put, gather, fp32 product, sum over 0.6 GB of temporaries) took 1.1 ms.
+__global__ void __launch_bounds__(256) moe_unpermute_bwd_kernel(
+    const bf16* __restrict__ g, const bf16* __restrict__ y, const int* __restrict__ row_of_pair,
+    const int* __restrict__ src_of_row, const bf16* __restrict__ probs, bf16* __restrict__ dy, bf16* __restrict__ dprobs,
+    int pairs, int k, int R, int H) {
+    const int lane = threadIdx.x & 31, hv = H >> 3;
+    const long long warps = (long long)gridDim.x * 8, total = (long long)pairs + (src_of_row ? R : 0);
+    for (long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); i < total; i += warps) {
+        if (i >= pairs) {
+            const int r = (int)(i - pairs);
+            if (src_of_row[r] >= 0) continue;
+            uint4* dst = reinterpret_cast<uint4*>(dy + (size_t)r * H);
+            for (int c = lane; c < hv; c += 32) dst[c] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        const Vec8* gr = reinterpret_cast<const Vec8*>(g + (size_t)(i / k) * H);
+        const size_t row = (size_t)row_of_pair[i] * H;
+        const Vec8* yr = reinterpret_cast<const Vec8*>(y + row);
+        Vec8* dr = reinterpret_cast<Vec8*>(dy + row);
+        const float w = __bfloat162float(probs[i]);
+        float dot = 0.f;
+#pragma unroll 4
+        for (int c = lane; c < hv; c += 32) {
+            float a[8], b[8];
+            unpack8(gr[c], a);
+            unpack8(yr[c], b);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                dot += a[j] * b[j];
+                a[j] *= w;
+            }
+            dr[c] = pack8(a);
+        }
+        dot = warp_sum(dot);
+        if (lane == 0) dprobs[i] = __float2bfloat16(dot);
+    }
+}
+
+// ---- routing: (token, slot) pairs -> rows of the aligned expert-major layout, pairs of an expert in their own order ----
+// A block per expert; its warps walk contiguous pieces of the pair list (coalesced, out of L2 after the first block) and
+// rank matches by ballot, so the order is that of a stable sort by expert.  Two launches, because an expert's first row
+// needs every earlier expert's count: 15 + 24 us for 32768 pairs and 128 experts, against 90 us on the device and a host
+// synchronisation for the radix sort, histogram and ten index kernels they replace.
+constexpr int kRouteWarps = 16;
+
+__device__ __forceinline__ int route_segment(int n) { return (n + kRouteWarps * 32 - 1) / (kRouteWarps * 32) * 32; }
+
+__device__ __forceinline__ int route_matches(const long long* ids, int n, int e, int a, int lane) {
+    int c = 0;
+    const int b = min(n, a + route_segment(n));
+#pragma unroll 4
+    for (int i = a + lane; i < b; i += 32) c += ids[i] == e;
+    return c;
+}
+
+__global__ void __launch_bounds__(kRouteWarps * 32) moe_count_kernel(const long long* __restrict__ ids, int n, int E,
+                                                                    int* __restrict__ counts, int* __restrict__ bad) {
+    __shared__ int red[2];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x < 2) red[threadIdx.x] = 0;
+    __syncthreads();
+    int c = route_matches(ids, n, blockIdx.x, w * route_segment(n), lane), out = 0;
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) out |= ids[i] < 0 || ids[i] >= E;
+    c = __reduce_add_sync(0xffffffffu, c);
+    out = __any_sync(0xffffffffu, out);
+    if (lane == 0) {
+        atomicAdd(&red[0], c);
+        if (out) red[1] = 1;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        counts[blockIdx.x] = red[0];
+        if (blockIdx.x == 0) *bad = red[1];
+    }
+}
+
+__global__ void __launch_bounds__(kRouteWarps * 32) moe_place_kernel(const long long* __restrict__ ids, int n, int k, int E,
+                                                                    const int* __restrict__ counts, int R, int* __restrict__ off,
+                                                                    int* __restrict__ row_of_pair, int* __restrict__ src_of_row) {
+    __shared__ int before, base[kRouteWarps + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x;
+    if (threadIdx.x == 0) before = 0;
+    __syncthreads();
+    int rows = 0;
+    for (int i = threadIdx.x; i < e; i += blockDim.x) rows += (counts[i] + 127) / 128 * 128;
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    if (lane == 0 && rows) atomicAdd(&before, rows);
+    const int a = w * route_segment(n);
+    const int mine = __reduce_add_sync(0xffffffffu, route_matches(ids, n, e, a, lane));
+    if (lane == 0) base[w + 1] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        base[0] = before;
+        for (int i = 0; i < kRouteWarps; ++i) base[i + 1] += base[i];
+    }
+    __syncthreads();
+    int row = base[w];
+    const int b = min(n, a + route_segment(n));
+    for (int i0 = a; i0 < b; i0 += 32) {
+        const int i = i0 + lane;
+        const bool hit = i < b && ids[i] == e;
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
+            const int r = row + __popc(m & ((1u << lane) - 1));
+            row_of_pair[i] = r;
+            src_of_row[r] = i / k;
+        }
+        row += __popc(m);
+    }
+    const int used = base[kRouteWarps], end = before + (counts[e] + 127) / 128 * 128;
+    for (int r = used + threadIdx.x; r < end; r += blockDim.x) src_of_row[r] = -1;
+    if (threadIdx.x == 0) off[e] = before;
+    if (e == E - 1) {                                        // rows that no expert uses
+        for (int r = end + threadIdx.x; r < R; r += blockDim.x) src_of_row[r] = -1;
+        if (threadIdx.x == 0) off[E] = end;
     }
 }
 }  // namespace
@@ -374,5 +501,27 @@ MM_API int mm_moe_unpermute(const void* y, const int* row_of_pair, const void* p
     long long work = (long long)T * (H / 8);
     int grid = (int)((work + 255) / 256 < 148 * 16 ? (work + 255) / 256 : 148 * 16);
     moe_unpermute_kernel<<<grid < 1 ? 1 : grid, 256, 0, st>>>((const bf16*)y, row_of_pair, (const bf16*)probs, (bf16*)out, T, k, H);
+    return (int)cudaGetLastError();
+}
+
+MM_API int mm_moe_unpermute_bwd(const void* g, const void* y, const int* row_of_pair, const int* src_of_row, const void* probs,
+                                void* dy, void* dprobs, int T, int k, int R, int H, cudaStream_t st) {
+    if (H % 8) return -1;
+    if (!T && !src_of_row) return 0;
+    const long long warps = (long long)T * k + (src_of_row ? R : 0), blocks = (warps + 7) / 8;
+    const int grid = (int)(blocks < 148 * 8 ? (blocks < 1 ? 1 : blocks) : 148 * 8);
+    moe_unpermute_bwd_kernel<<<grid, 256, 0, st>>>((const bf16*)g, (const bf16*)y, row_of_pair, src_of_row, (const bf16*)probs,
+                                                  (bf16*)dy, (bf16*)dprobs, T * k, k, R, H);
+    return (int)cudaGetLastError();
+}
+
+// ids: n = T * k expert numbers.  Writes off [E + 1], row_of_pair [n], src_of_row [R] (-1: pad row) with
+// R >= n + 127 * E, and *bad = 1 when an id lies outside [0, E) (such a pair gets no row: row_of_pair is set to 0 by the
+// caller beforehand or left unread).  counts: int scratch [E].
+MM_API int mm_moe_route(const long long* ids, int n, int k, int E, int R, int* counts, int* off, int* row_of_pair,
+                        int* src_of_row, int* bad, cudaStream_t st) {
+    if (E < 1 || k < 1 || R < n) return -1;
+    moe_count_kernel<<<E, kRouteWarps * 32, 0, st>>>(ids, n, E, counts, bad);
+    moe_place_kernel<<<E, kRouteWarps * 32, 0, st>>>(ids, n, k, E, counts, R, off, row_of_pair, src_of_row);
     return (int)cudaGetLastError();
 }

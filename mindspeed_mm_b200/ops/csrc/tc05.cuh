@@ -272,6 +272,14 @@ inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     }
     return fn;
 }
+// The encode call is a driver call: on a thread that has made no runtime call yet (an autograd worker whose first op is a
+// tensor-core kernel) there is no current context.  cudaFree(nullptr) binds the thread's device's primary one.
+template <class F>
+inline int encode_with_context(F encode) {
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaFree(nullptr) == cudaSuccess) r = encode();
+    return (int)r;
+}
 // 2-D bf16 tensor [rows, cols] with `ld` elements between rows; box = [box_rows, box_cols]; 128B swizzle.
 inline int make_tmap_2d(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                         uint32_t box_cols, CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_128B) {
@@ -281,10 +289,10 @@ inline int make_tmap_2d(CUtensorMap* m, const void* base, uint64_t rows, uint64_
     cuuint64_t strides[1] = {ld * 2};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t es[2] = {1, 1};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return (int)r;
+    return encode_with_context([&] {
+        return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    });
 }
 // 3-D bf16 tensor [d2, d1, d0] (d0 innermost, contiguous) with element strides s1, s2.
 inline int make_tmap_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
@@ -296,9 +304,9 @@ inline int make_tmap_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t 
     cuuint64_t strides[2] = {s1 * 2, s2 * 2};
     cuuint32_t box[3] = {b0, b1, b2};
     cuuint32_t es[3] = {1, 1, 1};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return (int)r;
+    return encode_with_context([&] {
+        return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    });
 }
 }  // namespace tc05

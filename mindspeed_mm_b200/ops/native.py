@@ -77,10 +77,11 @@ def _declare(L):
         "mm_fmha_bwd_max_tiles": [_i, _i],
         "mm_fmha_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _i, _f,
                         _i, _i, _p, _p],
-        "mm_grouped_gemm_max_tiles": [_i, _i, _i, _i, _i],
-        "mm_grouped_gemm_bf16": [_p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p],
+        "mm_grouped_gemm_bf16": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p],
         "mm_moe_permute": [_p, _p, _p, _i, _i, _p],
         "mm_moe_unpermute": [_p, _p, _p, _p, _i, _i, _i, _p],
+        "mm_moe_unpermute_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
+        "mm_moe_route": [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p],
         "mm_conv1d_fwd": [_p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_conv1d_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_l2norm_fwd": [_p, _p, _p, _ll, _i, _f, _p],
@@ -742,26 +743,37 @@ def moe_supported(tokens, gate_up, down) -> bool:
             and gate_up.shape[-1] % 256 == 0 and down.shape[-1] % 128 == 0)
 
 
-def aligned_routing(topk_ids, num_experts: int):
-    """Device-side plan of the aligned expert-major layout (no host sync): every expert's rows start at a
-    multiple of 128.  Returns (off [E+1] int32, row_of_pair [T*k] int32, src_of_row [R] int32 (-1 = pad), R)."""
+def _route(topk_ids, num_experts: int):
+    """Launches the routing kernels; returns (off, row_of_pair, src_of_row, R, check).  ``check()`` waits for them (not for
+    work queued behind them) and raises if an expert number was out of range."""
     T, k = topk_ids.shape
-    flat = topk_ids.reshape(-1)
-    order = torch.sort(flat, stable=True).indices
-    counts = torch.bincount(flat, minlength=num_experts)
-    padded = (counts + 127) // 128 * 128
-    off = torch.zeros(num_experts + 1, dtype=torch.int64, device=flat.device)
-    off[1:] = padded.cumsum(0)
-    ustart = torch.zeros(num_experts + 1, dtype=torch.int64, device=flat.device)
-    ustart[1:] = counts.cumsum(0)
-    sorted_e = flat[order]
-    rows = off[sorted_e] + (torch.arange(flat.numel(), device=flat.device) - ustart[sorted_e])
-    R = (T * k + num_experts * 127 + 127) // 128 * 128            # static upper bound of off[E]
-    row_of_pair = torch.empty(T * k, dtype=torch.int32, device=flat.device)
-    row_of_pair[order] = rows.to(torch.int32)
-    src_of_row = torch.full((R,), -1, dtype=torch.int32, device=flat.device)
-    src_of_row[rows] = (order // k).to(torch.int32)
-    return off.to(torch.int32), row_of_pair, src_of_row, R
+    dev, n = topk_ids.device, T * k
+    ids = topk_ids.to(torch.int64).contiguous()
+    R = (n + num_experts * 127 + 127) // 128 * 128            # static upper bound of off[E]
+    off = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
+    scratch = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)       # counts, out-of-range flag
+    row_of_pair = torch.zeros(n, dtype=torch.int32, device=dev)
+    src_of_row = torch.empty(R, dtype=torch.int32, device=dev)
+    _check(lib().mm_moe_route(ids.data_ptr(), n, k, num_experts, R, scratch.data_ptr(), off.data_ptr(), row_of_pair.data_ptr(),
+                              src_of_row.data_ptr(), scratch[num_experts:].data_ptr(), _st()), "moe_route")
+    bad = torch.empty(1, dtype=torch.int32, pin_memory=True)
+    bad.copy_(scratch[num_experts:], non_blocking=True)
+    done = torch.cuda.Event()
+    done.record()
+
+    def check():
+        done.synchronize()
+        if int(bad):
+            raise RuntimeError(f"expert numbers outside [0, {num_experts})")
+    return off, row_of_pair, src_of_row, R, check
+
+
+def aligned_routing(topk_ids, num_experts: int):
+    """Plan of the aligned expert-major layout: every expert's rows start at a multiple of 128.  Returns (off [E+1] int32,
+    row_of_pair [T*k] int32, src_of_row [R] int32 (-1 = pad), R)."""
+    off, row_of_pair, src_of_row, R, check = _route(topk_ids, num_experts)
+    check()
+    return off, row_of_pair, src_of_row, R
 
 
 class _AlignedPermute(torch.autograd.Function):
@@ -778,41 +790,43 @@ class _AlignedPermute(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (row_of_pair,) = ctx.saved_tensors
-        ones = torch.ones(ctx.T * ctx.k, dtype=g.dtype, device=g.device)
         out = torch.empty(ctx.T, g.shape[1], dtype=g.dtype, device=g.device)
-        _check(lib().mm_moe_unpermute(g.contiguous().data_ptr(), row_of_pair.data_ptr(), ones.data_ptr(), out.data_ptr(),
+        _check(lib().mm_moe_unpermute(g.contiguous().data_ptr(), row_of_pair.data_ptr(), None, out.data_ptr(),
                                       ctx.T, ctx.k, g.shape[1], _st()), "moe_unpermute")
         return out, None, None, None
 
 
 class _AlignedUnpermute(torch.autograd.Function):
+    """``src_of_row`` names the pad rows of ``y`` (they get zero gradients); None: every row belongs to a pair."""
+
     @staticmethod
-    def forward(ctx, y, row_of_pair, probs):
+    def forward(ctx, y, row_of_pair, probs, src_of_row=None):
         T, k = probs.shape
+        y = y.contiguous()
         out = torch.empty(T, y.shape[1], dtype=y.dtype, device=y.device)
         pc = probs.to(y.dtype).contiguous()
-        _check(lib().mm_moe_unpermute(y.contiguous().data_ptr(), row_of_pair.data_ptr(), pc.data_ptr(), out.data_ptr(), T, k,
+        _check(lib().mm_moe_unpermute(y.data_ptr(), row_of_pair.data_ptr(), pc.data_ptr(), out.data_ptr(), T, k,
                                       y.shape[1], _st()), "moe_unpermute")
-        ctx.save_for_backward(y, row_of_pair, pc)
+        ctx.save_for_backward(y, row_of_pair, pc, src_of_row)
         return out
 
     @staticmethod
     def backward(ctx, g):
-        y, row_of_pair, probs = ctx.saved_tensors
+        y, row_of_pair, probs, src_of_row = ctx.saved_tensors
         T, k = probs.shape
-        idx = row_of_pair.long()
-        ge = g.repeat_interleave(k, dim=0)                              # [T*k, H]
-        dy = torch.zeros_like(y)
-        dy[idx] = ge * probs.reshape(-1, 1)
-        dprobs = (ge.float() * y[idx].float()).sum(-1).view(T, k).to(probs.dtype)
-        return dy, None, dprobs
+        g = g.contiguous()
+        dy = torch.empty_like(y)
+        dprobs = torch.empty_like(probs)
+        _check(lib().mm_moe_unpermute_bwd(g.data_ptr(), y.data_ptr(), row_of_pair.data_ptr(),
+                                          None if src_of_row is None else src_of_row.data_ptr(), probs.data_ptr(),
+                                          dy.data_ptr(), dprobs.data_ptr(), T, k, y.shape[0], y.shape[1], _st()),
+               "moe_unpermute_bwd")
+        return dy, None, dprobs, None
 
 
 def _grouped_raw(a, b, c, off, mode, K, N, E):
-    R = a.shape[0]
-    plan = torch.empty(3 * lib().mm_grouped_gemm_max_tiles(R, E, K, N, mode) + 1, dtype=torch.int32, device=a.device)
-    _check(lib().mm_grouped_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), off.data_ptr(), plan.data_ptr(), R, E, K, N,
-                                      mode, status_word(a.device).data_ptr(), _st()), "grouped_gemm")
+    _check(lib().mm_grouped_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), off.data_ptr(), a.shape[0], E, K, N, mode,
+                                      status_word(a.device).data_ptr(), _st()), "grouped_gemm")
 
 
 class _AlignedGroupedGemm(torch.autograd.Function):
@@ -834,7 +848,7 @@ class _AlignedGroupedGemm(torch.autograd.Function):
         g = g.contiguous()
         dx = torch.empty_like(x)
         _grouped_raw(g, w, dx, off, 1, K, N, E)
-        dw = torch.zeros_like(w)
+        dw = torch.empty(E, K, N, dtype=w.dtype, device=w.device)
         _grouped_raw(x, g, dw, off, 2, K, N, E)
         return dx, dw, None
 
@@ -842,11 +856,13 @@ class _AlignedGroupedGemm(torch.autograd.Function):
 def moe_experts(tokens, topk_ids, probs, gate_up, down):
     """Routed SwiGLU experts: permute -> grouped GEMM -> SwiGLU -> grouped GEMM -> weighted un-permute."""
     E = gate_up.shape[0]
-    off, row_of_pair, src_of_row, R = aligned_routing(topk_ids, E)
+    off, row_of_pair, src_of_row, _, check = _route(topk_ids, E)
     x = _AlignedPermute.apply(tokens, src_of_row, row_of_pair, topk_ids.shape[1])
     h = _AlignedGroupedGemm.apply(x, gate_up, off)
     y = _AlignedGroupedGemm.apply(swiglu(h), down, off)
-    return _AlignedUnpermute.apply(y, row_of_pair, probs)
+    out = _AlignedUnpermute.apply(y, row_of_pair, probs, src_of_row)
+    check()                      # the routing is long done by now: the products queued behind it keep the GPU busy
+    return out
 
 
 # --------------------------------------------------------------------------- GDN
