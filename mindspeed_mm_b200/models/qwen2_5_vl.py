@@ -239,6 +239,12 @@ class Linear(nn.Module):
         return ops.linear(x, self.weight, self.bias, value_unused_in_backward)
 
 
+def _plain(*modules) -> bool:
+    """Exactly this file's Linear / RMSNorm, nothing hooked: their weights may be used without calling them."""
+    return not torch.nn.modules.module._has_any_global_hook() and all(
+        type(m) in (Linear, RMSNorm) and not (m._forward_hooks or m._forward_pre_hooks) for m in modules)
+
+
 class VisionBlock(nn.Module):
     def __init__(self, c: VisionConfig):
         super().__init__()
@@ -368,21 +374,24 @@ class DecoderLayer(nn.Module):
         """``cache`` (generation, one sequence): a dict that keeps this layer's rotated keys and the values of all
         tokens seen so far; the new tokens attend to them (causal mask aligned to the end of the key sequence)."""
         T = x.shape[0]
+        widths = [self.nq * self.hd, self.nkv * self.hd, self.nkv * self.hd]
+        if cache is not None:
+            n1, n2, p_qkv, p_o, p_down = self.input_layernorm, self.post_attention_layernorm, self.qkv_proj, self.o_proj, self.down_proj
+            # a wrapped or hooked projection (an adapter, an observer) is called as the module it is
+            plain = _plain(n1, n2, p_qkv, p_o, p_down) and p_o.bias is None and p_down.bias is None
+            qkv = ops.norm_linear(x, n1.weight, n1.eps, p_qkv.weight, p_qkv.bias) if plain else p_qkv(n1(x))
+            q, k, v = (t.view(T, -1, self.hd) for t in qkv.split(widths, dim=-1))
+            o = ops.attention_cached(q, k, v, cache, cos, sin).reshape(T, -1)
+            if plain:
+                x = ops.linear_add(o, p_o.weight, x)
+                return ops.linear_add(ops.norm_linear_swiglu(x, n2.weight, n2.eps, self.gate_up_proj.weight), p_down.weight, x)
+            x = x + p_o(o)
+            return x + p_down(ops.linear_swiglu(n2(x), self.gate_up_proj.weight))
         qkv = self.qkv_proj(self.input_layernorm(x))
-        q, k, v = qkv.split([self.nq * self.hd, self.nkv * self.hd, self.nkv * self.hd], dim=-1)
+        q, k, v = qkv.split(widths, dim=-1)
         q = ops.rope_rotate_half(q.view(T, self.nq, self.hd), cos, sin)
         k = ops.rope_rotate_half(k.view(T, self.nkv, self.hd), cos, sin)
         v = v.view(T, self.nkv, self.hd)
-        if cache is not None:
-            if "k" in cache:
-                k, v = torch.cat([cache["k"], k]), torch.cat([cache["v"], v])
-            cache["k"], cache["v"] = k, v
-            L = k.shape[0]
-            cu_q = torch.tensor([0, T], dtype=torch.int32, device=x.device)
-            cu_k = torch.tensor([0, L], dtype=torch.int32, device=x.device)
-            o = ops.attention_varlen(q, k, v, cu_q, cu_k, T, L, causal=True)
-            x = x + self.o_proj(o.reshape(T, -1))
-            return x + self.down_proj(ops.linear_swiglu(self.post_attention_layernorm(x), self.gate_up_proj.weight))
         o = ops.attention_varlen(q, k, v, cu_seqlens, cu_seqlens,
                                  max_seqlen, max_seqlen, causal=True)
         x = x + self.o_proj(o.reshape(T, -1))

@@ -210,13 +210,7 @@ class GatedAttention(nn.Module):
         k = self._rope(self.k_norm(k.reshape(T, self.nkv, self.hd)), cos, sin)
         v = v.reshape(T, self.nkv, self.hd)
         if cache is not None:
-            if "k" in cache:
-                k, v = torch.cat([cache["k"], k]), torch.cat([cache["v"], v])
-            cache["k"], cache["v"] = k, v
-            L = k.shape[0]
-            cu_q = torch.tensor([0, T], dtype=torch.int32, device=x.device)
-            cu_k = torch.tensor([0, L], dtype=torch.int32, device=x.device)
-            o = ops.attention_varlen(q, k, v, cu_q, cu_k, T, L, causal=True)
+            o = ops.attention_cached(q, k, v, cache)
         else:
             o = ops.attention_varlen(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen, causal=True)
         o = o.reshape(T, -1)

@@ -255,6 +255,50 @@ def attention_dense(q, k, v, causal: bool = False, softmax_scale: Optional[float
     return ref.attention_dense(q, k, v, causal, softmax_scale)
 
 
+def attention_cached(q, k, v, cache: dict, cos=None, sin=None):
+    """Generation, one sequence: appends the new tokens' keys (rotated with ``cos`` / ``sin`` like the queries, unless those
+    are None: then both come rotated) and values to ``cache["k"]`` / ``cache["v"]`` and attends to all of them, causal and
+    aligned to the end.  q [T, Nq, D], k / v [T, Nkv, D].  A few tokens (a decoding step) take one kernel."""
+    k_old, v_old = cache.get("k"), cache.get("v")
+    if _native(q) and _nat().decode_attention_supported(q, k, v, k_old, v_old, cos):
+        o, cache["k"], cache["v"] = _nat().decode_attention(q, k, v, k_old, v_old, cos, sin)
+        return o
+    if cos is not None:
+        q, k = rope_rotate_half(q, cos, sin), rope_rotate_half(k, cos, sin)
+    if k_old is not None:
+        k, v = torch.cat([k_old, k]), torch.cat([v_old, v])
+    cache["k"], cache["v"] = k, v
+    T, L = q.shape[0], k.shape[0]
+    # [0, n] made on the device: a copy from the host would make the host wait for everything queued so far
+    cu_q = torch.arange(0, T + 1, T, dtype=torch.int32, device=q.device)
+    cu_k = cu_q if L == T else torch.arange(0, L + 1, L, dtype=torch.int32, device=q.device)
+    return attention_varlen(q, k, v, cu_q, cu_k, T, L, causal=True)
+
+
+# --------------------------------------------------------------------------- generation: products of a few rows
+def norm_linear(x, norm_weight, eps, weight, bias=None):
+    """``linear(rms_norm(x), weight, bias)``; a few rows that keep no graph take one kernel."""
+    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_supported(x, weight) and _nat().skinny_supported(x, norm_weight, weight, bias):
+        return _nat().skinny_linear(x, weight, bias, norm_weight, eps)
+    return linear(rms_norm(x, norm_weight, eps), weight, bias)
+
+
+def norm_linear_swiglu(x, norm_weight, eps, weight_gate_up):
+    """``linear_swiglu(rms_norm(x), weight_gate_up)``; a few rows that keep no graph take one kernel."""
+    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_swiglu_supported(x, weight_gate_up) and \
+            _nat().skinny_supported(x, norm_weight, weight_gate_up):
+        return _nat().skinny_linear(x, weight_gate_up, None, norm_weight, eps, swiglu=True)
+    return linear_swiglu(rms_norm(x, norm_weight, eps), weight_gate_up)
+
+
+def linear_add(x, weight, residual):
+    """``residual + linear(x, weight)``; a few rows that keep no graph take one kernel."""
+    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_supported(x, weight) and residual.shape == (x.shape[0], weight.shape[0]) and \
+            _nat().skinny_supported(x, weight, residual):
+        return _nat().skinny_linear(x, weight, residual=residual)
+    return residual + linear(x, weight)
+
+
 # --------------------------------------------------------------------------- loss
 def linear_cross_entropy(h, weight, labels, ignore_index: int = -100, chunk: int = 2048):
     """Sum of token CE of ``h @ weight.T`` against ``labels`` without keeping [T, V] logits.

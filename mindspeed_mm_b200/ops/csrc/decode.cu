@@ -1,0 +1,486 @@
+// Generation with a key / value cache: a handful of new tokens against every weight and the whole cache.
+//
+// Both kernels are bound by HBM (each weight, key and value is used a few times only), and a step is a chain of some forty of
+// them, most of which take 4 to 40 us, so what counts beside the bytes is how fast a kernel fills the memory system and how
+// many there are.  Hence: products with M <= 4 rows stream the weights through CUDA cores instead of 128-row tensor-core tiles
+// (a 128 x 256 tile grid over 3584 columns is 14 CTAs, 1.8 TB/s); the RMSNorm in front, the bias, the SwiGLU and the residual
+// sum behind are part of the product; rotation, cache append and attention are one kernel.  All of them are launched with
+// programmatic stream serialisation: a kernel starts while its predecessor drains, asks L2 for its first weights (a hint, so a
+// predecessor that writes those weights is harmless) and waits for the predecessor before it reads anything.
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace {
+
+namespace cg = cooperative_groups;
+
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// After the wait, never before: a successor may then rely on everything in front of this kernel being complete.
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+__device__ __forceinline__ uint4 ld_once(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ float2 bf2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<bf162*>(&v)); }
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+    bf162 t = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&t);
+}
+
+template <class... P, class... A>
+int launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// ------------------------------------------------------------------------------------------ skinny product
+struct GemvParams {
+    const bf16 *x, *w, *bias, *norm, *res;
+    bf16* out;
+    long long ldx, ldw, ldr, ldo;
+    int N, K;                        // N: outputs (SWIGLU: half of the weight's rows)
+    float eps;
+};
+
+constexpr int kGemvWarps = 4, kGemvU = 4;
+
+// out[m, n] = act(norm(x)[m, :] . w[n, :] + bias[n]) + res[m, n].  A warp owns two weight rows (two neighbouring outputs; SWIGLU:
+// the gate and the up row of one output), lanes stride over K in 16-byte pieces, the next 4 pieces of both rows in flight while
+// the current ones are multiplied; x (normalised once per block) sits in shared memory as bf16, sums are fp32.
+// 128-thread blocks: 3584 outputs are 448 blocks, so the SMs differ by one block in four, not one in two.
+template <int M, bool SWIGLU, bool NORM>
+__global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(GemvParams p) {
+    extern __shared__ __align__(16) uint8_t gemv_smem[];
+    bf16* xs = reinterpret_cast<bf16*>(gemv_smem);                  // [M][K]
+    __shared__ float red[72];
+    const int lane = threadIdx.x & 31, nvec = p.K >> 3;
+    const int unit = blockIdx.x * kGemvWarps + (threadIdx.x >> 5), units = SWIGLU ? p.N : p.N >> 1;
+    const bool active = unit < units;
+    const int r0 = SWIGLU ? unit : 2 * unit, r1 = SWIGLU ? p.N + unit : r0 + 1;
+    const uint4* w0 = reinterpret_cast<const uint4*>(p.w + (size_t)(active ? r0 : 0) * p.ldw);
+    const uint4* w1 = reinterpret_cast<const uint4*>(p.w + (size_t)(active ? r1 : 0) * p.ldw);
+    if (active)
+        for (int i = lane * 8; i < nvec && i < 512; i += 256) {       // 128-byte lines, the first 8 KB of each row
+            prefetch_l2(w0 + i);
+            prefetch_l2(w1 + i);
+        }
+    wait_for_predecessor();
+    uint4 a[kGemvU], b[kGemvU];
+    auto load = [&](int c, uint4* u, uint4* v) {
+#pragma unroll
+        for (int j = 0; j < kGemvU; ++j) {
+            const int i = (c * kGemvU + j) * 32 + lane;
+            const bool in = active && i < nvec;
+            u[j] = in ? ld_once(w0 + i) : make_uint4(0, 0, 0, 0);
+            v[j] = in ? ld_once(w1 + i) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    load(0, a, b);
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const Vec8* xr = reinterpret_cast<const Vec8*>(p.x + m * p.ldx);
+        Vec8* dst = reinterpret_cast<Vec8*>(xs + (size_t)m * p.K);
+        if constexpr (NORM) {
+            float ss = 0.f;
+            for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) {
+                const Vec8 v = xr[i];
+                float f[8];
+                unpack8(v, f);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) ss += f[k] * f[k];
+                dst[i] = v;
+            }
+            ss = block_sum(ss, red);
+            const float rstd = rsqrtf(ss / (float)p.K + p.eps);
+            for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) {      // each thread re-reads what it wrote
+                float f[8], g[8];
+                unpack8(dst[i], f);
+                unpack8(reinterpret_cast<const Vec8*>(p.norm)[i], g);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) f[k] = f[k] * rstd * g[k];
+                dst[i] = pack8(f);
+            }
+        } else {
+            for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) dst[i] = xr[i];
+        }
+    }
+    __syncthreads();
+    let_successor_start();
+    float2 acc0[M], acc1[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) acc0[m] = acc1[m] = make_float2(0.f, 0.f);
+    const int chunks = (nvec + 32 * kGemvU - 1) / (32 * kGemvU);
+    for (int c = 0; c < chunks; ++c) {
+        uint4 na[kGemvU], nb[kGemvU];
+        if (c + 1 < chunks) load(c + 1, na, nb);
+#pragma unroll
+        for (int j = 0; j < kGemvU; ++j) {
+            const int i = (c * kGemvU + j) * 32 + lane;
+            const uint32_t ua[4] = {a[j].x, a[j].y, a[j].z, a[j].w}, ub[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const uint4 xv = i < nvec ? *reinterpret_cast<const uint4*>(xs + (size_t)m * p.K + i * 8) : make_uint4(0, 0, 0, 0);
+                const uint32_t ux[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 f = bf2(ux[k]);
+                    acc0[m] = __ffma2_rn(bf2(ua[k]), f, acc0[m]);
+                    acc1[m] = __ffma2_rn(bf2(ub[k]), f, acc1[m]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kGemvU; ++j) {
+            a[j] = na[j];
+            b[j] = nb[j];
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        float s0 = warp_sum(acc0[m].x + acc0[m].y), s1 = warp_sum(acc1[m].x + acc1[m].y);
+        if (lane || !active) continue;
+        bf16* o = p.out + m * p.ldo;
+        if constexpr (SWIGLU) {
+            o[r0] = __float2bfloat16(s0 / (1.f + __expf(-s0)) * s1);
+        } else {
+            if (p.bias) {
+                s0 += __bfloat162float(p.bias[r0]);
+                s1 += __bfloat162float(p.bias[r1]);
+            }
+            if (p.res) {
+                const float2 r = __bfloat1622float2(*reinterpret_cast<const bf162*>(p.res + m * p.ldr + r0));
+                s0 += r.x;
+                s1 += r.y;
+            }
+            *reinterpret_cast<bf162*>(o + r0) = __floats2bfloat162_rn(s0, s1);
+        }
+    }
+}
+
+template <int M, bool SWIGLU, bool NORM>
+int run_gemv(const GemvParams& p, cudaStream_t st) {
+    auto kern = gemv_kernel<M, SWIGLU, NORM>;
+    const size_t smem = (size_t)M * p.K * 2;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const int units = SWIGLU ? p.N : p.N / 2;
+    return launch_pdl(kern, dim3((units + kGemvWarps - 1) / kGemvWarps), kGemvWarps * 32, smem, 1, st, p);
+}
+
+template <int M>
+int run_gemv_m(const GemvParams& p, int swiglu, cudaStream_t st) {
+    if (swiglu) return p.norm ? run_gemv<M, true, true>(p, st) : run_gemv<M, true, false>(p, st);
+    return p.norm ? run_gemv<M, false, true>(p, st) : run_gemv<M, false, false>(p, st);
+}
+
+// ------------------------------------------------------------------------------------------ attention over the cache
+struct DecodeParams {
+    const bf16 *q, *k, *v;           // new tokens: [T, heads, 128] with token strides
+    const bf16 *cos, *sin;           // [T, 128] or null: q and k come rotated
+    const bf16 *k_old, *v_old;       // [past, Nkv, 128]
+    bf16 *k_new, *v_new;             // [past + T, Nkv, 128]: cache after the call
+    bf16* out;                       // [T, Nq, 128]
+    long long qs, ks, vs;
+    int T, past, Nq, Nkv;
+    float scale_log2;
+};
+
+constexpr int kDecWarps = 8, kDecD = 128, kDecRows = 16, kDecTile = 16;
+constexpr int kDecSmem = kDecWarps * kDecRows * (kDecD + 2) * 4;
+
+__device__ __forceinline__ void mma_16x8x16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// 32 consecutive elements [d0, d0 + 32) of one head of one new token, rotated (half rotation) if there are tables.
+__device__ __forceinline__ void load_row32(const bf16* row, const bf16* cosr, const bf16* sinr, int d0, uint4* dst) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int d = d0 + 8 * i;
+        Vec8 own = *reinterpret_cast<const Vec8*>(row + d);
+        if (cosr) {
+            float x[8], y[8], c[8], s[8];
+            unpack8(own, x);
+            unpack8(*reinterpret_cast<const Vec8*>(row + (d ^ 64)), y);
+            unpack8(*reinterpret_cast<const Vec8*>(cosr + d), c);
+            unpack8(*reinterpret_cast<const Vec8*>(sinr + d), s);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = d < 64 ? x[k] * c[k] - y[k] * s[k] : x[k] * c[k] + y[k] * s[k];
+            own = pack8(x);
+        }
+        dst[i] = *reinterpret_cast<uint4*>(&own);
+    }
+}
+
+// One cluster per key / value head, its CTAs split the keys, a warp takes every (CTAs x 8)-th run of 16 of them.  The T new tokens'
+// query heads of the group (T * Nq / Nkv <= 16) are the 16 rows of an mma.sync tile: the tensor cores are used only to spare the
+// cross-lane sums; the kernel moves keys and values.  Fragment order: a dot product may walk its dimension in any order, so a lane
+// of a quad takes 32 consecutive elements of its key (four 16-byte loads that are also the copy into the new cache), and for the
+// second product 16 consecutive elements of its four keys, paired across keys with a byte permute.  Every loaded piece is stored
+// to the new cache, rotated if it belongs to a new token, so the cache is read once instead of once for the append and once for
+// the attention.  Partial sums of the warps meet in shared memory, those of the CTAs in distributed shared memory: no workspace,
+// no second launch.
+// 9000 keys, 28 query and 4 key / value heads: see mm_decode_attention.
+__global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(DecodeParams p) {
+    extern __shared__ __align__(16) uint8_t dec_smem[];
+    float* part_o = reinterpret_cast<float*>(dec_smem);                       // [warp][row][128]
+    float* part_m = part_o + kDecWarps * kDecRows * kDecD;                    // [warp][row]
+    float* part_l = part_m + kDecWarps * kDecRows;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int splits = gridDim.x, split = blockIdx.x, kvh = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, g = lane >> 2;
+    const int G = p.Nq / p.Nkv, rows = p.T * G, L = p.past + p.T;
+    const size_t pitch = (size_t)p.Nkv * kDecD;
+    wait_for_predecessor();
+    let_successor_start();
+
+    // query fragments: rows g and g + 8 (row = token * G + head of the group), this quad lane's 32 dims
+    uint4 q0[4], q1[4];
+    int vis0 = 0, vis1 = 0;                                                    // keys the two rows may see
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q0[i] = q1[i] = make_uint4(0, 0, 0, 0);
+    if (g < rows) {
+        const int t = g / G;
+        vis0 = p.past + t + 1;
+        load_row32(p.q + t * p.qs + (size_t)(kvh * G + g % G) * kDecD, p.cos ? p.cos + t * kDecD : nullptr, p.sin + t * kDecD, quad * 32, q0);
+    }
+    if (g + 8 < rows) {
+        const int t = (g + 8) / G;
+        vis1 = p.past + t + 1;
+        load_row32(p.q + t * p.qs + (size_t)(kvh * G + (g + 8) % G) * kDecD, p.cos ? p.cos + t * kDecD : nullptr, p.sin + t * kDecD, quad * 32, q1);
+    }
+    const uint32_t* qa = reinterpret_cast<const uint32_t*>(q0);
+    const uint32_t* qb = reinterpret_cast<const uint32_t*>(q1);
+
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    float o[16][4];
+#pragma unroll
+    for (int n = 0; n < 16; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+
+    for (int k0 = (split * kDecWarps + warp) * kDecTile; k0 < L; k0 += splits * kDecWarps * kDecTile) {
+        float s[2][4];
+        // values first: their loads are in flight during the first product
+        uint4 vv[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int key = k0 + quad * 2 + (i & 1) + (i >> 1) * 8;
+            vv[i][0] = vv[i][1] = make_uint4(0, 0, 0, 0);
+            if (key < L) {
+                const bf16* src = key < p.past ? p.v_old + key * pitch + (size_t)kvh * kDecD
+                                               : p.v + (key - p.past) * p.vs + (size_t)kvh * kDecD;
+                vv[i][0] = ld_once(reinterpret_cast<const uint4*>(src + g * 16));
+                vv[i][1] = ld_once(reinterpret_cast<const uint4*>(src + g * 16 + 8));
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int key = k0 + h * 8 + g;
+            uint4 kk[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kk[i] = make_uint4(0, 0, 0, 0);
+            if (key < L) {
+                if (key < p.past) {
+                    const uint4* src = reinterpret_cast<const uint4*>(p.k_old + key * pitch + (size_t)kvh * kDecD + quad * 32);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) kk[i] = ld_once(src + i);
+                } else {
+                    const int t = key - p.past;
+                    load_row32(p.k + t * p.ks + (size_t)kvh * kDecD, p.cos ? p.cos + t * kDecD : nullptr, p.sin + t * kDecD, quad * 32, kk);
+                }
+                uint4* dst = reinterpret_cast<uint4*>(p.k_new + key * pitch + (size_t)kvh * kDecD + quad * 32);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dst[i] = kk[i];
+            }
+            const uint32_t* kr = reinterpret_cast<const uint32_t*>(kk);
+            s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t a[4] = {qa[2 * i], qb[2 * i], qa[2 * i + 1], qb[2 * i + 1]};
+                mma_16x8x16(s[h], a, kr[2 * i], kr[2 * i + 1]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int key = k0 + quad * 2 + (i & 1) + (i >> 1) * 8;
+            if (key < L) {
+                uint4* dst = reinterpret_cast<uint4*>(p.v_new + key * pitch + (size_t)kvh * kDecD + g * 16);
+                dst[0] = vv[i][0];
+                dst[1] = vv[i][1];
+            }
+        }
+        float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int key = k0 + h * 8 + quad * 2 + c;
+                s[h][c] = key < vis0 ? s[h][c] * p.scale_log2 : -INFINITY;
+                s[h][2 + c] = key < vis1 ? s[h][2 + c] * p.scale_log2 : -INFINITY;
+                x0 = fmaxf(x0, s[h][c]);
+                x1 = fmaxf(x1, s[h][2 + c]);
+            }
+#pragma unroll
+        for (int d = 1; d < 4; d <<= 1) {
+            x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, d));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, d));
+        }
+        const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+        const float u0 = n0 == -INFINITY ? 0.f : n0, u1 = n1 == -INFINITY ? 0.f : n1;
+        const float f0 = exp2f(m0 - u0), f1 = exp2f(m1 - u1);
+        m0 = n0;
+        m1 = n1;
+        l0 *= f0;
+        l1 *= f1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                s[h][c] = exp2f(s[h][c] - u0);
+                s[h][2 + c] = exp2f(s[h][2 + c] - u1);
+                l0 += s[h][c];
+                l1 += s[h][2 + c];
+            }
+        const uint32_t pa[4] = {pack2(s[0][0], s[0][1]), pack2(s[0][2], s[0][3]), pack2(s[1][0], s[1][1]), pack2(s[1][2], s[1][3])};
+        const uint32_t* v0 = reinterpret_cast<const uint32_t*>(vv[0]);
+        const uint32_t* v1 = reinterpret_cast<const uint32_t*>(vv[1]);
+        const uint32_t* v2 = reinterpret_cast<const uint32_t*>(vv[2]);
+        const uint32_t* v3 = reinterpret_cast<const uint32_t*>(vv[3]);
+#pragma unroll
+        for (int n = 0; n < 16; ++n) {                                         // output column n of this lane's group: dim g * 16 + n
+            const int i = n >> 1;
+            const uint32_t sel = n & 1 ? 0x7632 : 0x5410;
+            const uint32_t b0 = __byte_perm(v0[i], v1[i], sel), b1 = __byte_perm(v2[i], v3[i], sel);
+            o[n][0] *= f0;
+            o[n][1] *= f0;
+            o[n][2] *= f1;
+            o[n][3] *= f1;
+            mma_16x8x16(o[n], pa, b0, b1);
+        }
+    }
+    // Accumulator column of lane (g, quad) in product n: the output columns 2 * quad and 2 * quad + 1 of the tile, whose "column c"
+    // was loaded by the lanes with group c: dims c * 16 + n.
+#pragma unroll
+    for (int d = 1; d < 4; d <<= 1) {
+        l0 += __shfl_xor_sync(0xffffffffu, l0, d);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, d);
+    }
+    float* mo = part_o + (size_t)warp * kDecRows * kDecD;
+#pragma unroll
+    for (int n = 0; n < 16; ++n)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            mo[g * kDecD + (2 * quad + c) * 16 + n] = o[n][c];
+            mo[(g + 8) * kDecD + (2 * quad + c) * 16 + n] = o[n][2 + c];
+        }
+    if (quad == 0) {
+        part_m[warp * kDecRows + g] = m0;
+        part_m[warp * kDecRows + g + 8] = m1;
+        part_l[warp * kDecRows + g] = l0;
+        part_l[warp * kDecRows + g + 8] = l1;
+    }
+    __syncthreads();
+    // fold the warps of this CTA into warp 0's slots
+    for (int i = threadIdx.x; i < rows * kDecD; i += kDecWarps * 32) {
+        const int r = i / kDecD;
+        float m = -INFINITY;
+        for (int w = 0; w < kDecWarps; ++w) m = fmaxf(m, part_m[w * kDecRows + r]);
+        const float u = m == -INFINITY ? 0.f : m;
+        float acc = 0.f;
+        for (int w = 0; w < kDecWarps; ++w) acc += part_o[(size_t)w * kDecRows * kDecD + i] * exp2f(part_m[w * kDecRows + r] - u);
+        part_o[i] = acc;                                                       // only this thread reads or writes element i
+    }
+    __syncthreads();
+    if (threadIdx.x < rows) {
+        float m = -INFINITY, l = 0.f;
+        for (int w = 0; w < kDecWarps; ++w) m = fmaxf(m, part_m[w * kDecRows + threadIdx.x]);
+        const float u = m == -INFINITY ? 0.f : m;
+        for (int w = 0; w < kDecWarps; ++w) l += part_l[w * kDecRows + threadIdx.x] * exp2f(part_m[w * kDecRows + threadIdx.x] - u);
+        part_m[threadIdx.x] = m;
+        part_l[threadIdx.x] = l;
+    }
+    cluster.sync();
+    // fold the CTAs: each takes its share of the outputs (pairs of dims)
+    for (int i = split * kDecWarps * 32 + threadIdx.x; i < rows * (kDecD / 2); i += splits * kDecWarps * 32) {
+        const int r = i / (kDecD / 2), d = i % (kDecD / 2) * 2;
+        float m = -INFINITY;
+        for (int c = 0; c < splits; ++c) m = fmaxf(m, *cluster.map_shared_rank(part_m + r, c));
+        const float u = m == -INFINITY ? 0.f : m;
+        float l = 0.f, ax = 0.f, ay = 0.f;
+        for (int c = 0; c < splits; ++c) {
+            const float f = exp2f(*cluster.map_shared_rank(part_m + r, c) - u);
+            const float2 v = *reinterpret_cast<const float2*>(cluster.map_shared_rank(part_o + r * kDecD + d, c));
+            l += *cluster.map_shared_rank(part_l + r, c) * f;
+            ax += v.x * f;
+            ay += v.y * f;
+        }
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const int t = r / G, head = kvh * G + r % G;
+        *reinterpret_cast<bf162*>(p.out + ((size_t)t * p.Nq + head) * kDecD + d) = __floats2bfloat162_rn(ax * inv, ay * inv);
+    }
+    cluster.sync();                                                            // nobody leaves while its memory is read
+}
+
+}  // namespace
+
+// out[M, N] = swiglu?(norm?(x) @ W^T + bias?) + residual?  for M <= 4 rows.  norm: RMSNorm weight [K] or null; bias [N], res
+// [M, N]: null or bf16 (not with swiglu).  swiglu: W is [2N, K], gate rows then up rows.  K % 8 == 0, N % 2 == 0, leading
+// dimensions multiples of 8, 16-byte aligned bases, M * K <= 80 K elements (x is kept in shared memory).
+// Why M <= 4: 3584 x 3584 and 3584 x 18944 take 6.3 / 25.8 us at M = 1 (25 and 83 us as tensor-core tiles).
+MM_API int mm_gemv_bf16(const void* x, const void* w, const void* bias, const void* norm, const void* res, void* out, int M, int N,
+                        int K, long long ldx, long long ldw, long long ldr, long long ldo, float eps, int swiglu, cudaStream_t st) {
+    if (M < 1 || M > 4 || N < 1 || K < 1 || K % 8 || N % 2 || (ldx | ldw | ldr | ldo) % 8 || (long long)M * K > 80 * 1024) return -1;
+    if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out | (uintptr_t)norm) & 15 || ((uintptr_t)res & 3)) return -2;
+    if (swiglu && (bias || res)) return -3;
+    GemvParams p{(const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)norm, (const bf16*)res, (bf16*)out,
+                 ldx, ldw, ldr, ldo, N, K, eps};
+    switch (M) {
+        case 1: return run_gemv_m<1>(p, swiglu, st);
+        case 2: return run_gemv_m<2>(p, swiglu, st);
+        case 3: return run_gemv_m<3>(p, swiglu, st);
+        default: return run_gemv_m<4>(p, swiglu, st);
+    }
+}
+
+// Appends T new tokens to a cache and attends to it (causal, aligned to the end): k_new / v_new [past + T, Nkv, 128] are the old
+// cache followed by the new keys (rotated) and values.  T * Nq / Nkv <= 16; strides in elements, multiples of 8; 16-byte bases.
+MM_API int mm_decode_attention(const void* q, const void* k, const void* v, const void* cos, const void* sin, const void* k_old,
+                               const void* v_old, void* k_new, void* v_new, void* out, int T, int past, int Nq, int Nkv,
+                               long long qs, long long ks, long long vs, float scale, cudaStream_t st) {
+    if (T < 1 || past < 0 || Nkv < 1 || Nq % Nkv || (long long)T * (Nq / Nkv) > kDecRows || (qs | ks | vs) % 8 || Nkv > 65535) return -1;
+    const void* ptrs[] = {q, k, v, cos, sin, k_old, v_old, k_new, v_new, out};
+    for (const void* a : ptrs)
+        if ((uintptr_t)a & 15) return -2;
+    if (!cos != !sin) return -3;
+    DecodeParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, (const bf16*)cos, (const bf16*)sin, (const bf16*)k_old,
+                   (const bf16*)v_old, (bf16*)k_new, (bf16*)v_new, (bf16*)out, qs, ks, vs, T, past, Nq, Nkv,
+                   scale * 1.4426950408889634f};
+    // one run of 16 keys per warp before another CTA pays; 16 CTAs is the largest cluster
+    const int runs = (past + T + kDecTile * kDecWarps - 1) / (kDecTile * kDecWarps);
+    int splits = 1;
+    while (splits < 16 && splits < runs) splits *= 2;
+    cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return (int)e;
+    return launch_pdl(decode_attention_kernel, dim3(splits, Nkv), kDecWarps * 32, (size_t)kDecSmem, splits, st, p);
+}

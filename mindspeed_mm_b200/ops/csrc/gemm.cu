@@ -387,6 +387,16 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
 
 }  // namespace
 
+// csrc/decode.cu: products with up to 4 rows
+MM_API int mm_gemv_bf16(const void* x, const void* w, const void* bias, const void* norm, const void* res, void* out, int M, int N,
+                        int K, long long ldx, long long ldw, long long ldr, long long ldo, float eps, int swiglu, cudaStream_t st);
+
+namespace {
+// Up to 4 rows: the weights are streamed once through CUDA cores.  The line lies there because a fifth row makes the fp32
+// multiply-adds, not HBM, the limit (8 multiply-adds per weight element and SM cycle at 4 rows), and x has to fit shared memory.
+bool skinny(int M, int N, int K) { return M <= 4 && N % 2 == 0 && K % 8 == 0 && (long long)M * K <= 80 * 1024; }
+}  // namespace
+
 // lda/ldb/ldc: elements between consecutive rows of the tensors as laid out in memory.
 // Requirements: base pointers 16-byte aligned; ld* multiples of 8; `status` is a device int (0 = ok).
 MM_API int mm_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
@@ -394,6 +404,7 @@ MM_API int mm_gemm_bf16(const void* A, const void* B, void* C, const void* bias,
     if ((lda | ldb | ldc) % 8) return -1;
     if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return -2;
     if (M <= 0 || N <= 0 || K <= 0) return -3;
+    if (!a_mn && !b_mn && skinny(M, N, K)) return mm_gemv_bf16(A, B, bias, nullptr, nullptr, C, M, N, K, lda, ldb, 0, ldc, 0.f, 0, st);
 #define MM_DISPATCH(BN_)                                                                                          \
     if (!a_mn && !b_mn) return launch<BN_, false, false>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st);      \
     if (!a_mn && b_mn) return launch<BN_, false, true>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st);        \
@@ -413,6 +424,7 @@ MM_API int mm_gemm_swiglu_bf16(const void* A, const void* W, void* C, int M, int
     if ((lda | ldw | ldc) % 8) return -1;
     if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) return -2;
     if (M <= 0 || F <= 0 || K <= 0 || F % 128) return -3;
+    if (skinny(M, F, K)) return mm_gemv_bf16(A, W, nullptr, nullptr, nullptr, C, M, F, K, lda, ldw, 0, ldc, 0.f, 1, st);
     return launch<256, false, false, true>(A, W, C, nullptr, M, F, K, lda, ldw, ldc, status, st);
 }
 

@@ -70,6 +70,8 @@ def _declare(L):
         "mm_adamw": [_p, _p, _p, _p, _i, _p, _ll, _ll, _f, _f, _f, _f, _f, _f, _f, _f, _p, _p],
         "mm_gemm_bf16": [_p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _p, _p],
         "mm_gemm_swiglu_bf16": [_p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _p, _p],
+        "mm_gemv_bf16": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _ll, _f, _i, _p],
+        "mm_decode_attention": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _ll, _ll, _ll, _f, _p],
         "mm_ce_fwd_bwd": [_p, _ll, _p, _p, _i, _i, _i, _p],
         "mm_fmha_max_tiles": [_i, _i],
         "mm_fmha_set_fwd_variant": [_i],
@@ -488,6 +490,69 @@ def gemm_swiglu(x, w):
     _check(lib().mm_gemm_swiglu_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, F, K, a.stride(0), w.stride(0),
                                      out.stride(0), st.data_ptr(), _st()), "gemm_swiglu_bf16")
     return out.view(*shape[:-1], F)
+
+
+# --------------------------------------------------------------------------- generation (csrc/decode.cu)
+def skinny_supported(x, *tensors) -> bool:
+    """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies."""
+    return (x.dim() == 2 and 1 <= x.shape[0] <= 4 and x.shape[1] % 8 == 0 and x.numel() <= 80 * 1024 and _ok2d(x)
+            and all(t is None or (t.dtype == torch.bfloat16 and t.device == x.device) for t in tensors)
+            and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x,) + tensors)))
+
+
+def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=False):
+    """``act(rms_norm(x) @ w.T + bias) + residual`` for the rows :func:`skinny_supported` takes."""
+    if not _ok2d(w):
+        w = w.contiguous()
+    if bias is not None:
+        bias = bias.contiguous()
+    if norm is not None:
+        norm = norm.contiguous()
+        if norm.data_ptr() % 16:
+            norm = norm.clone()
+    if residual is not None and not _ok2d(residual):
+        residual = residual.contiguous()
+    M, K = x.shape
+    N = w.shape[0] // 2 if swiglu else w.shape[0]
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+    _check(lib().mm_gemv_bf16(x.data_ptr(), w.data_ptr(), None if bias is None else bias.data_ptr(),
+                              None if norm is None else norm.data_ptr(), None if residual is None else residual.data_ptr(),
+                              out.data_ptr(), M, N, K, x.stride(0), w.stride(0), 0 if residual is None else residual.stride(0),
+                              out.stride(0), eps, int(swiglu), _st()), "gemv_bf16")
+    return out
+
+
+def decode_attention_supported(q, k, v, k_old, v_old, cos) -> bool:
+    """Head dim 128, the new tokens' query heads of a group fill at most one 16-row tile, nothing keeps a graph."""
+    ts = [t for t in (q, k, v, k_old, v_old) if t is not None]
+    T, Nq, D = q.shape
+    return (os.environ.get("MM_B200_FMHA", "1") == "1" and D == 128 and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts)
+            and all(t.shape[1:] == k.shape[1:] and t.shape[2] == D for t in (v, k_old, v_old) if t is not None)
+            and k.shape[2] == D and k.shape[0] == v.shape[0] == T and (k_old is None or k_old.shape[0] == v_old.shape[0])
+            and T >= 1 and Nq % k.shape[1] == 0 and T * (Nq // k.shape[1]) <= 16 and (cos is None or tuple(cos.shape) == (T, D))
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)))
+
+
+def decode_attention(q, k, v, k_old, v_old, cos, sin):
+    """Rotates q and k (unless ``cos`` is None), appends k / v to the cache and attends to all of it.  Returns (out, keys, values)."""
+    q, k, v = _dense_heads(q), _dense_heads(k), _dense_heads(v)
+    T, Nq, D = q.shape
+    Nkv, past = k.shape[1], 0
+    if cos is not None:
+        cos, sin = cos.to(torch.bfloat16).contiguous(), sin.to(torch.bfloat16).contiguous()
+        if (cos.data_ptr() | sin.data_ptr()) % 16:
+            cos, sin = cos.clone(), sin.clone()
+    if k_old is not None:
+        k_old, v_old, past = k_old.contiguous(), v_old.contiguous(), k_old.shape[0]
+        if (k_old.data_ptr() | v_old.data_ptr()) % 16:
+            k_old, v_old = k_old.clone(), v_old.clone()
+    k_new, v_new = (torch.empty(past + T, Nkv, D, dtype=torch.bfloat16, device=q.device) for _ in range(2))
+    out = torch.empty(T, Nq, D, dtype=torch.bfloat16, device=q.device)
+    ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    _check(lib().mm_decode_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), ptr(cos), ptr(sin), ptr(k_old), ptr(v_old),
+                                     k_new.data_ptr(), v_new.data_ptr(), out.data_ptr(), T, past, Nq, Nkv, q.stride(0), k.stride(0),
+                                     v.stride(0), 1.0 / math.sqrt(D), _st()), "decode_attention")
+    return out, k_new, v_new
 
 
 def gemm_nn(a, b, out=None):

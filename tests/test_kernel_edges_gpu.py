@@ -62,3 +62,60 @@ def test_grouped_gemm_gradients_with_empty_experts(K, N):
         _close(dx[a:a + c], ge @ we.t(), rtol=2e-2, atol=2e-2 * N ** 0.5)
         _close(dw[e], xe.t() @ ge, rtol=2e-2, atol=2e-2 * c ** 0.5)
         a += c
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 136, 264), (2, 4608, 3584), (3, 24, 1032), (4, 256, 18944), (1, 3584, 18944), (5, 136, 264)])
+@pytest.mark.parametrize("norm,ends", [(False, "none"), (True, "bias"), (False, "residual"), (True, "swiglu")])
+def test_product_of_a_few_rows(M, N, K, norm, ends):
+    """Both sides of the 4-row rule (5 rows and a 4 x 18944 operand beyond the shared-memory bound run on tiles)."""
+    torch.manual_seed(M * 1000 + N)
+    x, g = torch.randn(M, K, device=DEV).bfloat16(), (1 + 0.1 * torch.randn(K, device=DEV)).bfloat16()
+    n = 2 * N if ends == "swiglu" else N
+    wide = torch.randn(n, K + 8, device=DEV).bfloat16() / K ** 0.5
+    w, b, r = wide[:, :K], torch.randn(n, device=DEV).bfloat16(), torch.randn(M, N, device=DEV).bfloat16()       # rows with a pitch
+    h = ref.rms_norm(x, g, 1e-6).float() if norm else x.float()
+    want = h @ w.float().t()
+    with torch.no_grad():
+        if ends == "swiglu":
+            got, want = ops.norm_linear_swiglu(x, g, 1e-6, w), ref.swiglu(want)
+        elif ends == "residual":
+            got, want = ops.linear_add(x, w, r), want + r.float()
+        elif ends == "bias":
+            got, want = ops.norm_linear(x, g, 1e-6, w, b), want + b.float()
+        else:
+            got = ops.linear(x, w)
+    # operands are the same bf16 values (the normalised rows may round differently by one ulp), sums are fp32: half an ulp of bf16
+    _close(got, want, rtol=8e-3, atol=4e-3)
+
+
+def test_product_of_a_few_rows_keeps_infinities_and_nan_to_their_outputs():
+    x, w = torch.zeros(1, 272, device=DEV).bfloat16(), torch.ones(16, 272, device=DEV).bfloat16()
+    x[0, -1], w[3, 5], w[4, 271] = float("inf"), float("nan"), -1
+    with torch.no_grad():
+        y = ops.linear(x, w)[0].float()
+    assert y[3].isnan() and y[4] == float("-inf") and (y[:3] == float("inf")).all() and (y[5:] == float("inf")).all()
+
+
+@pytest.mark.parametrize("T,past,Nq,Nkv", [(1, 0, 28, 4), (1, 1, 28, 4), (1, 15, 16, 16), (1, 127, 64, 4), (2, 128, 28, 4), (1, 129, 8, 8),
+                                           (4, 500, 8, 2), (1, 2047, 28, 4), (1, 9000, 28, 4), (3, 16383, 5, 1), (16, 40, 2, 2), (17, 40, 2, 2)])
+@pytest.mark.parametrize("rotate", [False, True])
+def test_attention_over_the_cache(T, past, Nq, Nkv, rotate):
+    """Every split of the keys over warps and CTAs, one to all rows of a tile, both sides of the 16-row rule."""
+    torch.manual_seed(past + T)
+    D = 128
+    qkv = torch.randn(T, (Nq + 2 * Nkv) * D, device=DEV).bfloat16()
+    q, k, v = (t.view(T, -1, D) for t in qkv.split([Nq * D, Nkv * D, Nkv * D], -1))
+    ang = torch.rand(T, D // 2, device=DEV).repeat(1, 2) * 6
+    cos, sin = (ang.cos().bfloat16(), ang.sin().bfloat16()) if rotate else (None, None)
+    old = {n: torch.randn(past, Nkv, D, device=DEV).bfloat16() for n in "kv"} if past else {}
+    cache = dict(old)
+    with torch.no_grad():
+        o = ops.attention_cached(q, k, v, cache, cos, sin)
+    qr, kr = (ref.rope_rotate_half(t, cos, sin) if rotate else t for t in (q, k))
+    keys, values = (torch.cat([old[n], t]) if past else t for n, t in (("k", kr), ("v", v)))
+    assert torch.equal(cache["v"], values) and cache["k"].shape == keys.shape
+    _close(cache["k"], keys, rtol=8e-3, atol=1e-6)                            # the rotation may round differently by one ulp
+    assert not past or torch.equal(cache["k"][:past], old["k"])
+    cu_q, cu_k = torch.tensor([0, T], device=DEV), torch.tensor([0, past + T], device=DEV)
+    want = ref.attention_varlen(qr.float(), keys.float(), values.float(), cu_q, cu_k, True)
+    _close(o, want, rtol=1e-2, atol=4e-3)                                     # probabilities and results are bf16
