@@ -69,9 +69,15 @@ def _native(x: torch.Tensor) -> bool:
     return x.is_cuda and _TIER == "native"
 
 
+_NATIVE = None
+
+
 def _nat():
-    from . import native
-    return native
+    global _NATIVE
+    if _NATIVE is None:
+        from . import native
+        _NATIVE = native
+    return _NATIVE
 
 
 # --------------------------------------------------------------------------- norms / elementwise

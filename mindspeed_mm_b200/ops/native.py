@@ -121,7 +121,40 @@ def status() -> dict:
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current stream (building a ``torch.cuda.Stream`` for it costs 3 us a launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class _NoGraph:
+    """Context of an autograd function that is run without a graph: takes what forward keeps and drops it."""
+    __slots__ = ()
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    def __setattr__(self, name, value):
+        pass
+
+
+_NO_GRAPH = _NoGraph()
+
+
+def _keeps_no_graph(args) -> bool:
+    grad = torch.is_grad_enabled()
+    for a in args:
+        if isinstance(a, torch.Tensor) and ((grad and a.requires_grad) or torch._C._functorch.is_functorch_wrapped_tensor(a)):
+            return False
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling())
+
+
+def _run(fn, *args):
+    """``fn.apply(*args)``.  Where nothing asks for a gradient and no transform, forward-mode level or tracer is active, the
+    forward is called directly: ``apply`` costs 15 us of host time a call, more than most kernels of a generation step or of a
+    prompt of a thousand tokens take (one token through 8 layers: 1484 -> 1235 us, a prompt of 1020 tokens with an image: 6604 -> 5725 us)."""
+    if _keeps_no_graph(args):
+        return fn.forward(_NO_GRAPH, *args)
+    return fn.apply(*args)
 
 
 def _eager(op: str, x, why: str):
@@ -213,7 +246,7 @@ def rms_norm(x, w, eps=1e-6):
         from . import reference
         _eager("rms_norm", x, f"H={x.shape[-1]}")
         return reference.rms_norm(x, w, eps)
-    return _RMSNorm.apply(x, w, eps)
+    return _run(_RMSNorm, x, w, eps)
 
 
 # --------------------------------------------------------------------------- SwiGLU
@@ -248,7 +281,7 @@ def swiglu(gu):
         from . import reference
         _eager("swiglu", gu, f"F={gu.shape[-1] // 2}")
         return reference.swiglu(gu)
-    return _SwiGLU.apply(gu)
+    return _run(_SwiGLU, gu)
 
 
 # --------------------------------------------------------------------------- RoPE
@@ -273,7 +306,7 @@ class _Gelu(torch.autograd.Function):
 
 def gelu(x, tanh: bool = True):
     """bf16 GELU (tanh approximation or exact erf form); element count a multiple of 8."""
-    return _Gelu.apply(x, bool(tanh))
+    return _run(_Gelu, x, bool(tanh))
 
 
 def _rope_call(x, cos, sin, interleaved, backward):
@@ -318,7 +351,7 @@ def rope(x, cos, sin, interleaved: bool):
             _eager("rope_rotate_half", x, f"D={D}")
             return reference.rope_rotate_half(x, cos, sin)
         cos, sin = cos.to(torch.bfloat16).contiguous(), sin.to(torch.bfloat16).contiguous()
-    return _Rope.apply(x, cos, sin, interleaved)
+    return _run(_Rope, x, cos, sin, interleaved)
 
 
 # --------------------------------------------------------------------------- adaLN
@@ -359,7 +392,7 @@ def layer_norm_modulate(x, scale, shift, eps=1e-6):
         from . import reference
         _eager("layer_norm_modulate", x, f"x {tuple(x.shape)} scale {tuple(scale.shape)}")
         return reference.layer_norm_modulate(x, scale, shift, eps)
-    return _LNMod.apply(x, scale.to(x.dtype), shift.to(x.dtype), eps)
+    return _run(_LNMod, x, scale.to(x.dtype), shift.to(x.dtype), eps)
 
 
 def layer_norm(x, weight=None, bias=None, eps=1e-6):
@@ -372,7 +405,7 @@ def layer_norm(x, weight=None, bias=None, eps=1e-6):
     else:
         scale = torch.zeros(1, H, dtype=x.dtype, device=x.device)
     shift = bias.to(x.dtype).view(1, H) if bias is not None else torch.zeros(1, H, dtype=x.dtype, device=x.device)
-    return _LNMod.apply(x.reshape(1, -1, H), scale, shift, eps).view(x.shape)
+    return _run(_LNMod, x.reshape(1, -1, H), scale, shift, eps).view(x.shape)
 
 
 class _GatedResidual(torch.autograd.Function):
@@ -401,7 +434,7 @@ def gated_residual(x, y, gate):
         from . import reference
         _eager("gated_residual", x, f"x {tuple(x.shape)} gate {tuple(gate.shape)}")
         return reference.gated_residual(x, y, gate)
-    return _GatedResidual.apply(x, y, gate.to(x.dtype))
+    return _run(_GatedResidual, x, y, gate.to(x.dtype))
 
 
 # --------------------------------------------------------------------------- AdamW
@@ -626,7 +659,7 @@ class _Linear(torch.autograd.Function):
 
 
 def linear(x, w, bias=None, skip_value=False):
-    return _Linear.apply(x, w, bias, skip_value)
+    return _run(_Linear, x, w, bias, skip_value)
 
 
 # --------------------------------------------------------------------------- not yet native
@@ -741,8 +774,8 @@ def attention_varlen(q, k, v, cu_q, cu_k, max_q, max_k, causal, scale, cache=Non
             store.append((out, lse))
             return out
         if mode == "replay" and store:
-            return _FMHA.apply(q, k, v, cu_q, cu_k, max_q, max_k, bool(causal), float(scale), store.pop(0))
-    return _FMHA.apply(q, k, v, cu_q, cu_k, max_q, max_k, bool(causal), float(scale))
+            return _run(_FMHA, q, k, v, cu_q, cu_k, max_q, max_k, bool(causal), float(scale), store.pop(0))
+    return _run(_FMHA, q, k, v, cu_q, cu_k, max_q, max_k, bool(causal), float(scale))
 
 
 def lce_supported(h, w) -> bool:
@@ -922,10 +955,10 @@ def moe_experts(tokens, topk_ids, probs, gate_up, down):
     """Routed SwiGLU experts: permute -> grouped GEMM -> SwiGLU -> grouped GEMM -> weighted un-permute."""
     E = gate_up.shape[0]
     off, row_of_pair, src_of_row, _, check = _route(topk_ids, E)
-    x = _AlignedPermute.apply(tokens, src_of_row, row_of_pair, topk_ids.shape[1])
-    h = _AlignedGroupedGemm.apply(x, gate_up, off)
-    y = _AlignedGroupedGemm.apply(swiglu(h), down, off)
-    out = _AlignedUnpermute.apply(y, row_of_pair, probs, src_of_row)
+    x = _run(_AlignedPermute, tokens, src_of_row, row_of_pair, topk_ids.shape[1])
+    h = _run(_AlignedGroupedGemm, x, gate_up, off)
+    y = _run(_AlignedGroupedGemm, swiglu(h), down, off)
+    out = _run(_AlignedUnpermute, y, row_of_pair, probs, src_of_row)
     check()                      # the routing is long done by now: the products queued behind it keep the GPU busy
     return out
 
@@ -973,7 +1006,7 @@ def conv1d_supported(x, w) -> bool:
 
 
 def causal_conv1d(x, w, activation, cu_seqlens):
-    return _CausalConv1d.apply(x, w, cu_seqlens, activation == "silu")
+    return _run(_CausalConv1d, x, w, cu_seqlens, activation == "silu")
 
 
 class _L2Norm(torch.autograd.Function):
@@ -1000,7 +1033,7 @@ class _L2Norm(torch.autograd.Function):
 
 
 def l2_norm(x, eps=1e-6):
-    return _L2Norm.apply(x, eps)
+    return _run(_L2Norm, x, eps)
 
 
 class _GatedRMSNorm(torch.autograd.Function):
@@ -1033,7 +1066,7 @@ class _GatedRMSNorm(torch.autograd.Function):
 
 
 def gated_rms_norm(x, z, w, eps=1e-6):
-    return _GatedRMSNorm.apply(x, z, w, eps)
+    return _run(_GatedRMSNorm, x, z, w, eps)
 
 
 def gdn_supported(q, v, chunk) -> bool:
