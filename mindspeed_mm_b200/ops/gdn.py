@@ -2,13 +2,13 @@
 
 The WY form splits the operator in two:
 
-* ``chunk_prologue`` -- everything local to a 64-token chunk (cumulative gates, the unit-triangular solve, ``u``,
-  ``w``, the decayed ``q`` / ``k`` and the masked intra-chunk attention).  It is plain batched PyTorch over all
-  chunks of all sequences at once, so autograd differentiates it.
+* the chunk prologue -- everything local to a 64-token chunk (cumulative gates, the unit-triangular solve, ``u``, ``w``, the
+  decayed ``q`` / ``k`` and the masked intra-chunk attention).  bf16 tensors on a GPU take the kernels of
+  ``csrc/gdn_prologue.cu`` in both directions; ``chunk_prologue`` is the batched PyTorch form, which autograd
+  differentiates (CPU, fp32 inputs, Kimi delta attention).
 * ``state_pass`` -- the walk over the chunks of a sequence, each needing the state its predecessor left.  On a GPU
-  the forward is the tcgen05 kernel of ``csrc/gdn.cu`` (state resident in tensor memory); on CPU a PyTorch loop with
-  the same inputs and outputs.  Its backward is written by hand: only ``dS`` has to be walked backwards over the
-  chunks, every other gradient is a batched product of saved per-chunk states.
+  the forward is the tcgen05 kernel of ``csrc/gdn.cu`` (state resident in tensor memory), the backward that of
+  ``csrc/gdn_bwd.cu``; on CPU a PyTorch loop with the same inputs and outputs.
 
 Operator parity: fla ``chunk_gated_delta_rule`` as called by the reference's Qwen3.5 gated-delta-net block
 (fsdp/models/qwen3_5/modeling_qwen3_5.py) with ``cu_seqlens`` packing.
@@ -229,10 +229,15 @@ def gated_delta_rule_varlen(q, k, v, g, beta, cu_seqlens, scale: Optional[float]
     scale = K ** -0.5 if scale is None else scale
     lay = _layout(cu_seqlens, q.device)
     needs_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v, g, beta))
-    if q.is_cuda and not needs_grad and K == 128 and v.shape[-1] == 128 and _native_tier():
-        # a pass that keeps no graph (inference, the first forward of a recomputed layer): the chunk-local prologue is one
-        # kernel that reads the packed tensors, then the tcgen05 state pass; nothing is scattered to a padded layout first
-        return _forward_native(q, k, v, g, beta, lay, scale)
+    if q.is_cuda and K == 128 and v.shape[-1] == 128 and _native_tier():
+        # chunk-local prologue (one kernel that reads the packed tensors) and tcgen05 state walk, in both directions.  With a
+        # graph only for bf16 q / k / v: the kernels read bf16 operands, and fp32 inputs keep their fp32 prologue below
+        if not needs_grad or (_native_bwd_ok() and all(t.dtype == torch.bfloat16 for t in (q, k, v))):
+            covered = lay.slot_of_tok.numel()
+            if covered > q.shape[0] or (needs_grad and covered != q.shape[0]):
+                raise RuntimeError(f"cu_seqlens covers {covered} tokens, the tensors hold {q.shape[0]}")
+            from . import native
+            return native._run(_GatedDelta, q, k, v, g, beta, lay, scale)
     qc, kc, vc = (lay.scatter(t.float()) for t in (q, k, v))
     gcn, bc = (lay.scatter(t.float()) for t in (g, beta))
     W, Qg, Kd, At, U, gamma = chunk_prologue(qc, kc, vc, gcn, bc, scale)
@@ -246,22 +251,62 @@ def _native_tier() -> bool:
     return get_tier() == "native"
 
 
-def _forward_native(q, k, v, g, beta, lay: ChunkLayout, scale: float):
-    from . import native
-    T, H, K = q.shape
-    V = v.shape[-1]
-    dev, NC = q.device, lay.NC
-    qb, kb, vb = (t.to(torch.bfloat16).contiguous() for t in (q, k, v))
-    gf, bf = g.float().contiguous(), beta.float().contiguous()
-    W, Qg, Kd, U = (torch.empty(H, NC, CHUNK, K if i < 3 else V, dtype=torch.bfloat16, device=dev) for i in range(4))
-    At = torch.empty(H, NC, CHUNK, CHUNK, dtype=torch.bfloat16, device=dev)
-    gamma = torch.empty(H, NC, dtype=torch.float32, device=dev)
-    native._check(native.lib().mm_gdn_prologue(
-        qb.data_ptr(), kb.data_ptr(), vb.data_ptr(), gf.data_ptr(), bf.data_ptr(), lay.chunk_tok0.data_ptr(),
-        lay.chunk_len.data_ptr(), W.data_ptr(), Qg.data_ptr(), Kd.data_ptr(), At.data_ptr(), U.data_ptr(), gamma.data_ptr(),
-        H, NC, float(scale), native._st()), "gdn_prologue")
-    O, _, _ = _state_pass_native(W, Qg, Kd, At, U, gamma, lay, False)
-    return lay.gather(O.reshape(H, NC * CHUNK, -1)).to(v.dtype)
+class _GatedDelta(torch.autograd.Function):
+    """The whole operator on packed tensors: prologue and state walk kernels forward, state walk and prologue kernels backward.
+    The backward prologue recomputes the chunk's scores and triangular inverse, so only bf16 operands are kept."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, lay, scale):
+        from . import native
+        T, H, K = q.shape
+        dev, NC = q.device, lay.NC
+        qb, kb, vb = (_aligned(t.to(torch.bfloat16).contiguous()) for t in (q, k, v))
+        gf, bf = g.float().contiguous(), beta.float().contiguous()
+        W, Qg, Kd, U = (torch.empty(H, NC, CHUNK, K, dtype=torch.bfloat16, device=dev) for _ in range(4))
+        At = torch.empty(H, NC, CHUNK, CHUNK, dtype=torch.bfloat16, device=dev)
+        gamma = torch.empty(H, NC, dtype=torch.float32, device=dev)
+        L = native.lib()
+        native._check(L.mm_gdn_prologue(
+            qb.data_ptr(), kb.data_ptr(), vb.data_ptr(), gf.data_ptr(), bf.data_ptr(), lay.chunk_tok0.data_ptr(),
+            lay.chunk_len.data_ptr(), W.data_ptr(), Qg.data_ptr(), Kd.data_ptr(), At.data_ptr(), U.data_ptr(), gamma.data_ptr(),
+            H, NC, float(scale), native._st()), "gdn_prologue")
+        keep = ctx is not native._NO_GRAPH
+        O, Vn, SprevT = _state_pass_native(W, Qg, Kd, At, U, gamma, lay, keep)
+        out = torch.empty(lay.T, H, K, dtype=torch.bfloat16, device=dev)
+        native._check(L.mm_gdn_layout(O.data_ptr(), out.data_ptr(), lay.chunk_tok0.data_ptr(), lay.chunk_len.data_ptr(), H, NC, 0,
+                                      native._st()), "gdn_layout")
+        if keep:
+            ctx.save_for_backward(qb, kb, vb, gf, bf, W, Qg, Kd, At, gamma, Vn, SprevT)
+            ctx.meta = (lay, scale, g.dtype, beta.dtype)
+        return out.to(v.dtype)
+
+    @staticmethod
+    def backward(ctx, dout):
+        from . import native
+        q, k, v, g, beta, W, Qg, Kd, At, gamma, Vn, SprevT = ctx.saved_tensors
+        lay, scale, g_dtype, beta_dtype = ctx.meta
+        T, H, K = q.shape
+        NC, dev, L, st = lay.NC, q.device, native.lib(), native._st()
+        dout = _aligned(dout.to(torch.bfloat16).contiguous())
+        dO, dVn = torch.empty_like(Vn), torch.empty_like(Vn)
+        GT = torch.empty_like(SprevT)
+        native._check(L.mm_gdn_layout(dout.data_ptr(), dO.data_ptr(), lay.chunk_tok0.data_ptr(), lay.chunk_len.data_ptr(), H, NC, 1, st),
+                      "gdn_layout")
+        native._check(L.mm_gdn_bwd(W.data_ptr(), Qg.data_ptr(), Kd.data_ptr(), At.data_ptr(), dO.data_ptr(), gamma.data_ptr(),
+                                   lay.seq_chunks.data_ptr(), dVn.data_ptr(), GT.data_ptr(), H, NC, lay.nseq, 0,
+                                   native.status_word(dev).data_ptr(), st), "gdn_bwd")
+        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+        dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
+        native._check(L.mm_gdn_prologue_bwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(), lay.chunk_tok0.data_ptr(), lay.chunk_len.data_ptr(),
+            dO.data_ptr(), Vn.data_ptr(), dVn.data_ptr(), SprevT.data_ptr(), GT.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+            dg.data_ptr(), dbeta.data_ptr(), H, NC, float(scale), st), "gdn_prologue_bwd")
+        return dq, dk, dv, dg.to(g_dtype), dbeta.to(beta_dtype), None, None
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """The layout and prologue kernels read 16-byte vectors."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def kda_chunk_prologue(q, k, v, g, beta, scale: float):

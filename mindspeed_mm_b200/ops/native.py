@@ -89,6 +89,8 @@ def _declare(L):
         "mm_l2norm_fwd": [_p, _p, _p, _ll, _i, _f, _p],
         "mm_l2norm_bwd": [_p, _p, _p, _p, _ll, _i, _p],
         "mm_gdn_prologue": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _f, _p],
+        "mm_gdn_prologue_bwd": [_p] * 17 + [_i, _i, _f, _p],
+        "mm_gdn_layout": [_p, _p, _p, _p, _i, _i, _i, _p],
         "mm_gdn_fwd": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p, _p],
         "mm_gdn_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p, _p],
         "mm_p2p_scatter_rows": [_p, _p, _p, _p, _p, _i, _i, _i, _p],
