@@ -36,6 +36,8 @@ struct FmhaParams {
     const int* tile_q0;
     const int* n_tiles;
     const int* tile_nseq;   // sequences covered by each tile (> 1: packed short sequences, block-diagonal mask)
+    const bf16* q;      // read directly (Q -> tensor memory) by the alternating kernel
+    long long q_ts;
     bf16* o;
     float* lse;         // [Nq, T]
     int T, Nq, Nkv, causal;
@@ -330,12 +332,13 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 #include "fmha_fwd_split.cuh"
+#include "fmha_fwd_alt.cuh"
 
-int g_fwd_variant = 0;   // 0: one softmax warpgroup; 1 / 2: split-softmax kernel with 2 / 4 compute warpgroups (fmha_fwd_split.cuh)
+int g_fwd_variant = 0;   // 0: one softmax warpgroup; 1, 2: split softmax (fmha_fwd_split.cuh); 3: by key length (see mm_fmha_fwd)
 
 }  // namespace
 
-// Selects the forward kernel for later calls (0 = default, 1 = split softmax).  Returns the previous value.
+// Selects the forward kernel for later calls (see above; the Python side sets 3).  Returns the previous value.
 MM_API int mm_fmha_set_fwd_variant(int v) {
     const int prev = g_fwd_variant;
     g_fwd_variant = v;
@@ -370,14 +373,22 @@ MM_API int mm_fmha_fwd(const void* q, const void* k, const void* v, void* o, flo
         cudaError_t e = cudaFuncSetAttribute(fmha_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(fmha_fwd_split_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fmha_fwd_alt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAltSmem);
         if (e != cudaSuccess) return (int)e;
         done = true;
     }
-    FmhaParams p{cu_q, cu_k, tile_seq, tile_q0, n_tiles, tile_nseq, (bf16*)o, lse, T, Nq, Nkv, causal, D,
+    FmhaParams p{cu_q, cu_k, tile_seq, tile_q0, n_tiles, tile_nseq, (const bf16*)q, q_ts, (bf16*)o, lse, T, Nq, Nkv, causal, D,
                  scale * 1.4426950408889634f, status};
     dim3 grid(max_tiles, Nq);
-    if (g_fwd_variant == 0)      // fallback: one softmax warpgroup, O folded in registers
+    // Long key sequences take the alternating groups: a key tile costs them 1650 clocks against 2440, but a CTA's set-up and end
+    // (12 warps, a second hand-over of the row sums) more.  Keys per sequence on average, split / alternating, 8192 tokens:
+    // 16 heads of 80: 512 keys 119.5 / 121.8 us, 1024 152 / 145, 2048 218 / 190, 1 x 4096 208 / 165; 12 heads of 128: 1024 158 / 157,
+    // 1 x 4096 182 / 156, 1 x 7800 461 / 388; 40 heads, 1 x 32760 24.3 / 20.2 ms.  Causal (half the tiles of a CTA on average):
+    // 28 heads, 2048 312 / 314, 1 x 4096 247 / 223.
+    const bool alternate = g_fwd_variant == 3 && Tk >= (causal ? 3072LL : 1024LL) * n_seqs;
+    if (alternate)
+        fmha_fwd_alt_kernel<<<grid, kAltThreads, kAltSmem, st>>>(tK, tV, p);
+    else if (g_fwd_variant == 0)      // fallback: one softmax warpgroup, O folded in registers
         fmha_fwd_kernel<<<grid, kThreads, kSmem, st>>>(tQ, tK, tV, p);
     else                         // default: split softmax, O accumulated in tensor memory with lazy rescaling
         fmha_fwd_split_kernel<2, true><<<grid, 64 + 256, kSmem, st>>>(tQ, tK, tV, p);

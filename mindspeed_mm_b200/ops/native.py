@@ -17,8 +17,9 @@ from . import build as _build
 
 _LIB = None
 _STATUS: dict = {}
-# forward attention kernel: 3 = split softmax, O accumulated in tensor memory with lazy rescaling
-# (csrc/fmha_fwd_split.cuh, default); 0 = one softmax warpgroup, O folded in registers (csrc/fmha_fwd.cu, fallback)
+# forward attention kernel: 3 (default) = by key length, alternating softmax groups (csrc/fmha_fwd_alt.cuh) for long keys, else
+# split softmax (csrc/fmha_fwd_split.cuh), both with O in tensor memory and lazy rescaling; 2 = always split softmax;
+# 0 = one softmax warpgroup, O folded in registers (csrc/fmha_fwd.cu, fallback)
 FMHA_FWD_VARIANT = int(os.environ.get("MM_B200_FMHA_FWD_VARIANT", "3"))
 LAUNCHES = 0  # native kernel launches issued through this module (bench reports it)
 

@@ -147,3 +147,26 @@ def test_gated_delta_rule_on_bf16_tensors(lens, H, gate):
         assert torch.equal(ops.gated_delta_rule_varlen(q, k, v, g, beta, cu, chunk=64), o)
     with pytest.raises(RuntimeError):
         ops.gated_delta_rule_varlen(q, k, v, g, beta, [0, T + 1], chunk=64)
+
+
+@pytest.mark.parametrize("lens_q,lens_k,nq,nkv,D,causal,grow", [
+    ([1024], [1024], 2, 2, 128, False, False), ([1023], [1023], 2, 2, 128, False, False),       # both sides of the key-length rule
+    ([1025], [1025], 4, 2, 80, False, True), ([4000, 129, 1], [4000, 129, 1], 2, 1, 72, False, True),
+    ([100, 1], [2047, 3], 4, 4, 128, False, True), ([1500, 40], [900, 1700], 2, 2, 8, False, False),
+    ([3072], [3072], 2, 2, 128, True, True), ([3071], [3071], 2, 2, 128, True, False), ([6200, 1], [6200, 1], 2, 1, 128, True, True),
+    ([130, 3], [6143, 300], 7, 1, 128, True, False)])
+def test_attention_over_long_keys(lens_q, lens_k, nq, nkv, D, causal, grow):
+    """Alternating softmax groups: odd and even numbers of key tiles, a last tile of any width, sequences with a single tile, and
+    scores that grow along the keys, so that the reference maximum moves and O is rescaled again and again."""
+    torch.manual_seed(sum(lens_q) + sum(lens_k))
+    Tq, Tk = sum(lens_q), sum(lens_k)
+    q, k, v = (torch.randn(t, n, D, device=DEV).bfloat16() for t, n in ((Tq, nq), (Tk, nkv), (Tk, nkv)))
+    if grow:
+        q = q.abs()
+        k = (k + torch.linspace(0.0, 40.0 / D ** 0.5, Tk, device=DEV)[:, None, None]).bfloat16()
+    cu = [torch.tensor([0] + l, device=DEV).cumsum(0).to(torch.int32) for l in (lens_q, lens_k)]
+    out, lse = native.fmha_forward(q, k, v, cu[0], cu[1], causal, D ** -0.5)
+    want, want_lse = ref.attention_varlen(q.float(), k.float(), v.float(), cu[0].cpu(), cu[1].cpu(), causal, return_lse=True)
+    native.check_status()
+    _close(out, want, rtol=1e-2, atol=4e-3)               # probabilities and results are bf16
+    assert float((lse - want_lse.reshape(lse.shape)).abs().max()) < 2e-3 * (1 + float(want_lse.abs().max()))
