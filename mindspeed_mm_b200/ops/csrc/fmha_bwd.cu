@@ -69,29 +69,15 @@ __global__ void fmha_delta_kernel(const bf16* __restrict__ o, const bf16* __rest
     if (lane == 0) delta[(size_t)(row % Nq) * T + row / Nq] = s;
 }
 
-__global__ void fmha_bwd_plan_kernel(const int* cu, int n_seqs, int* tile_seq, int* tile_r0, int* n_tiles, int* tile_nseq,
-                                     int max_tiles, int rows, int descending, int pack) {
-    if (threadIdx.x || blockIdx.x) return;
-    if (pack) {          // non-causal self-attention: short sequences share tiles
-        int n = 0;
-        for (int b = 0; b < n_seqs && n < max_tiles;) b = plan_packed(cu, n_seqs, b, rows, tile_seq, tile_r0, tile_nseq, n, max_tiles);
-        *n_tiles = n;
-        return;
-    }
-    int n = 0, longest = 0;
-    for (int b = 0; b < n_seqs; ++b) longest = max(longest, cu[b + 1] - cu[b]);
-    const int nt = (longest + rows - 1) / rows;
-    for (int k = 0; k < nt; ++k) {
-        const int t = descending ? nt - 1 - k : k;     // heavy tiles first
-        for (int b = 0; b < n_seqs && n < max_tiles; ++b)
-            if (t * rows < cu[b + 1] - cu[b]) {
-                tile_nseq[n] = 1;
-                tile_seq[n] = b;
-                tile_r0[n] = t * rows;
-                ++n;
-            }
-    }
-    *n_tiles = n;
+struct PlanOut {
+    const int* cu;
+    int *tile_seq, *tile_r0, *n_tiles, *tile_nseq;
+    int max_tiles;
+};
+// Block 0: query tiles, heavy ones first; block 1: key tiles (early ones see the most query tiles under a causal mask).
+__global__ void __launch_bounds__(kPlanThreads) fmha_bwd_plan_kernel(PlanOut q, PlanOut k, int n_seqs, int rows, int pack) {
+    const PlanOut& o = blockIdx.x ? k : q;
+    plan_tiles(o.cu, n_seqs, o.tile_seq, o.tile_r0, o.n_tiles, o.tile_nseq, o.max_tiles, rows, blockIdx.x == 0, pack);
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -630,9 +616,8 @@ MM_API int mm_fmha_bwd(const void* q, const void* k, const void* v, const void* 
     // short sequences share a tile when the mask allows it: non-causal, keys and queries the same packed sequences
     const int pack = !causal && cu_q == cu_k && T == Tk && variant != 0;
     fmha_delta_kernel<<<(unsigned)(((long long)T * Nq + 7) / 8), 256, 0, st>>>((const bf16*)o, (const bf16*)dO, delta, T, Nq, D);
-    fmha_bwd_plan_kernel<<<1, 32, 0, st>>>(cu_q, n_seqs, q_seq, q_r0, q_n, q_nseq, mq, 128, 1, pack);
-    // early key tiles see the most query tiles under a causal mask: emit them first
-    fmha_bwd_plan_kernel<<<1, 32, 0, st>>>(cu_k, n_seqs, k_seq, k_r0, k_n, k_nseq, mk, 128, 0, pack);
+    fmha_bwd_plan_kernel<<<2, kPlanThreads, 0, st>>>(PlanOut{cu_q, q_seq, q_r0, q_n, q_nseq, mq}, PlanOut{cu_k, k_seq, k_r0, k_n, k_nseq, mk},
+                                                     n_seqs, 128, pack);
     CUtensorMap tQ, tK, tV, tdO, tQ64, tdO64;
     int r;
     if ((r = make_tmap_3d(&tQ, q, D, Nq, T, D, q_ts, 64, 1, 128))) return 1000 + r;

@@ -46,28 +46,10 @@ struct FmhaParams {
     int* status;
 };
 
-__global__ void fmha_plan_kernel(const int* cu_q, int n_seqs, int* tile_seq, int* tile_q0, int* n_tiles, int* tile_nseq,
-                                 int max_tiles, int pack) {
-    if (threadIdx.x || blockIdx.x) return;
-    if (pack) {          // non-causal self-attention: short sequences share tiles (all tiles cost about the same)
-        int n = 0;
-        for (int b = 0; b < n_seqs && n < max_tiles;) b = plan_packed(cu_q, n_seqs, b, BQ, tile_seq, tile_q0, tile_nseq, n, max_tiles);
-        *n_tiles = n;
-        return;
-    }
-    // Later query tiles of a causal sequence have more key tiles: emit them first so the tail of the grid is
-    // made of short work items.
-    int n = 0, longest = 0;
-    for (int b = 0; b < n_seqs; ++b) longest = max(longest, cu_q[b + 1] - cu_q[b]);
-    for (int t = (longest + BQ - 1) / BQ - 1; t >= 0; --t)
-        for (int b = 0; b < n_seqs && n < max_tiles; ++b)
-            if (t * BQ < cu_q[b + 1] - cu_q[b]) {
-                tile_seq[n] = b;
-                tile_q0[n] = t * BQ;
-                tile_nseq[n] = 1;
-                ++n;
-            }
-    *n_tiles = n;
+// Later query tiles of a causal sequence have more key tiles: emit them first so the tail of the grid is made of short work items.
+__global__ void __launch_bounds__(kPlanThreads) fmha_plan_kernel(const int* cu_q, int n_seqs, int* tile_seq, int* tile_q0, int* n_tiles,
+                                                                int* tile_nseq, int max_tiles, int pack) {
+    plan_tiles(cu_q, n_seqs, tile_seq, tile_q0, n_tiles, tile_nseq, max_tiles, BQ, true, pack);
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -362,7 +344,7 @@ MM_API int mm_fmha_fwd(const void* q, const void* k, const void* v, void* o, flo
     int* tile_nseq = plan + 2 * max_tiles + 1;
     // short sequences share a tile when the mask allows it: non-causal, keys and queries the same packed sequences
     const int pack = !causal && cu_q == cu_k && T == Tk && g_fwd_variant != 0;
-    fmha_plan_kernel<<<1, 32, 0, st>>>(cu_q, n_seqs, tile_seq, tile_q0, n_tiles, tile_nseq, max_tiles, pack);
+    fmha_plan_kernel<<<1, kPlanThreads, 0, st>>>(cu_q, n_seqs, tile_seq, tile_q0, n_tiles, tile_nseq, max_tiles, pack);
     CUtensorMap tQ, tK, tV;
     int r;
     if ((r = make_tmap_3d(&tQ, q, D, Nq, T, D, q_ts, 64, 1, BQ))) return 1000 + r;
