@@ -59,14 +59,18 @@ struct GemvParams {
     float eps;
 };
 
-constexpr int kGemvWarps = 4, kGemvU = 4;
+constexpr int kGemvWarps = 4, kGemvU = 2;
 
-// out[m, n] = act(norm(x)[m, :] . w[n, :] + bias[n]) + res[m, n].  A warp owns two weight rows (two neighbouring outputs; SWIGLU:
-// the gate and the up row of one output), lanes stride over K in 16-byte pieces, the next 4 pieces of both rows in flight while
-// the current ones are multiplied; x (normalised once per block) sits in shared memory as bf16, sums are fp32.
-// 128-thread blocks: 3584 outputs are 448 blocks, so the SMs differ by one block in four, not one in two.
+__device__ __forceinline__ void copy_async(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+
+// out[m, n] = act(norm(x)[m, :] . w[n, :] + bias[n]) + res[m, n] for 2 to 4 rows (and one long row with a norm or SwiGLU).  A warp
+// owns two weight rows (two neighbouring outputs; SWIGLU: the gate and the up row of one output), lanes stride over K in 16-byte
+// pieces, the next ones of both rows in flight while the current ones are multiplied; x (normalised once per block) sits in shared
+// memory as bf16, sums are fp32.  128-thread blocks: 3584 outputs are 448 blocks, so the SMs differ by one block in four.
 template <int M, bool SWIGLU, bool NORM>
-__global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(GemvParams p) {
+__global__ void __launch_bounds__(kGemvWarps * 32, M == 1 ? 8 : 4) gemv_kernel(GemvParams p) {
     extern __shared__ __align__(16) uint8_t gemv_smem[];
     bf16* xs = reinterpret_cast<bf16*>(gemv_smem);                  // [M][K]
     __shared__ float red[72];
@@ -93,32 +97,35 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(GemvParams p) {
         }
     };
     load(0, a, b);
+    // every piece of x (and of the norm's weight) is in flight at once: one trip to L2, not one per loop step
+    bf16* ns = xs + (size_t)M * p.K;                                 // norm weight [K]
+    for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) {
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-        const Vec8* xr = reinterpret_cast<const Vec8*>(p.x + m * p.ldx);
-        Vec8* dst = reinterpret_cast<Vec8*>(xs + (size_t)m * p.K);
-        if constexpr (NORM) {
+        for (int m = 0; m < M; ++m) copy_async(xs + (size_t)m * p.K + i * 8, p.x + m * p.ldx + i * 8);
+        if constexpr (NORM) copy_async(ns + i * 8, p.norm + i * 8);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if constexpr (NORM) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {                                 // a thread works on the pieces that it copied
+            Vec8* row = reinterpret_cast<Vec8*>(xs + (size_t)m * p.K);
             float ss = 0.f;
             for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) {
-                const Vec8 v = xr[i];
                 float f[8];
-                unpack8(v, f);
+                unpack8(row[i], f);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) ss += f[k] * f[k];
-                dst[i] = v;
             }
             ss = block_sum(ss, red);
             const float rstd = rsqrtf(ss / (float)p.K + p.eps);
-            for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) {      // each thread re-reads what it wrote
+            for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) {
                 float f[8], g[8];
-                unpack8(dst[i], f);
-                unpack8(reinterpret_cast<const Vec8*>(p.norm)[i], g);
+                unpack8(row[i], f);
+                unpack8(reinterpret_cast<const Vec8*>(ns)[i], g);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) f[k] = f[k] * rstd * g[k];
-                dst[i] = pack8(f);
+                row[i] = pack8(f);
             }
-        } else {
-            for (int i = threadIdx.x; i < nvec; i += kGemvWarps * 32) dst[i] = xr[i];
         }
     }
     __syncthreads();
@@ -174,12 +181,194 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(GemvParams p) {
     }
 }
 
+// One row of x: the four warps of a block share pairs of weight rows (two neighbouring outputs; SWIGLU: the gate and the up row of
+// one output), a quarter of K each, with the next pair (or the next piece of a long row) in flight while this one is multiplied.
+// Nothing is staged: a thread's part of x stays in registers for all pairs of the block if the row is at most kRowK long, and is read
+// through L1, which the weights bypass, if it is longer.  With a norm a block sums the squares of x once, while its first weights are
+// on their way, and keeps the normalised x, rounded to bf16 like the norm kernel's result.
+constexpr int kSplitU = 4, kStep = kGemvWarps * kSplitU * 32;        // 16-byte pieces of a row per step
+constexpr int kRowK = kStep * 8;                                     // 4096
+constexpr int kRowBlocks = 148 * 4;
+
+struct RowLoads {
+    uint4 a[kSplitU], b[kSplitU];
+};
+
+__device__ __forceinline__ void multiply(const RowLoads& w, const uint4* x, float2& acc0, float2& acc1) {
+#pragma unroll
+    for (int j = 0; j < kSplitU; ++j) {
+        const uint32_t ua[4] = {w.a[j].x, w.a[j].y, w.a[j].z, w.a[j].w}, ub[4] = {w.b[j].x, w.b[j].y, w.b[j].z, w.b[j].w};
+        const uint32_t ux[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 f = bf2(ux[k]);
+            acc0 = __ffma2_rn(bf2(ua[k]), f, acc0);
+            acc1 = __ffma2_rn(bf2(ub[k]), f, acc1);
+        }
+    }
+}
+
+template <bool SWIGLU>
+__device__ __forceinline__ void finish_pair(const GemvParams& p, int pair, float2 s) {
+    if constexpr (SWIGLU) {
+        p.out[pair] = __float2bfloat16(s.x / (1.f + __expf(-s.x)) * s.y);
+    } else {
+        const int r = 2 * pair;
+        if (p.bias) {
+            s.x += __bfloat162float(p.bias[r]);
+            s.y += __bfloat162float(p.bias[r + 1]);
+        }
+        if (p.res) {
+            const float2 t = __bfloat1622float2(*reinterpret_cast<const bf162*>(p.res + r));
+            s.x += t.x;
+            s.y += t.y;
+        }
+        *reinterpret_cast<bf162*>(p.out + r) = __floats2bfloat162_rn(s.x, s.y);
+    }
+}
+
+// K <= kRowK.  One wave of blocks walks the pairs.
+template <bool SWIGLU, bool NORM>
+__global__ void __launch_bounds__(kGemvWarps * 32, 4) gemv_rows_kernel(GemvParams p) {
+    __shared__ float2 part[2][kGemvWarps];
+    __shared__ float red[72];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = p.K >> 3, pairs = SWIGLU ? p.N : p.N >> 1;
+    auto row = [&](int pair, int second) {
+        return reinterpret_cast<const uint4*>(p.w + (size_t)(SWIGLU ? pair + second * p.N : 2 * pair + second) * p.ldw);
+    };
+    for (int pair = blockIdx.x; pair < pairs && pair < blockIdx.x + 2 * (int)gridDim.x; pair += gridDim.x)      // the first two pairs
+        for (int i = threadIdx.x * 8; i < nvec; i += kGemvWarps * 256) {
+            prefetch_l2(row(pair, 0) + i);
+            prefetch_l2(row(pair, 1) + i);
+        }
+    wait_for_predecessor();
+    let_successor_start();
+    auto load = [&](int pair, RowLoads& w) {
+        const uint4 *w0 = row(pair, 0), *w1 = row(pair, 1);
+#pragma unroll
+        for (int j = 0; j < kSplitU; ++j) {
+            const int i = (warp * kSplitU + j) * 32 + lane;
+            w.a[j] = i < nvec ? ld_once(w0 + i) : make_uint4(0, 0, 0, 0);
+            w.b[j] = i < nvec ? ld_once(w1 + i) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    RowLoads cur, nxt;
+    load(blockIdx.x, cur);
+    uint4 x[kSplitU];
+#pragma unroll
+    for (int j = 0; j < kSplitU; ++j) {
+        const int i = (warp * kSplitU + j) * 32 + lane;
+        x[j] = i < nvec ? reinterpret_cast<const uint4*>(p.x)[i] : make_uint4(0, 0, 0, 0);
+    }
+    if constexpr (NORM) {
+        uint4 g[kSplitU];
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < kSplitU; ++j) {
+            const int i = (warp * kSplitU + j) * 32 + lane;
+            g[j] = i < nvec ? reinterpret_cast<const uint4*>(p.norm)[i] : make_uint4(0, 0, 0, 0);
+            float f[8];
+            unpack8(*reinterpret_cast<Vec8*>(&x[j]), f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) ss += f[k] * f[k];
+        }
+        const float rstd = rsqrtf(block_sum(ss, red) / (float)p.K + p.eps);
+#pragma unroll
+        for (int j = 0; j < kSplitU; ++j) {
+            float f[8], h[8];
+            unpack8(*reinterpret_cast<Vec8*>(&x[j]), f);
+            unpack8(*reinterpret_cast<Vec8*>(&g[j]), h);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) f[k] = f[k] * rstd * h[k];
+            *reinterpret_cast<Vec8*>(&x[j]) = pack8(f);
+            // past the end of the row the norm weight is zero; an infinite rstd must not turn that into NaN
+            if ((warp * kSplitU + j) * 32 + lane >= nvec) x[j] = make_uint4(0, 0, 0, 0);
+        }
+    }
+    int it = 0;
+    for (int pair = blockIdx.x; pair < pairs; pair += gridDim.x, ++it) {
+        if (pair + (int)gridDim.x < pairs) load(pair + gridDim.x, nxt);
+        float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+        multiply(cur, x, acc0, acc1);
+        const float s0 = warp_sum(acc0.x + acc0.y), s1 = warp_sum(acc1.x + acc1.y);
+        if (lane == 0) part[it & 1][warp] = make_float2(s0, s1);
+        __syncthreads();                        // (the other half of `part` is written next: its readers are behind this barrier)
+        if (threadIdx.x == (it & 3) * 32) {
+            float2 s = part[it & 1][0];
+#pragma unroll
+            for (int w = 1; w < kGemvWarps; ++w) {
+                s.x += part[it & 1][w].x;
+                s.y += part[it & 1][w].y;
+            }
+            finish_pair<SWIGLU>(p, pair, s);
+        }
+        cur = nxt;
+    }
+}
+
+// K > kRowK: a block per pair, the next step of both rows in flight.  3584 x 18944: 21.9 us, 6.2 TB/s (37 with a warp per pair, whose
+// 12 warps an SM kept 2 KB each in flight).
+__global__ void __launch_bounds__(kGemvWarps * 32) gemv_split_kernel(GemvParams p) {
+    __shared__ float2 part[kGemvWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = p.K >> 3, pair = blockIdx.x;
+    const uint4* w0 = reinterpret_cast<const uint4*>(p.w + (size_t)(2 * pair) * p.ldw);
+    const uint4* w1 = reinterpret_cast<const uint4*>(p.w + (size_t)(2 * pair + 1) * p.ldw);
+    const uint4* xv = reinterpret_cast<const uint4*>(p.x);
+    for (int i = threadIdx.x * 8; i < nvec && i < 1024; i += kGemvWarps * 256) {       // 128-byte lines, the first 16 KB of each row
+        prefetch_l2(w0 + i);
+        prefetch_l2(w1 + i);
+    }
+    wait_for_predecessor();
+    let_successor_start();
+    RowLoads cur, nxt;
+    uint4 x[kSplitU], nx[kSplitU];
+    auto load = [&](int c, RowLoads& w, uint4* t) {
+#pragma unroll
+        for (int j = 0; j < kSplitU; ++j) {
+            const int i = ((c * kGemvWarps + warp) * kSplitU + j) * 32 + lane;
+            const bool in = i < nvec;
+            w.a[j] = in ? ld_once(w0 + i) : make_uint4(0, 0, 0, 0);
+            w.b[j] = in ? ld_once(w1 + i) : make_uint4(0, 0, 0, 0);
+            t[j] = in ? xv[i] : make_uint4(0, 0, 0, 0);
+        }
+    };
+    load(0, cur, x);
+    float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+    const int chunks = (nvec + kStep - 1) / kStep;
+    for (int c = 0; c < chunks; ++c) {
+        if (c + 1 < chunks) load(c + 1, nxt, nx);
+        multiply(cur, x, acc0, acc1);
+        cur = nxt;
+#pragma unroll
+        for (int j = 0; j < kSplitU; ++j) x[j] = nx[j];
+    }
+    const float s0 = warp_sum(acc0.x + acc0.y), s1 = warp_sum(acc1.x + acc1.y);
+    if (lane == 0) part[warp] = make_float2(s0, s1);
+    __syncthreads();
+    if (threadIdx.x) return;
+    float2 s = part[0];
+#pragma unroll
+    for (int w = 1; w < kGemvWarps; ++w) {
+        s.x += part[w].x;
+        s.y += part[w].y;
+    }
+    finish_pair<false>(p, pair, s);
+}
+
 template <int M, bool SWIGLU, bool NORM>
 int run_gemv(const GemvParams& p, cudaStream_t st) {
+    if constexpr (M == 1) {
+        // one row: against a warp per pair, at the shapes of a 7B decoder layer: 4608 x 3584 with norm 12.2 -> 6.3 us, 3584 x 3584
+        // 9.1 -> 5.1, 37888 x 3584 with norm and SwiGLU 48.2 -> 40.2 (6.8 TB/s), 152064 x 3584 165 -> 155, 3584 x 18944 37 -> 22
+        const int pairs = SWIGLU ? p.N : p.N / 2;
+        if (p.K <= kRowK)
+            return launch_pdl(gemv_rows_kernel<SWIGLU, NORM>, dim3(pairs < kRowBlocks ? pairs : kRowBlocks), kGemvWarps * 32, (size_t)0, 1, st, p);
+        if (!SWIGLU && !NORM) return launch_pdl(gemv_split_kernel, dim3(pairs), kGemvWarps * 32, (size_t)0, 1, st, p);
+    }
     auto kern = gemv_kernel<M, SWIGLU, NORM>;
-    const size_t smem = (size_t)M * p.K * 2;
+    const size_t smem = (size_t)(M + NORM) * p.K * 2;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
         if (e != cudaSuccess) return (int)e;
     }
     const int units = SWIGLU ? p.N : p.N / 2;
@@ -445,11 +634,13 @@ __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(Dec
 
 // out[M, N] = swiglu?(norm?(x) @ W^T + bias?) + residual?  for M <= 4 rows.  norm: RMSNorm weight [K] or null; bias [N], res
 // [M, N]: null or bf16 (not with swiglu).  swiglu: W is [2N, K], gate rows then up rows.  K % 8 == 0, N % 2 == 0, leading
-// dimensions multiples of 8, 16-byte aligned bases, M * K <= 80 K elements (x is kept in shared memory).
-// Why M <= 4: 3584 x 3584 and 3584 x 18944 take 6.3 / 25.8 us at M = 1 (25 and 83 us as tensor-core tiles).
+// dimensions multiples of 8, 16-byte aligned bases, M * K <= 80 K elements (x, and with a norm its weight, in shared memory).
+// As tensor-core tiles 3584 x 3584 and 3584 x 18944 take 25 and 83 us for one row.
 MM_API int mm_gemv_bf16(const void* x, const void* w, const void* bias, const void* norm, const void* res, void* out, int M, int N,
                         int K, long long ldx, long long ldw, long long ldr, long long ldo, float eps, int swiglu, cudaStream_t st) {
-    if (M < 1 || M > 4 || N < 1 || K < 1 || K % 8 || N % 2 || (ldx | ldw | ldr | ldo) % 8 || (long long)M * K > 80 * 1024) return -1;
+    if (M < 1 || M > 4 || N < 1 || K < 1 || K % 8 || N % 2 || (ldx | ldw | ldr | ldo) % 8 || (long long)M * K > 80 * 1024 ||
+        (norm && (M + 1LL) * K > 112 * 1024))
+        return -1;
     if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out | (uintptr_t)norm) & 15 || ((uintptr_t)res & 3)) return -2;
     if (swiglu && (bias || res)) return -3;
     GemvParams p{(const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)norm, (const bf16*)res, (bf16*)out,
