@@ -19,7 +19,7 @@ template <int NV>
 __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const bf16* __restrict__ x,
                                                                    const bf16* __restrict__ w, bf16* __restrict__ y,
                                                                    float* __restrict__ rstd_out, int T, int H,
-                                                                   float eps) {
+                                                                   long long ldx, float eps) {
     __shared__ float red[72];
     const int nvec = H >> 3;
     // a thread owns the same columns in every row: its slice of the weight is read once, not once per row (re-reading it
@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const bf16* __
     // the next row's loads are issued before this row's reduction, so they are in flight across the block barrier
     Vec8 cache[NV];
     if (blockIdx.x < T) {
-        const Vec8* xr = reinterpret_cast<const Vec8*>(x + (size_t)blockIdx.x * H);
+        const Vec8* xr = reinterpret_cast<const Vec8*>(x + blockIdx.x * ldx);
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             int i = threadIdx.x + j * kRowThreads;
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const bf16* __
         Vec8 nxt[NV];
         const int nrow = row + gridDim.x;
         if (nrow < T) {
-            const Vec8* xn = reinterpret_cast<const Vec8*>(x + (size_t)nrow * H);
+            const Vec8* xn = reinterpret_cast<const Vec8*>(x + nrow * ldx);
 #pragma unroll
             for (int j = 0; j < NV; ++j) {
                 int i = threadIdx.x + j * kRowThreads;
@@ -90,7 +90,7 @@ template <int NV>
 __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_v16_kernel(const bf16* __restrict__ x,
                                                                        const bf16* __restrict__ w, bf16* __restrict__ y,
                                                                        float* __restrict__ rstd_out, int T, int H,
-                                                                       float eps) {
+                                                                       long long ldx, float eps) {
     __shared__ float red[72];
     const int nvec = H >> 4;
     Vec16 wc[NV], cache[NV];
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_v16_kernel(const bf16
         if (i < nvec) wc[j] = ld_v16(w + (size_t)i * 16);
     }
     if (blockIdx.x < T) {
-        const bf16* xr = x + (size_t)blockIdx.x * H;
+        const bf16* xr = x + blockIdx.x * ldx;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             int i = threadIdx.x + j * kRowThreads;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_v16_kernel(const bf16
         Vec16 nxt[NV];
         const int nrow = row + gridDim.x;
         if (nrow < T) {
-            const bf16* xn = x + (size_t)nrow * H;
+            const bf16* xn = x + nrow * ldx;
 #pragma unroll
             for (int j = 0; j < NV; ++j) {
                 int i = threadIdx.x + j * kRowThreads;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_bwd_kernel(const bf16* __rest
                                                                    const bf16* __restrict__ dy,
                                                                    const float* __restrict__ rstd_in,
                                                                    bf16* __restrict__ dx,
-                                                                   float* __restrict__ dw_partial, int T, int H) {
+                                                                   float* __restrict__ dw_partial, int T, int H, long long ldx) {
     __shared__ float red[72];
     const int nvec = H >> 3;
     float dwacc[NV][8];
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_bwd_kernel(const bf16* __rest
     constexpr bool kPrefetch = NV <= 2;
     Vec8 xc[NV], gc[NV];
     auto load_row = [&](int r, Vec8* xd, Vec8* gd) {
-        const Vec8* xr = reinterpret_cast<const Vec8*>(x + (size_t)r * H);
+        const Vec8* xr = reinterpret_cast<const Vec8*>(x + r * ldx);
         const Vec8* gr = reinterpret_cast<const Vec8*>(dy + (size_t)r * H);
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
@@ -644,6 +644,9 @@ __global__ void __launch_bounds__(kThreads) ln_mod_fwd_v16_kernel(const bf16* __
 
 // dx = rstd * (g - mean(g) - xhat * mean(g * xhat)), g = dy * (1 + scale);
 // dscale[b] += dy * xhat, dshift[b] += dy  -> per-CTA partials (CTA c handles rows of ONE batch entry).
+// NV = 16-byte vectors cached per thread: with the arrays of the widest row (4 vectors, 128 accumulators) every width ran at two
+// blocks an SM; 7800 rows of 1536 took 79 us, with one vector 31 us.
+template <int NV>
 __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ scale,
                                                               const bf16* __restrict__ dy,
                                                               const float* __restrict__ mean_in,
@@ -654,10 +657,10 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
     __shared__ float red[72];
     const int nvec = H >> 3;
     const int b = blockIdx.x / ctas_per_batch, lane_cta = blockIdx.x % ctas_per_batch;
-    float sc[kMaxVec][8], dsc[kMaxVec][8], dsh[kMaxVec][8];
+    float sc[NV][8], dsc[NV][8], dsh[NV][8];
     const Vec8* scp = reinterpret_cast<const Vec8*>(scale + (size_t)b * H);
 #pragma unroll
-    for (int j = 0; j < kMaxVec; ++j) {
+    for (int j = 0; j < NV; ++j) {
         int i = threadIdx.x + j * kThreads;
 #pragma unroll
         for (int k = 0; k < 8; ++k) dsc[j][k] = dsh[j][k] = 0.f;
@@ -668,10 +671,10 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
         const Vec8* xr = reinterpret_cast<const Vec8*>(x + row * H);
         const Vec8* gr = reinterpret_cast<const Vec8*>(dy + row * H);
         const float mean = mean_in[row], rstd = rstd_in[row];
-        float xh[kMaxVec][8], g[kMaxVec][8];
+        float xh[NV][8], g[NV][8];
         float m1 = 0.f, m2 = 0.f;
 #pragma unroll
-        for (int j = 0; j < kMaxVec; ++j) {
+        for (int j = 0; j < NV; ++j) {
             int i = threadIdx.x + j * kThreads;
             if (i < nvec) {
                 float a[8], d[8];
@@ -693,7 +696,7 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
         m2 /= (float)H;
         Vec8* dxr = reinterpret_cast<Vec8*>(dx + row * H);
 #pragma unroll
-        for (int j = 0; j < kMaxVec; ++j) {
+        for (int j = 0; j < NV; ++j) {
             int i = threadIdx.x + j * kThreads;
             if (i < nvec) {
                 float o[8];
@@ -706,7 +709,7 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
     float* o1 = dscale_partial + (size_t)blockIdx.x * H;
     float* o2 = dshift_partial + (size_t)blockIdx.x * H;
 #pragma unroll
-    for (int j = 0; j < kMaxVec; ++j) {
+    for (int j = 0; j < NV; ++j) {
         int i = threadIdx.x + j * kThreads;
         if (i < nvec) {
 #pragma unroll
@@ -718,14 +721,23 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
     }
 }
 
-// out[b, c] = sum_p partial[b*P + p, c]
-__global__ void fold_partials_batched_kernel(const float* __restrict__ partial, bf16* __restrict__ out, int P, int H) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y;
-    if (c >= H) return;
+// out[b, c] = sum over p of partial[b*P + p, c], for dscale (blockIdx.z = 0) and dshift; 32 lanes along c, 32 along p
+__global__ void __launch_bounds__(1024) fold_scale_shift_kernel(const float* __restrict__ p1, const float* __restrict__ p2,
+                                                               bf16* __restrict__ out1, bf16* __restrict__ out2, int P, int H) {
+    __shared__ float tile[32][33];
+    const int c = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y;
+    const float* partial = blockIdx.z ? p2 : p1;
     float s = 0.f;
-    for (int p = 0; p < P; ++p) s += partial[((size_t)b * P + p) * H + c];
-    out[(size_t)b * H + c] = __float2bfloat16(s);
+    if (c < H)
+        for (int p = threadIdx.y; p < P; p += 32) s += partial[((size_t)b * P + p) * H + c];
+    tile[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && c < H) {
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) t += tile[k][threadIdx.x];
+        (blockIdx.z ? out2 : out1)[(size_t)b * H + c] = __float2bfloat16(t);
+    }
 }
 
 // out = x + gate[b] * y   (x,y: [B*S, H]; gate: [B, H])
@@ -843,16 +855,18 @@ MM_API int mm_rmsnorm_set_v16(int on) {
     return 0;
 }
 
-MM_API int mm_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, int H, float eps,
-                          cudaStream_t st) {
-    if (H % 8 || H > kRowThreads * 8 * 8) return -1;
+// ldx: elements between rows of x (a column block of a wider matrix is read where it lies); y is dense.
+MM_API int mm_rmsnorm_fwd_ld(const void* x, long long ldx, const void* w, void* y, float* rstd, int T, int H, float eps,
+                             cudaStream_t st) {
+    if (H % 8 || ldx % 8 || H > kRowThreads * 8 * 8) return -1;
     // measured at 3584 (two vectors of 16 per thread): 0.86 -> 0.91 of the copy bandwidth; wider rows keep the 16-byte form
-    if (H % 16 == 0 && H <= kRowThreads * 2 * 16 && ((((uintptr_t)x | (uintptr_t)y | (uintptr_t)w)) & 31) == 0 && g_rms_fwd_v16) {
+    if (H % 16 == 0 && ldx % 16 == 0 && H <= kRowThreads * 2 * 16 && ((((uintptr_t)x | (uintptr_t)y | (uintptr_t)w)) & 31) == 0 &&
+        g_rms_fwd_v16) {
         const int nv16 = (H / 16 + kRowThreads - 1) / kRowThreads;
         static int h1 = 0, h2 = 0, h4 = 0;
 #define MM_RMS_FWD16(NV)                                                                                        \
     rmsnorm_fwd_v16_kernel<NV><<<resident_grid(rmsnorm_fwd_v16_kernel<NV>, kRowThreads, T, h##NV), kRowThreads, 0, st>>>( \
-        (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, T, H, eps)
+        (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, T, H, ldx, eps)
         if (nv16 <= 1) MM_RMS_FWD16(1);
         else if (nv16 <= 2) MM_RMS_FWD16(2);
         else MM_RMS_FWD16(4);
@@ -863,7 +877,7 @@ MM_API int mm_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, in
     static int g2 = 0, g4 = 0, g8 = 0;
 #define MM_RMS_FWD(NV)                                                                                  \
     rmsnorm_fwd_kernel<NV><<<resident_grid(rmsnorm_fwd_kernel<NV>, kRowThreads, T, g##NV), kRowThreads, 0, st>>>( \
-        (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, T, H, eps)
+        (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, T, H, ldx, eps)
     if (nv <= 2) MM_RMS_FWD(2);
     else if (nv <= 4) MM_RMS_FWD(4);
     else MM_RMS_FWD(8);
@@ -871,24 +885,33 @@ MM_API int mm_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, in
     return (int)cudaGetLastError();
 }
 
+MM_API int mm_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, int H, float eps, cudaStream_t st) {
+    return mm_rmsnorm_fwd_ld(x, H, w, y, rstd, T, H, eps, st);
+}
+
 MM_API int mm_rmsnorm_bwd_grid(int T) { return T < 148 * 6 ? T : 148 * 6; }
 
 // dw_partial: scratch of mm_rmsnorm_bwd_grid(T) * H floats.
-MM_API int mm_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, void* dx, void* dw,
-                          float* dw_partial, int T, int H, cudaStream_t st) {
-    if (H % 8 || H > kRowThreads * 8 * 8) return -1;
+MM_API int mm_rmsnorm_bwd_ld(const void* x, long long ldx, const void* w, const void* dy, const float* rstd, void* dx, void* dw,
+                             float* dw_partial, int T, int H, cudaStream_t st) {
+    if (H % 8 || ldx % 8 || H > kRowThreads * 8 * 8) return -1;
     static int g128 = 0, g256 = 0, g512 = 0;
     int grid = mm_rmsnorm_bwd_grid(T);      // the scratch holds that many partial rows; one resident wave may be fewer
 #define MM_RMS_BWD(TH)                                                                                              \
     grid = min(grid, resident_grid(rmsnorm_bwd_kernel<2, TH>, TH, T, g##TH));                                       \
     rmsnorm_bwd_kernel<2, TH><<<grid, TH, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd,          \
-                                                   (bf16*)dx, dw_partial, T, H)
+                                                   (bf16*)dx, dw_partial, T, H, ldx)
     if (H <= 128 * 16) { MM_RMS_BWD(128); }
     else if (H <= 256 * 16) { MM_RMS_BWD(256); }
     else { MM_RMS_BWD(512); }
 #undef MM_RMS_BWD
     fold_partials_kernel<<<(H + 31) / 32, dim3(32, 8), 0, st>>>(dw_partial, (bf16*)dw, grid, H);
     return (int)cudaGetLastError();
+}
+
+MM_API int mm_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, void* dx, void* dw, float* dw_partial,
+                          int T, int H, cudaStream_t st) {
+    return mm_rmsnorm_bwd_ld(x, H, w, dy, rstd, dx, dw, dw_partial, T, H, st);
 }
 
 MM_API int mm_swiglu_fwd(const void* in, void* out, long long T, int F, cudaStream_t st) {
@@ -981,11 +1004,15 @@ MM_API int mm_ln_mod_bwd(const void* x, const void* scale, const void* dy, const
     int per = mm_ln_mod_bwd_ctas(B, S);
     float* p1 = partials;
     float* p2 = partials + (size_t)B * per * H;
-    ln_mod_bwd_kernel<<<B * per, kThreads, 0, st>>>((const bf16*)x, (const bf16*)scale, (const bf16*)dy, mean, rstd,
-                                                    (bf16*)dx, p1, p2, S, H, per);
-    dim3 g((H + 255) / 256, B);
-    fold_partials_batched_kernel<<<g, 256, 0, st>>>(p1, (bf16*)dscale, per, H);
-    fold_partials_batched_kernel<<<g, 256, 0, st>>>(p2, (bf16*)dshift, per, H);
+    const int nv = (H / 8 + kThreads - 1) / kThreads;
+#define MM_LN_BWD(NV)                                                                                                     \
+    ln_mod_bwd_kernel<NV><<<B * per, kThreads, 0, st>>>((const bf16*)x, (const bf16*)scale, (const bf16*)dy, mean, rstd, (bf16*)dx, \
+                                                        p1, p2, S, H, per)
+    if (nv <= 1) MM_LN_BWD(1);
+    else if (nv <= 2) MM_LN_BWD(2);
+    else MM_LN_BWD(4);
+#undef MM_LN_BWD
+    fold_scale_shift_kernel<<<dim3((H + 31) / 32, B, 2), dim3(32, 32), 0, st>>>(p1, p2, (bf16*)dscale, (bf16*)dshift, per, H);
     return (int)cudaGetLastError();
 }
 
@@ -1061,10 +1088,10 @@ MM_API int mm_rmsnorm_bwd_noalloc(const void* x, const void* w, const void* dy, 
     const int grid = T < MM_NOALLOC_MAX_CTAS ? T : MM_NOALLOC_MAX_CTAS;
     if (H <= 128 * 16)
         rmsnorm_bwd_kernel<2, 128><<<grid, 128, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd,
-                                                         (bf16*)dx, partial, T, H);
+                                                         (bf16*)dx, partial, T, H, H);
     else
         rmsnorm_bwd_kernel<2, 256><<<grid, 256, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd,
-                                                         (bf16*)dx, partial, T, H);
+                                                         (bf16*)dx, partial, T, H, H);
     fold_partials_kernel<<<(H + 31) / 32, dim3(32, 8), 0, st>>>(partial, (bf16*)dw, grid, H);
     return (int)cudaGetLastError();
 }

@@ -47,6 +47,12 @@ def _row_group(H: int) -> bool:
 
 def _declare(L):
     sig = {
+        "mm_rmsnorm_fwd_ld": [_p, _ll, _p, _p, _p, _i, _i, _f, _p],
+        "mm_rmsnorm_bwd_ld": [_p, _ll, _p, _p, _p, _p, _p, _p, _i, _i, _p],
+        "mm_column_splits": [_i, _i, _i],
+        "mm_column_sum": [_p, _p, _p, _i, _i, _ll, _p],
+        "mm_gated_residual_bwd": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _p],
+        "mm_scale_bf16": [_p, _ll, _p, _p],
         "mm_rmsnorm_fwd": [_p, _p, _p, _p, _i, _i, _f, _p],
         "mm_rownorm_rms_fwd": [_p, _p, _p, _p, _ll, _i, _f, _p],
         "mm_rownorm_ln_mod_fwd": [_p, _p, _p, _p, _p, _p, _ll, _i, _i, _f, _p],
@@ -209,6 +215,11 @@ def check_status(device=None) -> int:
     return v
 
 
+def _pitch(x) -> int:
+    """Elements between the rows of a matrix (a single row's stride means nothing)."""
+    return x.stride(0) if x.shape[0] > 1 else x.shape[1]
+
+
 # --------------------------------------------------------------------------- RMSNorm
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
@@ -216,14 +227,17 @@ class _RMSNorm(torch.autograd.Function):
         shape = x.shape
         H = shape[-1]
         x2 = x.reshape(-1, H)
-        if not x2.is_contiguous():
+        if not x2.is_contiguous() and (_row_group(H) or not _ok2d(x2)):
             x2 = x2.contiguous()
         T = x2.shape[0]
-        y = torch.empty_like(x2)
+        y = torch.empty(T, H, dtype=x.dtype, device=x.device)
         rstd = torch.empty(T, dtype=torch.float32, device=x.device)
         wc = w.contiguous()
-        fn = lib().mm_rownorm_rms_fwd if _row_group(H) else lib().mm_rmsnorm_fwd
-        _check(fn(x2.data_ptr(), wc.data_ptr(), y.data_ptr(), rstd.data_ptr(), T, H, eps, _st()), "rmsnorm_fwd")
+        if _row_group(H):
+            rc = lib().mm_rownorm_rms_fwd(x2.data_ptr(), wc.data_ptr(), y.data_ptr(), rstd.data_ptr(), T, H, eps, _st())
+        else:       # rows may lie apart (the query or key columns of a fused projection): no copy of them is made
+            rc = lib().mm_rmsnorm_fwd_ld(x2.data_ptr(), _pitch(x2), wc.data_ptr(), y.data_ptr(), rstd.data_ptr(), T, H, eps, _st())
+        _check(rc, "rmsnorm_fwd")
         ctx.save_for_backward(x2, wc, rstd)
         ctx.shape = shape
         return y.view(shape)
@@ -235,11 +249,11 @@ class _RMSNorm(torch.autograd.Function):
         dy2 = dy.reshape(T, H)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        dx = torch.empty_like(x2)
+        dx = torch.empty(T, H, dtype=x2.dtype, device=x2.device)
         dw = torch.empty_like(w)
         grid = lib().mm_rmsnorm_bwd_grid(T)
         partial = torch.empty(grid * H, dtype=torch.float32, device=x2.device)
-        _check(lib().mm_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
+        _check(lib().mm_rmsnorm_bwd_ld(x2.data_ptr(), _pitch(x2), w.data_ptr(), dy2.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
                                     dw.data_ptr(), partial.data_ptr(), T, H, _st()), "rmsnorm_bwd")
         return dx.view(ctx.shape), dw, None
 
@@ -427,9 +441,14 @@ class _GatedResidual(torch.autograd.Function):
     def backward(ctx, dout):
         y, g = ctx.saved_tensors
         B, S, H = y.shape
-        dy = dout * g.view(B, 1, H)
-        dg = (dout.float() * y.float()).sum(1).to(g.dtype).view(ctx.gshape)
-        return dout, dy, dg
+        if torch.is_grad_enabled():          # create_graph: the gradient itself is differentiated
+            return dout, dout * g.view(B, 1, H), (dout.float() * y.float()).sum(1).to(g.dtype).view(ctx.gshape)
+        dc, y, g = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (dout.contiguous(), y, g))
+        dy, dg = torch.empty_like(y), torch.empty_like(g)
+        partial = torch.empty(B * lib().mm_column_splits(S, H, B) * H, dtype=torch.float32, device=y.device)
+        _check(lib().mm_gated_residual_bwd(dc.data_ptr(), y.data_ptr(), g.data_ptr(), dy.data_ptr(), dg.data_ptr(), partial.data_ptr(),
+                                           B, S, H, _st()), "gated_residual_bwd")
+        return dout, dy, dg.view(ctx.gshape)
 
 
 def gated_residual(x, y, gate):
@@ -622,6 +641,18 @@ def gemm_tn(a, b, out=None):
 _BWD_NATIVE = os.environ.get("MM_B200_GEMM_BWD", "1") == "1"
 
 
+def column_sum(x):
+    """Sum over the rows of a bf16 matrix (a bias gradient), fp32 inside.  The four bias gradients of a vision block on 8192 patches
+    (218 MB): 94 us as ``torch.sum``, 69 us in these two kernels."""
+    rows, cols = x.shape
+    if rows < 1 or cols % 8 or not _ok2d(x):
+        return torch.sum(x, 0, dtype=torch.float32).to(x.dtype)
+    out = torch.empty(cols, dtype=x.dtype, device=x.device)
+    partial = torch.empty(lib().mm_column_splits(rows, cols, 1) * cols, dtype=torch.float32, device=x.device)
+    _check(lib().mm_column_sum(x.data_ptr(), out.data_ptr(), partial.data_ptr(), rows, cols, x.stride(0), _st()), "column_sum")
+    return out
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias, skip_value=False):
@@ -657,7 +688,7 @@ class _Linear(torch.autograd.Function):
             else:
                 dw = gemm_tn(dy2, x2) if _BWD_NATIVE else dy2.t() @ x2
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = torch.sum(dy2, 0, dtype=torch.float32).to(dy2.dtype)
+            db = column_sum(dy2)
         return dx, dw, db, None
 
 
@@ -825,8 +856,12 @@ class _LinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         dh, dw = ctx.saved_tensors
-        gs = g.to(dh.dtype)
-        return dh.mul_(gs), dw.mul_(gs), None, None, None
+        gs = g.float().reshape(1)
+        for t in (dh, dw):
+            _check(lib().mm_scale_bf16(t.data_ptr(), t.numel(), gs.data_ptr(), _st()), "scale_bf16")
+        # written behind autograd's back: a second backward through the same forward stays an error
+        torch.autograd.graph.increment_version((dh, dw))
+        return dh, dw, None, None, None
 
 
 def linear_cross_entropy(h, w, labels, ignore_index=-100, chunk=8192):

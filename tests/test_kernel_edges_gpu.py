@@ -170,3 +170,92 @@ def test_attention_over_long_keys(lens_q, lens_k, nq, nkv, D, causal, grow):
     native.check_status()
     _close(out, want, rtol=1e-2, atol=4e-3)               # probabilities and results are bf16
     assert float((lse - want_lse.reshape(lse.shape)).abs().max()) < 2e-3 * (1 + float(want_lse.abs().max()))
+
+
+@pytest.mark.parametrize("rows,cols,pitch", [(1, 8, 8), (3, 264, 264), (33, 256, 512), (8192, 1280, 1280), (1000, 6912, 6920), (40000, 16, 16)])
+def test_column_sums(rows, cols, pitch):
+    torch.manual_seed(rows)
+    x = torch.randn(rows, pitch, device=DEV).bfloat16()[:, :cols]
+    # fp32 sums rounded once to bf16
+    _close(native.column_sum(x), x.double().sum(0), rtol=4e-3, atol=1e-3)
+
+
+@pytest.mark.parametrize("B,S,H", [(1, 1, 8), (2, 7, 264), (1, 7800, 1536), (3, 100, 5120)])
+def test_gated_residual_gradients(B, S, H):
+    torch.manual_seed(S)
+    x, y, do = (torch.randn(B, S, H, device=DEV).bfloat16().requires_grad_(i < 2) for i in range(3))
+    gate = torch.randn(B, 1, H, device=DEV).bfloat16().requires_grad_()
+    dx, dy, dg = torch.autograd.grad(ops.gated_residual(x, y, gate), [x, y, gate], do)
+    assert torch.equal(dx, do) and torch.equal(dy, do * gate.detach())
+    _close(dg, (do.double() * y.detach().double()).sum(1, keepdim=True), rtol=4e-3, atol=1e-3)
+
+
+@pytest.mark.parametrize("n", [8, 16, 40, 4096 + 8])
+@pytest.mark.parametrize("scale", [1.0, 1.0 / 3, float("inf")])
+def test_scaling_in_place(n, scale):
+    x = torch.randn(n, device=DEV).bfloat16()
+    want = (x.float() * torch.tensor(scale, device=DEV)).bfloat16()
+    s = torch.tensor([scale], device=DEV)
+    assert native.lib().mm_scale_bf16(x.data_ptr(), n, s.data_ptr(), native._st()) == 0
+    assert torch.equal(x, want)
+
+
+def test_cross_entropy_refuses_a_second_backward():
+    h, w = torch.randn(16, 64, device=DEV).bfloat16().requires_grad_(), torch.randn(256, 64, device=DEV).bfloat16().requires_grad_()
+    loss, _ = ops.linear_cross_entropy(h, w, torch.arange(16, device=DEV))
+    loss.backward(retain_graph=True)
+    with pytest.raises(RuntimeError):
+        loss.backward()
+
+
+@pytest.mark.parametrize("T,H", [(1, 264), (5, 264), (300, 1536), (64, 3584), (7, 5120), (3, 8192)])
+def test_rms_norm_of_columns_of_a_wider_matrix(T, H):
+    """Rows that lie apart are normalised in place, with the gradients of a dense matrix."""
+    torch.manual_seed(H)
+    wide, w = torch.randn(T, 3 * H, device=DEV).bfloat16().requires_grad_(), (1 + 0.1 * torch.randn(H, device=DEV)).bfloat16().requires_grad_()
+    dy = torch.randn(T, H, device=DEV).bfloat16()
+    got = ops.rms_norm(wide[:, H:2 * H], w)
+    dwide, dw = torch.autograd.grad(got, [wide, w], dy)
+    dense = wide.detach()[:, H:2 * H].contiguous().requires_grad_()
+    want = ops.rms_norm(dense, w)
+    ddense, dw2 = torch.autograd.grad(want, [dense, w], dy)
+    assert torch.equal(got, want) and torch.equal(dwide[:, H:2 * H], ddense) and torch.equal(dw, dw2)
+    assert not dwide[:, :H].any() and not dwide[:, 2 * H:].any()
+
+
+@pytest.mark.parametrize("B,S,H", [(2, 5, 64 * 8), (1, 777, 2048), (1, 40, 2056), (2, 33, 4104), (1, 3, 8192)])
+def test_layer_norm_modulate_gradients(B, S, H):
+    """Each number of vectors per thread of the backward kernel."""
+    torch.manual_seed(H)
+    x, sc, sh = torch.randn(B, S, H, device=DEV).bfloat16(), torch.randn(B, 1, H, device=DEV).bfloat16(), torch.randn(B, 1, H, device=DEV).bfloat16()
+    dy = torch.randn(B, S, H, device=DEV).bfloat16()
+    leaf = [t.clone().requires_grad_() for t in (x, sc, sh)]
+    got = torch.autograd.grad(ops.layer_norm_modulate(*leaf), leaf, dy)
+    leaf = [t.float().requires_grad_() for t in (x, sc, sh)]
+    want = torch.autograd.grad(ref.layer_norm_modulate(*leaf), leaf, dy.float())
+    for a, b in zip(got, want):
+        _close(a, b, rtol=1e-2, atol=4e-3)
+
+
+@pytest.mark.parametrize("lens,causal", [([64] * 9, False), ([1] * 300, False), ([127, 1, 128, 129, 0, 5, 300], False), ([1, 255, 257, 0, 128, 700], True),
+                                         ([3] * 5000, False), ([2] * 4500, True)])
+def test_attention_tile_lists(lens, causal):
+    """Packed and plain tile lists: empty sequences, exact multiples of a tile, more sequences than the cached offsets."""
+    torch.manual_seed(len(lens))
+    T, D, N = sum(lens), 64, 2
+    q, k, v = (torch.randn(T, N, D, device=DEV).bfloat16().requires_grad_() for _ in range(3))
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    do = torch.randn(T, N, D, device=DEV).bfloat16()
+    o = ops.attention_varlen(q, k, v, cu, cu, max(lens), max(lens), causal=causal)
+    got = torch.autograd.grad(o, [q, k, v], do)
+    # one masked product over all tokens states the same
+    seq = torch.repeat_interleave(torch.arange(len(lens), device=DEV), torch.tensor(lens, device=DEV))
+    leaf = [t.detach().float().requires_grad_() for t in (q, k, v)]
+    mask = seq[:, None] == seq[None]
+    if causal:
+        mask &= torch.arange(T, device=DEV)[:, None] >= torch.arange(T, device=DEV)[None]
+    s = (torch.einsum("qnd,knd->nqk", leaf[0], leaf[1]) * D ** -0.5).masked_fill(~mask, float("-inf"))
+    want = torch.einsum("nqk,knd->qnd", s.softmax(-1), leaf[2])
+    _close(o.detach(), want.detach(), rtol=1e-2, atol=8e-3)
+    for a, b in zip(got, torch.autograd.grad(want, leaf, do.float())):
+        _close(a, b, rtol=2e-2, atol=2e-2)
