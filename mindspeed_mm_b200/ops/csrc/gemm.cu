@@ -58,7 +58,24 @@ struct Params {
     // the whole row can then be applied after the columns have been scattered to other GPUs)
     float* stats = nullptr;
     int n_slots = 1, per_slot = 0;
+    // split tail (see split_plan): tiles from `full` on are cut along K into `parts` items whose fp32 sums go to `ws`
+    int full = 0, parts = 1;
+    float* ws = nullptr;
 };
+
+// One entry of a CTA's list: a tile and the part of K that it covers.
+struct Item {
+    int tile, kb0, kb1, slot;      // slot: tile-sized block of `ws`, or -1: the whole tile, stored as output
+};
+
+__device__ __forceinline__ int item_count(const Params& p, int n_tiles) { return p.ws ? p.full + (n_tiles - p.full) * p.parts : n_tiles; }
+
+__device__ __forceinline__ Item item_at(const Params& p, int i, int n_tiles, int k_blocks) {
+    if (!p.ws || i < p.full) return {i, 0, k_blocks, -1};
+    // neighbours in the list are neighbouring tiles over the same part of K, so that they share operand tiles in L2
+    const int rem = n_tiles - p.full, t = (i - p.full) % rem, part = (i - p.full) / rem;
+    return {p.full + t, part * k_blocks / p.parts, (part + 1) * k_blocks / p.parts, t * p.parts + part};
+}
 
 constexpr int kMaxDst = 8;
 struct TMapSet {
@@ -102,6 +119,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const int n_blocks = SWIGLU ? p.N / 128 : (p.N + BN - 1) / BN;
     const int n_tiles = m_blocks * n_blocks;
     const int k_blocks = (p.K + BK - 1) / BK;
+    const int n_items = item_count(p, n_tiles);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
@@ -133,10 +151,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
+                const Item item = item_at(p, i, n_tiles, k_blocks);
                 int mb, nb;
-                tile_coords(tile, m_blocks, n_blocks, p.group_m, mb, nb);
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                tile_coords(item.tile, m_blocks, n_blocks, p.group_m, mb, nb);
+                for (int kb = item.kb0; kb < item.kb1; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
                         atomicExch(p.status, MM_TIMEOUT_TMA);
                         ok = false;
@@ -177,7 +196,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             uint32_t phase = 0;
             int it = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++it) {
+            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x, ++it) {
+                const Item item = item_at(p, i, n_tiles, k_blocks);
                 const int acc = it & 1;
                 if (!mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag)) {
                     atomicExch(p.status, MM_TIMEOUT_MMA);
@@ -185,7 +205,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 }
                 fence_after_sync();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                for (int kb = item.kb0; kb < item.kb1; ++kb) {
                     if (!mbar_wait(&full[stage], phase, abort_flag)) {
                         atomicExch(p.status, MM_TIMEOUT_MMA);
                         ok = false;
@@ -202,7 +222,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                                                  : smem_desc_sw128(a0 + k * 32, 16, 1024);
                         const uint64_t db = B_MN ? smem_desc_sw128(b0 + k * 2048, BK * 128, 1024)
                                                  : smem_desc_sw128(b0 + k * 32, 16, 1024);
-                        mma_ss(d_tmem, da, db, idesc, (kb | k) ? 1u : 0u);
+                        mma_ss(d_tmem, da, db, idesc, (kb != item.kb0 || k) ? 1u : 0u);
                     }
                     mma_commit(&empty[stage]);  // slot reusable once these MMAs have read it
                     if (++stage == C::kStages) {
@@ -220,9 +240,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const bool issuer = threadIdx.x == 64;
         int it = 0;
         int slab_count = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
+        for (int i = blockIdx.x; i < n_items; i += gridDim.x, ++it) {
+            const Item item = item_at(p, i, n_tiles, k_blocks);
             int mb, nb;
-            tile_coords(tile, m_blocks, n_blocks, p.group_m, mb, nb);
+            tile_coords(item.tile, m_blocks, n_blocks, p.group_m, mb, nb);
             const int acc = it & 1;
             if (!mbar_wait(&tfull[acc], (it >> 1) & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
             // make the go / no-go decision identical for all 128 epilogue threads before any bar.sync below
@@ -233,6 +254,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             fence_after_sync();
             const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
             constexpr int kSlabs = SWIGLU ? 2 : BN / 64;
+            if (!SWIGLU && item.slot >= 0) {
+                // [column / 4][row][4]: the lanes of a warp write neighbouring rows of a column group
+                float4* dst = reinterpret_cast<float4*>(p.ws) + (size_t)item.slot * (BM * BN / 4) + row;
+#pragma unroll 1
+                for (int slab = 0; slab < kSlabs; ++slab) {
+                    uint32_t r[64];
+                    tmem_ld_32x32(t_row + slab * 64, r);
+                    tmem_ld_32x32(t_row + slab * 64 + 32, r + 32);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 16; ++c)
+                        dst[(slab * 16 + c) * BM] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
+                                                                __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
+                }
+                fence_before_sync();
+                mbar_arrive(&tempty[acc]);
+                continue;
+            }
 #pragma unroll 1
             for (int slab = 0; slab < kSlabs; ++slab, ++slab_count) {
                 uint8_t* buf = sC + (slab_count & 1) * (BM * 128);
@@ -323,6 +362,74 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
 }
 
+// ---- split tail ----
+// 168 tiles on 148 SMs take two rounds, the second one with 20 CTAs at work.  The tiles behind the last whole round are therefore cut
+// along K into `parts` items each, so that ceil(rem * parts / 148) rounds of a 1 / parts tile follow; the items leave fp32 sums in a
+// workspace and a second kernel adds them in their order, adds the bias and rounds, exactly once, to bf16.  No CTA waits for another.
+struct SplitPlan {
+    int full, parts;
+};
+
+// parts: the number that the estimate below makes fastest, 1 if the gain is under 4 us.  A 64-deep step of a 128 x 256 tile takes
+// 0.44 us (1.4 PFLOP/s over 148 SMs); an item's sums are written and read once at about 4 TB/s, a further launch and the shorter
+// main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and lost 2 us).
+// Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 220 / 150 us, 405 x 3584 x 37888 (56) 216 / 122,
+// 8192 x 3584 x 18944 (896) 828 / 761, 8192 x 3584 x 152064 8636 / 6268, 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.
+inline SplitPlan split_plan(int M, int N, int K, int BN, int sms) {
+    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK, rem = tiles % sms;
+    SplitPlan best{tiles, 1};
+    if (!rem) return best;
+    const double unit = kb * 0.44 * BN / 256;
+    double least = unit - 4.0;
+    for (int parts = 2; parts <= 16 && kb / parts >= 4; ++parts) {
+        const int rounds = (rem * parts + sms - 1) / sms;
+        const double t = unit * rounds / parts + 6.0 + rem * parts * (BM * BN * 8e-6 / 4.0);
+        if (t < least) {
+            least = t;
+            best = {tiles - rem, parts};
+        }
+    }
+    return best;
+}
+
+inline int sm_count() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    return sms;
+}
+
+// C tile = bf16(sum over the parts of the workspace + bias); a thread makes 8 columns of a row
+template <int BN>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ ws, bf16* __restrict__ C, const bf16* __restrict__ bias,
+                                                        int M, int N, long long ldc, int full, int parts, int group_m) {
+    const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM, t = blockIdx.y;      // cg: group of 8 columns
+    int mb, nb;
+    tile_coords(full + t, (M + BM - 1) / BM, (N + BN - 1) / BN, group_m, mb, nb);
+    const int m = mb * BM + row, n = nb * BN + cg * 8;
+    if (m >= M || n >= N) return;
+    const float4* src = reinterpret_cast<const float4*>(ws) + (size_t)t * parts * (BM * BN / 4) + (size_t)(2 * cg) * BM + row;
+    float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+    for (int q = 0; q < parts; ++q) {
+        const float4 a = src[(size_t)q * (BM * BN / 4)], b = src[(size_t)q * (BM * BN / 4) + BM];
+        f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+        f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+    }
+    bf16* dst = C + (size_t)m * ldc + n;
+    if (n + 8 <= N) {
+        if (bias)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) f[k] += __bfloat162float(bias[n + k]);
+        *reinterpret_cast<Vec8*>(dst) = pack8(f);
+    } else {
+        for (int k = 0; n + k < N; ++k) dst[k] = __float2bfloat16(f[k] + (bias ? __bfloat162float(bias[n + k]) : 0.f));
+    }
+}
+
 struct Route {
     int mode = 0, blk = 0, world = 1, rank = 0, row_off = 0;
     void* const* dst = nullptr;     // mode != 0: `world` destination base pointers (peer-mapped)
@@ -333,7 +440,7 @@ struct Route {
 
 template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false>
 int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
-           long long ldc, int* status, cudaStream_t st, const Route& rt = Route()) {
+           long long ldc, int* status, cudaStream_t st, const Route& rt = Route(), float* ws = nullptr, long long ws_bytes = 0) {
     using C = Cfg<BN>;
     CUtensorMap tA, tB;
     TMapSet tC;
@@ -371,15 +478,21 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
         done = true;
     }
     const int m_blocks = (M + BM - 1) / BM, n_blocks = SWIGLU ? N / 128 : (N + BN - 1) / BN;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
-    const int tiles = m_blocks * n_blocks;
+    const int sms = sm_count(), tiles = m_blocks * n_blocks;
     Params p{M, N, K, (const bf16*)bias, status, 8, rt.mode, rt.blk, rt.world, rt.rank, rt.mode == 1 ? 0 : rt.row_off,
              rt.stats, rt.n_slots, rt.n_slots > 0 ? N / rt.n_slots : N};
+    const SplitPlan plan = !SWIGLU && ws && rt.mode == 0 ? split_plan(M, N, K, BN, sms) : SplitPlan{tiles, 1};
+    const int rem = tiles - plan.full;
+    if (plan.parts > 1 && (long long)rem * plan.parts * BM * BN * 4 <= ws_bytes) {
+        p.full = plan.full;
+        p.parts = plan.parts;
+        p.ws = ws;
+        const int items = plan.full + rem * plan.parts;
+        kern<<<items < sms ? items : sms, kThreads, C::kSmem, st>>>(tA, tB, tC, p);
+        sum_parts_kernel<BN><<<dim3(BM * BN / 8 / 256, rem), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full, plan.parts,
+                                                                           p.group_m);
+        return (int)cudaGetLastError();
+    }
     const int grid = tiles < sms ? tiles : sms;
     kern<<<grid, kThreads, C::kSmem, st>>>(tA, tB, tC, p);
     return (int)cudaGetLastError();
@@ -397,24 +510,41 @@ namespace {
 bool skinny(int M, int N, int K) { return M <= 4 && N % 2 == 0 && K % 8 == 0 && (long long)M * K <= 80 * 1024; }
 }  // namespace
 
+// Bytes of workspace with which mm_gemm_bf16_ws splits the tail of this product along K (0: it would not).
+MM_API long long mm_gemm_ws_bytes(int M, int N, int K, int a_mn, int b_mn, int bn) {
+    if (M <= 0 || N <= 0 || K <= 0 || (!a_mn && !b_mn && skinny(M, N, K))) return 0;
+    const int BN = bn == 128 ? 128 : 256;
+    const SplitPlan plan = split_plan(M, N, K, BN, sm_count());
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    return plan.parts > 1 ? (tiles - plan.full) * plan.parts * BM * BN * 4 : 0;
+}
+
 // lda/ldb/ldc: elements between consecutive rows of the tensors as laid out in memory.
 // Requirements: base pointers 16-byte aligned; ld* multiples of 8; `status` is a device int (0 = ok).
-MM_API int mm_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
-                        long long ldb, long long ldc, int a_mn, int b_mn, int bn, int* status, cudaStream_t st) {
+// ws: null, or workspace of mm_gemm_ws_bytes (16-byte aligned), used by this call alone.
+MM_API int mm_gemm_bf16_ws(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
+                           long long ldb, long long ldc, int a_mn, int b_mn, int bn, int* status, void* ws, long long ws_bytes,
+                           cudaStream_t st) {
     if ((lda | ldb | ldc) % 8) return -1;
-    if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return -2;
+    if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C | (uintptr_t)ws) & 15) return -2;
     if (M <= 0 || N <= 0 || K <= 0) return -3;
     if (!a_mn && !b_mn && skinny(M, N, K)) return mm_gemv_bf16(A, B, bias, nullptr, nullptr, C, M, N, K, lda, ldb, 0, ldc, 0.f, 0, st);
-#define MM_DISPATCH(BN_)                                                                                          \
-    if (!a_mn && !b_mn) return launch<BN_, false, false>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st);      \
-    if (!a_mn && b_mn) return launch<BN_, false, true>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st);        \
-    if (a_mn && !b_mn) return launch<BN_, true, false>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st);        \
-    return launch<BN_, true, true>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st);
+    float* w = (float*)ws;
+#define MM_DISPATCH(BN_)                                                                                                              \
+    if (!a_mn && !b_mn) return launch<BN_, false, false>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st, Route(), w, ws_bytes);      \
+    if (!a_mn && b_mn) return launch<BN_, false, true>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st, Route(), w, ws_bytes);        \
+    if (a_mn && !b_mn) return launch<BN_, true, false>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st, Route(), w, ws_bytes);        \
+    return launch<BN_, true, true>(A, B, C, bias, M, N, K, lda, ldb, ldc, status, st, Route(), w, ws_bytes);
     if (bn == 128) {
         MM_DISPATCH(128)
     }
     MM_DISPATCH(256)
 #undef MM_DISPATCH
+}
+
+MM_API int mm_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda, long long ldb,
+                        long long ldc, int a_mn, int b_mn, int bn, int* status, cudaStream_t st) {
+    return mm_gemm_bf16_ws(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, bn, status, nullptr, 0, st);
 }
 
 

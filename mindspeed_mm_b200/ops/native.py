@@ -76,6 +76,8 @@ def _declare(L):
         "mm_gated_residual": [_p, _p, _p, _p, _ll, _i, _i, _p],
         "mm_adamw": [_p, _p, _p, _p, _i, _p, _ll, _ll, _f, _f, _f, _f, _f, _f, _f, _f, _p, _p],
         "mm_gemm_bf16": [_p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _p, _p],
+        "mm_gemm_bf16_ws": [_p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _p, _p, _ll, _p],
+        "mm_gemm_ws_bytes": [_i, _i, _i, _i, _i, _i],
         "mm_gemm_swiglu_bf16": [_p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _p, _p],
         "mm_gemv_bf16": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _ll, _f, _i, _p],
         "mm_decode_attention": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _ll, _ll, _ll, _f, _p],
@@ -118,7 +120,7 @@ def _declare(L):
         if hasattr(L, name):
             fn = getattr(L, name)
             fn.argtypes = args
-            fn.restype = _i
+            fn.restype = _ll if name == "mm_gemm_ws_bytes" else _i
             _STATUS[name] = True
         else:
             _STATUS[name] = False
@@ -497,8 +499,11 @@ def _gemm_raw(a, b, out, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, bn=None):
     if bn is None:
         bn = 256 if N >= 256 else 128
     st = status_word(a.device)
-    rc = lib().mm_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), None if bias is None else bias.data_ptr(),
-                            M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), bn, st.data_ptr(), _st())
+    L = lib()
+    nbytes = L.mm_gemm_ws_bytes(M, N, K, int(a_mn), int(b_mn), bn)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
+    rc = L.mm_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), None if bias is None else bias.data_ptr(), M, N, K, lda, ldb,
+                           ldc, int(a_mn), int(b_mn), bn, st.data_ptr(), None if ws is None else ws.data_ptr(), nbytes, _st())
     _check(rc, "gemm_bf16")
 
 

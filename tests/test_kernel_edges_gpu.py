@@ -259,3 +259,25 @@ def test_attention_tile_lists(lens, causal):
     _close(o.detach(), want.detach(), rtol=1e-2, atol=8e-3)
     for a, b in zip(got, torch.autograd.grad(want, leaf, do.float())):
         _close(a, b, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K,splits", [(1421, 3584, 3600, True), (1409, 3592, 4104, True), (1, 264, 18952, None), (5, 8, 18944, True), (136, 520, 8200, True),
+                                          (128 * 148, 256, 8192, False), (128 * 149, 256, 8192, True), (128, 256, 256, False)])
+def test_products_with_a_split_tail(layout, M, N, K, splits):
+    """Ragged rows, columns and depths, a lone tail and one behind whole rounds; both sides of the rule."""
+    if layout == "tn" and M % 8:
+        M = M // 8 * 8 + 8                                        # the rows are the contiguous dimension there
+    torch.manual_seed(M)
+    a = torch.randn((K, M) if layout == "tn" else (M, K), device=DEV).bfloat16()
+    b = torch.randn((N, K) if layout == "nt" else (K, N), device=DEV).bfloat16()
+    bias = torch.randn(N, device=DEV).bfloat16() if layout == "nt" else None
+    nbytes = native.lib().mm_gemm_ws_bytes(M, N, K, int(layout == "tn"), int(layout != "nt"), 256 if N >= 256 else 128)
+    assert splits is None or (nbytes > 0) == splits
+    got = {"nt": lambda: native.gemm_nt(a, b, bias), "nn": lambda: native.gemm_nn(a, b), "tn": lambda: native.gemm_tn(a, b)}[layout]()
+    want = (a.float().t() if layout == "tn" else a.float()) @ (b.float().t() if layout == "nt" else b.float())
+    if bias is not None:
+        want += bias.float()
+    native.check_status()
+    # exact products, fp32 sums (of any order), one rounding to bf16: half an ulp, and the order's error at K = 18952
+    _close(got, want, rtol=4.5e-3, atol=2e-3 * K ** 0.5 / 100)
