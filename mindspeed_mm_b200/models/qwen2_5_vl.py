@@ -411,6 +411,8 @@ class LMHead(nn.Module):
     def forward(self, x, labels=None, prenormed: bool = False, norm_only: bool = False):
         """``prenormed``: ``x`` already went through a final norm of its own (multi-token-prediction block);
         ``norm_only``: return the normalised hidden states instead of logits / loss."""
+        if labels is None and not prenormed and not norm_only and _plain(self.norm):
+            return ops.norm_linear(x, self.norm.weight, self.norm.eps, self.weight)
         h = x if prenormed else self.norm(x)
         if norm_only:
             return h
@@ -508,7 +510,7 @@ class Qwen25VLModel(nn.Module):
             x = x.index_copy(0, img_pos, v.to(x.dtype))
         cos, sin = batch.get("rope_cos"), batch.get("rope_sin")
         if cos is None:
-            cos, sin = ops.ref.mrope_cos_sin(batch["position_ids"], t.head_dim, t.rope_theta, t.mrope_section)
+            cos, sin = ops.mrope_tables(batch["position_ids"], t.head_dim, t.rope_theta, t.mrope_section, x.dtype)
         cos, sin = cos.to(x.dtype), sin.to(x.dtype)
         for i, layer in enumerate(self.layers):
             if kv_cache is not None:

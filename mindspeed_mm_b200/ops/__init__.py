@@ -147,6 +147,15 @@ def rope_interleaved(x, cos, sin):
     return ref.rope_interleaved(x, cos, sin)
 
 
+def mrope_tables(position_ids, head_dim: int, theta: float, mrope_section, dtype):
+    """Multimodal rotary tables (cos, sin), [T, head_dim] in ``dtype``, from positions [3, T] (see ``reference.mrope_cos_sin``)."""
+    if _native(position_ids) and dtype == torch.bfloat16 and position_ids.dtype == torch.int64 and tuple(position_ids.shape[:1]) == (3,) \
+            and position_ids.dim() == 2 and position_ids.shape[1] > 0 and head_dim % 2 == 0 and len(mrope_section) == 3:
+        return _nat().mrope_tables(position_ids, head_dim, theta, mrope_section)
+    cos, sin = ref.mrope_cos_sin(position_ids, head_dim, theta, mrope_section)
+    return cos.to(dtype), sin.to(dtype)
+
+
 def l2_norm(x, eps: float = 1e-6):
     if _native(x) and x.dtype == torch.bfloat16 and x.shape[-1] <= 256:
         return _nat().l2_norm(x, eps)

@@ -8,6 +8,7 @@
 // programmatic stream serialisation: a kernel starts while its predecessor drains, asks L2 for its first weights (a hint, so a
 // predecessor that writes those weights is harmless) and waits for the predecessor before it reads anything.
 #include <cooperative_groups.h>
+#include <math.h>
 
 #include "common.cuh"
 
@@ -381,6 +382,24 @@ int run_gemv_m(const GemvParams& p, int swiglu, cudaStream_t st) {
     return p.norm ? run_gemv<M, false, true>(p, st) : run_gemv<M, false, false>(p, st);
 }
 
+// ------------------------------------------------------------------------------------------ rotary tables
+// cos / sin [T, 2 * half] (both halves alike, bf16) of angle position[axis(i)][t] / theta^(i / half), axis by section.  In 64 bits: an
+// angle reaches the position itself (thousands of radians), and T * half values are nothing next to the launches of the ten
+// element-wise kernels that made them before, each of which a decoding step waited for.
+__global__ void __launch_bounds__(128) rotary_tables_kernel(const long long* __restrict__ pos, bf16* __restrict__ cosb, bf16* __restrict__ sinb,
+                                                           int T, int half, int s0, int s1, int s2, double log2_theta) {
+    const int n = T * half;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const int t = j / half, i = j % half, axis = i < s0 ? 0 : i < s0 + s1 ? 1 : i < s0 + s1 + s2 ? 2 : 0;
+        double s, c;
+        sincos((double)pos[(size_t)axis * T + t] * exp2(-log2_theta * i / half), &s, &c);
+        const bf16 cb = __float2bfloat16((float)c), sb = __float2bfloat16((float)s);
+        const size_t at = (size_t)t * 2 * half + i;
+        cosb[at] = cosb[at + half] = cb;
+        sinb[at] = sinb[at + half] = sb;
+    }
+}
+
 // ------------------------------------------------------------------------------------------ attention over the cache
 struct DecodeParams {
     const bf16 *q, *k, *v;           // new tokens: [T, heads, 128] with token strides
@@ -651,6 +670,15 @@ MM_API int mm_gemv_bf16(const void* x, const void* w, const void* bias, const vo
         case 3: return run_gemv_m<3>(p, swiglu, st);
         default: return run_gemv_m<4>(p, swiglu, st);
     }
+}
+
+// pos: int64 [3, T]; cosb / sinb: bf16 [T, 2 * half]; sections as in the caller's model (sum <= half; what is left follows axis 0).
+MM_API int mm_rotary_tables(const long long* pos, void* cosb, void* sinb, int T, int half, int s0, int s1, int s2, double theta,
+                            cudaStream_t st) {
+    if (T < 1 || half < 1 || (long long)T * half > 0x7fffffff || theta <= 0) return -1;
+    const int blocks = (T * half + 127) / 128;
+    rotary_tables_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 128, 0, st>>>(pos, (bf16*)cosb, (bf16*)sinb, T, half, s0, s1, s2, log2(theta));
+    return (int)cudaGetLastError();
 }
 
 // Appends T new tokens to a cache and attends to it (causal, aligned to the end): k_new / v_new [past + T, Nkv, 128] are the old

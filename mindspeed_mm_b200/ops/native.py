@@ -80,6 +80,7 @@ def _declare(L):
         "mm_gemm_ws_bytes": [_i, _i, _i, _i, _i, _i],
         "mm_gemm_swiglu_bf16": [_p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _p, _p],
         "mm_gemv_bf16": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _ll, _f, _i, _p],
+        "mm_rotary_tables": [_p, _p, _p, _i, _i, _i, _i, _i, C.c_double, _p],
         "mm_decode_attention": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _ll, _ll, _ll, _f, _p],
         "mm_ce_fwd_bwd": [_p, _ll, _p, _p, _i, _i, _i, _p],
         "mm_fmha_max_tiles": [_i, _i],
@@ -553,6 +554,16 @@ def gemm_swiglu(x, w):
 
 
 # --------------------------------------------------------------------------- generation (csrc/decode.cu)
+def mrope_tables(position_ids, head_dim, theta, section):
+    """bf16 rotary tables [T, head_dim] of int64 positions [3, T], computed in 64 bits by one kernel."""
+    pos = position_ids.contiguous()
+    T = pos.shape[1]
+    cos, sin = (torch.empty(T, head_dim, dtype=torch.bfloat16, device=pos.device) for _ in range(2))
+    _check(lib().mm_rotary_tables(pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, head_dim // 2, *section, float(theta), _st()),
+           "rotary_tables")
+    return cos, sin
+
+
 def skinny_supported(x, *tensors) -> bool:
     """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies."""
     return (x.dim() == 2 and 1 <= x.shape[0] <= 4 and x.shape[1] % 8 == 0 and x.numel() <= 80 * 1024 and _ok2d(x)

@@ -281,3 +281,18 @@ def test_products_with_a_split_tail(layout, M, N, K, splits):
     native.check_status()
     # exact products, fp32 sums (of any order), one rounding to bf16: half an ulp, and the order's error at K = 18952
     _close(got, want, rtol=4.5e-3, atol=2e-3 * K ** 0.5 / 100)
+
+
+@pytest.mark.parametrize("T,D,section,theta", [(1, 128, (16, 24, 24), 1e6), (77, 64, (8, 12, 12), 1e4), (3, 16, (2, 1, 1), 1e7), (5000, 128, (16, 24, 20), 1e6)])
+def test_rotary_tables(T, D, section, theta):
+    """Positions up to 130 000: the table is that of a 64-bit angle, rounded once."""
+    pos = torch.randint(0, 130000, (3, T), device=DEV)
+    cos, sin = ops.mrope_tables(pos, D, theta, section, torch.bfloat16)
+    i = torch.arange(D // 2, device=DEV)
+    axis = (i >= section[0]).long() + (i >= section[0] + section[1]).long()
+    axis[i >= sum(section)] = 0
+    ang = pos.double()[axis].t() * theta ** (-i.double() / (D // 2))
+    ang = torch.cat([ang, ang], -1)
+    # one rounding (two where the 64-bit value is rounded to 32 bits first)
+    for got, want in ((cos, ang.cos()), (sin, ang.sin())):
+        assert float((got.double() - want).abs().max()) <= 2 ** -9 + 1e-6
