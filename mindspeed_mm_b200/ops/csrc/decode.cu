@@ -449,7 +449,6 @@ __device__ __forceinline__ void load_row32(const bf16* row, const bf16* cosr, co
 // to the new cache, rotated if it belongs to a new token, so the cache is read once instead of once for the append and once for
 // the attention.  Partial sums of the warps meet in shared memory, those of the CTAs in distributed shared memory: no workspace,
 // no second launch.
-// 9000 keys, 28 query and 4 key / value heads: see mm_decode_attention.
 __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(DecodeParams p) {
     extern __shared__ __align__(16) uint8_t dec_smem[];
     float* part_o = reinterpret_cast<float*>(dec_smem);                       // [warp][row][128]
@@ -460,8 +459,47 @@ __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(Dec
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, g = lane >> 2;
     const int G = p.Nq / p.Nkv, rows = p.T * G, L = p.past + p.T;
     const size_t pitch = (size_t)p.Nkv * kDecD;
+    const int first = (split * kDecWarps + warp) * kDecTile, stride = splits * kDecWarps * kDecTile;
+    for (int k0 = first; k0 < p.past; k0 += stride) {              // this warp's part of the old cache (128-byte lines) on its way to L2
+        const int key = k0 + (lane >> 1);
+        if (key < p.past) {
+            const size_t at = key * pitch + (size_t)kvh * kDecD + (lane & 1) * 64;
+            prefetch_l2(p.k_old + at);
+            prefetch_l2(p.v_old + at);
+        }
+    }
     wait_for_predecessor();
     let_successor_start();
+
+    // keys k0 .. k0 + 15: the lane's 32 elements of keys g and g + 8, its 16 elements of values 2 * quad (+ 1, + 8, + 9)
+    auto fetch = [&](int k0, uint4 (*kk)[4], uint4 (*vv)[2]) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int key = k0 + h * 8 + g;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kk[h][i] = make_uint4(0, 0, 0, 0);
+            if (key < p.past) {
+                const uint4* src = reinterpret_cast<const uint4*>(p.k_old + key * pitch + (size_t)kvh * kDecD + quad * 32);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) kk[h][i] = ld_once(src + i);
+            } else if (key < L) {
+                const int t = key - p.past;
+                load_row32(p.k + t * p.ks + (size_t)kvh * kDecD, p.cos ? p.cos + t * kDecD : nullptr, p.sin + t * kDecD, quad * 32, kk[h]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int key = k0 + quad * 2 + (i & 1) + (i >> 1) * 8;
+            vv[i][0] = vv[i][1] = make_uint4(0, 0, 0, 0);
+            if (key < L) {
+                const bf16* src = key < p.past ? p.v_old + key * pitch + (size_t)kvh * kDecD : p.v + (key - p.past) * p.vs + (size_t)kvh * kDecD;
+                vv[i][0] = ld_once(reinterpret_cast<const uint4*>(src + g * 16));
+                vv[i][1] = ld_once(reinterpret_cast<const uint4*>(src + g * 16 + 8));
+            }
+        }
+    };
+    uint4 kk[2][4], vv[4][2];
+    if (first < L) fetch(first, kk, vv);                           // in flight while the queries are read and rotated
 
     // query fragments: rows g and g + 8 (row = token * G + head of the group), this quad lane's 32 dims
     uint4 q0[4], q1[4];
@@ -486,41 +524,19 @@ __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(Dec
 #pragma unroll
     for (int n = 0; n < 16; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
 
-    for (int k0 = (split * kDecWarps + warp) * kDecTile; k0 < L; k0 += splits * kDecWarps * kDecTile) {
+    for (int k0 = first; k0 < L; k0 += stride) {
         float s[2][4];
-        // values first: their loads are in flight during the first product
-        uint4 vv[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int key = k0 + quad * 2 + (i & 1) + (i >> 1) * 8;
-            vv[i][0] = vv[i][1] = make_uint4(0, 0, 0, 0);
-            if (key < L) {
-                const bf16* src = key < p.past ? p.v_old + key * pitch + (size_t)kvh * kDecD
-                                               : p.v + (key - p.past) * p.vs + (size_t)kvh * kDecD;
-                vv[i][0] = ld_once(reinterpret_cast<const uint4*>(src + g * 16));
-                vv[i][1] = ld_once(reinterpret_cast<const uint4*>(src + g * 16 + 8));
-            }
-        }
+        uint4 nk[2][4], nv[4][2];
+        if (k0 + stride < L) fetch(k0 + stride, nk, nv);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int key = k0 + h * 8 + g;
-            uint4 kk[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) kk[i] = make_uint4(0, 0, 0, 0);
             if (key < L) {
-                if (key < p.past) {
-                    const uint4* src = reinterpret_cast<const uint4*>(p.k_old + key * pitch + (size_t)kvh * kDecD + quad * 32);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) kk[i] = ld_once(src + i);
-                } else {
-                    const int t = key - p.past;
-                    load_row32(p.k + t * p.ks + (size_t)kvh * kDecD, p.cos ? p.cos + t * kDecD : nullptr, p.sin + t * kDecD, quad * 32, kk);
-                }
                 uint4* dst = reinterpret_cast<uint4*>(p.k_new + key * pitch + (size_t)kvh * kDecD + quad * 32);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dst[i] = kk[i];
+                for (int i = 0; i < 4; ++i) dst[i] = kk[h][i];
             }
-            const uint32_t* kr = reinterpret_cast<const uint32_t*>(kk);
+            const uint32_t* kr = reinterpret_cast<const uint32_t*>(kk[h]);
             s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -585,6 +601,15 @@ __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(Dec
             o[n][3] *= f1;
             mma_16x8x16(o[n], pa, b0, b1);
         }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kk[h][i] = nk[h][i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            vv[i][0] = nv[i][0];
+            vv[i][1] = nv[i][1];
+        }
     }
     // Accumulator column of lane (g, quad) in product n: the output columns 2 * quad and 2 * quad + 1 of the tile, whose "column c"
     // was loaded by the lanes with group c: dims c * 16 + n.
@@ -608,41 +633,69 @@ __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(Dec
         part_l[warp * kDecRows + g + 8] = l1;
     }
     __syncthreads();
-    // fold the warps of this CTA into warp 0's slots
-    for (int i = threadIdx.x; i < rows * kDecD; i += kDecWarps * 32) {
-        const int r = i / kDecD;
-        float m = -INFINITY;
+    // fold the warps of this CTA into warp 0's slots; the 8 factors of a row are made once, not by every element
+    __shared__ float fac[16][kDecRows], all_m[kDecRows], all_l[kDecRows];      // fac: by warp here, by CTA below
+    if (threadIdx.x < rows) {
+        const int r = threadIdx.x;
+        float m = -INFINITY, l = 0.f;
+#pragma unroll
         for (int w = 0; w < kDecWarps; ++w) m = fmaxf(m, part_m[w * kDecRows + r]);
         const float u = m == -INFINITY ? 0.f : m;
-        float acc = 0.f;
-        for (int w = 0; w < kDecWarps; ++w) acc += part_o[(size_t)w * kDecRows * kDecD + i] * exp2f(part_m[w * kDecRows + r] - u);
-        part_o[i] = acc;                                                       // only this thread reads or writes element i
+#pragma unroll
+        for (int w = 0; w < kDecWarps; ++w) {
+            const float f = exp2f(part_m[w * kDecRows + r] - u);
+            fac[w][r] = f;
+            l += part_l[w * kDecRows + r] * f;
+        }
+        all_m[r] = m;
+        all_l[r] = l;
     }
     __syncthreads();
-    if (threadIdx.x < rows) {
-        float m = -INFINITY, l = 0.f;
-        for (int w = 0; w < kDecWarps; ++w) m = fmaxf(m, part_m[w * kDecRows + threadIdx.x]);
-        const float u = m == -INFINITY ? 0.f : m;
-        for (int w = 0; w < kDecWarps; ++w) l += part_l[w * kDecRows + threadIdx.x] * exp2f(part_m[w * kDecRows + threadIdx.x] - u);
-        part_m[threadIdx.x] = m;
-        part_l[threadIdx.x] = l;
+    for (int i = threadIdx.x; i < rows * (kDecD / 4); i += kDecWarps * 32) {
+        const int r = i / (kDecD / 4);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < kDecWarps; ++w) {
+            const float4 v = reinterpret_cast<const float4*>(part_o + (size_t)w * kDecRows * kDecD)[i];
+            const float f = fac[w][r];
+            acc.x += v.x * f;
+            acc.y += v.y * f;
+            acc.z += v.z * f;
+            acc.w += v.w * f;
+        }
+        reinterpret_cast<float4*>(part_o)[i] = acc;                            // only this thread reads or writes element i
     }
     cluster.sync();
     // fold the CTAs: each takes its share of the outputs (pairs of dims)
+    if (threadIdx.x < rows) {
+        const int r = threadIdx.x;
+        float m = -INFINITY, l = 0.f, ms[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            ms[c] = c < splits ? *cluster.map_shared_rank(all_m + r, c) : -INFINITY;
+            m = fmaxf(m, ms[c]);
+        }
+        const float u = m == -INFINITY ? 0.f : m;
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+            if (c < splits) {
+                const float f = exp2f(ms[c] - u);
+                fac[c][r] = f;
+                l += *cluster.map_shared_rank(all_l + r, c) * f;
+            }
+        part_l[r] = l > 0.f ? 1.f / l : 0.f;
+    }
+    __syncthreads();
     for (int i = split * kDecWarps * 32 + threadIdx.x; i < rows * (kDecD / 2); i += splits * kDecWarps * 32) {
         const int r = i / (kDecD / 2), d = i % (kDecD / 2) * 2;
-        float m = -INFINITY;
-        for (int c = 0; c < splits; ++c) m = fmaxf(m, *cluster.map_shared_rank(part_m + r, c));
-        const float u = m == -INFINITY ? 0.f : m;
-        float l = 0.f, ax = 0.f, ay = 0.f;
+        float ax = 0.f, ay = 0.f;
+#pragma unroll 4
         for (int c = 0; c < splits; ++c) {
-            const float f = exp2f(*cluster.map_shared_rank(part_m + r, c) - u);
             const float2 v = *reinterpret_cast<const float2*>(cluster.map_shared_rank(part_o + r * kDecD + d, c));
-            l += *cluster.map_shared_rank(part_l + r, c) * f;
-            ax += v.x * f;
-            ay += v.y * f;
+            ax += v.x * fac[c][r];
+            ay += v.y * fac[c][r];
         }
-        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const float inv = part_l[r];
         const int t = r / G, head = kvh * G + r % G;
         *reinterpret_cast<bf162*>(p.out + ((size_t)t * p.Nq + head) * kDecD + d) = __floats2bfloat162_rn(ax * inv, ay * inv);
     }
@@ -694,10 +747,12 @@ MM_API int mm_decode_attention(const void* q, const void* k, const void* v, cons
     DecodeParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, (const bf16*)cos, (const bf16*)sin, (const bf16*)k_old,
                    (const bf16*)v_old, (bf16*)k_new, (bf16*)v_new, (bf16*)out, qs, ks, vs, T, past, Nq, Nkv,
                    scale * 1.4426950408889634f};
-    // one run of 16 keys per warp before another CTA pays; 16 CTAs is the largest cluster
+    // one run of 16 keys per warp before another CTA pays; 16 CTAs is the largest cluster.  More CTAs than SMs are worth it for long
+    // caches only: 16 key / value heads, 16 CTAs each against 8: 2000 keys 32.4 / 28.1 us, 9000 76 / 79, 16000 111 / 132.  28 query and
+    // 4 key / value heads: 311 keys 11.1 us, 2000 12.1, 9000 26.5.
     const int runs = (past + T + kDecTile * kDecWarps - 1) / (kDecTile * kDecWarps);
     int splits = 1;
-    while (splits < 16 && splits < runs) splits *= 2;
+    while (splits < 16 && splits < runs && (splits * 2 * Nkv <= 148 || runs >= 64)) splits *= 2;
     cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
