@@ -138,11 +138,11 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             mbar_init(&v_full[i], 1);
             mbar_init(&v_empty[i], 1);
             mbar_init(&s_full[i], 1);
-            mbar_init(&s_empty[i], 256);
+            mbar_init(&s_empty[i], 8);                // one arrival per warp
         }
         mbar_init(dp_full, 1);
-        mbar_init(dp_empty, 256);
-        mbar_init(ds_full, 256);
+        mbar_init(dp_empty, 8);
+        mbar_init(ds_full, 8);
         mbar_init(dq_full, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -271,28 +271,39 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tmem_ld_32x32(tdP + half * 64 + lane_off + 32, d + 32);
             tmem_wait_ld();
             fence_before_sync();
-            mbar_arrive(&s_empty[st]);
-            mbar_arrive(dp_empty);
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&s_empty[st]);
+                mbar_arrive(dp_empty);
+            }
             const int kbase = j * 128 + half * 64;
             const int limit = !row_ok ? -1 : (p.causal ? min(k_len - 1, qi + diag) : vis_hi - 1);
             // packed fp32 math (two columns per instruction): dS = exp2(S * scale - lse) * (dP - delta)
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2), nd2 = make_float2(-dlt, -dlt);
-            const bool tile_masked = kbase + 63 > limit || nseq > 1;   // some column of this row is hidden (or the row is padding)
+            // some column of a row of this warp is hidden (or the row is padding)
+            const bool tile_masked = __any_sync(0xffffffffu, kbase + 63 > limit || nseq > 1);
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
                 const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sc2, nl2);
                 const float2 g = __fadd2_rn(make_float2(__uint_as_float(d[2 * i]), __uint_as_float(d[2 * i + 1])), nd2);
-                float2 ds = __fmul2_rn(make_float2(exp2f(x.x), exp2f(x.y)), g);
-                if (tile_masked) {
-                    if (kbase + 2 * i > limit || kbase + 2 * i < vis_lo) ds.x = 0.f;
-                    if (kbase + 2 * i + 1 > limit || kbase + 2 * i + 1 < vis_lo) ds.y = 0.f;
-                }
-                d[i] = pack2(ds.x, ds.y);
+                const float2 ds = __fmul2_rn(make_float2(exp2f(x.x), exp2f(x.y)), g);
+                r[2 * i] = __float_as_uint(ds.x);
+                r[2 * i + 1] = __float_as_uint(ds.y);
             }
+            // a pass of its own: inside the loop above the compares ran, predicated, for every tile, and registers spilled (dQ, dK and dV
+            // of 16 heads, D = 80, sequences of 1564, 1276 and 5120: 0.978 ms before, 0.946 ms with these passes here and in dK/dV)
+            if (tile_masked) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i)
+                    if (kbase + i > limit || kbase + i < vis_lo) r[i] = 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) d[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
             tmem_st_32x32(t_row, d);             // over the first 32 of the 64 fp32 columns this thread just read
             tmem_wait_st();
             fence_before_sync();
-            mbar_arrive(ds_full);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ds_full);
         }
         bf16* dst = p.dq + ((size_t)(q_begin + qi) * p.Nq + head) * p.D + half * 64;
         if (ok && n_kv > 0 && mbar_wait(dq_full, 0, abort_flag)) {

@@ -6,10 +6,12 @@
 //     dP^T_i = V dO_i^T         128 x 128 x 128   SS   -> TMEM columns [128, 256)
 //     dV    += P^T_i  dO_i      128 x 128 x 128   TS   (P^T_i  written by the row threads over their own S^T columns)
 //     dK    += dS^T_i Q_i       128 x 128 x 128   TS   (dS^T_i written over their own dP^T columns)
-// All four products have N = 128, so every tcgen05.mma runs at the full 64 clocks (the 64-row steps of the default
-// kernel pay 48 clocks for N = 64 products, i.e. 1.5x for S^T and dP^T) and the operand traffic from shared memory
-// drops from 256 KB to 192 KB per 128 query rows.  S^T and dP^T are single-buffered; the tensor pipe is kept busy by the
-// issue order   S_0 dP_0 | dV_i S_{i+1} dK_i dP_{i+1} | ...   in which the product that follows a wait never depends on
+// All four products have N = 128: the 64-row steps of the default kernel read 256 KB of operands from shared memory per
+// 128 query rows, these 192 KB.  Bound by the issue of the products: clock stamps show 130 clocks for each of the 16
+// tcgen05.mma of S^T and dP^T (both operands in shared memory) and 72 for each of the 16 of dV and dK (A in tensor
+// memory), 3230 of the 3550 clocks of a step.  dQ, dK and dV of 12 heads x 7800 x 7800 x 128 took 1.356 ms; 1.283 ms
+// once the masks had a pass of their own (4150 clocks a step); 1.204 ms with two buffers for the statistics.
+// S^T and dP^T are single-buffered; the tensor pipe is kept busy by the issue order   S_0 dP_0 | dV_i S_{i+1} dK_i dP_{i+1} | ...   in which the product that follows a wait never depends on
 // the row threads' other phase: while they turn S_{i+1} into P_{i+1}, the pipe runs dK_i and dP_{i+1}; while they turn
 // dP_{i+1} into dS_{i+1}, it runs dV_{i+1} and S_{i+2}.
 //
@@ -23,7 +25,11 @@
 
 constexpr int kRingQ128 = 3;    // Q_i is needed first (S^T_i) and released last (dK_i): it gets the deeper ring
 constexpr int kRingDO128 = 2;
-constexpr int kSmemDkv128 = (2 + kRingQ128 + kRingDO128) * kTile + 2 * 128 * 4 + 256 + 1024;    // K, V, Q ring, dO ring, stats, barriers, align
+// K, V, Q ring, dO ring, statistics (two buffers), barriers, alignment: dynamic shared memory starts 1024-aligned (behind the 1 KB
+// that the system keeps), which the kernel checks, since a full kilobyte of slack does not fit
+constexpr int kSlackDkv128 = 768;
+constexpr int kSmemDkv128 = (2 + kRingQ128 + kRingDO128) * kTile + 2 * 2 * 128 * 4 + 256 + kSlackDkv128;
+static_assert(kSmemDkv128 <= 227 * 1024, "shared memory of a CTA");
 
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -32,13 +38,16 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     constexpr int BQ = 128;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    if (smem - smem_raw > kSlackDkv128) {
+        if (threadIdx.x == 0) atomicExch(p.status, MM_TIMEOUT_TMA);
+        return;
+    }
     uint8_t* sK = smem;
     uint8_t* sV = sK + kTile;
     uint8_t* sQ = sV + kTile;                     // [kRingQ128]
     uint8_t* sdO = sQ + kRingQ128 * kTile;        // [kRingDO128]
-    float* s_lse = reinterpret_cast<float*>(sdO + kRingDO128 * kTile);     // [128]
-    float* s_dlt = s_lse + BQ;                                              // [128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s_dlt + BQ);
+    float* s_stat = reinterpret_cast<float*>(sdO + kRingDO128 * kTile);    // [2][-lse * log2(e) | -delta][128]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s_stat + 4 * BQ);
     uint64_t* kv_full = bars + 0;
     uint64_t* q_full = bars + 1;                  // [kRingQ128]
     uint64_t* q_empty = q_full + kRingQ128;       // [kRingQ128]
@@ -81,8 +90,8 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         mbar_init(s_full, 1);
         mbar_init(dp_full, 1);
-        mbar_init(p_full, 256);
-        mbar_init(ds_full, 256);
+        mbar_init(p_full, 8);                         // one arrival per warp
+        mbar_init(ds_full, 8);
         mbar_init(acc_full, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -182,24 +191,29 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         int vis_lo = 0, vis_hi = q_len;                  // queries that see this key (packed tiles: its own sequence)
         if (nseq > 1) packed_row_range(p.cu_k, seq, nseq, k_begin + kj, k_begin, vis_lo, vis_hi);
         const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-        // per-column statistics (lse from threads 0..127, delta from 128..255) are fetched one tile ahead
+        // per-column statistics (lse from threads 0..127, delta from 128..255), negated for the packed additions: fetched two
+        // tiles ahead, written to shared memory one ahead
         auto load_stat = [&](int it) -> float {
             const int head = head0 + it / per_head;
             const int qi = min((i_min + it % per_head) * BQ + (tid2 & 127), q_len - 1);
             const size_t idx = (size_t)head * p.T + q_begin + qi;
-            return tid2 < 128 ? p.lse[idx] * kLog2e : p.delta[idx];
+            return tid2 < 128 ? p.lse[idx] * -kLog2e : -p.delta[idx];
         };
-        float pre = n_it > 0 ? load_stat(0) : 0.f;
+        if (n_it > 0) s_stat[tid2] = load_stat(0);
+        float pre = n_it > 1 ? load_stat(1) : 0.f;
         bool ok = true;
         for (int it = 0; it < n_it; ++it) {
             const uint32_t par = it & 1;
             const int qbase = (i_min + it % per_head) * BQ;
-            // the statistics buffer is single: everybody must be done with tile it - 1 before it is overwritten
+            // everybody is done with tile it - 1, whose buffer takes the next tile's statistics, and sees those of this tile
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (tid2 < 128) s_lse[tid2] = pre;
-            else s_dlt[tid2 - 128] = pre;
-            if (it + 1 < n_it) pre = load_stat(it + 1);
-            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (it + 1 < n_it) s_stat[((it + 1) & 1) * 2 * BQ + tid2] = pre;
+            if (it + 2 < n_it) pre = load_stat(it + 2);
+            // read before the scores are there: behind them the tensor core's operand reads keep shared memory busy, and 16 reads
+            // in the middle of the exponentials made these 1850 clocks instead of 1070
+            float4 ls[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) ls[i] = reinterpret_cast<const float4*>(s_stat + (it & 1) * 2 * BQ + half * 64)[i];
             if (ok && !mbar_wait(s_full, par, abort_flag)) ok = false;
             if (!ok) continue;
             fence_after_sync();
@@ -211,23 +225,23 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             // visible query columns for this key: qi < q_len and (not causal or kj <= qi + diag)
             const int c_lo = !row_ok ? BQ : (p.causal ? max(0, kj - diag - qbase) : max(0, vis_lo - qbase));
             const int c_hi = min(BQ, vis_hi - qbase);
-            const float* ls = s_lse + half * 64;
-            const float* dl = s_dlt + half * 64;
+            // (16-byte reads: a scalar read per column would be as many load instructions as there are exponentials)
+            const float4* dl = reinterpret_cast<const float4*>(s_stat + (it & 1) * 2 * BQ + BQ + half * 64);
             // packed fp32 math (two query columns per instruction): P = exp2(S^T * scale - lse)
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-            const bool col_masked = c_lo > half * 64 || c_hi < half * 64 + 64;
+            const bool col_masked = __any_sync(0xffffffffu, c_lo > half * 64 || c_hi < half * 64 + 64);
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-                const float2 x = __ffma2_rn(make_float2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2,
-                                            make_float2(-ls[2 * i], -ls[2 * i + 1]));
-                float2 pr = make_float2(exp2f(x.x), exp2f(x.y));
-                if (col_masked) {
-                    const int cc = half * 64 + 2 * i;
-                    if (cc < c_lo || cc >= c_hi) pr.x = 0.f;
-                    if (cc + 1 < c_lo || cc + 1 >= c_hi) pr.y = 0.f;
-                }
-                s[2 * i] = __float_as_uint(pr.x);
-                s[2 * i + 1] = __float_as_uint(pr.y);
+                const float4 l4 = ls[i >> 1];
+                const float2 l2 = i & 1 ? make_float2(l4.z, l4.w) : make_float2(l4.x, l4.y);
+                const float2 x = __ffma2_rn(make_float2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, l2);
+                s[2 * i] = __float_as_uint(exp2f(x.x));
+                s[2 * i + 1] = __float_as_uint(exp2f(x.y));
+            }
+            if (col_masked) {            // a pass of its own: inside the loop above the compares ran, predicated, for every tile
+#pragma unroll
+                for (int i = 0; i < 64; ++i)
+                    if (half * 64 + i < c_lo || half * 64 + i >= c_hi) s[i] = 0;
             }
             {
                 uint32_t pw[32];
@@ -236,7 +250,8 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 tmem_st_32x32(t_s, pw);                  // over the first 32 of the 64 fp32 columns this thread has just read
                 tmem_wait_st();
                 fence_before_sync();
-                mbar_arrive(p_full);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_full);
             }
             if (!mbar_wait(dp_full, par, abort_flag)) { ok = false; continue; }
             fence_after_sync();
@@ -248,15 +263,17 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 uint32_t dw[32];
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {               // dS = P * (dP - delta)
-                    const float2 g = __fadd2_rn(make_float2(__uint_as_float(d[2 * i]), __uint_as_float(d[2 * i + 1])),
-                                                make_float2(-dl[2 * i], -dl[2 * i + 1]));
+                    const float4 d4 = dl[i >> 1];
+                    const float2 d2 = i & 1 ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y);
+                    const float2 g = __fadd2_rn(make_float2(__uint_as_float(d[2 * i]), __uint_as_float(d[2 * i + 1])), d2);
                     const float2 ds = __fmul2_rn(make_float2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), g);
                     dw[i] = pack2(ds.x, ds.y);
                 }
                 tmem_st_32x32(t_d, dw);
                 tmem_wait_st();
                 fence_before_sync();
-                mbar_arrive(ds_full);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ds_full);
             }
         }
         bf16* dvp = p.dv + ((size_t)(k_begin + kj) * out_heads + out_head) * p.D + half * 64;
