@@ -167,11 +167,7 @@ class GatedDeltaNet(nn.Module):
         proj = self.in_proj(x)
         qkv, z, b, a = proj.split([self.conv_dim, self.value_dim, self.hv, self.hv], dim=-1)
         qkv = ops.causal_conv1d(qkv, self.conv_weight.to(qkv.dtype), None, "silu", cu_seqlens)
-        q, k, v = qkv.split([self.key_dim, self.key_dim, self.value_dim], dim=-1)
-        rep = self.hv // self.hk
-        q = ops.l2_norm(q.reshape(T, self.hk, self.dk)).repeat_interleave(rep, dim=1)
-        k = ops.l2_norm(k.reshape(T, self.hk, self.dk)).repeat_interleave(rep, dim=1)
-        v = v.reshape(T, self.hv, self.dv)
+        q, k, v = ops.delta_heads(qkv, self.hk, self.hv, self.dk, self.dv)
         beta = torch.sigmoid(b.float())
         g = -torch.exp(self.A_log.float()) * F.softplus(a.float() + self.dt_bias.float())
         o = ops.gated_delta_rule_varlen(q, k, v, g, beta, cu_seqlens, chunk=self.c.gdn_chunk)

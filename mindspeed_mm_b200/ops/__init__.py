@@ -163,6 +163,17 @@ def l2_norm(x, eps: float = 1e-6):
     return ref.l2_norm(x, eps)
 
 
+def delta_heads(qkv, hk: int, hv: int, dk: int, dv: int):
+    """``q | k | v`` of ``hk`` key and ``hv`` value heads [T, 2 hk dk + hv dv] as the delta rule takes them: q and k L2-normalised
+    and repeated to ``hv`` heads."""
+    if _native(qkv) and _nat().delta_heads_supported(qkv, hk, hv, dk, dv):
+        return _nat().delta_heads(qkv, hk, hv, dv)
+    T = qkv.shape[0]
+    q, k, v = qkv.split([hk * dk, hk * dk, hv * dv], dim=-1)
+    q, k = (l2_norm(t.reshape(T, hk, dk)).repeat_interleave(hv // hk, dim=1) for t in (q, k))
+    return q, k, v.reshape(T, hv, dv)
+
+
 def gated_rms_norm(x, z, weight, eps: float = 1e-6):
     """``rmsnorm(x) * weight * silu(z)`` over the last dim, in ``z``'s dtype (``x`` may be the fp32 output of the delta rule)."""
     D = x.shape[-1]

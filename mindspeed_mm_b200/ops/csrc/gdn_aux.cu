@@ -1,8 +1,11 @@
 // Auxiliary kernels of the gated-delta-net layer on packed sequences:
 //   causal_conv1d (depthwise, kernel <= 8, optional SiLU, restarts at every sequence boundary) forward and backward,
+//   delta_heads (the step between the convolution and the delta rule) forward and backward,
 //   l2norm over the head dim (forward and backward; the gated RMSNorm of the layer's output lives in rownorm.cu).
-// x is [T, D] bf16 with the channel dim contiguous: a thread owns 8 channels (16 bytes) and walks a strip of
-// tokens keeping the last K-1 inputs in registers, so every input is read once.
+// x is [T, D] bf16 with the channel dim contiguous and ldx elements between tokens: the convolution reads its columns of
+// the fused projection in place (the seven copies of columns and heads in a training step of the layer, 4096 tokens, took
+// 261 us).  A thread owns 8 channels (16 bytes) and walks a strip of tokens keeping the last K-1 inputs in registers, so
+// every input is read once.
 #include "common.cuh"
 
 namespace {
@@ -16,7 +19,7 @@ constexpr int kStrip = 32;   // tokens per thread strip
 constexpr int kChunk = 8;
 
 template <int K, bool SILU>
-__global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w,
                                                          const int* __restrict__ seq_start, bf16* __restrict__ y, int T,
                                                          int D) {
     const int dv = D >> 3;
@@ -33,7 +36,7 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict_
 #pragma unroll
     for (int i = 0; i < K - 1; ++i) {
         const int t = t0 - (K - 1) + i;
-        if (t >= 0 && t >= s0) unpack8(reinterpret_cast<const Vec8*>(x + (size_t)t * D)[c], hist[i]);
+        if (t >= 0 && t >= s0) unpack8(reinterpret_cast<const Vec8*>(x + t * ldx)[c], hist[i]);
         else
 #pragma unroll
             for (int j = 0; j < 8; ++j) hist[i][j] = 0.f;
@@ -44,7 +47,7 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict_
 #pragma unroll
         for (int u = 0; u < kChunk; ++u)
             if (tc + u < t1) {
-                in[u] = reinterpret_cast<const Vec8*>(x + (size_t)(tc + u) * D)[c];
+                in[u] = reinterpret_cast<const Vec8*>(x + (tc + u) * ldx)[c];
                 st[u] = seq_start[tc + u];
             }
 #pragma unroll
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict_
 // ring, and dx of token u - (K-1) is complete when u has been visited.  Weight gradients count outputs of the own strip
 // only, so strips do not double count; they leave through fp32 atomics.
 template <int K, bool SILU>
-__global__ void __launch_bounds__(128) conv1d_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(128) conv1d_bwd_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w,
                                                          const int* __restrict__ seq_start, const int* __restrict__ seq_end,
                                                          const bf16* __restrict__ dy, bf16* __restrict__ dx,
                                                          float* __restrict__ dw, int T, int D) {
@@ -105,7 +108,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const bf16* __restrict_
 #pragma unroll
     for (int i = 0; i < K - 1; ++i) {
         const int t = t0 - (K - 1) + i;
-        if (t >= 0 && t >= s0) unpack8(reinterpret_cast<const Vec8*>(x + (size_t)t * D)[c], hist[i]);
+        if (t >= 0 && t >= s0) unpack8(reinterpret_cast<const Vec8*>(x + t * ldx)[c], hist[i]);
         else
 #pragma unroll
             for (int j = 0; j < 8; ++j) hist[i][j] = 0.f;
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const bf16* __restrict_
                 for (int i = 0; i < K - 1; ++i)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) hist[i][j] = 0.f;
-            unpack8(reinterpret_cast<const Vec8*>(x + (size_t)u * D)[c], hist[K - 1]);
+            unpack8(reinterpret_cast<const Vec8*>(x + u * ldx)[c], hist[K - 1]);
             float g[8];
             unpack8(reinterpret_cast<const Vec8*>(dy + (size_t)u * D)[c], g);
             if (SILU) {
@@ -215,7 +218,102 @@ __global__ void l2norm_bwd_kernel(const bf16* __restrict__ y, const bf16* __rest
     for (int i = lane; i < D; i += 32) dx[row * D + i] = __float2bfloat16(r * (gv[i >> 5] - yv[i >> 5] * dot));
 }
 
+
+// ---- the heads of the delta rule out of the convolution's result x [T, 2 hk 128 + vvec 8] = q | k | v, one CTA per token:
+// q and k of hk heads L2-normalised and written rep times each (the value heads outnumber them), v copied.  Memory-bound: every byte
+// is read and written once, where columns copied out, rows normalised, heads repeated and v copied out were seven passes; backward,
+// the repeats' gradients are summed in fp32, go through the norm and land with dv in the one gradient of x.  T = 4096, hk = 16,
+// 32 value heads: 30 us forward, where norm and copies took 160, and 35 us backward, where sums, norm and concatenation took 124.
+constexpr int kHeadVec = 16;      // 16-byte vectors of a 128-wide head: half a warp per row
+
+__device__ __forceinline__ float half_warp_sum(float v) {
+#pragma unroll
+    for (int o = kHeadVec / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__global__ void __launch_bounds__(256) delta_heads_fwd_kernel(const Vec8* __restrict__ x, Vec8* __restrict__ q, Vec8* __restrict__ k,
+                                                              Vec8* __restrict__ v, float* __restrict__ rnorm, int hk, int rep, int vvec,
+                                                              float eps) {
+    const size_t t = blockIdx.x;
+    const int nn = 2 * hk * kHeadVec, W = nn + vvec;      // nn is a multiple of 32: a warp has rows to normalise or values, not both
+    const Vec8* src = x + t * W;
+    for (int i = threadIdx.x; i < W; i += 256) {
+        Vec8 in = src[i];
+        if (i >= nn) {
+            v[t * vvec + (i - nn)] = in;
+            continue;
+        }
+        float f[8];
+        unpack8(in, f);
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+        const float r = rsqrtf(half_warp_sum(ss) + eps);
+        const int row = i / kHeadVec, c = i % kHeadVec;
+        if (c == 0) rnorm[t * 2 * hk + row] = r;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] *= r;
+        in = pack8(f);
+        Vec8* dst = (row < hk ? q : k) + (t * hk + row % hk) * rep * kHeadVec + c;
+        for (int j = 0; j < rep; ++j) dst[j * kHeadVec] = in;
+    }
+}
+
+__global__ void __launch_bounds__(256) delta_heads_bwd_kernel(const Vec8* __restrict__ q, const Vec8* __restrict__ k,
+                                                              const float* __restrict__ rnorm, const Vec8* __restrict__ dq,
+                                                              const Vec8* __restrict__ dk, const Vec8* __restrict__ dv,
+                                                              Vec8* __restrict__ dx, int hk, int rep, int vvec) {
+    const size_t t = blockIdx.x;
+    const int nn = 2 * hk * kHeadVec, W = nn + vvec;
+    Vec8* dst = dx + t * W;
+    for (int i = threadIdx.x; i < W; i += 256) {
+        if (i >= nn) {
+            dst[i] = dv[t * vvec + (i - nn)];
+            continue;
+        }
+        const int row = i / kHeadVec, c = i % kHeadVec;
+        const size_t at = (t * hk + row % hk) * rep * kHeadVec + c;
+        const Vec8* gsrc = (row < hk ? dq : dk) + at;
+        float y[8], g[8];
+        unpack8((row < hk ? q : k)[at], y);
+        unpack8(gsrc[0], g);
+        for (int j = 1; j < rep; ++j) {
+            float h[8];
+            unpack8(gsrc[j * kHeadVec], h);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) g[e] += h[e];
+        }
+        float dot = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dot += y[e] * g[e];
+        dot = half_warp_sum(dot);
+        const float r = rnorm[t * 2 * hk + row];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) g[e] = r * (g[e] - y[e] * dot);
+        dst[i] = pack8(g);
+    }
+}
+
 }  // namespace
+
+// x: bf16 [T, 2 hk 128 + v_width], q, k: [T, hk * rep, 128], v: [T, v_width], rnorm: fp32 [T, 2 hk]; all dense, 16-byte aligned.
+MM_API int mm_delta_heads_fwd(const void* x, void* q, void* k, void* v, float* rnorm, int T, int hk, int rep, int v_width, float eps,
+                              cudaStream_t st) {
+    if (v_width % 8 || hk < 1 || rep < 1) return -1;
+    if (T == 0) return 0;
+    delta_heads_fwd_kernel<<<T, 256, 0, st>>>((const Vec8*)x, (Vec8*)q, (Vec8*)k, (Vec8*)v, rnorm, hk, rep, v_width / 8, eps);
+    return (int)cudaGetLastError();
+}
+
+MM_API int mm_delta_heads_bwd(const void* q, const void* k, const float* rnorm, const void* dq, const void* dk, const void* dv, void* dx,
+                              int T, int hk, int rep, int v_width, cudaStream_t st) {
+    if (v_width % 8 || hk < 1 || rep < 1) return -1;
+    if (T == 0) return 0;
+    delta_heads_bwd_kernel<<<T, 256, 0, st>>>((const Vec8*)q, (const Vec8*)k, rnorm, (const Vec8*)dq, (const Vec8*)dk, (const Vec8*)dv,
+                                              (Vec8*)dx, hk, rep, v_width / 8);
+    return (int)cudaGetLastError();
+}
 
 #define MM_CONV_K(MACRO)                  \
     switch (K) {                          \
@@ -229,28 +327,30 @@ __global__ void l2norm_bwd_kernel(const bf16* __restrict__ y, const bf16* __rest
         default: MACRO(8); break;         \
     }
 
-MM_API int mm_conv1d_fwd(const void* x, const void* w, const int* seq_start, void* y, int T, int D, int K, int silu, cudaStream_t st) {
-    if (D % 8 || K > kMaxK || K < 1) return -1;
+// ldx: elements between the tokens of x, a multiple of 8.
+MM_API int mm_conv1d_fwd(const void* x, long long ldx, const void* w, const int* seq_start, void* y, int T, int D, int K, int silu,
+                         cudaStream_t st) {
+    if (D % 8 || ldx % 8 || K > kMaxK || K < 1) return -1;
     dim3 grid((D / 8 + 127) / 128, (T + kStrip - 1) / kStrip);
 #define MM_CONV_FWD(KK)                                                                                                   \
-    if (silu) conv1d_fwd_kernel<KK, true><<<grid, 128, 0, st>>>((const bf16*)x, (const bf16*)w, seq_start, (bf16*)y, T, D); \
-    else conv1d_fwd_kernel<KK, false><<<grid, 128, 0, st>>>((const bf16*)x, (const bf16*)w, seq_start, (bf16*)y, T, D)
+    if (silu) conv1d_fwd_kernel<KK, true><<<grid, 128, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, (bf16*)y, T, D); \
+    else conv1d_fwd_kernel<KK, false><<<grid, 128, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, (bf16*)y, T, D)
     MM_CONV_K(MM_CONV_FWD)
 #undef MM_CONV_FWD
     return (int)cudaGetLastError();
 }
 
 // dw: fp32 [D, K], zeroed by the caller (accumulated with atomics).
-MM_API int mm_conv1d_bwd(const void* x, const void* w, const int* seq_start, const int* seq_end, const void* dy, void* dx,
+MM_API int mm_conv1d_bwd(const void* x, long long ldx, const void* w, const int* seq_start, const int* seq_end, const void* dy, void* dx,
                          float* dw, int T, int D, int K, int silu, cudaStream_t st) {
-    if (D % 8 || K > kMaxK || K < 1) return -1;
+    if (D % 8 || ldx % 8 || K > kMaxK || K < 1) return -1;
     dim3 grid((D / 8 + 127) / 128, (T + kStrip - 1) / kStrip);
 #define MM_CONV_BWD(KK)                                                                                                  \
     if (silu)                                                                                                            \
-        conv1d_bwd_kernel<KK, true><<<grid, 128, 0, st>>>((const bf16*)x, (const bf16*)w, seq_start, seq_end,           \
+        conv1d_bwd_kernel<KK, true><<<grid, 128, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, seq_end,           \
                                                           (const bf16*)dy, (bf16*)dx, dw, T, D);                         \
     else                                                                                                                 \
-        conv1d_bwd_kernel<KK, false><<<grid, 128, 0, st>>>((const bf16*)x, (const bf16*)w, seq_start, seq_end,          \
+        conv1d_bwd_kernel<KK, false><<<grid, 128, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, seq_end,          \
                                                            (const bf16*)dy, (bf16*)dx, dw, T, D)
     MM_CONV_K(MM_CONV_BWD)
 #undef MM_CONV_BWD

@@ -165,10 +165,19 @@ __device__ __forceinline__ void store8(void* base, size_t vec, const float* f) {
     }
 }
 
+// Where row `row` of z starts: z is [rows / zh, zh, H] with ldz elements between its tokens, so that the gate's columns of a fused
+// projection are read in place and not copied out first.  zh = 1, ldz = H: dense rows.
+__device__ __forceinline__ size_t gate_row(long long row, int zh, long long ldz, int H) {
+    if (zh == 1) return (size_t)(row * ldz);
+    const unsigned t = (unsigned)row / (unsigned)zh, h = (unsigned)row - t * (unsigned)zh;
+    return (size_t)t * ldz + (size_t)h * H;
+}
+
 template <int G, bool XF32>
 __global__ void __launch_bounds__(kBlock) gated_rms_fwd_kernel(const void* __restrict__ x, const bf16* __restrict__ z,
                                                               const bf16* __restrict__ w, bf16* __restrict__ y,
-                                                              float* __restrict__ rstd_out, long long rows, int H, float eps) {
+                                                              float* __restrict__ rstd_out, long long rows, int H, int zh, long long ldz,
+                                                              float eps) {
     constexpr int kRowsPerBlock = kBlock / G;
     const int nvec = H >> 3;
     const int gl = threadIdx.x % G;
@@ -191,7 +200,7 @@ __global__ void __launch_bounds__(kBlock) gated_rms_fwd_kernel(const void* __res
         const float r = rsqrtf(ss / (float)H + eps);
         if (gl == 0 && rstd_out) rstd_out[row] = r;
         float zz[8], o[8];
-        unpack8(reinterpret_cast<const Vec8*>(z + (size_t)row * H)[gl], zz);
+        unpack8(reinterpret_cast<const Vec8*>(z + gate_row(row, zh, ldz, H))[gl], zz);
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] = f[k] * r * wv[k] * zz[k] / (1.f + __expf(-zz[k]));
         reinterpret_cast<Vec8*>(y + (size_t)row * H)[gl] = pack8(o);
@@ -203,7 +212,7 @@ __global__ void __launch_bounds__(kBlock) gated_rms_bwd_kernel(const void* __res
                                                               const bf16* __restrict__ w, const bf16* __restrict__ dy,
                                                               const float* __restrict__ rstd_in, void* __restrict__ dx,
                                                               bf16* __restrict__ dz, float* __restrict__ dw, long long rows,
-                                                              int H) {
+                                                              int H, int zh, long long ldz) {
     constexpr int kRowsPerBlock = kBlock / G;
     __shared__ float sdw[256];
     const int nvec = H >> 3;
@@ -225,7 +234,7 @@ __global__ void __launch_bounds__(kBlock) gated_rms_bwd_kernel(const void* __res
             r = rstd_in[row];
             load8<XF32>(x, (size_t)row * nvec + gl, n);
             unpack8(reinterpret_cast<const Vec8*>(dy + (size_t)row * H)[gl], g);
-            unpack8(reinterpret_cast<const Vec8*>(z + (size_t)row * H)[gl], zz);
+            unpack8(reinterpret_cast<const Vec8*>(z + gate_row(row, zh, ldz, H))[gl], zz);
             float dzv[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -256,8 +265,8 @@ __global__ void __launch_bounds__(kBlock) gated_rms_bwd_kernel(const void* __res
 
 template <bool XF32>
 int gated_launch(bool bwd, const void* x, const void* z, const void* w, void* y_or_dy, float* rstd, void* dx, void* dz,
-                 float* dw, long long rows, int H, float eps, cudaStream_t st) {
-    if (H % 8 || H < 8 || H > 256) return -1;
+                 float* dw, long long rows, int H, int zh, long long ldz, float eps, cudaStream_t st) {
+    if (H % 8 || H < 8 || H > 256 || zh < 1 || ldz % 8 || (zh > 1 && rows > 0x7fffffffLL)) return -1;
     const int nvec = H / 8;
 #define MM_GR(G)                                                                                                           \
     {                                                                                                                      \
@@ -266,10 +275,10 @@ int gated_launch(bool bwd, const void* x, const void* z, const void* w, void* y_
         if (grid == 0) return 0;                                                                                           \
         if (!bwd)                                                                                                          \
             gated_rms_fwd_kernel<G, XF32><<<grid, kBlock, 0, st>>>(x, (const bf16*)z, (const bf16*)w, (bf16*)y_or_dy, rstd, \
-                                                                  rows, H, eps);                                           \
+                                                                  rows, H, zh, ldz, eps);                                  \
         else                                                                                                               \
             gated_rms_bwd_kernel<G, XF32><<<grid, kBlock, 0, st>>>(x, (const bf16*)z, (const bf16*)w,                       \
-                                                                  (const bf16*)y_or_dy, rstd, dx, (bf16*)dz, dw, rows, H); \
+                                                                  (const bf16*)y_or_dy, rstd, dx, (bf16*)dz, dw, rows, H, zh, ldz); \
         return (int)cudaGetLastError();                                                                                    \
     }
     if (nvec <= 4) MM_GR(4)
@@ -281,18 +290,19 @@ int gated_launch(bool bwd, const void* x, const void* z, const void* w, void* y_
 
 }  // namespace
 
-// y = rmsnorm(x) * w * silu(z).  x fp32 (x_f32 = 1) or bf16; rstd [rows] fp32 (optional in the forward).
+// y = rmsnorm(x) * w * silu(z).  x fp32 (x_f32 = 1) or bf16; rstd [rows] fp32 (optional in the forward).  z: zh rows a token, ldz
+// elements (a multiple of 8) between tokens; the other tensors are dense.
 MM_API int mm_gated_rms_fwd(const void* x, int x_f32, const void* z, const void* w, void* y, float* rstd, long long rows,
-                            int H, float eps, cudaStream_t st) {
-    return x_f32 ? gated_launch<true>(false, x, z, w, y, rstd, nullptr, nullptr, nullptr, rows, H, eps, st)
-                 : gated_launch<false>(false, x, z, w, y, rstd, nullptr, nullptr, nullptr, rows, H, eps, st);
+                            int H, int zh, long long ldz, float eps, cudaStream_t st) {
+    return x_f32 ? gated_launch<true>(false, x, z, w, y, rstd, nullptr, nullptr, nullptr, rows, H, zh, ldz, eps, st)
+                 : gated_launch<false>(false, x, z, w, y, rstd, nullptr, nullptr, nullptr, rows, H, zh, ldz, eps, st);
 }
 
 // dx (x's type), dz (bf16), dw (fp32 [H], zeroed by the caller; accumulated with atomics).
 MM_API int mm_gated_rms_bwd(const void* x, int x_f32, const void* z, const void* w, const void* dy, const float* rstd,
-                            void* dx, void* dz, float* dw, long long rows, int H, cudaStream_t st) {
-    return x_f32 ? gated_launch<true>(true, x, z, w, const_cast<void*>(dy), const_cast<float*>(rstd), dx, dz, dw, rows, H, 0.f, st)
-                 : gated_launch<false>(true, x, z, w, const_cast<void*>(dy), const_cast<float*>(rstd), dx, dz, dw, rows, H, 0.f, st);
+                            void* dx, void* dz, float* dw, long long rows, int H, int zh, long long ldz, cudaStream_t st) {
+    return x_f32 ? gated_launch<true>(true, x, z, w, const_cast<void*>(dy), const_cast<float*>(rstd), dx, dz, dw, rows, H, zh, ldz, 0.f, st)
+                 : gated_launch<false>(true, x, z, w, const_cast<void*>(dy), const_cast<float*>(rstd), dx, dz, dw, rows, H, zh, ldz, 0.f, st);
 }
 
 // y = x * rsqrt(mean(x^2) + eps) * w;  rstd (optional) [rows] keeps the factor for the backward.

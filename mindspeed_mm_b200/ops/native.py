@@ -57,8 +57,8 @@ def _declare(L):
         "mm_rownorm_rms_fwd": [_p, _p, _p, _p, _ll, _i, _f, _p],
         "mm_rownorm_ln_mod_fwd": [_p, _p, _p, _p, _p, _p, _ll, _i, _i, _f, _p],
         "mm_rownorm_l2_fwd": [_p, _p, _p, _ll, _i, _f, _p],
-        "mm_gated_rms_fwd": [_p, _i, _p, _p, _p, _p, _ll, _i, _f, _p],
-        "mm_gated_rms_bwd": [_p, _i, _p, _p, _p, _p, _p, _p, _p, _ll, _i, _p],
+        "mm_gated_rms_fwd": [_p, _i, _p, _p, _p, _p, _ll, _i, _i, _ll, _f, _p],
+        "mm_gated_rms_bwd": [_p, _i, _p, _p, _p, _p, _p, _p, _p, _ll, _i, _i, _ll, _p],
         "mm_rmsnorm_bwd_grid": [_i],
         "mm_sq_norm_blocks": [],
         "mm_rmsnorm_set_v16": [_i],
@@ -94,8 +94,10 @@ def _declare(L):
         "mm_moe_unpermute": [_p, _p, _p, _p, _i, _i, _i, _p],
         "mm_moe_unpermute_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_moe_route": [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p],
-        "mm_conv1d_fwd": [_p, _p, _p, _p, _i, _i, _i, _i, _p],
-        "mm_conv1d_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
+        "mm_delta_heads_fwd": [_p, _p, _p, _p, _p, _i, _i, _i, _i, _f, _p],
+        "mm_delta_heads_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
+        "mm_conv1d_fwd": [_p, _ll, _p, _p, _p, _i, _i, _i, _i, _p],
+        "mm_conv1d_bwd": [_p, _ll, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_l2norm_fwd": [_p, _p, _p, _ll, _i, _f, _p],
         "mm_l2norm_bwd": [_p, _p, _p, _p, _ll, _i, _p],
         "mm_gdn_prologue": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _f, _p],
@@ -1032,10 +1034,13 @@ class _CausalConv1d(torch.autograd.Function):
     def forward(ctx, x, w, cu_seqlens, silu):
         T, D = x.shape
         K = w.shape[-1]
-        x, w = x.contiguous(), w.contiguous()
+        # the convolution's columns of a fused projection are read where they are
+        if x.stride(1) != 1 or _pitch(x) % 8 or x.data_ptr() % 16:
+            x = x.contiguous()
+        w = w.contiguous()
         start, end = _seq_bounds(cu_seqlens, T, x.device)
-        y = torch.empty_like(x)
-        _check(lib().mm_conv1d_fwd(x.data_ptr(), w.data_ptr(), start.data_ptr(), y.data_ptr(), T, D, K, int(silu), _st()),
+        y = torch.empty(T, D, dtype=x.dtype, device=x.device)
+        _check(lib().mm_conv1d_fwd(x.data_ptr(), _pitch(x), w.data_ptr(), start.data_ptr(), y.data_ptr(), T, D, K, int(silu), _st()),
                "conv1d_fwd")
         ctx.save_for_backward(x, w, start, end)
         ctx.silu = silu
@@ -1047,9 +1052,9 @@ class _CausalConv1d(torch.autograd.Function):
         T, D = x.shape
         K = w.shape[-1]
         dy = dy.contiguous()
-        dx = torch.empty_like(x)
+        dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
         dw = torch.zeros(D, K, dtype=torch.float32, device=x.device)
-        _check(lib().mm_conv1d_bwd(x.data_ptr(), w.data_ptr(), start.data_ptr(), end.data_ptr(), dy.data_ptr(),
+        _check(lib().mm_conv1d_bwd(x.data_ptr(), _pitch(x), w.data_ptr(), start.data_ptr(), end.data_ptr(), dy.data_ptr(),
                                    dx.data_ptr(), dw.data_ptr(), T, D, K, int(ctx.silu), _st()), "conv1d_bwd")
         return dx, dw.to(w.dtype), None, None
 
@@ -1090,20 +1095,59 @@ def l2_norm(x, eps=1e-6):
     return _run(_L2Norm, x, eps)
 
 
+class _DeltaHeads(torch.autograd.Function):
+    """``q | k | v`` columns to the delta rule's heads: q and k L2-normalised and repeated, v as it is, each dense."""
+
+    @staticmethod
+    def forward(ctx, x, hk, hv, dv, eps):
+        T, dev = x.shape[0], x.device
+        q, k = (torch.empty(T, hv, 128, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        v = torch.empty(T, hv, dv, dtype=torch.bfloat16, device=dev)
+        r = torch.empty(T, 2 * hk, dtype=torch.float32, device=dev)
+        _check(lib().mm_delta_heads_fwd(x.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), r.data_ptr(), T, hk, hv // hk, hv * dv,
+                                        eps, _st()), "delta_heads_fwd")
+        ctx.save_for_backward(q, k, r)
+        return q, k, v
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        q, k, r = ctx.saved_tensors
+        T, hk, v_width = q.shape[0], r.shape[1] // 2, dv.shape[1] * dv.shape[2]
+        dq, dk, dv = (g if g.is_contiguous() and g.data_ptr() % 16 == 0 else g.clone(memory_format=torch.contiguous_format) for g in (dq, dk, dv))
+        dx = torch.empty(T, 2 * hk * 128 + v_width, dtype=torch.bfloat16, device=q.device)
+        _check(lib().mm_delta_heads_bwd(q.data_ptr(), k.data_ptr(), r.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                        dx.data_ptr(), T, hk, q.shape[1] // hk, v_width, _st()), "delta_heads_bwd")
+        return dx, None, None, None, None
+
+
+def delta_heads_supported(x, hk, hv, dk, dv) -> bool:
+    return (x.dim() == 2 and x.dtype == torch.bfloat16 and dk == 128 and hv % hk == 0 and dv % 8 == 0 and x.is_contiguous()
+            and x.data_ptr() % 16 == 0 and x.shape[1] == 2 * hk * dk + hv * dv)
+
+
+def delta_heads(x, hk, hv, dv, eps=1e-6):
+    return _run(_DeltaHeads, x, hk, hv, dv, eps)
+
+
 class _GatedRMSNorm(torch.autograd.Function):
     """``rmsnorm(x) * w * silu(z)`` over the last dim (<= 256): x fp32 or bf16, z / w / result bf16."""
 
     @staticmethod
     def forward(ctx, x, z, w, eps):
         D = x.shape[-1]
-        x2, z2, wc = x.reshape(-1, D).contiguous(), z.reshape(-1, D).contiguous(), w.contiguous()
+        x2, wc = x.reshape(-1, D).contiguous(), w.contiguous()
         rows = x2.shape[0]
+        # z of [tokens, heads, D] with dense heads may have its tokens apart (the gate's columns of a fused projection)
+        if z.dim() == 3 and z.stride(2) == 1 and z.stride(1) == D and z.stride(0) % 8 == 0 and z.data_ptr() % 16 == 0 and rows < 2 ** 31:
+            z2, zh, ldz = z, z.shape[1], z.stride(0)
+        else:
+            z2, zh, ldz = z.reshape(-1, D).contiguous(), 1, D
         y = torch.empty(rows, D, dtype=torch.bfloat16, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         _check(lib().mm_gated_rms_fwd(x2.data_ptr(), int(x2.dtype == torch.float32), z2.data_ptr(), wc.data_ptr(), y.data_ptr(),
-                                      rstd.data_ptr(), rows, D, eps, _st()), "gated_rms_fwd")
+                                      rstd.data_ptr(), rows, D, zh, ldz, eps, _st()), "gated_rms_fwd")
         ctx.save_for_backward(x2, z2, wc, rstd)
-        ctx.shapes = (x.shape, z.shape)
+        ctx.shapes, ctx.gate_rows = (x.shape, z.shape), (zh, ldz)
         return y.view(z.shape)
 
     @staticmethod
@@ -1111,10 +1155,10 @@ class _GatedRMSNorm(torch.autograd.Function):
         x2, z2, wc, rstd = ctx.saved_tensors
         rows, D = x2.shape
         dy2 = dy.reshape(rows, D).contiguous()
-        dx, dz = torch.empty_like(x2), torch.empty_like(z2)
+        dx, dz = torch.empty_like(x2), torch.empty(rows, D, dtype=z2.dtype, device=z2.device)
         dw = torch.zeros(D, dtype=torch.float32, device=x2.device)
         _check(lib().mm_gated_rms_bwd(x2.data_ptr(), int(x2.dtype == torch.float32), z2.data_ptr(), wc.data_ptr(), dy2.data_ptr(),
-                                      rstd.data_ptr(), dx.data_ptr(), dz.data_ptr(), dw.data_ptr(), rows, D, _st()),
+                                      rstd.data_ptr(), dx.data_ptr(), dz.data_ptr(), dw.data_ptr(), rows, D, *ctx.gate_rows, _st()),
                "gated_rms_bwd")
         return dx.view(ctx.shapes[0]), dz.view(ctx.shapes[1]), dw.to(wc.dtype), None
 

@@ -296,3 +296,44 @@ def test_rotary_tables(T, D, section, theta):
     # one rounding (two where the 64-bit value is rounded to 32 bits first)
     for got, want in ((cos, ang.cos()), (sin, ang.sin())):
         assert float((got.double() - want).abs().max()) <= 2 ** -9 + 1e-6
+
+
+@pytest.mark.parametrize("T,hk,hv,dv", [(1, 1, 1, 8), (130, 2, 6, 128), (65, 16, 32, 128), (3, 3, 3, 72), (257, 1, 5, 24)])
+def test_delta_heads(T, hk, hv, dv):
+    """One head, odd repeats, values narrower than a warp's share: against the same steps in fp32."""
+    torch.manual_seed(T)
+    x = torch.randn(T, 2 * hk * 128 + hv * dv, device=DEV).bfloat16()
+    x[0, :128] = 0                                                # a row without a norm
+    x.requires_grad_()
+    leaf = x.detach().float().requires_grad_()
+    assert native.delta_heads_supported(x, hk, hv, 128, dv)
+    got = ops.delta_heads(x, hk, hv, 128, dv)
+    rows = ref.l2_norm(leaf[:, :2 * hk * 128].reshape(T, 2, hk, 128)).repeat_interleave(hv // hk, dim=2)
+    want = (rows[:, 0], rows[:, 1], leaf[:, 2 * hk * 128:].reshape(T, hv, dv))
+    for a, b in zip(got, want):
+        _close(a.detach(), b.detach(), rtol=2 ** -8, atol=0)      # one rounding to bf16
+    do = [torch.randn_like(t) for t in got]
+    do[0][0] = 0                                                  # (its gradient is 1000 times the others')
+    (a,), (b,) = torch.autograd.grad(got, [x], do), torch.autograd.grad(want, [leaf], [t.float() for t in do])
+    # one rounding of the result; y is read rounded: 2^-9 of |g| |y| over the row's norm
+    _close(a, b, rtol=2 ** -7, atol=0)
+
+
+@pytest.mark.parametrize("T,D,extra", [(1, 8, 0), (70, 264, 8), (33, 1032, 24), (129, 64, 3)])
+def test_convolution_and_gate_on_columns_of_a_wider_matrix(T, D, extra):
+    """Columns read in place (and copied where their pitch or their start does not allow it) give what dense ones give."""
+    torch.manual_seed(T)
+    wide = torch.randn(T, D + extra, device=DEV).bfloat16()
+    cu = torch.tensor([0, T // 3, T], device=DEV)
+    w = torch.randn(D, 4, device=DEV).bfloat16()
+    for lo in sorted({0, extra // 2, extra}):
+        outs = []
+        for x in (wide[:, lo:lo + D], wide[:, lo:lo + D].clone()):
+            x = x.detach().requires_grad_()
+            y = ops.causal_conv1d(x, w, None, "silu", cu)
+            outs.append([y.detach(), *torch.autograd.grad(y, [x], torch.ones_like(y))])
+            z = x.detach().view(T, -1, 8).requires_grad_()
+            o = torch.linspace(-2, 2, T * D, device=DEV).bfloat16().view(T, -1, 8)
+            y = ops.gated_rms_norm(o, z, w.view(-1)[:8])
+            outs[-1] += [y.detach(), *torch.autograd.grad(y, [z], torch.ones_like(y))]
+        assert all(torch.equal(a, b) for a, b in zip(*outs))
