@@ -83,104 +83,158 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict_
 // One pass over u = t0 .. t1 + K - 2 (the strip plus the K-1 outputs after it that still used its inputs): x[u] and dy[u]
 // are read once, the pre-activation comes from the sliding history as in the forward, the last K values of dpre sit in a
 // ring, and dx of token u - (K-1) is complete when u has been visited.  Weight gradients count outputs of the own strip
-// only, so strips do not double count; they leave through fp32 atomics.
+// only, so strips do not double count.
+// Was bound by the latency of its loads (60% of the stalls; the registers of the windows leave 12 warps an SM), so: 4 channels a
+// thread, tokens in chunks of four that are copied into shared memory three chunks ahead (each thread waits for its own copies
+// only), their bounds read once a strip, and the weight gradients of the block's four strips added up in shared memory, from where
+// they leave as consecutive fp32 atomics (a thread's own sums were 4.2 million, each in a 128-byte line of its own).  4096 x 8192,
+// K = 4: 160 us before, 74 us now, behind a flush of L2; memory allows 29.
+constexpr int kBwdWarps = 4;      // strips of a block: a warp has 128 channels of one
+constexpr int kBwdChunk = 4;
+constexpr int kBwdStages = 4;
+
+__device__ __forceinline__ void copy_async8(void* smem, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void unpack4(const uint2& v, float* f) {
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+    f[0] = lo.x, f[1] = lo.y, f[2] = hi.x, f[3] = hi.y;
+}
+
 template <int K, bool SILU>
-__global__ void __launch_bounds__(128) conv1d_bwd_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w,
-                                                         const int* __restrict__ seq_start, const int* __restrict__ seq_end,
-                                                         const bf16* __restrict__ dy, bf16* __restrict__ dx,
-                                                         float* __restrict__ dw, int T, int D) {
-    const int dv = D >> 3;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= dv) return;
-    const int t0 = blockIdx.y * kStrip, t1 = min(T, t0 + kStrip);
-    float wk[K][8], dwacc[K][8];
+__global__ void __launch_bounds__(32 * kBwdWarps) conv1d_bwd_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w,
+                                                                    const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+                                                                    const bf16* __restrict__ dy, bf16* __restrict__ dx,
+                                                                    float* __restrict__ dw, int T, int D) {
+    constexpr int CH = 4;
+    __shared__ uint2 stage[kBwdWarps][kBwdStages * kBwdChunk][2][32];       // x and dy of a token
+    __shared__ int bounds[kBwdWarps][2][kStrip + kMaxK];                      // where the sequences of tokens t0, t0 + 1, ... start and end
+    static_assert(32 * CH * kMaxK * sizeof(float) <= sizeof(stage[0]), "weight gradients lie over the stages");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = blockIdx.x * 32 * CH, c = c0 + lane * CH;
+    const int t0 = (blockIdx.y * kBwdWarps + warp) * kStrip, t1 = min(T, t0 + kStrip);
+    float dwacc[K][CH];
 #pragma unroll
     for (int k = 0; k < K; ++k)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            wk[k][j] = __bfloat162float(w[(size_t)(c * 8 + j) * K + k]);
-            dwacc[k][j] = 0.f;
+        for (int j = 0; j < CH; ++j) dwacc[k][j] = 0.f;
+    for (int i = lane; i < kStrip + K - 1; i += 32)
+        if (t0 + i < T) {
+            bounds[warp][0][i] = seq_start[t0 + i];
+            bounds[warp][1][i] = min(T, seq_end[t0 + i]);
         }
-    float hist[K][8];     // inputs u-(K-1) .. u (zero before the start of u's sequence)
-    float ring[K][8];     // ring[i] = dpre[u - (K-1) + i]
-    int ring_t[K];        // the output token each ring slot holds (-1: none)
-    const int s0 = seq_start[t0];
+    __syncwarp();
+    if (c < D && t0 < T) {
+        float wk[K][CH];
 #pragma unroll
-    for (int i = 0; i < K - 1; ++i) {
-        const int t = t0 - (K - 1) + i;
-        if (t >= 0 && t >= s0) unpack8(reinterpret_cast<const Vec8*>(x + t * ldx)[c], hist[i]);
-        else
+        for (int k = 0; k < K; ++k)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) hist[i][j] = 0.f;
-    }
+            for (int j = 0; j < CH; ++j) wk[k][j] = __bfloat162float(w[(size_t)(c + j) * K + k]);
+        const bf16* xc = x + c;
+        const bf16* gc = dy + c;
+        const int u_end = min(T, t1 + K - 1);         // one past the last output that used an input of the strip
+        uint2 (*mine)[2][32] = stage[warp];
+        auto fetch = [&](int chunk) {
 #pragma unroll
-    for (int i = 0; i < K; ++i) {
-        ring_t[i] = -1;
+            for (int i = 0; i < kBwdChunk; ++i) {
+                const int u = t0 + chunk * kBwdChunk + i;
+                if (u < u_end) {
+                    uint2 (*slot)[32] = mine[chunk % kBwdStages * kBwdChunk + i];
+                    copy_async8(&slot[0][lane], xc + u * ldx);
+                    copy_async8(&slot[1][lane], gc + (size_t)u * D);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ring[i][j] = 0.f;
-    }
-    const int u_end = min(T, t1 + K - 1);
-    for (int u = t0; u < u_end + K - 1; ++u) {
-        // shift the ring; slot K-1 receives dpre[u] (or nothing once u is past the last output that matters)
+        for (int i = 0; i < kBwdStages - 1; ++i) fetch(i);
+        float hist[K][CH];     // inputs u-(K-1) .. u (zero before the start of u's sequence)
+        float ring[K][CH];     // ring[i] = dpre[u - (K-1) + i]
+        const int s0 = seq_start[t0];
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+#pragma unroll
+            for (int j = 0; j < CH; ++j) hist[i][j] = ring[i][j] = 0.f;
 #pragma unroll
         for (int i = 0; i < K - 1; ++i) {
-            ring_t[i] = ring_t[i + 1];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ring[i][j] = ring[i + 1][j];
+            const int t = t0 - (K - 1) + i;
+            if (t >= 0 && t >= s0) unpack4(*reinterpret_cast<const uint2*>(xc + t * ldx), hist[i]);
         }
-        ring_t[K - 1] = -1;
-        if (u < u_end) {
-            if (seq_start[u] == u)
+        for (int chunk = 0, uc = t0; uc < t1 + K - 1; ++chunk, uc += kBwdChunk) {
+            fetch(chunk + kBwdStages - 1);            // (an empty group past the end) over the slots that the last chunk left
+            asm volatile("cp.async.wait_group %0;" ::"n"(kBwdStages - 1) : "memory");
+#pragma unroll
+            for (int b = 0; b < kBwdChunk; ++b) {
+                const int u = uc + b, t = u - (K - 1);
 #pragma unroll
                 for (int i = 0; i < K - 1; ++i)
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) hist[i][j] = 0.f;
-            unpack8(reinterpret_cast<const Vec8*>(x + u * ldx)[c], hist[K - 1]);
-            float g[8];
-            unpack8(reinterpret_cast<const Vec8*>(dy + (size_t)u * D)[c], g);
-            if (SILU) {
+                    for (int j = 0; j < CH; ++j) ring[i][j] = ring[i + 1][j];
+                if (u < u_end) {
+                    uint2 (*slot)[32] = mine[chunk % kBwdStages * kBwdChunk + b];
+                    if (bounds[warp][0][u - t0] == u)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float pre = 0.f;
+                        for (int i = 0; i < K - 1; ++i)
 #pragma unroll
-                    for (int k = 0; k < K; ++k) pre += wk[k][j] * hist[k][j];
-                    const float sg = 1.f / (1.f + __expf(-pre));
-                    g[j] = g[j] * sg * (1.f + pre * (1.f - sg));
+                            for (int j = 0; j < CH; ++j) hist[i][j] = 0.f;
+                    unpack4(slot[0][lane], hist[K - 1]);
+                    float g[CH];
+                    unpack4(slot[1][lane], g);
+                    if (SILU) {
+#pragma unroll
+                        for (int j = 0; j < CH; ++j) {
+                            float pre = 0.f;
+#pragma unroll
+                            for (int k = 0; k < K; ++k) pre += wk[k][j] * hist[k][j];
+                            const float sg = 1.f / (1.f + __expf(-pre));
+                            g[j] = g[j] * sg * (1.f + pre * (1.f - sg));
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) ring[K - 1][j] = g[j];
+                    if (u < t1)           // weight gradient of the own strip's outputs
+#pragma unroll
+                        for (int k = 0; k < K; ++k)
+#pragma unroll
+                            for (int j = 0; j < CH; ++j) dwacc[k][j] += g[j] * hist[k][j];
+#pragma unroll
+                    for (int i = 0; i < K - 1; ++i)
+#pragma unroll
+                        for (int j = 0; j < CH; ++j) hist[i][j] = hist[i + 1][j];
+                }
+                // input token t has now seen all its outputs t .. t + K - 1 (ring slots 0 .. K-1), as far as its sequence goes
+                if (t >= t0 && t < t1) {
+                    const int e = bounds[warp][1][t - t0];
+                    float acc[CH];
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) acc[j] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < K; ++i)            // slot i holds output t + i, which used x[t] with tap K-1-i
+                        if (t + i < e)
+#pragma unroll
+                            for (int j = 0; j < CH; ++j) acc[j] += wk[K - 1 - i][j] * ring[i][j];
+                    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(acc[0], acc[1]), __floats2bfloat162_rn(acc[2], acc[3])};
+                    *reinterpret_cast<uint2*>(dx + (size_t)t * D + c) = *reinterpret_cast<uint2*>(o);
                 }
             }
-            ring_t[K - 1] = u;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ring[K - 1][j] = g[j];
-            if (u < t1)           // weight gradient of the own strip's outputs
-#pragma unroll
-                for (int k = 0; k < K; ++k)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) dwacc[k][j] += g[j] * hist[k][j];
-#pragma unroll
-            for (int i = 0; i < K - 1; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) hist[i][j] = hist[i + 1][j];
-        }
-        // input token t = u - (K-1) has now seen all its outputs t .. t + K - 1 (ring slots 0 .. K-1)
-        const int t = u - (K - 1);
-        if (t >= t0 && t < t1) {
-            const int e = seq_end[t];
-            float acc[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-#pragma unroll
-            for (int i = 0; i < K; ++i) {          // slot i holds output t + i, which used x[t] with tap K-1-i
-                if (ring_t[i] == t + i && t + i < e)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] += wk[K - 1 - i][j] * ring[i][j];
-            }
-            reinterpret_cast<Vec8*>(dx + (size_t)t * D)[c] = pack8(acc);
         }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    float* sdw = reinterpret_cast<float*>(stage[warp]);
 #pragma unroll
-    for (int k = 0; k < K; ++k)
+    for (int j = 0; j < CH; ++j)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(&dw[(size_t)(c * 8 + j) * K + k], dwacc[k][j]);
+        for (int k = 0; k < K; ++k) sdw[(lane * CH + j) * K + k] = dwacc[k][j];
+    __syncthreads();
+    const int n = min(32 * CH, D - c0) * K;
+    for (int i = threadIdx.x; i < n; i += 32 * kBwdWarps) {
+        float sum = 0.f;
+#pragma unroll
+        for (int r = 0; r < kBwdWarps; ++r) sum += reinterpret_cast<const float*>(stage[r])[i];
+        atomicAdd(&dw[(size_t)c0 * K + i], sum);
+    }
 }
 
 // ---- l2norm over the last dim (D <= 256, one warp per row)
@@ -344,13 +398,13 @@ MM_API int mm_conv1d_fwd(const void* x, long long ldx, const void* w, const int*
 MM_API int mm_conv1d_bwd(const void* x, long long ldx, const void* w, const int* seq_start, const int* seq_end, const void* dy, void* dx,
                          float* dw, int T, int D, int K, int silu, cudaStream_t st) {
     if (D % 8 || ldx % 8 || K > kMaxK || K < 1) return -1;
-    dim3 grid((D / 8 + 127) / 128, (T + kStrip - 1) / kStrip);
+    dim3 grid((D + 127) / 128, (T + kStrip * kBwdWarps - 1) / (kStrip * kBwdWarps));
 #define MM_CONV_BWD(KK)                                                                                                  \
     if (silu)                                                                                                            \
-        conv1d_bwd_kernel<KK, true><<<grid, 128, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, seq_end,           \
+        conv1d_bwd_kernel<KK, true><<<grid, 32 * kBwdWarps, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, seq_end,           \
                                                           (const bf16*)dy, (bf16*)dx, dw, T, D);                         \
     else                                                                                                                 \
-        conv1d_bwd_kernel<KK, false><<<grid, 128, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, seq_end,          \
+        conv1d_bwd_kernel<KK, false><<<grid, 32 * kBwdWarps, 0, st>>>((const bf16*)x, ldx, (const bf16*)w, seq_start, seq_end,          \
                                                            (const bf16*)dy, (bf16*)dx, dw, T, D)
     MM_CONV_K(MM_CONV_BWD)
 #undef MM_CONV_BWD

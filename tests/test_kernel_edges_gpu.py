@@ -337,3 +337,21 @@ def test_convolution_and_gate_on_columns_of_a_wider_matrix(T, D, extra):
             y = ops.gated_rms_norm(o, z, w.view(-1)[:8])
             outs[-1] += [y.detach(), *torch.autograd.grad(y, [z], torch.ones_like(y))]
         assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("lens,D,K,silu", [([1], 8, 1, True), ([100, 27], 136, 8, True), ([31, 1, 0, 97], 264, 2, False), ([129, 2, 169], 72, 5, True),
+                                           ([32] * 5, 128, 4, True)])
+def test_convolution_backward_at_strip_edges(lens, D, K, silu):
+    """Strips of 32 tokens, four a block, 128 channels a warp: short tails, sequences that end at and around the edges, every K."""
+    torch.manual_seed(K)
+    T = sum(lens)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0)
+    x, dy = (torch.randn(T, D, device=DEV).bfloat16() for _ in range(2))
+    w = torch.randn(D, K, device=DEV).bfloat16()
+    leaf, want = [], []
+    for cast, f in ((lambda t: t, ops.causal_conv1d), (lambda t: t.float(), ref.causal_conv1d)):
+        leaf = [cast(t).detach().requires_grad_() for t in (x, w)]
+        y = f(*leaf, None, "silu" if silu else None, cu if cast(x) is x else cu.unique().tolist())     # (the oracle takes no empty sequence)
+        want.append(torch.autograd.grad(y, leaf, cast(dy)))
+    for a, b in zip(*want):
+        _close(a, b, rtol=2 ** -8, atol=1e-5)                     # fp32 sums, one rounding to bf16
