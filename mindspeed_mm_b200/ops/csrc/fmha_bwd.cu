@@ -43,6 +43,7 @@ struct BwdParams {
     int D;                  // head dim of the tensors in global memory (<= HD); shared-memory tiles stay HD wide
     float scale, scale_log2;
     int* status;
+    int heads_first;        // see attention_grid
     int split;              // dK/dV kernel: 1 = one CTA per QUERY head writing partial dk / dv [Tk, Nq, 128]
 };
 
@@ -92,7 +93,7 @@ constexpr int kSmemDq = (2 + kRingK + 2) * kTile + 1024 + 1024;
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
-    if ((int)blockIdx.x >= *p.n_tiles) return;     // whole CTA leaves before any barrier or TMEM allocation
+    if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;     // whole CTA leaves before any barrier or TMEM allocation
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
@@ -115,11 +116,11 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seq = p.tile_seq[blockIdx.x];
-    const int q0 = p.tile_r0[blockIdx.x];
-    const int nseq = p.tile_nseq[blockIdx.x];
+    const int seq = p.tile_seq[tile_of(p.heads_first)];
+    const int q0 = p.tile_r0[tile_of(p.heads_first)];
+    const int nseq = p.tile_nseq[tile_of(p.heads_first)];
     constexpr bool live = true;
-    const int head = blockIdx.y;
+    const int head = head_of(p.heads_first);
     const int kv_head = head / (p.Nq / p.Nkv);
     const int q_begin = p.cu_q[seq], q_len = p.cu_q[seq + nseq] - q_begin;
     const int k_begin = p.cu_k[seq], k_len = p.cu_k[seq + nseq] - k_begin;
@@ -353,7 +354,7 @@ constexpr int kSmemDkv = 2 * kTile + 2 * kRing * kQTile + 2048 + 1024;
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
-    if ((int)blockIdx.x >= *p.n_tiles) return;
+    if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sK = smem;
@@ -374,13 +375,13 @@ fmha_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seq = p.tile_seq[blockIdx.x];
-    const int kv0 = p.tile_r0[blockIdx.x];
+    const int seq = p.tile_seq[tile_of(p.heads_first)];
+    const int kv0 = p.tile_r0[tile_of(p.heads_first)];
     const int Gfull = p.Nq / p.Nkv;
-    const int kv_head = p.split ? blockIdx.y / Gfull : blockIdx.y;
-    const int head0 = p.split ? blockIdx.y : kv_head * Gfull;     // first query head this CTA walks
+    const int kv_head = p.split ? head_of(p.heads_first) / Gfull : head_of(p.heads_first);
+    const int head0 = p.split ? head_of(p.heads_first) : kv_head * Gfull;     // first query head this CTA walks
     const int G = p.split ? 1 : Gfull;                              // ... and how many
-    const int out_heads = p.split ? p.Nq : p.Nkv, out_head = blockIdx.y;
+    const int out_heads = p.split ? p.Nq : p.Nkv, out_head = head_of(p.heads_first);
     const int q_begin = p.cu_q[seq], q_len = p.cu_q[seq + 1] - q_begin;
     const int k_begin = p.cu_k[seq], k_len = p.cu_k[seq + 1] - k_begin;
     const int diag = k_len - q_len;
@@ -640,19 +641,21 @@ MM_API int mm_fmha_bwd(const void* q, const void* k, const void* v, const void* 
     if (cudaFuncSetAttribute(fmha_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDq) != cudaSuccess) return -3;
     if (cudaFuncSetAttribute(fmha_bwd_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDkv) != cudaSuccess) return -3;
     BwdParams p{cu_q, cu_k, q_seq, q_r0, q_nseq, q_n, lse, delta, (bf16*)dq, (bf16*)dk, (bf16*)dv, T, Tk, Nq, Nkv, causal, D, scale,
-                scale * kLog2e, status, split_heads};
+                scale * kLog2e, status, heads_go_first(causal, mq), split_heads};
     BwdParams pk = p;
     pk.tile_seq = k_seq;
     pk.tile_r0 = k_r0;
     pk.tile_nseq = k_nseq;
     pk.n_tiles = k_n;
-    fmha_bwd_dq_kernel<<<dim3(mq, Nq), 320, kSmemDq, st>>>(tQ, tK, tV, tdO, p);
+    pk.heads_first = heads_go_first(causal, mk);
+    const dim3 k_grid = attention_grid(pk.heads_first, mk, split_heads ? Nq : Nkv);
+    fmha_bwd_dq_kernel<<<attention_grid(p.heads_first, mq, Nq), 320, kSmemDq, st>>>(tQ, tK, tV, tdO, p);
     if (variant != 0) {      // dK/dV over 128-row query steps: all four products at N = 128
         if (cudaFuncSetAttribute(fmha_bwd_dkv128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDkv128) != cudaSuccess)
             return -3;
-        fmha_bwd_dkv128_kernel<<<dim3(mk, split_heads ? Nq : Nkv), 320, kSmemDkv128, st>>>(tQ, tK, tV, tdO, pk);
+        fmha_bwd_dkv128_kernel<<<k_grid, 320, kSmemDkv128, st>>>(tQ, tK, tV, tdO, pk);
         return (int)cudaGetLastError();
     }
-    fmha_bwd_dkv_kernel<<<dim3(mk, split_heads ? Nq : Nkv), 320, kSmemDkv, st>>>(tQ64, tK, tV, tdO64, pk);
+    fmha_bwd_dkv_kernel<<<k_grid, 320, kSmemDkv, st>>>(tQ64, tK, tV, tdO64, pk);
     return (int)cudaGetLastError();
 }

@@ -11,9 +11,10 @@
 // tcgen05.mma of S^T and dP^T (both operands in shared memory) and 72 for each of the 16 of dV and dK (A in tensor
 // memory), 3230 of the 3550 clocks of a step.  dQ, dK and dV of 12 heads x 7800 x 7800 x 128 took 1.356 ms; 1.283 ms
 // once the masks had a pass of their own (4150 clocks a step); 1.204 ms with two buffers for the statistics.
-// S^T and dP^T are single-buffered; the tensor pipe is kept busy by the issue order   S_0 dP_0 | dV_i S_{i+1} dK_i dP_{i+1} | ...   in which the product that follows a wait never depends on
-// the row threads' other phase: while they turn S_{i+1} into P_{i+1}, the pipe runs dK_i and dP_{i+1}; while they turn
-// dP_{i+1} into dS_{i+1}, it runs dV_{i+1} and S_{i+2}.
+// S^T and dP^T are single-buffered; the tensor pipe is kept busy by the issue order
+//     S_0 dP_0 | dV_i S_{i+1} dK_i dP_{i+1} | ...
+// in which the product that follows a wait never depends on the row threads' other phase: while they turn S_{i+1} into
+// P_{i+1}, the pipe runs dK_i and dP_{i+1}; while they turn dP_{i+1} into dS_{i+1}, it runs dV_{i+1} and S_{i+2}.
 //
 //   warp 0      TMA: K, V once; Q_i into a 3-deep and dO_i into a 2-deep ring (Q is released by dK_i, dO by dV_i)
 //   warp 1      MMA issuer
@@ -34,7 +35,7 @@ static_assert(kSmemDkv128 <= 227 * 1024, "shared memory of a CTA");
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
-    if ((int)blockIdx.x >= *p.n_tiles) return;
+    if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     constexpr int BQ = 128;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -62,14 +63,14 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seq = p.tile_seq[blockIdx.x];
-    const int kv0 = p.tile_r0[blockIdx.x];
+    const int seq = p.tile_seq[tile_of(p.heads_first)];
+    const int kv0 = p.tile_r0[tile_of(p.heads_first)];
     const int Gfull = p.Nq / p.Nkv;
-    const int kv_head = p.split ? blockIdx.y / Gfull : blockIdx.y;
-    const int head0 = p.split ? blockIdx.y : kv_head * Gfull;
+    const int kv_head = p.split ? head_of(p.heads_first) / Gfull : head_of(p.heads_first);
+    const int head0 = p.split ? head_of(p.heads_first) : kv_head * Gfull;
     const int G = p.split ? 1 : Gfull;
-    const int out_heads = p.split ? p.Nq : p.Nkv, out_head = blockIdx.y;
-    const int nseq = p.tile_nseq[blockIdx.x];          // > 1: consecutive short sequences packed into this tile
+    const int out_heads = p.split ? p.Nq : p.Nkv, out_head = head_of(p.heads_first);
+    const int nseq = p.tile_nseq[tile_of(p.heads_first)];          // > 1: consecutive short sequences packed into this tile
     const int q_begin = p.cu_q[seq], q_len = p.cu_q[seq + nseq] - q_begin;
     const int k_begin = p.cu_k[seq], k_len = p.cu_k[seq + nseq] - k_begin;
     const int diag = k_len - q_len;

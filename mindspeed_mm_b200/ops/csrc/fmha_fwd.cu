@@ -44,6 +44,7 @@ struct FmhaParams {
     int D;              // head dim of the tensors in global memory (<= HD)
     float scale_log2;   // softmax scale * log2(e)
     int* status;
+    int heads_first;    // see attention_grid
 };
 
 // Later query tiles of a causal sequence have more key tiles: emit them first so the tail of the grid is made of short work items.
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(kPlanThreads) fmha_plan_kernel(const int* cu_q
 __global__ void __launch_bounds__(kThreads, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaParams p) {
-    if ((int)blockIdx.x >= *p.n_tiles) return;
+    if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
@@ -79,9 +80,9 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float* l_final = alpha_ring + 2 * 128;                      // [128]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seq = p.tile_seq[blockIdx.x];
-    const int q0 = p.tile_q0[blockIdx.x];
-    const int head = blockIdx.y;
+    const int seq = p.tile_seq[tile_of(p.heads_first)];
+    const int q0 = p.tile_q0[tile_of(p.heads_first)];
+    const int head = head_of(p.heads_first);
     const int kv_head = head / (p.Nq / p.Nkv);
     const int q_begin = p.cu_q[seq], q_len = p.cu_q[seq + 1] - q_begin;
     const int k_begin = p.cu_k[seq], k_len = p.cu_k[seq + 1] - k_begin;
@@ -360,8 +361,8 @@ MM_API int mm_fmha_fwd(const void* q, const void* k, const void* v, void* o, flo
         done = true;
     }
     FmhaParams p{cu_q, cu_k, tile_seq, tile_q0, n_tiles, tile_nseq, (const bf16*)q, q_ts, (bf16*)o, lse, T, Nq, Nkv, causal, D,
-                 scale * 1.4426950408889634f, status};
-    dim3 grid(max_tiles, Nq);
+                 scale * 1.4426950408889634f, status, heads_go_first(causal, max_tiles)};
+    const dim3 grid = attention_grid(p.heads_first, max_tiles, Nq);
     // Long key sequences take the alternating groups: a key tile costs them 1650 clocks against 2440, but a CTA's set-up and end
     // (12 warps, a second hand-over of the row sums) more.  Keys per sequence on average, split / alternating, 8192 tokens:
     // 16 heads of 80: 512 keys 119.5 / 121.8 us, 1024 152 / 145, 2048 218 / 190, 1 x 4096 208 / 165; 12 heads of 128: 1024 158 / 157,

@@ -29,7 +29,7 @@ constexpr int kAltSmem = (kAltK + kAltV) * kTileBytes + 256 + 4 * 128 * 4 + 1024
 
 __global__ void __launch_bounds__(kAltThreads, 1)
 fmha_fwd_alt_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, FmhaParams p) {
-    if ((int)blockIdx.x >= *p.n_tiles) return;
+    if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sK = smem;
@@ -50,8 +50,8 @@ fmha_fwd_alt_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     float* l_part = m_ref + 2 * 128;                                                      // [group][128]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seq = p.tile_seq[blockIdx.x], q0 = p.tile_q0[blockIdx.x], nseq = p.tile_nseq[blockIdx.x];
-    const int head = blockIdx.y, kv_head = head / (p.Nq / p.Nkv);
+    const int seq = p.tile_seq[tile_of(p.heads_first)], q0 = p.tile_q0[tile_of(p.heads_first)], nseq = p.tile_nseq[tile_of(p.heads_first)];
+    const int head = head_of(p.heads_first), kv_head = head / (p.Nq / p.Nkv);
     const int q_begin = p.cu_q[seq], q_len = p.cu_q[seq + nseq] - q_begin;
     const int k_begin = p.cu_k[seq], k_len = p.cu_k[seq + nseq] - k_begin;
     const int diag = k_len - q_len;                      // causal: key j visible to query i iff j <= i + diag
