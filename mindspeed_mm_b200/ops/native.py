@@ -1139,7 +1139,7 @@ class _GatedRMSNorm(torch.autograd.Function):
         rows = x2.shape[0]
         # z of [tokens, heads, D] with dense heads may have its tokens apart (the gate's columns of a fused projection)
         if z.dim() == 3 and z.stride(2) == 1 and z.stride(1) == D and z.stride(0) % 8 == 0 and z.data_ptr() % 16 == 0 and rows < 2 ** 31:
-            z2, zh, ldz = z, z.shape[1], z.stride(0)
+            z2, zh, ldz = z, max(1, z.shape[1]), z.stride(0)
         else:
             z2, zh, ldz = z.reshape(-1, D).contiguous(), 1, D
         y = torch.empty(rows, D, dtype=torch.bfloat16, device=x.device)

@@ -355,3 +355,12 @@ def test_convolution_backward_at_strip_edges(lens, D, K, silu):
         want.append(torch.autograd.grad(y, leaf, cast(dy)))
     for a, b in zip(*want):
         _close(a, b, rtol=2 ** -8, atol=1e-5)                     # fp32 sums, one rounding to bf16
+
+
+@pytest.mark.parametrize("T,h", [(0, 4), (5, 0), (0, 0)])
+def test_gate_without_rows(T, h):
+    """No tokens or no heads: nothing to do, forward and backward."""
+    x, z = (torch.randn(T, h, 64, device=DEV).bfloat16().requires_grad_() for _ in range(2))
+    y = ops.gated_rms_norm(x, z, torch.ones(64, device=DEV).bfloat16())
+    dx, dz = torch.autograd.grad(y, [x, z], torch.ones_like(y))
+    assert y.shape == dx.shape == dz.shape == (T, h, 64)
