@@ -149,8 +149,7 @@ def rope_interleaved(x, cos, sin):
 
 def mrope_tables(position_ids, head_dim: int, theta: float, mrope_section, dtype):
     """Multimodal rotary tables (cos, sin), [T, head_dim] in ``dtype``, from positions [3, T] (see ``reference.mrope_cos_sin``)."""
-    if _native(position_ids) and dtype == torch.bfloat16 and position_ids.dtype == torch.int64 and tuple(position_ids.shape[:1]) == (3,) \
-            and position_ids.dim() == 2 and position_ids.shape[1] > 0 and head_dim % 2 == 0 and len(mrope_section) == 3:
+    if _native(position_ids) and _nat().mrope_tables_supported(position_ids, head_dim, mrope_section, dtype):
         return _nat().mrope_tables(position_ids, head_dim, theta, mrope_section)
     cos, sin = ref.mrope_cos_sin(position_ids, head_dim, theta, mrope_section)
     return cos.to(dtype), sin.to(dtype)
@@ -236,8 +235,7 @@ def linear_swiglu(x, weight_gate_up):
     """``swiglu(x @ W_gate_up.T)``.  On the native tier a pass that keeps no graph (the first forward of a recomputed
     unit, inference) runs one kernel with the activation as the GEMM epilogue; a pass that will be differentiated keeps
     the pre-activation for the backward and runs GEMM and activation kernels."""
-    if _native(x) and x.dtype == torch.bfloat16 and \
-            not (torch.is_grad_enabled() and (x.requires_grad or weight_gate_up.requires_grad)) and \
+    if _native(x) and x.dtype == torch.bfloat16 and _nat()._keeps_no_graph((x, weight_gate_up)) and \
             _nat().gemm_swiglu_supported(x, weight_gate_up):
         return _nat().gemm_swiglu(x, weight_gate_up)
     return swiglu(linear(x, weight_gate_up))
@@ -286,7 +284,7 @@ def attention_cached(q, k, v, cache: dict, cos=None, sin=None):
     are None: then both come rotated) and values to ``cache["k"]`` / ``cache["v"]`` and attends to all of them, causal and
     aligned to the end.  q [T, Nq, D], k / v [T, Nkv, D].  A few tokens (a decoding step) take one kernel."""
     k_old, v_old = cache.get("k"), cache.get("v")
-    if _native(q) and _nat().decode_attention_supported(q, k, v, k_old, v_old, cos):
+    if _native(q) and _nat().decode_attention_supported(q, k, v, k_old, v_old, cos, sin):
         o, cache["k"], cache["v"] = _nat().decode_attention(q, k, v, k_old, v_old, cos, sin)
         return o
     if cos is not None:

@@ -556,6 +556,12 @@ def gemm_swiglu(x, w):
 
 
 # --------------------------------------------------------------------------- generation (csrc/decode.cu)
+# These kernels are called outside of an autograd function, so each rule below asks for a call that keeps no graph.
+def mrope_tables_supported(position_ids, head_dim, section, dtype) -> bool:
+    return (dtype == torch.bfloat16 and position_ids.dtype == torch.int64 and position_ids.dim() == 2 and position_ids.shape[0] == 3
+            and position_ids.shape[1] > 0 and head_dim % 2 == 0 and len(section) == 3 and _keeps_no_graph((position_ids,)))
+
+
 def mrope_tables(position_ids, head_dim, theta, section):
     """bf16 rotary tables [T, head_dim] of int64 positions [3, T], computed in 64 bits by one kernel."""
     pos = position_ids.contiguous()
@@ -568,9 +574,9 @@ def mrope_tables(position_ids, head_dim, theta, section):
 
 def skinny_supported(x, *tensors) -> bool:
     """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies."""
-    return (x.dim() == 2 and 1 <= x.shape[0] <= 4 and x.shape[1] % 8 == 0 and x.numel() <= 80 * 1024 and _ok2d(x)
-            and all(t is None or (t.dtype == torch.bfloat16 and t.device == x.device) for t in tensors)
-            and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x,) + tensors)))
+    return (_keeps_no_graph((x,) + tensors) and x.dim() == 2 and 1 <= x.shape[0] <= 4 and x.shape[1] % 8 == 0
+            and x.numel() <= 80 * 1024 and _ok2d(x)
+            and all(t is None or (t.dtype == torch.bfloat16 and t.device == x.device) for t in tensors))
 
 
 def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=False):
@@ -595,15 +601,15 @@ def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=Fal
     return out
 
 
-def decode_attention_supported(q, k, v, k_old, v_old, cos) -> bool:
+def decode_attention_supported(q, k, v, k_old, v_old, cos, sin=None) -> bool:
     """Head dim 128, the new tokens' query heads of a group fill at most one 16-row tile, nothing keeps a graph."""
     ts = [t for t in (q, k, v, k_old, v_old) if t is not None]
     T, Nq, D = q.shape
-    return (os.environ.get("MM_B200_FMHA", "1") == "1" and D == 128 and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts)
+    return (_keeps_no_graph(ts + [cos, sin]) and os.environ.get("MM_B200_FMHA", "1") == "1" and D == 128
+            and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts)
             and all(t.shape[1:] == k.shape[1:] and t.shape[2] == D for t in (v, k_old, v_old) if t is not None)
             and k.shape[2] == D and k.shape[0] == v.shape[0] == T and (k_old is None or k_old.shape[0] == v_old.shape[0])
-            and T >= 1 and Nq % k.shape[1] == 0 and T * (Nq // k.shape[1]) <= 16 and (cos is None or tuple(cos.shape) == (T, D))
-            and not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)))
+            and T >= 1 and Nq % k.shape[1] == 0 and T * (Nq // k.shape[1]) <= 16 and (cos is None or tuple(cos.shape) == (T, D)))
 
 
 def decode_attention(q, k, v, k_old, v_old, cos, sin):
@@ -897,19 +903,29 @@ def moe_supported(tokens, gate_up, down) -> bool:
             and gate_up.shape[-1] % 256 == 0 and down.shape[-1] % 128 == 0)
 
 
+class _Route(torch.autograd.Function):
+    """Routing kernels as an autograd function, so that a tracer records them (there is nothing to differentiate)."""
+
+    @staticmethod
+    def forward(ctx, topk_ids, num_experts):
+        T, k = topk_ids.shape
+        dev, n = topk_ids.device, T * k
+        ids = topk_ids.to(torch.int64).contiguous()
+        R = (n + num_experts * 127 + 127) // 128 * 128            # static upper bound of off[E]
+        off = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
+        scratch = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)       # counts, out-of-range flag
+        row_of_pair = torch.zeros(n, dtype=torch.int32, device=dev)
+        src_of_row = torch.empty(R, dtype=torch.int32, device=dev)
+        _check(lib().mm_moe_route(ids.data_ptr(), n, k, num_experts, R, scratch.data_ptr(), off.data_ptr(), row_of_pair.data_ptr(),
+                                  src_of_row.data_ptr(), scratch[num_experts:].data_ptr(), _st()), "moe_route")
+        return off, row_of_pair, src_of_row, scratch
+
+
 def _route(topk_ids, num_experts: int):
     """Launches the routing kernels; returns (off, row_of_pair, src_of_row, R, check).  ``check()`` waits for them (not for
     work queued behind them) and raises if an expert number was out of range."""
-    T, k = topk_ids.shape
-    dev, n = topk_ids.device, T * k
-    ids = topk_ids.to(torch.int64).contiguous()
-    R = (n + num_experts * 127 + 127) // 128 * 128            # static upper bound of off[E]
-    off = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
-    scratch = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)       # counts, out-of-range flag
-    row_of_pair = torch.zeros(n, dtype=torch.int32, device=dev)
-    src_of_row = torch.empty(R, dtype=torch.int32, device=dev)
-    _check(lib().mm_moe_route(ids.data_ptr(), n, k, num_experts, R, scratch.data_ptr(), off.data_ptr(), row_of_pair.data_ptr(),
-                              src_of_row.data_ptr(), scratch[num_experts:].data_ptr(), _st()), "moe_route")
+    off, row_of_pair, src_of_row, scratch = _run(_Route, topk_ids, int(num_experts))
+    R = src_of_row.shape[0]
     bad = torch.empty(1, dtype=torch.int32, pin_memory=True)
     bad.copy_(scratch[num_experts:], non_blocking=True)
     done = torch.cuda.Event()

@@ -364,3 +364,25 @@ def test_gate_without_rows(T, h):
     y = ops.gated_rms_norm(x, z, torch.ones(64, device=DEV).bfloat16())
     dx, dz = torch.autograd.grad(y, [x, z], torch.ones_like(y))
     assert y.shape == dx.shape == dz.shape == (T, h, 64)
+
+
+@pytest.mark.parametrize("name", ["product", "attention", "tables", "experts", "swiglu"])
+def test_a_recorded_trace_computes_again(name):
+    """A trace of a call that keeps no graph runs the kernels on the inputs of its replay."""
+    bf = lambda *s: torch.randn(*s, device=DEV).bfloat16()  # noqa: E731
+    w, g, gate_up, down, tab, probs = bf(64, 256), bf(256), bf(4, 256, 512) / 16, bf(4, 256, 256) / 16, bf(1, 128), torch.rand(64, 2, device=DEV).bfloat16()
+    f, make = {"product": (lambda x: ops.norm_linear(x, g, 1e-6, w), lambda: (bf(2, 256),)),
+               "attention": (lambda q, k, v: ops.attention_cached(q, k, v, {}, tab, tab), lambda: (bf(1, 4, 128), bf(1, 2, 128), bf(1, 2, 128))),
+               "tables": (lambda p: ops.mrope_tables(p, 128, 1e6, (16, 24, 24), torch.bfloat16)[0], lambda: (torch.randint(0, 99, (3, 7), device=DEV),)),
+               "experts": (lambda x, i: native.moe_experts(x, i, probs, gate_up, down), lambda: (bf(64, 256), torch.randint(0, 4, (64, 2), device=DEV))),
+               "swiglu": (lambda x: ops.linear_swiglu(x, gate_up[0]), lambda: (bf(8, 512),))}[name]
+    with torch.no_grad():
+        m, args = torch.jit.trace(f, make(), check_trace=False), make()
+        # the tables' general path computes its angles in 32 bits
+        _close(m(*args), f(*args), rtol=8e-3, atol=4e-3)
+
+
+def test_forward_mode_is_refused_where_no_rule_for_it_exists():
+    with torch.autograd.forward_ad.dual_level(), pytest.raises(NotImplementedError):
+        x = torch.autograd.forward_ad.make_dual(torch.randn(1, 256, device=DEV).bfloat16(), torch.randn(1, 256, device=DEV).bfloat16())
+        ops.norm_linear(x, torch.ones(256, device=DEV).bfloat16(), 1e-6, torch.randn(64, 256, device=DEV).bfloat16())

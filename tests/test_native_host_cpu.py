@@ -1,4 +1,5 @@
 """Host side of the native ops: when an op may skip its autograd function."""
+import pytest
 import torch
 import torch.autograd.forward_ad as fwad
 
@@ -31,3 +32,30 @@ def test_only_calls_without_graph_transform_or_tracer_skip_the_autograd_function
     y = native._run(_Double, p, 2)
     assert torch.equal(torch.autograd.grad(y.sum(), p)[0], torch.full((3,), 2.0))
     assert torch.equal(native._run(_Double, x, 2), x * 2) and not native._run(_Double, x, 2).requires_grad
+
+
+def _rules():
+    """The rules of the kernels that are called without an autograd function, each on a call that it takes."""
+    bf = lambda *s: torch.randn(*s).bfloat16()  # noqa: E731
+    x, w, q, kv, old, tab = bf(2, 256), bf(64, 256), bf(1, 4, 128), bf(1, 2, 128), bf(9, 2, 128), bf(1, 128)
+    return {"product": (lambda t: native.skinny_supported(t, w, None), x),
+            "product, norm weight": (lambda t: native.skinny_supported(x, t, w), bf(256)),
+            "cached attention": (lambda t: native.decode_attention_supported(t, kv, kv, old, old, tab, tab), q),
+            "cached attention, tables": (lambda t: native.decode_attention_supported(q, kv, kv, old, old, tab, t), tab),
+            "rotary tables": (lambda t: native.mrope_tables_supported(t, 128, (16, 24, 24), torch.bfloat16), torch.arange(21).view(3, 7))}
+
+
+@pytest.mark.parametrize("name", list(_rules()))
+def test_kernels_called_without_an_autograd_function_ask_for_a_plain_call(name):
+    rule, t = _rules()[name]
+    assert rule(t)
+    seen = []
+    torch.func.vmap(lambda u: seen.append(rule(u)) or u)(torch.stack([t, t]))
+    torch.jit.trace(lambda u: seen.append(rule(u)) or u + 0, (t,), check_trace=False)
+    if t.is_floating_point():
+        with fwad.dual_level():
+            seen.append(rule(fwad.make_dual(t, t.clone())))
+        seen.append(rule(t.clone().requires_grad_()))
+        with torch.no_grad():
+            assert rule(t.clone().requires_grad_())
+    assert len(seen) >= 2 and not any(seen)
