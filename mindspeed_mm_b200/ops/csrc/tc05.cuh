@@ -87,13 +87,16 @@ __device__ __forceinline__ void packed_row_range(const int* cu, int first, int n
 //   pack: sequences in their order; one of at least `rows` rows is cut into tiles, a shorter one shares its tile with as many
 //         following ones as fit (the greedy walk is serial in the tiles; all threads look for the ends).
 //   else: tiles of all sequences by their position t in the sequence, `descending` from the last one (causal attention: the tiles
-//         with most work first); a tile's place is the number of tiles in front of it, counted over the sequences by a warp
-//         per sequence, so nothing is serial in the number of tiles.
-// (One thread with the offsets in global memory took 20 us for 128 windows and 8 us for four sequences of 2048; now 9 and 2.5.)
-constexpr int kPlanThreads = 256, kPlanCache = 4096;
+//         with most work first).  Position by position, the block keeps the sequences that reach it and ranks them by ballot, which is
+//         linear in the tiles; once kPlanFew sequences or fewer are left, their tiles find their places independently of one another.
+// Offsets that reach past the tensors make more tiles than the list holds; none is listed then.
+// Forward / backward in us, causal, 2 heads of 64: one thread with the offsets in global memory; every tile counting the tiles of all
+// sequences; this.  4 x 2048: 42 / 148, 37 / 126, 37 / 121.  512 x 16: 85 / 181, 697 / 1769, 59 / 112.  4096 x 2: 608 / 1273,
+// 41030 / 105651, 321 / 642.  128 windows of 64 without a mask: 42 / 113 with one thread, 31 / 100 now.
+constexpr int kPlanThreads = 256, kPlanWarps = kPlanThreads / 32, kPlanCache = 4096, kPlanFew = 32;
 __device__ __forceinline__ void plan_tiles(const int* cu, int n_seqs, int* tile_seq, int* tile_r0, int* n_tiles, int* tile_nseq,
                                            int max_tiles, int rows, bool descending, bool pack) {
-    __shared__ int cached[kPlanCache + 1];
+    __shared__ int cached[kPlanCache + 1], list[kPlanCache];
     const bool fits = n_seqs <= kPlanCache;
     if (fits)
         for (int i = threadIdx.x; i <= n_seqs; i += kPlanThreads) cached[i] = cu[i];
@@ -102,19 +105,18 @@ __device__ __forceinline__ void plan_tiles(const int* cu, int n_seqs, int* tile_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (pack) {
         // where a tile that starts at sequence b ends, for every b; the walk from end to end is then a read per tile
-        __shared__ int ends[kPlanCache];
         auto end_of = [&](int b) {
             int e = b + 1;
             while (e < n_seqs && off[e + 1] - off[b] <= rows) ++e;
             return e;
         };
         if (fits)
-            for (int b = threadIdx.x; b < n_seqs; b += kPlanThreads) ends[b] = end_of(b);
+            for (int b = threadIdx.x; b < n_seqs; b += kPlanThreads) list[b] = end_of(b);
         __syncthreads();
         if (warp) return;
         int n = 0;
         for (int b = 0; b < n_seqs && n < max_tiles;) {
-            const int len = off[b + 1] - off[b], end = fits ? ends[b] : end_of(b);
+            const int len = off[b + 1] - off[b], end = fits ? list[b] : end_of(b);
             if (len >= rows) {
                 const int cut = min((len + rows - 1) / rows, max_tiles - n);
                 for (int t = lane; t < cut; t += 32) {
@@ -137,27 +139,63 @@ __device__ __forceinline__ void plan_tiles(const int* cu, int n_seqs, int* tile_
         if (lane == 0) *n_tiles = n;
         return;
     }
-    auto tiles = [&](int b) { return (off[b + 1] - off[b] + rows - 1) / rows; };
-    for (int b = warp; b < n_seqs; b += kPlanThreads / 32) {
-        const int mine = tiles(b);
-        for (int t = lane; t < mine; t += 32) {
-            int place = 0;
-            for (int o = 0; o < n_seqs; ++o) {
-                const int n = tiles(o);
-                place += descending ? max(0, n - t - 1) : min(n, t);
-                place += o < b && n > t;
+    __shared__ int warp_count[kPlanWarps], few_seq[kPlanFew], few_tiles[kPlanFew];
+    __shared__ unsigned long long sum;
+    auto tiles = [&](int b) { return max(0, (off[b + 1] - off[b] + rows - 1) / rows); };
+    if (threadIdx.x == 0) sum = 0;
+    __syncthreads();
+    unsigned long long mine = 0;
+    for (int b = threadIdx.x; b < n_seqs; b += kPlanThreads) mine += tiles(b);
+    if (mine) atomicAdd(&sum, mine);
+    __syncthreads();
+    const int total = sum <= (unsigned long long)max_tiles ? (int)sum : 0;
+    if (threadIdx.x == 0) *n_tiles = total;
+    if (!total) return;
+    auto place = [&](int k) { return descending ? total - 1 - k : k; };      // of the k-th tile by rising position
+    auto put = [&](int k, int b, int t) {
+        const int at = place(k);
+        tile_seq[at] = b;
+        tile_r0[at] = t * rows;
+        tile_nseq[at] = 1;
+    };
+    // count: sequences with more than t - 1 tiles, in `list` or, where that is too short, in the tile list at position t - 1
+    int t = 0, count = n_seqs, k0 = 0, before_k0 = 0;
+    auto candidate = [&](int i) { return t == 0 ? i : fits ? list[i] : tile_seq[place(before_k0 + i)]; };
+    while (count > kPlanFew) {
+        int kept = 0;
+        for (int i0 = 0; i0 < count; i0 += kPlanThreads) {
+            const int i = i0 + threadIdx.x, b = i < count ? candidate(i) : 0;
+            const bool keep = i < count && tiles(b) > t;
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) warp_count[warp] = __popc(m);
+            __syncthreads();                         // the candidates of this stretch are read, too: `list` is compacted in place
+            int rank = kept + __popc(m & ((1u << lane) - 1));
+            for (int w = 0; w < kPlanWarps; ++w) {
+                if (w < warp) rank += warp_count[w];
+                kept += warp_count[w];
             }
-            if (place >= max_tiles) continue;
-            tile_seq[place] = b;
-            tile_r0[place] = t * rows;
-            tile_nseq[place] = 1;
+            if (keep) {
+                if (fits) list[rank] = b;
+                put(k0 + rank, b, t);
+            }
+            __syncthreads();
         }
+        before_k0 = k0;
+        k0 += kept;
+        count = kept;
+        ++t;
     }
-    if (threadIdx.x == 0) {
-        int n = 0;
-        for (int b = 0; b < n_seqs; ++b) n += tiles(b);
-        *n_tiles = min(n, max_tiles);
+    if (threadIdx.x < count) {
+        few_seq[threadIdx.x] = candidate(threadIdx.x);
+        few_tiles[threadIdx.x] = tiles(few_seq[threadIdx.x]);
     }
+    __syncthreads();
+    for (int i = warp; i < count; i += kPlanWarps)
+        for (int pos = t + lane; pos < few_tiles[i]; pos += 32) {
+            int k = k0;
+            for (int o = 0; o < count; ++o) k += max(0, min(few_tiles[o], pos) - t) + (o < i && few_tiles[o] > pos);
+            put(k, few_seq[i], pos);
+        }
 }
 
 // Grid of an attention kernel and a block's place in it.  Causal tiles cost what they see and stand in their list from long to short:

@@ -386,3 +386,37 @@ def test_forward_mode_is_refused_where_no_rule_for_it_exists():
     with torch.autograd.forward_ad.dual_level(), pytest.raises(NotImplementedError):
         x = torch.autograd.forward_ad.make_dual(torch.randn(1, 256, device=DEV).bfloat16(), torch.randn(1, 256, device=DEV).bfloat16())
         ops.norm_linear(x, torch.ones(256, device=DEV).bfloat16(), 1e-6, torch.randn(64, 256, device=DEV).bfloat16())
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 257, 4096, 4097])
+@pytest.mark.parametrize("longest", [1, 300, 2000])
+def test_tile_lists_name_every_tile_once_longest_first(n, longest):
+    """The list as the planner writes it: one to all positions kept by ballot, both places where the sequences left are kept."""
+    g = torch.Generator().manual_seed(n + longest)
+    lens = torch.randint(0, longest + 1, (n,), generator=g) * (torch.rand(n, generator=g) < 0.7)
+    if longest == 2000 and n > 300:
+        lens[60:] = lens[60:] % 130                                          # a few long ones among many short ones
+    lens[0] = longest
+    T, cu = int(lens.sum()), torch.nn.functional.pad(lens.cumsum(0), (1, 0)).to(torch.int32).to(DEV)
+    L, q = native.lib(), torch.randn(T, 1, 8, device=DEV).bfloat16()
+    most = L.mm_fmha_max_tiles(T, n)
+    plan, o, lse = torch.full((3 * most + 1,), -1, dtype=torch.int32, device=DEV), torch.empty_like(q), torch.empty(1, T, device=DEV)
+    assert L.mm_fmha_fwd(q.data_ptr(), q.data_ptr(), q.data_ptr(), o.data_ptr(), lse.data_ptr(), cu.data_ptr(), cu.data_ptr(), plan.data_ptr(), T, T, n, 1, 1,
+                         8, 8, 8, 8, 1, 1.0, native.status_word(q.device).data_ptr(), native._st()) == 0
+    native.check_status()
+    count = int(plan[2 * most])
+    seq, row = plan[:count].tolist(), plan[most:most + count].tolist()
+    assert sorted(zip(seq, row)) == [(b, r) for b, l in enumerate(lens.tolist()) for r in range(0, l, 128)]
+    assert row == sorted(row, reverse=True) and set(plan[2 * most + 1:2 * most + 1 + count].tolist()) == {1}
+
+
+def test_planning_many_short_sequences_takes_no_longer_than_their_attention_by_orders():
+    """4096 causal sequences of 2: 0.6 ms on one thread, 41 ms where each tile counted the tiles of every sequence."""
+    q, cu = torch.randn(8192, 2, 64, device=DEV).bfloat16(), torch.arange(0, 8193, 2, dtype=torch.int32, device=DEV)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    native.fmha_forward(q, q, q, cu, cu, True, 0.125)
+    a.record()
+    native.fmha_forward(q, q, q, cu, cu, True, 0.125)
+    b.record()
+    torch.cuda.synchronize()
+    assert a.elapsed_time(b) < 5
