@@ -262,7 +262,8 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int j = 0; j < n_kv; ++j) {
             const int st = j & 1;
             const uint32_t ph = (j >> 1) & 1;
-            if (!mbar_wait(&s_full[st], ph, abort_flag) || !mbar_wait(dp_full, j & 1, abort_flag)) { ok = false; break; }
+            // (the votes keep the warp together: what follows are whole-warp instructions, also when a wait gives up in some lanes only)
+            if (!__all_sync(0xffffffffu, mbar_wait(&s_full[st], ph, abort_flag) && mbar_wait(dp_full, j & 1, abort_flag))) { ok = false; break; }
             fence_after_sync();
             uint32_t r[64], d[64];
             const uint32_t t_row = tS + st * 128 + half * 64 + lane_off;
@@ -307,7 +308,8 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (lane == 0) mbar_arrive(ds_full);
         }
         bf16* dst = p.dq + ((size_t)(q_begin + qi) * p.Nq + head) * p.D + half * 64;
-        if (ok && n_kv > 0 && mbar_wait(dq_full, 0, abort_flag)) {
+        if (ok && n_kv > 0) ok = __all_sync(0xffffffffu, mbar_wait(dq_full, 0, abort_flag));
+        if (ok && n_kv > 0) {
             fence_after_sync();
 #pragma unroll
             for (int c = 0; c < 2; ++c) {

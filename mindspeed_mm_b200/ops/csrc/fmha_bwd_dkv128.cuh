@@ -215,7 +215,8 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             float4 ls[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) ls[i] = reinterpret_cast<const float4*>(s_stat + (it & 1) * 2 * BQ + half * 64)[i];
-            if (ok && !mbar_wait(s_full, par, abort_flag)) ok = false;
+            // (the votes keep the warp together: what follows are whole-warp instructions, also when a wait gives up in some lanes only)
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(s_full, par, abort_flag));
             if (!ok) continue;
             fence_after_sync();
             uint32_t s[64];
@@ -254,7 +255,7 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(p_full);
             }
-            if (!mbar_wait(dp_full, par, abort_flag)) { ok = false; continue; }
+            if (!__all_sync(0xffffffffu, mbar_wait(dp_full, par, abort_flag))) { ok = false; continue; }
             fence_after_sync();
             {
                 uint32_t d[64];
@@ -279,7 +280,8 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         bf16* dvp = p.dv + ((size_t)(k_begin + kj) * out_heads + out_head) * p.D + half * 64;
         bf16* dkp = p.dk + ((size_t)(k_begin + kj) * out_heads + out_head) * p.D + half * 64;
-        if (ok && n_it > 0 && mbar_wait(acc_full, 0, abort_flag)) {
+        if (ok && n_it > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag));
+        if (ok && n_it > 0) {
             fence_after_sync();
 #pragma unroll
             for (int c = 0; c < 2; ++c) {

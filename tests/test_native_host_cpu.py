@@ -1,4 +1,6 @@
 """Host side of the native ops: when an op may skip its autograd function."""
+import os
+
 import pytest
 import torch
 import torch.autograd.forward_ad as fwad
@@ -59,3 +61,15 @@ def test_kernels_called_without_an_autograd_function_ask_for_a_plain_call(name):
         with torch.no_grad():
             assert rule(t.clone().requires_grad_())
     assert len(seen) >= 2 and not any(seen)
+
+
+@pytest.mark.parametrize("name,role", [("fmha_bwd.cu", "// two warpgroups of 128 threads: both own all 128 query rows"),
+                                       ("fmha_bwd_dkv128.cuh", "- row threads (warps 2..9)"), ("fmha_fwd_alt.cuh", "- softmax (warps 4..11)")])
+def test_waits_in_front_of_whole_warp_instructions_are_voted(name, role):
+    """A bounded wait may give up in some lanes of a warp only; these threads then run __syncwarp, votes and tensor-memory accesses
+    of the whole warp, so every one of their waits has to be decided by the warp.  Read off the source: the waits cannot be made to fail."""
+    with open(os.path.join(os.path.dirname(native.__file__), "csrc", name)) as f:
+        text = f.read()
+    begin = text.index(role)
+    waits = [ln for ln in text[begin:text.index("atomicExch(p.status, MM_TIMEOUT_EPI)", begin)].splitlines() if "mbar_wait(" in ln]
+    assert len(waits) >= 2 and all("__all_sync(0xffffffffu, mbar_wait(" in ln for ln in waits)
