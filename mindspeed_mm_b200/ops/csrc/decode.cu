@@ -61,6 +61,7 @@ struct GemvParams {
 };
 
 constexpr int kGemvWarps = 4, kGemvU = 2;
+constexpr int kGemvStatic = 72 * 4;                                  // static shared memory of gemv_kernel; counts towards the 48 KB
 
 __device__ __forceinline__ void copy_async(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
@@ -74,7 +75,7 @@ template <int M, bool SWIGLU, bool NORM>
 __global__ void __launch_bounds__(kGemvWarps * 32, M == 1 ? 8 : 4) gemv_kernel(GemvParams p) {
     extern __shared__ __align__(16) uint8_t gemv_smem[];
     bf16* xs = reinterpret_cast<bf16*>(gemv_smem);                  // [M][K]
-    __shared__ float red[72];
+    __shared__ float red[kGemvStatic / 4];
     const int lane = threadIdx.x & 31, nvec = p.K >> 3;
     const int unit = blockIdx.x * kGemvWarps + (threadIdx.x >> 5), units = SWIGLU ? p.N : p.N >> 1;
     const bool active = unit < units;
@@ -368,7 +369,7 @@ int run_gemv(const GemvParams& p, cudaStream_t st) {
     }
     auto kern = gemv_kernel<M, SWIGLU, NORM>;
     const size_t smem = (size_t)(M + NORM) * p.K * 2;
-    if (smem > 48 * 1024) {
+    if (smem + kGemvStatic > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
         if (e != cudaSuccess) return (int)e;
     }

@@ -90,6 +90,18 @@ def test_product_of_a_few_rows(M, N, K, norm, ends):
     _close(got, want, rtol=8e-3, atol=4e-3)
 
 
+@pytest.mark.parametrize("M,K", [(1, 12208), (1, 12216), (1, 12288), (1, 12296), (2, 8144), (2, 8192), (2, 8200), (3, 6144), (4, 4912), (1, 57344), (2, 38224)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_normalised_rows_around_the_shared_memory_limits(M, K, swiglu):
+    """x and the norm's weight in shared memory: up to, at and beyond the 48 KB that need no opt-in, and the most a block can have."""
+    torch.manual_seed(K)
+    x, g, w = torch.randn(M, K, device=DEV).bfloat16(), (1 + 0.1 * torch.randn(K, device=DEV)).bfloat16(), torch.randn(256, K, device=DEV).bfloat16() / K ** 0.5
+    want = ref.rms_norm(x, g, 1e-6).float() @ w.float().t()
+    with torch.no_grad():
+        got = ops.norm_linear_swiglu(x, g, 1e-6, w) if swiglu else ops.norm_linear(x, g, 1e-6, w)
+    _close(got, ref.swiglu(want) if swiglu else want, rtol=8e-3, atol=4e-3)
+
+
 def test_product_of_a_few_rows_keeps_infinities_and_nan_to_their_outputs():
     x, w = torch.zeros(1, 272, device=DEV).bfloat16(), torch.ones(16, 272, device=DEV).bfloat16()
     x[0, -1], w[3, 5], w[4, 271] = float("inf"), float("nan"), -1
