@@ -302,7 +302,7 @@ def attention_cached(q, k, v, cache: dict, cos=None, sin=None):
 # --------------------------------------------------------------------------- generation: products of a few rows
 def norm_linear(x, norm_weight, eps, weight, bias=None):
     """``linear(rms_norm(x), weight, bias)``; a few rows that keep no graph take one kernel."""
-    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_supported(x, weight) and _nat().skinny_supported(x, norm_weight, weight, bias):
+    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_supported(x, weight) and _nat().skinny_supported(x, weight, bias, norm=norm_weight):
         return _nat().skinny_linear(x, weight, bias, norm_weight, eps)
     return linear(rms_norm(x, norm_weight, eps), weight, bias)
 
@@ -310,7 +310,7 @@ def norm_linear(x, norm_weight, eps, weight, bias=None):
 def norm_linear_swiglu(x, norm_weight, eps, weight_gate_up):
     """``linear_swiglu(rms_norm(x), weight_gate_up)``; a few rows that keep no graph take one kernel."""
     if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_swiglu_supported(x, weight_gate_up) and \
-            _nat().skinny_supported(x, norm_weight, weight_gate_up):
+            _nat().skinny_supported(x, weight_gate_up, norm=norm_weight):
         return _nat().skinny_linear(x, weight_gate_up, None, norm_weight, eps, swiglu=True)
     return linear_swiglu(rms_norm(x, norm_weight, eps), weight_gate_up)
 

@@ -707,7 +707,8 @@ __global__ void __launch_bounds__(kDecWarps * 32, 1) decode_attention_kernel(Dec
 
 // out[M, N] = swiglu?(norm?(x) @ W^T + bias?) + residual?  for M <= 4 rows.  norm: RMSNorm weight [K] or null; bias [N], res
 // [M, N]: null or bf16 (not with swiglu).  swiglu: W is [2N, K], gate rows then up rows.  K % 8 == 0, N % 2 == 0, leading
-// dimensions multiples of 8, 16-byte aligned bases, M * K <= 80 K elements (x, and with a norm its weight, in shared memory).
+// dimensions multiples of 8, 16-byte aligned bases, M * K <= 80 K elements and with a norm (M + 1) * K <= 112 K (x and the norm's
+// weight in shared memory; native.skinny_supported asks for the same).
 // As tensor-core tiles 3584 x 3584 and 3584 x 18944 take 25 and 83 us for one row.
 MM_API int mm_gemv_bf16(const void* x, const void* w, const void* bias, const void* norm, const void* res, void* out, int M, int N,
                         int K, long long ldx, long long ldw, long long ldr, long long ldo, float eps, int swiglu, cudaStream_t st) {

@@ -572,11 +572,14 @@ def mrope_tables(position_ids, head_dim, theta, section):
     return cos, sin
 
 
-def skinny_supported(x, *tensors) -> bool:
-    """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies."""
-    return (_keeps_no_graph((x,) + tensors) and x.dim() == 2 and 1 <= x.shape[0] <= 4 and x.shape[1] % 8 == 0
-            and x.numel() <= 80 * 1024 and _ok2d(x)
-            and all(t is None or (t.dtype == torch.bfloat16 and t.device == x.device) for t in tensors))
+def skinny_supported(x, *tensors, norm=None) -> bool:
+    """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies.  The sizes are
+    mm_gemv_bf16's own rule: x, and with a norm its weight too, have to fit a block's shared memory."""
+    if not _keeps_no_graph((x, norm) + tensors) or x.dim() != 2:
+        return False
+    M, K = x.shape
+    return (1 <= M <= 4 and K % 8 == 0 and M * K <= 80 * 1024 and (norm is None or (M + 1) * K <= 112 * 1024) and _ok2d(x)
+            and all(t is None or (t.dtype == torch.bfloat16 and t.device == x.device) for t in (norm,) + tensors))
 
 
 def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=False):

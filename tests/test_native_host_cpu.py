@@ -41,7 +41,7 @@ def _rules():
     bf = lambda *s: torch.randn(*s).bfloat16()  # noqa: E731
     x, w, q, kv, old, tab = bf(2, 256), bf(64, 256), bf(1, 4, 128), bf(1, 2, 128), bf(9, 2, 128), bf(1, 128)
     return {"product": (lambda t: native.skinny_supported(t, w, None), x),
-            "product, norm weight": (lambda t: native.skinny_supported(x, t, w), bf(256)),
+            "product, norm weight": (lambda t: native.skinny_supported(x, w, norm=t), bf(256)),
             "cached attention": (lambda t: native.decode_attention_supported(t, kv, kv, old, old, tab, tab), q),
             "cached attention, tables": (lambda t: native.decode_attention_supported(q, kv, kv, old, old, tab, t), tab),
             "rotary tables": (lambda t: native.mrope_tables_supported(t, 128, (16, 24, 24), torch.bfloat16), torch.arange(21).view(3, 7))}
@@ -73,3 +73,12 @@ def test_waits_in_front_of_whole_warp_instructions_are_voted(name, role):
     begin = text.index(role)
     waits = [ln for ln in text[begin:text.index("atomicExch(p.status, MM_TIMEOUT_EPI)", begin)].splitlines() if "mbar_wait(" in ln]
     assert len(waits) >= 2 and all("__all_sync(0xffffffffu, mbar_wait(" in ln for ln in waits)
+
+
+@pytest.mark.parametrize("M,K,norm,takes", [(1, 57344, True, True), (1, 57352, True, False), (1, 57352, False, True), (2, 38224, True, True),
+                                            (2, 38232, True, False), (4, 20480, False, True), (4, 20488, False, False), (3, 27304, True, True),
+                                            (3, 27312, True, False), (5, 64, False, False)])
+def test_products_of_a_few_rows_that_fit_shared_memory(M, K, norm, takes):
+    """M * K up to 80 K elements, and (M + 1) * K up to 112 K where a norm's weight is held beside x."""
+    x, w = torch.zeros(M, K, dtype=torch.bfloat16), torch.zeros(16, K, dtype=torch.bfloat16)
+    assert native.skinny_supported(x, w, norm=torch.zeros(K, dtype=torch.bfloat16) if norm else None) is takes
