@@ -593,7 +593,7 @@ def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=Fal
         if norm.data_ptr() % 16:
             norm = norm.clone()
     if residual is not None and not _ok2d(residual):
-        residual = residual.contiguous()
+        residual = residual.clone(memory_format=torch.contiguous_format)     # also where it only starts off an aligned address
     M, K = x.shape
     N = w.shape[0] // 2 if swiglu else w.shape[0]
     out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)

@@ -104,6 +104,14 @@ def test_normalised_rows_around_the_shared_memory_limits(M, K, swiglu):
     _close(got, ref.swiglu(want) if swiglu else want, rtol=8e-3, atol=4e-3)
 
 
+@pytest.mark.parametrize("start,pitch", [(1, 64), (2, 64), (3, 72), (8, 71)])
+def test_residual_of_a_few_rows_may_start_anywhere(start, pitch):
+    x, w, buf = torch.randn(2, 256, device=DEV).bfloat16(), torch.randn(64, 256, device=DEV).bfloat16() / 16, torch.randn(200, device=DEV).bfloat16()
+    r = buf[start:].as_strided((2, 64), (pitch, 1))
+    with torch.no_grad():
+        _close(ops.linear_add(x, w, r), x.float() @ w.float().t() + r.float(), rtol=8e-3, atol=4e-3)
+
+
 def test_product_of_a_few_rows_keeps_infinities_and_nan_to_their_outputs():
     x, w = torch.zeros(1, 272, device=DEV).bfloat16(), torch.ones(16, 272, device=DEV).bfloat16()
     x[0, -1], w[3, 5], w[4, 271] = float("inf"), float("nan"), -1
