@@ -240,9 +240,11 @@ class Linear(nn.Module):
 
 
 def _plain(*modules) -> bool:
-    """Exactly this file's Linear / RMSNorm, nothing hooked: their weights may be used without calling them."""
+    """Exactly this file's Linear / RMSNorm, nothing hooked, compiled or with a forward of its own (an adapter, a wrapper set on the
+    instance): their weights may be used without calling them."""
     return not torch.nn.modules.module._has_any_global_hook() and all(
-        type(m) in (Linear, RMSNorm) and not (m._forward_hooks or m._forward_pre_hooks) for m in modules)
+        type(m) in (Linear, RMSNorm) and "forward" not in m.__dict__ and getattr(m, "_compiled_call_impl", None) is None
+        and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) for m in modules)
 
 
 class VisionBlock(nn.Module):

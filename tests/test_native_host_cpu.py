@@ -5,6 +5,7 @@ import pytest
 import torch
 import torch.autograd.forward_ad as fwad
 
+from mindspeed_mm_b200.models.qwen2_5_vl import DecoderLayer, LMHead, TextConfig
 from mindspeed_mm_b200.ops import native
 
 
@@ -82,3 +83,35 @@ def test_products_of_a_few_rows_that_fit_shared_memory(M, K, norm, takes):
     """M * K up to 80 K elements, and (M + 1) * K up to 112 K where a norm's weight is held beside x."""
     x, w = torch.zeros(M, K, dtype=torch.bfloat16), torch.zeros(16, K, dtype=torch.bfloat16)
     assert native.skinny_supported(x, w, norm=torch.zeros(K, dtype=torch.bfloat16) if norm else None) is takes
+
+
+@pytest.mark.parametrize("name", ["input_layernorm", "post_attention_layernorm", "qkv_proj", "o_proj", "down_proj", "norm"])
+@pytest.mark.parametrize("how", ["forward", "forward_hook", "pre_hook", "backward_hook", "adapter"])
+def test_wrapped_modules_are_called_in_the_generation_path(name, how):
+    """The generation path uses the weights of plain modules; one that something was attached to is called."""
+    torch.manual_seed(0)
+    c = TextConfig(num_layers=1, hidden_size=32, intermediate_size=64, num_attention_heads=4, num_key_value_heads=2, vocab_size=48)
+    layer, head = DecoderLayer(c), LMHead(c)
+    for p in (*layer.parameters(), *head.parameters()):
+        torch.nn.init.normal_(p, std=0.1)
+    owner, calls = (head, []) if name == "norm" else (layer, [])
+    m = getattr(owner, name)
+    if how == "forward":
+        inner = m.forward
+        m.forward = lambda *a, **k: calls.append(1) or inner(*a, **k)
+    elif how == "forward_hook":
+        m.register_forward_hook(lambda *a: calls.append(1))
+    elif how == "pre_hook":
+        m.register_forward_pre_hook(lambda *a: calls.append(1))
+    elif how == "backward_hook":
+        m.register_full_backward_hook(lambda *a: calls.append(1))
+    else:
+        class Adapter(type(m)):
+            def forward(self, *a, **k):
+                calls.append(1)
+                return super().forward(*a, **k)
+        m.__class__ = Adapter
+    x = torch.randn(3, 32, requires_grad=True)
+    y = head(x) if name == "norm" else layer(x, torch.ones(3, 8), torch.zeros(3, 8), None, None, cache={})
+    y.sum().backward()
+    assert calls
