@@ -6,15 +6,16 @@ namespace {
 constexpr int kWarps = 8, kCols = 256;      // a warp reads 256 columns of a row (16 bytes a lane), a block 8 rows at a time
 
 // partial[b][split][c] = sum over the rows of batch b that the split walks of x[r][c] (times y[r][c] if GATED, which also writes
-// out = x * gate[b]).  Blocks: (column group, row split, batch); the warps of a block take every 8th row, four rows in flight each,
+// out = x * gate[b]).  Blocks: (batch and column group, row split); the warps of a block take every 8th row, four rows in flight each,
 // and meet in shared memory.  Rows are split so that the grid fills the SMs whatever the width is: 8192 x 3840 -> 15 x 40 blocks.
 template <bool GATED>
 __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y,
                                                                 const bf16* __restrict__ gate, bf16* __restrict__ out,
                                                                 float* __restrict__ partial, int rows, int cols, long long ldx) {
     __shared__ float tile[kWarps][kCols + 4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * kCols + lane * 8;
-    const int split = blockIdx.y, splits = gridDim.y, b = blockIdx.z;
+    const int groups = (cols + kCols - 1) / kCols, b = blockIdx.x / groups, c0 = (blockIdx.x - b * groups) * kCols;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = c0 + lane * 8;
+    const int split = blockIdx.y, splits = gridDim.y;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (c < cols) {
         const bf16* xb = x + (size_t)b * rows * ldx + c;
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __r
 #pragma unroll
     for (int k = 0; k < 8; ++k) tile[warp][lane * 8 + k] = acc[k];
     __syncthreads();
-    const int col = blockIdx.x * kCols + threadIdx.x;
+    const int col = c0 + threadIdx.x;
     if (col < cols) {
         float s = 0.f;
 #pragma unroll
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __r
 // sums[b][c] = sum over the splits, in their order
 __global__ void __launch_bounds__(256) fold_splits_kernel(const float* __restrict__ partial, bf16* __restrict__ sums, int splits, int cols) {
     __shared__ float tile[8][33];
-    const int c = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y;
+    const int groups = (cols + 31) / 32, b = blockIdx.x / groups, c = (blockIdx.x - b * groups) * 32 + threadIdx.x;
     float s = 0.f;
     if (c < cols)
 #pragma unroll 4
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(256) scale_kernel(bf16* __restrict__ x, long l
 }
 
 int splits_of(int rows, int cols, int batches) {
+    if (rows < 1 || cols < 1 || batches < 1) return 1;
     const long long groups = (long long)((cols + kCols - 1) / kCols) * batches;
     long long s = (148 * 4 + groups - 1) / groups;                   // four blocks an SM
     const long long most = (rows + kWarps * 4 - 1) / (kWarps * 4);     // at least four rows a warp
@@ -105,22 +107,26 @@ MM_API int mm_column_sum(const void* x, void* sums, float* partial, int rows, in
     if (cols % 8 || ldx % 8 || ((uintptr_t)x & 15)) return -1;
     if (rows < 1 || cols < 1) return -2;
     const int splits = splits_of(rows, cols, 1);
-    column_sum_kernel<false><<<dim3((cols + kCols - 1) / kCols, splits, 1), kWarps * 32, 0, st>>>((const bf16*)x, nullptr, nullptr, nullptr,
+    column_sum_kernel<false><<<dim3((cols + kCols - 1) / kCols, splits), kWarps * 32, 0, st>>>((const bf16*)x, nullptr, nullptr, nullptr,
                                                                                                   partial, rows, cols, ldx);
-    fold_splits_kernel<<<dim3((cols + 31) / 32, 1), dim3(32, 8), 0, st>>>(partial, (bf16*)sums, splits, cols);
+    fold_splits_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, st>>>(partial, (bf16*)sums, splits, cols);
     return (int)cudaGetLastError();
 }
 
 // Backward of x + gate[b] * y: dy = dout * gate[b], dgate[b, c] = sum over the rows of dout * y (fp32 inside).  dout, y, dy: dense
-// [batches, rows, cols]; one pass over dout and y.
+// [batches, rows, cols]; one pass over dout and y.  Nothing to sum over (rows == 0): zeros.
 MM_API int mm_gated_residual_bwd(const void* dout, const void* y, const void* gate, void* dy, void* dgate, float* partial, int batches,
                                  int rows, int cols, cudaStream_t st) {
-    if (cols % 8 || batches > 65535 || ((uintptr_t)dout | (uintptr_t)y | (uintptr_t)gate | (uintptr_t)dy) & 15) return -1;
-    if (rows < 1 || cols < 1 || batches < 1) return -2;
+    if (cols % 8 || ((uintptr_t)dout | (uintptr_t)y | (uintptr_t)gate | (uintptr_t)dy) & 15) return -1;
+    if (rows < 0 || cols < 0 || batches < 0) return -2;
+    if (!batches || !cols) return 0;
+    if (!rows) return (int)cudaMemsetAsync(dgate, 0, (size_t)batches * cols * sizeof(bf16), st);
+    const long long blocks = (long long)batches * ((cols + 31) / 32);       // a gate per token is as many batches as there are tokens
+    if (blocks > 0x7fffffffLL) return -2;
     const int splits = splits_of(rows, cols, batches);
-    column_sum_kernel<true><<<dim3((cols + kCols - 1) / kCols, splits, batches), kWarps * 32, 0, st>>>(
+    column_sum_kernel<true><<<dim3(batches * ((cols + kCols - 1) / kCols), splits), kWarps * 32, 0, st>>>(
         (const bf16*)dout, (const bf16*)y, (const bf16*)gate, (bf16*)dy, partial, rows, cols, cols);
-    fold_splits_kernel<<<dim3((cols + 31) / 32, batches), dim3(32, 8), 0, st>>>(partial, (bf16*)dgate, splits, cols);
+    fold_splits_kernel<<<(int)blocks, dim3(32, 8), 0, st>>>(partial, (bf16*)dgate, splits, cols);
     return (int)cudaGetLastError();
 }
 
