@@ -715,7 +715,8 @@ class _Linear(torch.autograd.Function):
             else:
                 dw = gemm_tn(dy2, x2) if _BWD_NATIVE else dy2.t() @ x2
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = column_sum(dy2)
+            # create_graph: the sum itself is differentiated
+            db = torch.sum(dy2, 0, dtype=torch.float32).to(dy2.dtype) if torch.is_grad_enabled() else column_sum(dy2)
         return dx, dw, db, None
 
 
@@ -883,6 +884,9 @@ class _LinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         dh, dw = ctx.saved_tensors
+        if torch.is_grad_enabled():          # create_graph: the scaling itself is differentiated
+            gs = g.to(dh.dtype)
+            return dh.mul_(gs), dw.mul_(gs), None, None, None
         gs = g.float().reshape(1)
         for t in (dh, dw):
             _check(lib().mm_scale_bf16(t.data_ptr(), t.numel(), gs.data_ptr(), _st()), "scale_bf16")
@@ -987,6 +991,10 @@ class _AlignedUnpermute(torch.autograd.Function):
     def backward(ctx, g):
         y, row_of_pair, probs, src_of_row = ctx.saved_tensors
         T, k = probs.shape
+        if torch.is_grad_enabled():          # create_graph: the gradient itself is differentiated
+            ge = g.repeat_interleave(k, dim=0)
+            dy = torch.zeros_like(y).index_copy(0, row_of_pair.long(), ge * probs.reshape(-1, 1))
+            return dy, None, (ge.float() * y[row_of_pair.long()].float()).sum(-1).view(T, k).to(probs.dtype), None
         g = g.contiguous()
         dy = torch.empty_like(y)
         dprobs = torch.empty_like(probs)

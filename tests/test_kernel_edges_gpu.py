@@ -446,3 +446,26 @@ def test_planning_many_short_sequences_takes_no_longer_than_their_attention_by_o
     b.record()
     torch.cuda.synchronize()
     assert a.elapsed_time(b) < 5
+
+
+@pytest.mark.parametrize("name", ["bias", "loss", "unpermute", "gate"])
+def test_gradients_that_are_linear_in_the_incoming_one_can_be_differentiated(name):
+    """create_graph: the derivative of a gradient by a factor in front of the op's result is the gradient itself."""
+    bf = lambda *s: torch.randn(*s, device=DEV).bfloat16().requires_grad_()  # noqa: E731
+    s = torch.ones((), device=DEV, requires_grad=True)
+    x, w, b, h, vocab, y, gate = bf(16, 64), bf(32, 64), bf(32), bf(16, 64), bf(256, 64), bf(128, 64), bf(2, 1, 64)
+    probs, rows = torch.rand(64, 2, device=DEV).bfloat16().requires_grad_(), torch.arange(128, device=DEV, dtype=torch.int32).flip(0)
+    c = torch.randn(8192, device=DEV)
+    out, leaves = {"bias": lambda: (ops.linear(x, w, b), [b]), "loss": lambda: (ops.linear_cross_entropy(h, vocab, torch.arange(16, device=DEV))[0], [h, vocab]),
+                   "unpermute": lambda: (native._AlignedUnpermute.apply(y, rows, probs), [y, probs]),
+                   "gate": lambda: (ops.gated_residual(y.view(2, 64, 64), y.view(2, 64, 64), gate), [gate])}[name]()
+    plain = torch.autograd.grad((out.float().view(-1) * c[:out.numel()] if out.dim() else out * 1.0).sum(), leaves, retain_graph=name != "loss")
+    if name == "loss":                       # its gradients are scaled in place: once per forward
+        out = ops.linear_cross_entropy(h, vocab, torch.arange(16, device=DEV))[0]
+    grads = torch.autograd.grad((out.float().view(-1) * c[:out.numel()] * s if out.dim() else out * s).sum(), leaves, create_graph=True)
+    for a, g in zip(plain, grads):
+        _close(g.detach(), a, rtol=8e-3, atol=4e-3)
+        v = torch.randn_like(g)
+        (ds,) = torch.autograd.grad(g, [s], v, retain_graph=True)
+        want = (a.float() * v.float()).sum()
+        assert float((ds - want).abs()) <= 2e-2 * float((a.float() * v.float()).norm()) + 1e-3
