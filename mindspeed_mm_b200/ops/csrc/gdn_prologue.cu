@@ -117,8 +117,8 @@ __device__ __forceinline__ void load_gates(const float* g, const float* beta, lo
     if (threadIdx.x == 0) before = 0.f;
     gc[r] = before + a;
     gc[r + 1] = before + a + b;
-    eg[r] = __expf(gc[r]);
-    eg[r + 1] = __expf(gc[r + 1]);
+    eg[r] = expf(gc[r]);
+    eg[r + 1] = expf(gc[r + 1]);
     bt[r] = r < len ? beta[(tok0 + r) * H + head] : 0.f;
     bt[r + 1] = r + 1 < len ? beta[(tok0 + r + 1) * H + head] : 0.f;
 }
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prologue_kernel(
                 float at[2];
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const float dec = j + e <= i ? __expf(gc[i] - gc[j + e]) : 0.f;
+                    const float dec = j + e <= i ? expf(gc[i] - gc[j + e]) : 0.f;
                     sA[i * LT + j + e] = j + e < i ? bt[i] * s[n][2 * h + e] * dec : 0.f;
                     at[e] = p[n][2 * h + e] * dec * scale;
                 }
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prologue_kernel(
         float fq[8], fk[8];
         unpack8(*reinterpret_cast<const Vec8*>(sQ + r * LB + c8), fq);
         unpack8(*reinterpret_cast<const Vec8*>(sK + r * LB + c8), fk);
-        const float a = scale * eg[r], b = __expf(last - gc[r]);
+        const float a = scale * eg[r], b = expf(last - gc[r]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             fq[e] *= a;
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_prologue_bwd_kernel(
     clear<8>(aq);
     clear<4>(dat);
     warp_product<false, true, 8>(ak, sVN, LB, m0, sG, LB, n0, 0, D);
-    scale_rows(ak, __expf(gl - gc[ri]), __expf(gl - gc[ri + 8]));
+    scale_rows(ak, expf(gl - gc[ri]), expf(gl - gc[ri + 8]));
     row_dot(ak, sK, slot + (0 + wn) * C, m0, n0);                     // <dKd, Kd>
     warp_product<false, true, 8>(aq, sDO, LB, m0, sS, LB, n0, 0, D);
     scale_rows(aq, scale * e0, scale * e1);
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_prologue_bwd_kernel(
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int i = ri + (e >> 1) * 8, j = h0 + n * 8 + (lane & 3) * 2 + (e & 1);
-            const float dec = j <= i ? __expf(gc[i] - gc[j]) : 0.f;
+            const float dec = j <= i ? expf(gc[i] - gc[j]) : 0.f;
             s[n][e] = j < i ? s[n][e] * dec : 0.f;                    // S D, strictly lower
             dat[n][e] *= dec * scale;                                 // dP, so that dAt At = dP (q_i . k_j)
             sA[i * LT + j] = s[n][e] * bt[i];
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_prologue_bwd_kernel(
                     (h ? be1 : be0) += E;
                     (h ? rr1 : rr0) += R;
                     col += R;
-                    put_split(sp, i, j, j < i ? da * beta_i * __expf(gc[i] - gc[j]) : 0.f);
+                    put_split(sp, i, j, j < i ? da * beta_i * expf(gc[i] - gc[j]) : 0.f);
                     put_split(sp2, i, j, dat[n][e]);
                 }
 #pragma unroll

@@ -171,6 +171,19 @@ def test_gated_delta_rule_on_bf16_tensors(lens, H, gate):
         ops.gated_delta_rule_varlen(q, k, v, g, beta, [0, T + 1], chunk=64)
 
 
+def test_decay_of_a_chunk_is_an_fp32_exponential():
+    """Gates whose sums are exact in fp32: what is left is the exponential's own error, 2 ulp and not one that grows with the sum."""
+    H, K, z = 64, 128, dict(dtype=torch.bfloat16, device=DEV)
+    q = torch.nn.functional.normalize(torch.randn(64, H, K, device=DEV), dim=-1).bfloat16()
+    g = (-torch.arange(1, H + 1, device=DEV, dtype=torch.float32) / 64).expand(64, H).contiguous()      # sums of -1 .. -64
+    W, Qg, Kd, U, At = *(torch.empty(H, 1, 64, K, **z) for _ in range(4)), torch.empty(H, 1, 64, 64, **z)
+    gamma, at = torch.empty(H, 1, device=DEV), [torch.tensor([i], dtype=torch.int32, device=DEV) for i in (0, 64)]
+    assert native.lib().mm_gdn_prologue(q.data_ptr(), q.data_ptr(), q.data_ptr(), g.data_ptr(), torch.ones_like(g).data_ptr(), at[0].data_ptr(), at[1].data_ptr(),
+                                        W.data_ptr(), Qg.data_ptr(), Kd.data_ptr(), At.data_ptr(), U.data_ptr(), gamma.data_ptr(), H, 1, 1.0, native._st()) == 0
+    want = (-torch.arange(1, H + 1, device=DEV, dtype=torch.float64)).exp()
+    assert float((gamma[:, 0].double() / want - 1).abs().max()) <= 2.5 * 2 ** -23
+
+
 @pytest.mark.parametrize("lens_q,lens_k,nq,nkv,D,causal,grow", [
     ([1024], [1024], 2, 2, 128, False, False), ([1023], [1023], 2, 2, 128, False, False),       # both sides of the key-length rule
     ([1025], [1025], 4, 2, 80, False, True), ([4000, 129, 1], [4000, 129, 1], 2, 1, 72, False, True),
