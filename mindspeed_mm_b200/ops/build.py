@@ -21,8 +21,15 @@ LIBNAME = "libmm_b200_ops.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xptxas", "-v", "--use_fast_math",
+    "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
 ]
+# Sources whose fp32 functions are the full ones: under --use_fast_math expf() is the fast exponential, whose relative error grows
+# with its argument, and these replace PyTorch forms that had the full one.
+FULL_MATH = ("gdn_prologue.cu",)
+
+
+def _flags(src: str) -> list:
+    return NVCC_FLAGS if src in FULL_MATH else [*NVCC_FLAGS, "--use_fast_math"]
 
 
 def _nvcc() -> str:
@@ -46,7 +53,7 @@ def _digest() -> str:
         if f.endswith((".cu", ".cuh", ".h")):
             h.update(f.encode())
             h.update(open(os.path.join(CSRC, f), "rb").read())
-    h.update(" ".join(NVCC_FLAGS).encode())
+            h.update(" ".join(_flags(f)).encode())
     return h.hexdigest()
 
 
@@ -65,7 +72,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     def one(src):
         obj = os.path.join(LIBDIR, src[:-3] + ".o")
-        cmd = [nvcc, *NVCC_FLAGS, "-I", CSRC, "-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [nvcc, *_flags(src), "-I", CSRC, "-c", os.path.join(CSRC, src), "-o", obj]
         r = subprocess.run(cmd, capture_output=True, text=True)
         logs[src] = r.stdout + r.stderr
         if r.returncode != 0:

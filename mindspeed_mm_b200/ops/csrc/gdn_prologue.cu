@@ -10,7 +10,7 @@
 // rows past the end of a sequence's last chunk are zero (beta = g = 0), so they leave T, U, W and the state untouched.
 // Outputs are bf16 [H, NC, 64, *] (what the tcgen05 state-pass kernel reads) and gamma fp32 [H, NC].
 //
-// Arithmetic is fp32 throughout, on the tensor cores where that costs nothing: in every 64 x 64 x 128 product one operand is a
+// Arithmetic is fp32 throughout (exponentials too: this file is built without fast math), on the tensor cores where that costs nothing: in every 64 x 64 x 128 product one operand is a
 // bf16 tensor as it is in memory (q, k, v, dVn, ...), and the other, if it is fp32 (T, dS, dP, with beta and the gates folded into
 // its columns), is split into three bf16 terms that hold all 24 bits of it; products of bf16 numbers are exact in the fp32
 // accumulator.  (mma.sync, not tcgen05: the operands are 64 rows high and come out of registers and shared memory in between
@@ -175,7 +175,7 @@ __device__ __forceinline__ void store_rows(const float (*acc)[4], bf16* dst, lon
 }
 
 // Two CTAs fit an SM, so one CTA's loads and substitution run beside the other's products.  Bound by the chain of phases (load,
-// scores, inverse, two products) of a CTA.  2144 chunks x heads (4096 tokens, 32 heads): 124 us; about 900 us with every product
+// scores, inverse, two products) of a CTA.  2144 chunks x heads (4096 tokens, 32 heads): 126 us; about 900 us with every product
 // on CUDA cores from odd-stride fp32 tiles and a 64-row substitution by one thread per column.
 __global__ void __launch_bounds__(kThreads, 2) gdn_prologue_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, const float* __restrict__ g,
@@ -305,8 +305,8 @@ __device__ __forceinline__ void scale_rows(float (*acc)[4], float a, float b) {
 //   dS = dA beta_i D    dP = dAt D scale    dk = dS k + dS^T k + dP^T q + beta exp(gc) T^T dW + exp(gl - gc) dKd
 //   dq = dP k + scale exp(gc) dQg           dv = beta T^T dU
 // T, A and the two score matrices are recomputed; nothing of the chunk is kept in fp32 between the passes.  One CTA an SM (eleven
-// 64 x 128 tiles of shared memory); bound like the forward by its chain of phases.  2144 chunks x heads: 396 us, where the batched
-// products, casts, scatters and autograd through the PyTorch prologue took 4.6 ms.
+// 64 x 128 tiles of shared memory); bound like the forward by its chain of phases.  2144 chunks x heads: 409 us, where the batched
+// products, casts, scatters and autograd through the PyTorch prologue took 4.6 ms (395 with the fast exponential).
 __global__ void __launch_bounds__(kThreads, 1) gdn_prologue_bwd_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, const float* __restrict__ g,
     const float* __restrict__ beta, const int* __restrict__ chunk_tok0, const int* __restrict__ chunk_len,
