@@ -256,7 +256,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             mbar_arrive(&p_full[st]);
         }
         l_final[row] = l;
-        if (ok && qi < q_len && n_kv > 0)
+        if (ok && qi < q_len)
             p.lse[(size_t)head * p.T + q_begin + qi] = (m == -INFINITY) ? -INFINITY : m * 0.6931471805599453f + logf(l);
         mbar_arrive(fin);
         if (!ok && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
@@ -288,7 +288,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             fence_before_sync();
             mbar_arrive(&o_empty[st]);
         }
-        if (ok && mbar_wait(fin, 0, abort_flag) && qi < q_len && n_kv > 0) {
+        if (ok && mbar_wait(fin, 0, abort_flag) && qi < q_len) {      // zeros where no key is visible
             const float lsum = l_final[row];
             const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
             bf16* dst = p.o + ((size_t)(q_begin + qi) * p.Nq + head) * p.D;

@@ -285,6 +285,12 @@ fmha_fwd_alt_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             if (grp == 0 && qi < q_len)
                 p.lse[(size_t)head * p.T + q_begin + qi] = (m_fin == -INFINITY) ? -INFINITY : m_fin * 0.6931471805599453f + logf(lsum);
         }
+        if (n_kv == 0 && qi < q_len) {                   // no key is visible to this tile
+            bf16* dst = p.o + ((size_t)(q_begin + qi) * p.Nq + head) * p.D + grp * 64;
+            for (int g = 0; g < 8; ++g)
+                if (grp * 64 + g * 8 < p.D) reinterpret_cast<uint4*>(dst)[g] = make_uint4(0, 0, 0, 0);
+            if (grp == 0) p.lse[(size_t)head * p.T + q_begin + qi] = -INFINITY;
+        }
         if (!ok && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
     }
 

@@ -330,7 +330,7 @@ fmha_fwd_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         named_barrier_sync(1, kCompute);
         atomicAdd(&l_sum[row], l);
         named_barrier_sync(1, kCompute);
-        if (ok && qi < q_len && n_kv > 0) {
+        if (ok && qi < q_len) {                              // zeros where no key is visible
             const float lsum = l_sum[row];
             const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
             if (half == 0)

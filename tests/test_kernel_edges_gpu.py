@@ -482,3 +482,24 @@ def test_gradients_that_are_linear_in_the_incoming_one_can_be_differentiated(nam
         (ds,) = torch.autograd.grad(g, [s], v, retain_graph=True)
         want = (a.float() * v.float()).sum()
         assert float((ds - want).abs()) <= 2e-2 * float((a.float() * v.float()).norm()) + 1e-3
+
+
+@pytest.mark.parametrize("lens_q,lens_k,causal", [([400], [100], True), ([10, 300, 10], [0, 300, 7], False), ([10, 300], [0, 4000], False),
+                                                  ([4000, 10], [3500, 3500], True)])
+@pytest.mark.parametrize("D", [72, 128])
+def test_rows_that_see_no_key_are_zero(lens_q, lens_k, causal, D):
+    """Whole tiles of them, too, in both forward kernels; their gradients are zero."""
+    torch.manual_seed(sum(lens_q))
+    q, k, v = (torch.randn(sum(t), 2, D, device=DEV).bfloat16().requires_grad_() for t in (lens_q, lens_k, lens_k))
+    cu = [torch.tensor([0] + l, device=DEV).cumsum(0).to(torch.int32) for l in (lens_q, lens_k)]
+    poison = [torch.full((sum(lens_q), 2, 128), float("nan"), device=DEV) for _ in range(4)]       # what the allocator hands out next
+    del poison
+    out, lse = native.fmha_forward(q.detach(), k.detach(), v.detach(), *cu, causal, D ** -0.5)
+    want, want_lse = ref.attention_varlen(q.detach().float(), k.detach().float(), v.detach().float(), cu[0].cpu(), cu[1].cpu(), causal, return_lse=True)
+    hidden = want_lse[0] == float("-inf")
+    assert hidden.any() and torch.equal(lse == float("-inf"), want_lse == float("-inf")) and not out[hidden].any()
+    _close(out[~hidden], want[~hidden], rtol=1e-2, atol=4e-3)
+    o = ops.attention_varlen(q, k, v, *cu, max(lens_q), max(lens_k), causal=causal)
+    dq, dk, dv = torch.autograd.grad(o, [q, k, v], torch.randn_like(o))
+    native.check_status()
+    assert not dq[hidden].any() and all(bool(t.isfinite().all()) for t in (dq, dk, dv))
