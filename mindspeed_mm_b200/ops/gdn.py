@@ -260,7 +260,7 @@ class _GatedDelta(torch.autograd.Function):
         from . import native
         T, H, K = q.shape
         dev, NC = q.device, lay.NC
-        qb, kb, vb = (_aligned(t.to(torch.bfloat16).contiguous()) for t in (q, k, v))
+        qb, kb, vb = (native._dense(t.to(torch.bfloat16)) for t in (q, k, v))
         gf, bf = g.float().contiguous(), beta.float().contiguous()
         W, Qg, Kd, U = (torch.empty(H, NC, CHUNK, K, dtype=torch.bfloat16, device=dev) for _ in range(4))
         At = torch.empty(H, NC, CHUNK, CHUNK, dtype=torch.bfloat16, device=dev)
@@ -287,7 +287,7 @@ class _GatedDelta(torch.autograd.Function):
         lay, scale, g_dtype, beta_dtype = ctx.meta
         T, H, K = q.shape
         NC, dev, L, st = lay.NC, q.device, native.lib(), native._st()
-        dout = _aligned(dout.to(torch.bfloat16).contiguous())
+        dout = native._dense(dout.to(torch.bfloat16))
         dO, dVn = torch.empty_like(Vn), torch.empty_like(Vn)
         GT = torch.empty_like(SprevT)
         native._check(L.mm_gdn_layout(dout.data_ptr(), dO.data_ptr(), lay.chunk_tok0.data_ptr(), lay.chunk_len.data_ptr(), H, NC, 1, st),
@@ -302,11 +302,6 @@ class _GatedDelta(torch.autograd.Function):
             dO.data_ptr(), Vn.data_ptr(), dVn.data_ptr(), SprevT.data_ptr(), GT.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
             dg.data_ptr(), dbeta.data_ptr(), H, NC, float(scale), st), "gdn_prologue_bwd")
         return dq, dk, dv, dg.to(g_dtype), dbeta.to(beta_dtype), None, None
-
-
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    """The layout and prologue kernels read 16-byte vectors."""
-    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def kda_chunk_prologue(q, k, v, g, beta, scale: float):

@@ -225,6 +225,12 @@ def _pitch(x) -> int:
     return x.stride(0) if x.shape[0] > 1 else x.shape[1]
 
 
+def _dense(t):
+    """Contiguous and 16-byte aligned, as kernels with vector loads take it (a single row of a wider matrix is contiguous wherever
+    it starts, and .contiguous() returns it as it is)."""
+    return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 # --------------------------------------------------------------------------- RMSNorm
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
@@ -232,12 +238,12 @@ class _RMSNorm(torch.autograd.Function):
         shape = x.shape
         H = shape[-1]
         x2 = x.reshape(-1, H)
-        if not x2.is_contiguous() and (_row_group(H) or not _ok2d(x2)):
-            x2 = x2.contiguous()
+        if _row_group(H) or not _ok2d(x2):
+            x2 = _dense(x2)
         T = x2.shape[0]
         y = torch.empty(T, H, dtype=x.dtype, device=x.device)
         rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-        wc = w.contiguous()
+        wc = _dense(w)
         if _row_group(H):
             rc = lib().mm_rownorm_rms_fwd(x2.data_ptr(), wc.data_ptr(), y.data_ptr(), rstd.data_ptr(), T, H, eps, _st())
         else:       # rows may lie apart (the query or key columns of a fused projection): no copy of them is made
@@ -251,9 +257,7 @@ class _RMSNorm(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w, rstd = ctx.saved_tensors
         T, H = x2.shape
-        dy2 = dy.reshape(T, H)
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
+        dy2 = _dense(dy.reshape(T, H))
         dx = torch.empty(T, H, dtype=x2.dtype, device=x2.device)
         dw = torch.empty_like(w)
         grid = lib().mm_rmsnorm_bwd_grid(T)
@@ -995,7 +999,7 @@ class _AlignedUnpermute(torch.autograd.Function):
             ge = g.repeat_interleave(k, dim=0)
             dy = torch.zeros_like(y).index_copy(0, row_of_pair.long(), ge * probs.reshape(-1, 1))
             return dy, None, (ge.float() * y[row_of_pair.long()].float()).sum(-1).view(T, k).to(probs.dtype), None
-        g = g.contiguous()
+        g = _dense(g)
         dy = torch.empty_like(y)
         dprobs = torch.empty_like(probs)
         _check(lib().mm_moe_unpermute_bwd(g.data_ptr(), y.data_ptr(), row_of_pair.data_ptr(),
@@ -1063,7 +1067,7 @@ class _CausalConv1d(torch.autograd.Function):
         K = w.shape[-1]
         # the convolution's columns of a fused projection are read where they are
         if x.stride(1) != 1 or _pitch(x) % 8 or x.data_ptr() % 16:
-            x = x.contiguous()
+            x = _dense(x)
         w = w.contiguous()
         start, end = _seq_bounds(cu_seqlens, T, x.device)
         y = torch.empty(T, D, dtype=x.dtype, device=x.device)
@@ -1078,7 +1082,7 @@ class _CausalConv1d(torch.autograd.Function):
         x, w, start, end = ctx.saved_tensors
         T, D = x.shape
         K = w.shape[-1]
-        dy = dy.contiguous()
+        dy = _dense(dy)
         dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
         dw = torch.zeros(D, K, dtype=torch.float32, device=x.device)
         _check(lib().mm_conv1d_bwd(x.data_ptr(), _pitch(x), w.data_ptr(), start.data_ptr(), end.data_ptr(), dy.data_ptr(),
@@ -1140,7 +1144,7 @@ class _DeltaHeads(torch.autograd.Function):
     def backward(ctx, dq, dk, dv):
         q, k, r = ctx.saved_tensors
         T, hk, v_width = q.shape[0], r.shape[1] // 2, dv.shape[1] * dv.shape[2]
-        dq, dk, dv = (g if g.is_contiguous() and g.data_ptr() % 16 == 0 else g.clone(memory_format=torch.contiguous_format) for g in (dq, dk, dv))
+        dq, dk, dv = _dense(dq), _dense(dk), _dense(dv)
         dx = torch.empty(T, 2 * hk * 128 + v_width, dtype=torch.bfloat16, device=q.device)
         _check(lib().mm_delta_heads_bwd(q.data_ptr(), k.data_ptr(), r.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                                         dx.data_ptr(), T, hk, q.shape[1] // hk, v_width, _st()), "delta_heads_bwd")
@@ -1162,13 +1166,13 @@ class _GatedRMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, z, w, eps):
         D = x.shape[-1]
-        x2, wc = x.reshape(-1, D).contiguous(), w.contiguous()
+        x2, wc = _dense(x.reshape(-1, D)), _dense(w)
         rows = x2.shape[0]
         # z of [tokens, heads, D] with dense heads may have its tokens apart (the gate's columns of a fused projection)
         if z.dim() == 3 and z.stride(2) == 1 and z.stride(1) == D and z.stride(0) % 8 == 0 and z.data_ptr() % 16 == 0 and rows < 2 ** 31:
             z2, zh, ldz = z, max(1, z.shape[1]), z.stride(0)
         else:
-            z2, zh, ldz = z.reshape(-1, D).contiguous(), 1, D
+            z2, zh, ldz = _dense(z.reshape(-1, D)), 1, D
         y = torch.empty(rows, D, dtype=torch.bfloat16, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         _check(lib().mm_gated_rms_fwd(x2.data_ptr(), int(x2.dtype == torch.float32), z2.data_ptr(), wc.data_ptr(), y.data_ptr(),
@@ -1181,7 +1185,7 @@ class _GatedRMSNorm(torch.autograd.Function):
     def backward(ctx, dy):
         x2, z2, wc, rstd = ctx.saved_tensors
         rows, D = x2.shape
-        dy2 = dy.reshape(rows, D).contiguous()
+        dy2 = _dense(dy.reshape(rows, D))
         dx, dz = torch.empty_like(x2), torch.empty(rows, D, dtype=z2.dtype, device=z2.device)
         dw = torch.zeros(D, dtype=torch.float32, device=x2.device)
         _check(lib().mm_gated_rms_bwd(x2.data_ptr(), int(x2.dtype == torch.float32), z2.data_ptr(), wc.data_ptr(), dy2.data_ptr(),

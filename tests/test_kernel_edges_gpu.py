@@ -358,7 +358,7 @@ def test_delta_heads(T, hk, hv, dv):
     _close(a, b, rtol=2 ** -7, atol=0)
 
 
-@pytest.mark.parametrize("T,D,extra", [(1, 8, 0), (70, 264, 8), (33, 1032, 24), (129, 64, 3)])
+@pytest.mark.parametrize("T,D,extra", [(1, 8, 0), (1, 64, 3), (1, 264, 8), (70, 264, 8), (33, 1032, 24), (129, 64, 3)])
 def test_convolution_and_gate_on_columns_of_a_wider_matrix(T, D, extra):
     """Columns read in place (and copied where their pitch or their start does not allow it) give what dense ones give."""
     torch.manual_seed(T)
@@ -503,3 +503,16 @@ def test_rows_that_see_no_key_are_zero(lens_q, lens_k, causal, D):
     dq, dk, dv = torch.autograd.grad(o, [q, k, v], torch.randn_like(o))
     native.check_status()
     assert not dq[hidden].any() and all(bool(t.isfinite().all()) for t in (dq, dk, dv))
+
+
+@pytest.mark.parametrize("T,H", [(1, 64), (1, 264), (1, 3584), (3, 264)])
+@pytest.mark.parametrize("start", [1, 3, 8])
+def test_rms_norm_of_rows_that_start_anywhere(T, H, start):
+    """A single row is contiguous wherever it starts; so is what a gradient may be a view of."""
+    x, w, dy = (torch.randn(T * H + start, device=DEV).bfloat16()[start:].view(T, H) for _ in range(3))
+    outs = []
+    for a, b, g in ((x, w[0], dy), (x.clone(), w[0].clone(), dy.clone())):
+        a, b = a.detach().requires_grad_(), b.detach().requires_grad_()
+        y = ops.rms_norm(a, b)
+        outs.append([y.detach(), *torch.autograd.grad(y, [a, b], g)])
+    assert all(torch.equal(p, q) for p, q in zip(*outs))
