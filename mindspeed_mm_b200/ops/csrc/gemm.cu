@@ -373,8 +373,8 @@ struct SplitPlan {
 // parts: the number that the estimate below makes fastest, 1 if the gain is under 4 us.  A 64-deep step of a 128 x 256 tile takes
 // 0.44 us (1.4 PFLOP/s over 148 SMs); an item's sums are written and read once at about 4 TB/s, a further launch and the shorter
 // main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and lost 2 us).
-// Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 220 / 150 us, 405 x 3584 x 37888 (56) 216 / 122,
-// 8192 x 3584 x 18944 (896) 828 / 761, 8192 x 3584 x 152064 8636 / 6268, 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.
+// Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 218 / 151 us, 405 x 3584 x 37888 (56) 216 / 122,
+// 8192 x 3584 x 18944 (896) 828 / 776, 8192 x 3584 x 152064 (7 rounds become 6 and a part) 6920 / 6210, 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.
 inline SplitPlan split_plan(int M, int N, int K, int BN, int sms) {
     const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK, rem = tiles % sms;
     SplitPlan best{tiles, 1};
@@ -521,7 +521,7 @@ MM_API long long mm_gemm_ws_bytes(int M, int N, int K, int a_mn, int b_mn, int b
 
 // lda/ldb/ldc: elements between consecutive rows of the tensors as laid out in memory.
 // Requirements: base pointers 16-byte aligned; ld* multiples of 8; `status` is a device int (0 = ok).
-// ws: null, or workspace of mm_gemm_ws_bytes (16-byte aligned), used by this call alone.
+// ws: null (the tile list is not split), or workspace of mm_gemm_ws_bytes (16-byte aligned), used by this call alone.
 MM_API int mm_gemm_bf16_ws(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
                            long long ldb, long long ldc, int a_mn, int b_mn, int bn, int* status, void* ws, long long ws_bytes,
                            cudaStream_t st) {
@@ -541,12 +541,6 @@ MM_API int mm_gemm_bf16_ws(const void* A, const void* B, void* C, const void* bi
     MM_DISPATCH(256)
 #undef MM_DISPATCH
 }
-
-MM_API int mm_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda, long long ldb,
-                        long long ldc, int a_mn, int b_mn, int bn, int* status, cudaStream_t st) {
-    return mm_gemm_bf16_ws(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, bn, status, nullptr, 0, st);
-}
-
 
 // C[M, F] = silu(A W_gate^T) * (A W_up^T) with W = [W_gate; W_up] stored as one [2F, K] matrix.  F % 128 == 0.
 MM_API int mm_gemm_swiglu_bf16(const void* A, const void* W, void* C, int M, int F, int K, long long lda, long long ldw,

@@ -75,7 +75,6 @@ def _declare(L):
         "mm_ln_mod_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _p],
         "mm_gated_residual": [_p, _p, _p, _p, _ll, _i, _i, _p],
         "mm_adamw": [_p, _p, _p, _p, _i, _p, _ll, _ll, _f, _f, _f, _f, _f, _f, _f, _f, _p, _p],
-        "mm_gemm_bf16": [_p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _p, _p],
         "mm_gemm_bf16_ws": [_p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _p, _p, _ll, _p],
         "mm_gemm_ws_bytes": [_i, _i, _i, _i, _i, _i],
         "mm_gemm_swiglu_bf16": [_p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _p, _p],
