@@ -242,9 +242,14 @@ class Linear(nn.Module):
 def _plain(*modules) -> bool:
     """Exactly this file's Linear / RMSNorm, nothing hooked, compiled or with a forward of its own (an adapter, a wrapper set on the
     instance): their weights may be used without calling them."""
-    return not torch.nn.modules.module._has_any_global_hook() and all(
-        type(m) in (Linear, RMSNorm) and "forward" not in m.__dict__ and getattr(m, "_compiled_call_impl", None) is None
-        and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) for m in modules)
+    if torch.nn.modules.module._has_any_global_hook():
+        return False
+    for m in modules:
+        d = m.__dict__
+        if (type(m) not in (Linear, RMSNorm) or "forward" in d or d.get("_compiled_call_impl") is not None or d["_forward_hooks"]
+                or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]):
+            return False
+    return True
 
 
 class VisionBlock(nn.Module):

@@ -302,24 +302,28 @@ def attention_cached(q, k, v, cache: dict, cos=None, sin=None):
 # --------------------------------------------------------------------------- generation: products of a few rows
 def norm_linear(x, norm_weight, eps, weight, bias=None):
     """``linear(rms_norm(x), weight, bias)``; a few rows that keep no graph take one kernel."""
-    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_supported(x, weight) and _nat().skinny_supported(x, weight, bias, norm=norm_weight):
-        return _nat().skinny_linear(x, weight, bias, norm_weight, eps)
+    if x.is_cuda and _TIER == "native":
+        nat = _nat()
+        if nat.skinny_supported(x, weight, bias, norm=norm_weight) and nat.gemm_supported(x, weight):
+            return nat.skinny_linear(x, weight, bias, norm_weight, eps)
     return linear(rms_norm(x, norm_weight, eps), weight, bias)
 
 
 def norm_linear_swiglu(x, norm_weight, eps, weight_gate_up):
     """``linear_swiglu(rms_norm(x), weight_gate_up)``; a few rows that keep no graph take one kernel."""
-    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_swiglu_supported(x, weight_gate_up) and \
-            _nat().skinny_supported(x, weight_gate_up, norm=norm_weight):
-        return _nat().skinny_linear(x, weight_gate_up, None, norm_weight, eps, swiglu=True)
+    if x.is_cuda and _TIER == "native":
+        nat = _nat()
+        if nat.skinny_supported(x, weight_gate_up, norm=norm_weight) and nat.gemm_swiglu_supported(x, weight_gate_up):
+            return nat.skinny_linear(x, weight_gate_up, None, norm_weight, eps, swiglu=True)
     return linear_swiglu(rms_norm(x, norm_weight, eps), weight_gate_up)
 
 
 def linear_add(x, weight, residual):
     """``residual + linear(x, weight)``; a few rows that keep no graph take one kernel."""
-    if _native(x) and x.dtype == torch.bfloat16 and _nat().gemm_supported(x, weight) and residual.shape == (x.shape[0], weight.shape[0]) and \
-            _nat().skinny_supported(x, weight, residual):
-        return _nat().skinny_linear(x, weight, residual=residual)
+    if x.is_cuda and _TIER == "native":
+        nat = _nat()
+        if nat.skinny_supported(x, weight, residual) and nat.gemm_supported(x, weight) and residual.shape == (x.shape[0], weight.shape[0]):
+            return nat.skinny_linear(x, weight, residual=residual)
     return residual + linear(x, weight)
 
 

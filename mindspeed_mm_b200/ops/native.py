@@ -152,13 +152,36 @@ class _NoGraph:
 _NO_GRAPH = _NoGraph()
 
 
+# bound once: looking them up costs more than calling them, and a generation step asks some fifty times
+_compiling, _transforms, _tracing = torch.compiler.is_compiling, torch._C._are_functorch_transforms_active, torch._C._get_tracing_state
+_wrapped, _forward_ad, _grad_enabled = torch._C._functorch.is_functorch_wrapped_tensor, torch.autograd.forward_ad, torch.is_grad_enabled
+
+
+def _plain_mode() -> bool:
+    """No transform, forward-mode level, tracer or compiler is active."""
+    return not (_compiling() or _transforms() or _forward_ad._current_level >= 0 or _tracing() is not None)
+
+
 def _keeps_no_graph(args) -> bool:
-    grad = torch.is_grad_enabled()
+    if not _plain_mode():
+        return False
+    grad = _grad_enabled()
     for a in args:
-        if isinstance(a, torch.Tensor) and ((grad and a.requires_grad) or torch._C._functorch.is_functorch_wrapped_tensor(a)):
+        if isinstance(a, torch.Tensor) and ((grad and a.requires_grad) or _wrapped(a)):
             return False
-    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
-                or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling())
+    return True
+
+
+def _plain_bf16(tensors) -> bool:
+    """:func:`_keeps_no_graph` of tensors (or None) that have to be bf16 on one device."""
+    if not _plain_mode():
+        return False
+    grad, bf16, dev, tensor = _grad_enabled(), torch.bfloat16, tensors[0].get_device(), torch.Tensor
+    for t in tensors:
+        # (a functorch wrapper is never a Parameter, which most of these are)
+        if t is not None and (t.dtype is not bf16 or t.get_device() != dev or (grad and t.requires_grad) or (type(t) is tensor and _wrapped(t))):
+            return False
+    return True
 
 
 def _run(fn, *args):
@@ -514,7 +537,8 @@ def _gemm_raw(a, b, out, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, bn=None):
 
 
 def _ok2d(t):
-    return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    st = t.stride()
+    return len(st) == 2 and st[1] == 1 and st[0] % 8 == 0 and t.data_ptr() % 16 == 0
 
 
 def gemm_supported(x, w) -> bool:
@@ -578,11 +602,12 @@ def mrope_tables(position_ids, head_dim, theta, section):
 def skinny_supported(x, *tensors, norm=None) -> bool:
     """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies.  The sizes are
     mm_gemv_bf16's own rule: x, and with a norm its weight too, have to fit a block's shared memory."""
-    if not _keeps_no_graph((x, norm) + tensors) or x.dim() != 2:
+    if x.dim() != 2:
         return False
     M, K = x.shape
-    return (1 <= M <= 4 and K % 8 == 0 and M * K <= 80 * 1024 and (norm is None or (M + 1) * K <= 112 * 1024) and _ok2d(x)
-            and all(t is None or (t.dtype == torch.bfloat16 and t.device == x.device) for t in (norm,) + tensors))
+    if not 1 <= M <= 4 or K % 8 or M * K > 80 * 1024 or (norm is not None and (M + 1) * K > 112 * 1024):
+        return False
+    return _plain_bf16((x, norm, *tensors)) and _ok2d(x)
 
 
 def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=False):
@@ -592,9 +617,7 @@ def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=Fal
     if bias is not None:
         bias = bias.contiguous()
     if norm is not None:
-        norm = norm.contiguous()
-        if norm.data_ptr() % 16:
-            norm = norm.clone()
+        norm = _dense(norm)
     if residual is not None and not _ok2d(residual):
         residual = residual.clone(memory_format=torch.contiguous_format)     # also where it only starts off an aligned address
     M, K = x.shape
@@ -609,13 +632,15 @@ def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=Fal
 
 def decode_attention_supported(q, k, v, k_old, v_old, cos, sin=None) -> bool:
     """Head dim 128, the new tokens' query heads of a group fill at most one 16-row tile, nothing keeps a graph."""
-    ts = [t for t in (q, k, v, k_old, v_old) if t is not None]
     T, Nq, D = q.shape
-    return (_keeps_no_graph(ts + [cos, sin]) and os.environ.get("MM_B200_FMHA", "1") == "1" and D == 128
-            and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts)
-            and all(t.shape[1:] == k.shape[1:] and t.shape[2] == D for t in (v, k_old, v_old) if t is not None)
-            and k.shape[2] == D and k.shape[0] == v.shape[0] == T and (k_old is None or k_old.shape[0] == v_old.shape[0])
-            and T >= 1 and Nq % k.shape[1] == 0 and T * (Nq // k.shape[1]) <= 16 and (cos is None or tuple(cos.shape) == (T, D)))
+    Tk, Nkv, Dk = k.shape
+    if D != 128 or Dk != D or not 1 <= T == Tk or v.shape != k.shape or Nq % Nkv or T * (Nq // Nkv) > 16:
+        return False
+    if k_old is not None and (k_old.shape != v_old.shape or k_old.shape[1:] != k.shape[1:]):
+        return False
+    if cos is not None and tuple(cos.shape) != (T, D):
+        return False
+    return os.environ.get("MM_B200_FMHA", "1") == "1" and _plain_bf16((q, k, v, k_old, v_old)) and _keeps_no_graph((cos, sin))
 
 
 def decode_attention(q, k, v, k_old, v_old, cos, sin):
@@ -624,13 +649,9 @@ def decode_attention(q, k, v, k_old, v_old, cos, sin):
     T, Nq, D = q.shape
     Nkv, past = k.shape[1], 0
     if cos is not None:
-        cos, sin = cos.to(torch.bfloat16).contiguous(), sin.to(torch.bfloat16).contiguous()
-        if (cos.data_ptr() | sin.data_ptr()) % 16:
-            cos, sin = cos.clone(), sin.clone()
+        cos, sin = _dense(cos.to(torch.bfloat16)), _dense(sin.to(torch.bfloat16))
     if k_old is not None:
-        k_old, v_old, past = k_old.contiguous(), v_old.contiguous(), k_old.shape[0]
-        if (k_old.data_ptr() | v_old.data_ptr()) % 16:
-            k_old, v_old = k_old.clone(), v_old.clone()
+        k_old, v_old, past = _dense(k_old), _dense(v_old), k_old.shape[0]
     k_new, v_new = (torch.empty(past + T, Nkv, D, dtype=torch.bfloat16, device=q.device) for _ in range(2))
     out = torch.empty(T, Nq, D, dtype=torch.bfloat16, device=q.device)
     ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
@@ -739,8 +760,8 @@ def fmha_supported(q, k, v) -> bool:
 def _dense_heads(t):
     """[T, N, D] with unit stride on D, D between heads and an 8-element aligned token stride (views into a
     fused qkv tensor qualify); anything else is copied."""
-    T, N, D = t.shape
-    if t.stride(2) != 1 or t.stride(1) != D or t.stride(0) % 8 or t.data_ptr() % 16:
+    st = t.stride()
+    if st[2] != 1 or st[1] != t.shape[2] or st[0] % 8 or t.data_ptr() % 16:
         t = t.contiguous()
     return t
 
