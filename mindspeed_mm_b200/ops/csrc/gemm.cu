@@ -507,7 +507,12 @@ MM_API int mm_gemv_bf16(const void* x, const void* w, const void* bias, const vo
 namespace {
 // Up to 4 rows: the weights are streamed once through CUDA cores.  The line lies there because a fifth row makes the fp32
 // multiply-adds, not HBM, the limit (8 multiply-adds per weight element and SM cycle at 4 rows), and x has to fit shared memory.
-bool skinny(int M, int N, int K) { return M <= 4 && N % 2 == 0 && K % 8 == 0 && (long long)M * K <= 80 * 1024; }
+// Four rows are at that limit: where the 128 x 256 tiles of the weight's `rows` rows keep half of the SMs busy, tiles are as fast or
+// faster (18944 x 3584: 44 us both ways, 37888 x 3584 67 against 73, 152064 x 3584 198 against 243; 8192 x 8192 64 against 56;
+// three rows 202 against 195 at 152064 x 3584).
+bool skinny(int M, int rows, int K) {
+    return M <= 4 && rows % 2 == 0 && K % 8 == 0 && (long long)M * K <= 80 * 1024 && (M < 4 || rows < 74 * 256);
+}
 }  // namespace
 
 // Bytes of workspace with which mm_gemm_bf16_ws splits the tail of this product along K (0: it would not).
@@ -548,7 +553,7 @@ MM_API int mm_gemm_swiglu_bf16(const void* A, const void* W, void* C, int M, int
     if ((lda | ldw | ldc) % 8) return -1;
     if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) return -2;
     if (M <= 0 || F <= 0 || K <= 0 || F % 128) return -3;
-    if (skinny(M, F, K)) return mm_gemv_bf16(A, W, nullptr, nullptr, nullptr, C, M, F, K, lda, ldw, 0, ldc, 0.f, 1, st);
+    if (skinny(M, 2 * F, K)) return mm_gemv_bf16(A, W, nullptr, nullptr, nullptr, C, M, F, K, lda, ldw, 0, ldc, 0.f, 1, st);
     return launch<256, false, false, true>(A, W, C, nullptr, M, F, K, lda, ldw, ldc, status, st);
 }
 

@@ -599,15 +599,16 @@ def mrope_tables(position_ids, head_dim, theta, section):
     return cos, sin
 
 
-def skinny_supported(x, *tensors, norm=None) -> bool:
+def skinny_supported(x, w, *tensors, norm=None) -> bool:
     """Up to 4 bf16 rows that keep no graph: the product kernel of csrc/decode.cu with its fused ends applies.  The sizes are
-    mm_gemv_bf16's own rule: x, and with a norm its weight too, have to fit a block's shared memory."""
+    mm_gemv_bf16's own rule: x, and with a norm its weight too, have to fit a block's shared memory; and four rows against a weight
+    whose tiles keep half of the SMs busy are left to the tensor cores (``skinny`` in csrc/gemm.cu)."""
     if x.dim() != 2:
         return False
     M, K = x.shape
-    if not 1 <= M <= 4 or K % 8 or M * K > 80 * 1024 or (norm is not None and (M + 1) * K > 112 * 1024):
+    if not 1 <= M <= 4 or K % 8 or M * K > 80 * 1024 or (norm is not None and (M + 1) * K > 112 * 1024) or (M == 4 and w.shape[0] >= 74 * 256):
         return False
-    return _plain_bf16((x, norm, *tensors)) and _ok2d(x)
+    return _plain_bf16((x, w, norm, *tensors)) and _ok2d(x)
 
 
 def skinny_linear(x, w, bias=None, norm=None, eps=0.0, residual=None, swiglu=False):

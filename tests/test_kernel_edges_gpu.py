@@ -66,10 +66,12 @@ def test_grouped_gemm_gradients_with_empty_experts(K, N):
         a += c
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 136, 264), (2, 4608, 3584), (3, 24, 1032), (4, 256, 18944), (1, 3584, 18944), (5, 136, 264)])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 136, 264), (2, 4608, 3584), (3, 24, 1032), (4, 256, 18944), (1, 3584, 18944), (5, 136, 264),
+                                   (4, 18816, 264), (4, 18944, 264), (3, 18944, 264), (4, 9344, 264), (4, 9472, 264)])
 @pytest.mark.parametrize("norm,ends", [(False, "none"), (True, "bias"), (False, "residual"), (True, "swiglu")])
 def test_product_of_a_few_rows(M, N, K, norm, ends):
-    """Both sides of the 4-row rule (5 rows run on tiles); 4 x 18944 is close to the most that the kernel takes."""
+    """Both sides of the 4-row rule (5 rows run on tiles, and 4 rows against 18944 or more weight rows, which SwiGLU has twice of);
+    4 x 18944 is close to the most that the kernel takes."""
     torch.manual_seed(M * 1000 + N)
     x, g = torch.randn(M, K, device=DEV).bfloat16(), (1 + 0.1 * torch.randn(K, device=DEV)).bfloat16()
     n = 2 * N if ends == "swiglu" else N

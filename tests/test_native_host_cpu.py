@@ -115,3 +115,9 @@ def test_wrapped_modules_are_called_in_the_generation_path(name, how):
     y = head(x) if name == "norm" else layer(x, torch.ones(3, 8), torch.zeros(3, 8), None, None, cache={})
     y.sum().backward()
     assert calls
+
+
+def test_four_rows_against_a_wide_weight_take_tiles():
+    x = torch.zeros(4, 16, dtype=torch.bfloat16)
+    takes = [native.skinny_supported(x[:m], torch.zeros(n, 16, dtype=torch.bfloat16)) for m, n in ((4, 18936), (4, 18944), (3, 18944))]
+    assert takes == [True, False, True]
