@@ -371,19 +371,23 @@ struct SplitPlan {
 };
 
 // parts: the number that the estimate below makes fastest, 1 if the gain is under 4 us.  A 64-deep step of a 128 x 256 tile takes
-// 0.44 us (1.4 PFLOP/s over 148 SMs); an item's sums are written and read once at about 4 TB/s, a further launch and the shorter
-// main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and lost 2 us).
+// 0.44 us (1.4 PFLOP/s over 148 SMs), and no product is over before its operands have come once at 6.2 TB/s: a single row of tiles
+// over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about 4 TB/s, a
+// further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
+// lost 2 us).
 // Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 218 / 151 us, 405 x 3584 x 37888 (56) 216 / 122,
-// 8192 x 3584 x 18944 (896) 828 / 776, 8192 x 3584 x 152064 (7 rounds become 6 and a part) 6920 / 6210, 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.
+// 8192 x 3584 x 18944 (896) 828 / 776, 8192 x 3584 x 152064 (7 rounds become 6 and a part) 6920 / 6210, 3840 x 1280 x 8192 (150)
+// 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands: 85 x 25368 x 27344 247 / 279, 126 x 26744 x 24168 251 / 271.
 inline SplitPlan split_plan(int M, int N, int K, int BN, int sms) {
-    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK, rem = tiles % sms;
+    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK, full = tiles / sms, rem = tiles % sms;
     SplitPlan best{tiles, 1};
     if (!rem) return best;
-    const double unit = kb * 0.44 * BN / 256;
-    double least = unit - 4.0;
+    const double unit = kb * 0.44 * BN / 256, operands = 2.0 * K * ((double)M + N) / 6.2e6;
+    auto at_least = [&](double t) { return t > operands ? t : operands; };
+    double least = at_least(unit * (full + 1)) - 4.0;
     for (int parts = 2; parts <= 16 && kb / parts >= 4; ++parts) {
         const int rounds = (rem * parts + sms - 1) / sms;
-        const double t = unit * rounds / parts + 6.0 + rem * parts * (BM * BN * 8e-6 / 4.0);
+        const double t = at_least(unit * full + unit * rounds / parts) + 6.0 + rem * parts * (BM * BN * 8e-6 / 4.0);
         if (t < least) {
             least = t;
             best = {tiles - rem, parts};

@@ -304,9 +304,10 @@ def test_attention_tile_lists(lens, causal):
 
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K,splits", [(1421, 3584, 3600, True), (1409, 3592, 4104, True), (1, 264, 18952, None), (5, 8, 18944, True), (136, 520, 8200, True),
-                                          (128 * 148, 256, 8192, False), (128 * 149, 256, 8192, True), (128, 256, 256, False)])
+                                          (128 * 148, 256, 8192, False), (128 * 149, 256, 8192, True), (128, 256, 256, False), (85, 25368, 8200, False)])
 def test_products_with_a_split_tail(layout, M, N, K, splits):
-    """Ragged rows, columns and depths, a lone tail and one behind whole rounds; both sides of the rule."""
+    """Ragged rows, columns and depths, a lone tail and one behind whole rounds; both sides of the rule (one row of tiles over a large
+    weight is bound by its bytes and stays whole)."""
     if layout == "tn" and M % 8:
         M = M // 8 * 8 + 8                                        # the rows are the contiguous dimension there
     torch.manual_seed(M)
