@@ -93,6 +93,7 @@ def _declare(L):
         "mm_moe_unpermute": [_p, _p, _p, _p, _i, _i, _i, _p],
         "mm_moe_unpermute_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_moe_route": [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p],
+        "mm_moe_route_scratch": [_i, _i],
         "mm_delta_heads_fwd": [_p, _p, _p, _p, _p, _i, _i, _i, _i, _f, _p],
         "mm_delta_heads_bwd": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_conv1d_fwd": [_p, _ll, _p, _p, _p, _i, _i, _i, _i, _p],
@@ -122,7 +123,7 @@ def _declare(L):
         if hasattr(L, name):
             fn = getattr(L, name)
             fn.argtypes = args
-            fn.restype = _ll if name == "mm_gemm_ws_bytes" else _i
+            fn.restype = _ll if name in ("mm_gemm_ws_bytes", "mm_moe_route_scratch") else _i
             _STATUS[name] = True
         else:
             _STATUS[name] = False
@@ -945,21 +946,22 @@ class _Route(torch.autograd.Function):
         ids = topk_ids.to(torch.int64).contiguous()
         R = (n + num_experts * 127 + 127) // 128 * 128            # static upper bound of off[E]
         off = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
-        scratch = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)       # counts, out-of-range flag
-        row_of_pair = torch.zeros(n, dtype=torch.int32, device=dev)
+        scratch = torch.empty(lib().mm_moe_route_scratch(n, num_experts), dtype=torch.int32, device=dev)
+        rows = torch.zeros(n + 1, dtype=torch.int32, device=dev)                    # rows of the pairs, out-of-range flag
+        row_of_pair, bad = rows[:n], rows[n:]
         src_of_row = torch.empty(R, dtype=torch.int32, device=dev)
         _check(lib().mm_moe_route(ids.data_ptr(), n, k, num_experts, R, scratch.data_ptr(), off.data_ptr(), row_of_pair.data_ptr(),
-                                  src_of_row.data_ptr(), scratch[num_experts:].data_ptr(), _st()), "moe_route")
-        return off, row_of_pair, src_of_row, scratch
+                                  src_of_row.data_ptr(), bad.data_ptr(), _st()), "moe_route")
+        return off, row_of_pair, src_of_row, bad
 
 
 def _route(topk_ids, num_experts: int):
     """Launches the routing kernels; returns (off, row_of_pair, src_of_row, R, check).  ``check()`` waits for them (not for
     work queued behind them) and raises if an expert number was out of range."""
-    off, row_of_pair, src_of_row, scratch = _run(_Route, topk_ids, int(num_experts))
+    off, row_of_pair, src_of_row, flag = _run(_Route, topk_ids, int(num_experts))
     R = src_of_row.shape[0]
     bad = torch.empty(1, dtype=torch.int32, pin_memory=True)
-    bad.copy_(scratch[num_experts:], non_blocking=True)
+    bad.copy_(flag, non_blocking=True)
     done = torch.cuda.Event()
     done.record()
 

@@ -20,10 +20,15 @@ def _close(a, b, rtol, atol):
     assert float((a - b).norm()) <= rtol * float(b.norm()) + 0.25 * atol * a.numel() ** 0.5
 
 
-@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (1, 8, 8), (37, 2, 5), (513, 8, 128), (4096, 3, 300)])
-def test_moe_routing_matches_a_stable_sort(T, k, E):
+@pytest.mark.parametrize("T,k,E", [(0, 2, 3), (1, 1, 1), (1, 8, 8), (37, 2, 5), (128, 8, 9), (513, 8, 128), (4096, 3, 300), (341, 3, 300), (40000, 8, 7),
+                                   (40000, 8, 513), (300, 2, 6000), (300, 2, 6001), (70, 1, 20000)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_moe_routing_matches_a_stable_sort(T, k, E, skew):
+    """One chunk of pairs and several, more chunks than threads of the scan, blocks of eight warps and of one; all pairs of one expert."""
     g = torch.Generator().manual_seed(T)
     ids = torch.randint(0, max(1, E - 2), (T, k), generator=g)               # the last experts stay empty where E > 2
+    if skew:
+        ids[:] = E // 2
     off, row_of_pair, src_of_row, R = (t.cpu() if torch.is_tensor(t) else t for t in native.aligned_routing(ids.to(DEV), E))
     flat = ids.reshape(-1)
     counts = torch.bincount(flat, minlength=E)
@@ -36,9 +41,12 @@ def test_moe_routing_matches_a_stable_sort(T, k, E):
 
 
 def test_moe_routing_refuses_expert_numbers_out_of_range():
-    for wrong in (-1, 4):
-        with pytest.raises(RuntimeError):
-            native.aligned_routing(torch.tensor([[0, wrong]], device=DEV), 4)
+    for wrong in (-1, 4, 2 ** 40):
+        for before in (0, 3000):
+            ids = torch.zeros(before + 1, 2, dtype=torch.int64, device=DEV)
+            ids[-1, 1] = wrong
+            with pytest.raises(RuntimeError):
+                native.aligned_routing(ids, 4)
 
 
 @pytest.mark.parametrize("K,N", [(256, 128), (128, 256), (384, 512)])
