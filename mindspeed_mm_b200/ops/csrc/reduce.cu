@@ -3,31 +3,43 @@
 
 namespace {
 
-constexpr int kWarps = 8, kCols = 256;      // a warp reads 256 columns of a row (16 bytes a lane), a block 8 rows at a time
+constexpr int kWarps = 8, kCols = 256;      // a warp reads 256 columns of a row (16 bytes a lane), or several rows of a narrower matrix
+constexpr int kFlight = 8;                  // rows that a lane has in flight
+
+// Lanes of a warp that share a row: a power of two, 32 from 256 columns on.
+__host__ __device__ __forceinline__ int lanes_per_row(int cols) {
+    int n = 1;
+    while (n < 32 && n * 8 < cols) n *= 2;
+    return n;
+}
 
 // partial[b][split][c] = sum over the rows of batch b that the split walks of x[r][c] (times y[r][c] if GATED, which also writes
-// out = x * gate[b]).  Blocks: (batch and column group, row split); the warps of a block take every 8th row, four rows in flight each,
-// and meet in shared memory.  Rows are split so that the grid fills the SMs whatever the width is: 8192 x 3840 -> 15 x 40 blocks.
+// out = x * gate[b]).  Blocks: (batch and column group, row split); the warps of a block take every 8th row (or group of rows of a
+// narrow matrix) and meet in shared memory.  Rows are split so that the grid fills the SMs whatever the width is (see splits_of).
+// Bound by HBM.  Plain sums have eight rows a lane in flight, asked for before the first is added: 75600 x 13824 347 us, 75600 x 5120
+// 146, 300000 x 8 15; 476, 187 and 46 in a loop unrolled four times with a row per warp whatever its width, 370, 182 and 20 as
+// torch.sum.  With a gate, which reads two rows and writes one, that loop stays: 1 x 32760 x 5120 183 us, 228 with eight in flight.
 template <bool GATED>
 __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y,
                                                                 const bf16* __restrict__ gate, bf16* __restrict__ out,
                                                                 float* __restrict__ partial, int rows, int cols, long long ldx) {
     __shared__ float tile[kWarps][kCols + 4];
     const int groups = (cols + kCols - 1) / kCols, b = blockIdx.x / groups, c0 = (blockIdx.x - b * groups) * kCols;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = c0 + lane * 8;
-    const int split = blockIdx.y, splits = gridDim.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per_row = lanes_per_row(cols), sub = lane / per_row, at_once = 32 / per_row;
+    const int c = c0 + (lane - sub * per_row) * 8, split = blockIdx.y, splits = gridDim.y;
+    const long long step = (long long)splits * kWarps * at_once;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (c < cols) {
         const bf16* xb = x + (size_t)b * rows * ldx + c;
         float g[8];
         if constexpr (GATED) unpack8(*reinterpret_cast<const Vec8*>(gate + (size_t)b * cols + c), g);
+        long long r = (long long)(split * kWarps + warp) * at_once + sub;
+        if constexpr (GATED) {
 #pragma unroll 4
-        for (int r = split * kWarps + warp; r < rows; r += splits * kWarps) {
-            float f[8];
-            unpack8(*reinterpret_cast<const Vec8*>(xb + (size_t)r * ldx), f);
-            if constexpr (GATED) {
+            for (; r < rows; r += step) {
                 const size_t at = ((size_t)b * rows + r) * cols + c;
-                float h[8];
+                float f[8], h[8];
+                unpack8(*reinterpret_cast<const Vec8*>(xb + r * ldx), f);
                 unpack8(*reinterpret_cast<const Vec8*>(y + at), h);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
@@ -35,14 +47,30 @@ __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __r
                     f[k] *= g[k];
                 }
                 *reinterpret_cast<Vec8*>(out + at) = pack8(f);
-            } else {
+            }
+        } else {
+            for (; r < rows; r += kFlight * step) {
+                Vec8 v[kFlight];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] += f[k];
+                for (int j = 0; j < kFlight; ++j)
+                    if (r + j * step < rows) v[j] = *reinterpret_cast<const Vec8*>(xb + (r + j * step) * ldx);
+#pragma unroll
+                for (int j = 0; j < kFlight; ++j) {
+                    if (r + j * step >= rows) break;
+                    float f[8];
+                    unpack8(v[j], f);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[k] += f[k];
+                }
             }
         }
     }
+    for (int o = per_row; o < 32; o <<= 1)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) tile[warp][lane * 8 + k] = acc[k];
+        for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    if (sub == 0)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) tile[warp][lane * 8 + k] = acc[k];
     __syncthreads();
     const int col = c0 + threadIdx.x;
     if (col < cols) {
@@ -87,11 +115,11 @@ __global__ void __launch_bounds__(256) scale_kernel(bf16* __restrict__ x, long l
     for (long long i = (n & ~15LL) + first; i < n; i += stride) x[i] = __float2bfloat16(__bfloat162float(x[i]) * s);
 }
 
-int splits_of(int rows, int cols, int batches) {
+int splits_of(int rows, int cols, int batches, bool gated) {
     if (rows < 1 || cols < 1 || batches < 1) return 1;
-    const long long groups = (long long)((cols + kCols - 1) / kCols) * batches;
-    long long s = (148 * 4 + groups - 1) / groups;                   // four blocks an SM
-    const long long most = (rows + kWarps * 4 - 1) / (kWarps * 4);     // at least four rows a warp
+    const long long groups = (long long)((cols + kCols - 1) / kCols) * batches, at_once = 32 / lanes_per_row(cols) * kWarps;
+    long long s = (148 * (gated ? 4 : 8) + groups - 1) / groups;     // blocks an SM: 8 for plain sums (4: 75600 x 13824 392 us, 8: 347)
+    const long long most = (rows + at_once * 4 - 1) / (at_once * 4);   // at least four rows a lane
     s = s < most ? s : most;
     return (int)(s < 1 ? 1 : s);
 }
@@ -99,14 +127,14 @@ int splits_of(int rows, int cols, int batches) {
 }  // namespace
 
 // Row splits, i.e. scratch of batches * splits * cols floats for the two entries below.
-MM_API int mm_column_splits(int rows, int cols, int batches) { return splits_of(rows, cols, batches); }
+MM_API int mm_column_splits(int rows, int cols, int batches, int gated) { return splits_of(rows, cols, batches, gated != 0); }
 
 // sums[c] (bf16) = sum over r of x[r, c], fp32 inside.  x: [rows, cols] bf16 with ldx elements between rows; cols and ldx multiples
 // of 8, 16-byte aligned.  8192 x (3840 + 1280 + 6912 + 1280): see native.py.
 MM_API int mm_column_sum(const void* x, void* sums, float* partial, int rows, int cols, long long ldx, cudaStream_t st) {
     if (cols % 8 || ldx % 8 || ((uintptr_t)x & 15)) return -1;
     if (rows < 1 || cols < 1) return -2;
-    const int splits = splits_of(rows, cols, 1);
+    const int splits = splits_of(rows, cols, 1, false);
     column_sum_kernel<false><<<dim3((cols + kCols - 1) / kCols, splits), kWarps * 32, 0, st>>>((const bf16*)x, nullptr, nullptr, nullptr,
                                                                                                   partial, rows, cols, ldx);
     fold_splits_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, st>>>(partial, (bf16*)sums, splits, cols);
@@ -117,13 +145,13 @@ MM_API int mm_column_sum(const void* x, void* sums, float* partial, int rows, in
 // [batches, rows, cols]; one pass over dout and y.  Nothing to sum over (rows == 0): zeros.
 MM_API int mm_gated_residual_bwd(const void* dout, const void* y, const void* gate, void* dy, void* dgate, float* partial, int batches,
                                  int rows, int cols, cudaStream_t st) {
-    if (cols % 8 || ((uintptr_t)dout | (uintptr_t)y | (uintptr_t)gate | (uintptr_t)dy) & 15) return -1;
+    if (cols % 8 || ((uintptr_t)dout | (uintptr_t)y | (uintptr_t)gate | (uintptr_t)dy | (uintptr_t)dgate) & 15) return -1;
     if (rows < 0 || cols < 0 || batches < 0) return -2;
     if (!batches || !cols) return 0;
     if (!rows) return (int)cudaMemsetAsync(dgate, 0, (size_t)batches * cols * sizeof(bf16), st);
-    const long long blocks = (long long)batches * ((cols + 31) / 32);       // a gate per token is as many batches as there are tokens
+    const long long blocks = (long long)batches * ((cols + 31) / 32);
     if (blocks > 0x7fffffffLL) return -2;
-    const int splits = splits_of(rows, cols, batches);
+    const int splits = splits_of(rows, cols, batches, true);
     column_sum_kernel<true><<<dim3(batches * ((cols + kCols - 1) / kCols), splits), kWarps * 32, 0, st>>>(
         (const bf16*)dout, (const bf16*)y, (const bf16*)gate, (bf16*)dy, partial, rows, cols, cols);
     fold_splits_kernel<<<(int)blocks, dim3(32, 8), 0, st>>>(partial, (bf16*)dgate, splits, cols);

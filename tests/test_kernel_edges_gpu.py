@@ -217,8 +217,10 @@ def test_attention_over_long_keys(lens_q, lens_k, nq, nkv, D, causal, grow):
     assert float((lse - want_lse.reshape(lse.shape)).abs().max()) < 2e-3 * (1 + float(want_lse.abs().max()))
 
 
-@pytest.mark.parametrize("rows,cols,pitch", [(1, 8, 8), (3, 264, 264), (33, 256, 512), (8192, 1280, 1280), (1000, 6912, 6920), (40000, 16, 16)])
+@pytest.mark.parametrize("rows,cols,pitch", [(1, 8, 8), (3, 264, 264), (33, 256, 512), (8192, 1280, 1280), (1000, 6912, 6920), (40000, 16, 16), (9, 8, 16),
+                                             (5000, 24, 32), (777, 128, 128), (777, 136, 136), (65000, 248, 256)])
 def test_column_sums(rows, cols, pitch):
+    """One to 32 lanes a row, the last row of a lane's eight, columns of a wider matrix."""
     torch.manual_seed(rows)
     x = torch.randn(rows, pitch, device=DEV).bfloat16()[:, :cols]
     # fp32 sums rounded once to bf16
@@ -227,7 +229,7 @@ def test_column_sums(rows, cols, pitch):
 
 @pytest.mark.parametrize("B,S,H", [(1, 1, 8), (2, 7, 264), (1, 7800, 1536), (3, 100, 5120), (70000, 1, 264), (2, 0, 64), (0, 3, 64)])
 def test_gated_residual_gradients(B, S, H):
-    """A gate per token is 70000 batches; without rows the gate's gradient is zero."""
+    """A gate per token is 70000 batches; without rows its gradient is zero."""
     torch.manual_seed(S)
     x, y, do = (torch.randn(B, S, H, device=DEV).bfloat16().requires_grad_(i < 2) for i in range(3))
     gate = torch.randn(B, 1, H, device=DEV).bfloat16().requires_grad_()
