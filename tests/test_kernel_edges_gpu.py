@@ -227,9 +227,9 @@ def test_column_sums(rows, cols, pitch):
     _close(native.column_sum(x), x.double().sum(0), rtol=4e-3, atol=1e-3)
 
 
-@pytest.mark.parametrize("B,S,H", [(1, 1, 8), (2, 7, 264), (1, 7800, 1536), (3, 100, 5120), (70000, 1, 264), (2, 0, 64), (0, 3, 64)])
+@pytest.mark.parametrize("B,S,H", [(1, 1, 8), (2, 7, 264), (1, 7800, 1536), (3, 100, 5120), (70000, 1, 264), (300, 7, 264), (300, 8, 264), (2, 0, 64), (0, 3, 64)])
 def test_gated_residual_gradients(B, S, H):
-    """A gate per token is 70000 batches; without rows its gradient is zero."""
+    """Both sides of the rule for short batches (7 and 8 rows); a gate per token is 70000 batches; without rows its gradient is zero."""
     torch.manual_seed(S)
     x, y, do = (torch.randn(B, S, H, device=DEV).bfloat16().requires_grad_(i < 2) for i in range(3))
     gate = torch.randn(B, 1, H, device=DEV).bfloat16().requires_grad_()
