@@ -274,9 +274,9 @@ def test_rms_norm_of_columns_of_a_wider_matrix(T, H):
     assert not dwide[:, :H].any() and not dwide[:, 2 * H:].any()
 
 
-@pytest.mark.parametrize("B,S,H", [(2, 5, 64 * 8), (1, 777, 2048), (1, 40, 2056), (2, 33, 4104), (1, 3, 8192)])
+@pytest.mark.parametrize("B,S,H", [(2, 5, 64 * 8), (1, 777, 2048), (1, 40, 2056), (2, 33, 4104), (1, 3, 8192), (18, 32, 264), (19, 32, 264), (700, 2, 264)])
 def test_layer_norm_modulate_gradients(B, S, H):
-    """Each number of vectors per thread of the backward kernel."""
+    """Each number of vectors per thread of the backward kernel; both folds of its partial sums, over 32 and 31 to one rows."""
     torch.manual_seed(H)
     x, sc, sh = torch.randn(B, S, H, device=DEV).bfloat16(), torch.randn(B, 1, H, device=DEV).bfloat16(), torch.randn(B, 1, H, device=DEV).bfloat16()
     dy = torch.randn(B, S, H, device=DEV).bfloat16()
