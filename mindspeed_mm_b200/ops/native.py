@@ -1183,6 +1183,15 @@ def delta_heads(x, hk, hv, dv, eps=1e-6):
     return _run(_DeltaHeads, x, hk, hv, dv, eps)
 
 
+def _gate_rows(z, D):
+    """The gate as the kernels read it: (tensor, rows a token, elements between tokens).  [tokens, heads, D] with dense heads may have
+    its tokens apart (the gate's columns of a fused projection); anything else is dense rows."""
+    st = z.stride()
+    if len(st) == 3 and st[2] == 1 and st[1] == D and st[0] % 8 == 0 and z.data_ptr() % 16 == 0 and z.shape[0] * z.shape[1] < 2 ** 31:
+        return z, max(1, z.shape[1]), st[0]
+    return _dense(z.reshape(-1, D)), 1, D
+
+
 class _GatedRMSNorm(torch.autograd.Function):
     """``rmsnorm(x) * w * silu(z)`` over the last dim (<= 256): x fp32 or bf16, z / w / result bf16."""
 
@@ -1191,28 +1200,25 @@ class _GatedRMSNorm(torch.autograd.Function):
         D = x.shape[-1]
         x2, wc = _dense(x.reshape(-1, D)), _dense(w)
         rows = x2.shape[0]
-        # z of [tokens, heads, D] with dense heads may have its tokens apart (the gate's columns of a fused projection)
-        if z.dim() == 3 and z.stride(2) == 1 and z.stride(1) == D and z.stride(0) % 8 == 0 and z.data_ptr() % 16 == 0 and rows < 2 ** 31:
-            z2, zh, ldz = z, max(1, z.shape[1]), z.stride(0)
-        else:
-            z2, zh, ldz = _dense(z.reshape(-1, D)), 1, D
+        z2, zh, ldz = _gate_rows(z, D)
         y = torch.empty(rows, D, dtype=torch.bfloat16, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         _check(lib().mm_gated_rms_fwd(x2.data_ptr(), int(x2.dtype == torch.float32), z2.data_ptr(), wc.data_ptr(), y.data_ptr(),
                                       rstd.data_ptr(), rows, D, zh, ldz, eps, _st()), "gated_rms_fwd")
         ctx.save_for_backward(x2, z2, wc, rstd)
-        ctx.shapes, ctx.gate_rows = (x.shape, z.shape), (zh, ldz)
+        ctx.shapes = (x.shape, z.shape)
         return y.view(z.shape)
 
     @staticmethod
     def backward(ctx, dy):
         x2, z2, wc, rstd = ctx.saved_tensors
         rows, D = x2.shape
+        z2, zh, ldz = _gate_rows(z2, D)        # read off what was saved: a hook (offload to the host) gives back a dense copy
         dy2 = _dense(dy.reshape(rows, D))
         dx, dz = torch.empty_like(x2), torch.empty(rows, D, dtype=z2.dtype, device=z2.device)
         dw = torch.zeros(D, dtype=torch.float32, device=x2.device)
         _check(lib().mm_gated_rms_bwd(x2.data_ptr(), int(x2.dtype == torch.float32), z2.data_ptr(), wc.data_ptr(), dy2.data_ptr(),
-                                      rstd.data_ptr(), dx.data_ptr(), dz.data_ptr(), dw.data_ptr(), rows, D, *ctx.gate_rows, _st()),
+                                      rstd.data_ptr(), dx.data_ptr(), dz.data_ptr(), dw.data_ptr(), rows, D, zh, ldz, _st()),
                "gated_rms_bwd")
         return dx.view(ctx.shapes[0]), dz.view(ctx.shapes[1]), dw.to(wc.dtype), None
 

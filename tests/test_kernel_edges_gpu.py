@@ -529,3 +529,17 @@ def test_rms_norm_of_rows_that_start_anywhere(T, H, start):
         y = ops.rms_norm(a, b)
         outs.append([y.detach(), *torch.autograd.grad(y, [a, b], g)])
     assert all(torch.equal(p, q) for p, q in zip(*outs))
+
+
+def test_columns_of_a_wider_matrix_offloaded_to_the_host_and_back():
+    """What is saved where it lies comes back dense; the gradients stay the same."""
+    from mindspeed_mm_b200.runtime.features import ActivationOffload
+    wide, w, cw, o = (torch.randn(*s, device=DEV).bfloat16() for s in ((33, 1536), (512,), (512, 4), (33, 4, 128)))
+    outs = []
+    for enabled in (False, True):
+        x = wide[:, 512:1024].detach().requires_grad_()
+        with ActivationOffload(enabled=enabled, min_bytes=0) as a:
+            ys = [ops.rms_norm(x, w), ops.causal_conv1d(x, cw, None, "silu", None), ops.gated_rms_norm(o, x.view(33, 4, 128), w[:128])]
+        assert (a.bytes_offloaded > 0) == enabled
+        outs.append([g for y in ys for g in torch.autograd.grad(y, [x], torch.ones_like(y))])
+    assert all(torch.equal(p, q) for p, q in zip(*outs))

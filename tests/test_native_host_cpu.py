@@ -121,3 +121,31 @@ def test_four_rows_against_a_wide_weight_take_tiles():
     x = torch.zeros(4, 16, dtype=torch.bfloat16)
     takes = [native.skinny_supported(x[:m], torch.zeros(n, 16, dtype=torch.bfloat16)) for m, n in ((4, 18936), (4, 18944), (3, 18944))]
     assert takes == [True, False, True]
+
+
+@pytest.mark.parametrize("name", ["rms_norm", "causal_conv1d", "gated_rms_norm"])
+def test_backward_reads_the_layout_of_what_the_hooks_give_back(name, monkeypatch):
+    """Columns of a wider matrix are saved as they lie; saved-tensor hooks (activations offloaded to the host) return dense copies.
+    The pitch that the backward kernel gets has to be the one of the tensor it gets."""
+    calls = {}
+
+    class Fake:
+        def __getattr__(self, fn):
+            return lambda *a: calls.__setitem__(fn, a) or (1 if fn.endswith("_grid") else 0)
+    monkeypatch.setattr(native, "lib", lambda: Fake())
+    monkeypatch.setattr(native, "_st", lambda: 0)
+    wide = torch.randn(6, 3 * 512).bfloat16()
+    x, w = wide[:, 512:1024].detach().requires_grad_(), torch.randn(512).bfloat16()
+    back, given = [], {}
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: back.append(t.clone(memory_format=torch.contiguous_format)) or back[-1]):
+        if name == "rms_norm":
+            y, ld = native.rms_norm(x, w), lambda a: (a[0], a[1])
+        elif name == "causal_conv1d":
+            y, ld = native.causal_conv1d(x, torch.randn(512, 4).bfloat16(), "silu", None), lambda a: (a[0], a[1])
+        else:
+            z = x.detach().view(6, 4, 128).requires_grad_()
+            y, ld = native.gated_rms_norm(torch.randn(6, 4, 128).bfloat16(), z, torch.randn(128).bfloat16()), lambda a: (a[2], a[9] if len(a) == 12 else a[12])
+        assert ld(next(a for fn, a in calls.items() if "_fwd" in fn))[1] == 3 * 512           # read in place
+        y.backward(torch.ones_like(y))
+    pointer, pitch = ld(next(a for fn, a in calls.items() if "_bwd" in fn and not fn.endswith("_grid")))
+    assert any(t.data_ptr() == pointer for t in back) and pitch == 512
