@@ -238,6 +238,11 @@ def gated_delta_rule_varlen(q, k, v, g, beta, cu_seqlens, scale: Optional[float]
                 raise RuntimeError(f"cu_seqlens covers {covered} tokens, the tensors hold {q.shape[0]}")
             from . import native
             return native._run(_GatedDelta, q, k, v, g, beta, lay, scale)
+    return _by_prologue(q, k, v, g, beta, lay, scale)
+
+
+def _by_prologue(q, k, v, g, beta, lay: ChunkLayout, scale: float):
+    """The operator with the prologue in PyTorch, which autograd differentiates."""
     qc, kc, vc = (lay.scatter(t.float()) for t in (q, k, v))
     gcn, bc = (lay.scatter(t.float()) for t in (g, beta))
     W, Qg, Kd, At, U, gamma = chunk_prologue(qc, kc, vc, gcn, bc, scale)
@@ -276,15 +281,23 @@ class _GatedDelta(torch.autograd.Function):
         native._check(L.mm_gdn_layout(O.data_ptr(), out.data_ptr(), lay.chunk_tok0.data_ptr(), lay.chunk_len.data_ptr(), H, NC, 0,
                                       native._st()), "gdn_layout")
         if keep:
-            ctx.save_for_backward(qb, kb, vb, gf, bf, W, Qg, Kd, At, gamma, Vn, SprevT)
-            ctx.meta = (lay, scale, g.dtype, beta.dtype)
+            ctx.save_for_backward(q, k, v, g, beta, W, Qg, Kd, At, gamma, Vn, SprevT)
+            ctx.meta = (lay, scale)
         return out.to(v.dtype)
 
     @staticmethod
     def backward(ctx, dout):
         from . import native
         q, k, v, g, beta, W, Qg, Kd, At, gamma, Vn, SprevT = ctx.saved_tensors
-        lay, scale, g_dtype, beta_dtype = ctx.meta
+        lay, scale = ctx.meta
+        if torch.is_grad_enabled():          # create_graph: the gradient itself is differentiated, as far as the prologue goes
+            needs = ctx.needs_input_grad[:5]
+            grads = iter(torch.autograd.grad(_by_prologue(q, k, v, g, beta, lay, scale), [t for t, n in zip((q, k, v, g, beta), needs) if n],
+                                             dout, create_graph=True))
+            return (*(next(grads) if n else None for n in needs), None, None)
+        g_dtype, beta_dtype = g.dtype, beta.dtype
+        q, k, v = (native._dense(t) for t in (q, k, v))
+        g, beta = g.float().contiguous(), beta.float().contiguous()
         T, H, K = q.shape
         NC, dev, L, st = lay.NC, q.device, native.lib(), native._st()
         dout = native._dense(dout.to(torch.bfloat16))

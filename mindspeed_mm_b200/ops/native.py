@@ -1171,6 +1171,8 @@ class _DeltaHeads(torch.autograd.Function):
         dx = torch.empty(T, 2 * hk * 128 + v_width, dtype=torch.bfloat16, device=q.device)
         _check(lib().mm_delta_heads_bwd(q.data_ptr(), k.data_ptr(), r.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                                         dx.data_ptr(), T, hk, q.shape[1] // hk, v_width, _st()), "delta_heads_bwd")
+        if torch.is_grad_enabled():          # create_graph: the values' columns are dv itself
+            dx = torch.cat([dx[:, :2 * hk * 128], dv.reshape(T, v_width)], 1)
         return dx, None, None, None, None
 
 

@@ -543,3 +543,23 @@ def test_columns_of_a_wider_matrix_offloaded_to_the_host_and_back():
         assert (a.bytes_offloaded > 0) == enabled
         outs.append([g for y in ys for g in torch.autograd.grad(y, [x], torch.ones_like(y))])
     assert all(torch.equal(p, q) for p, q in zip(*outs))
+
+
+def test_delta_rule_gradients_keep_a_graph_where_they_had_one():
+    """create_graph: through the prologue of the delta rule, and through the values of its heads."""
+    torch.manual_seed(0)
+    T, H, cu = 130, 2, [0, 70, 130]
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, H, 128, device=DEV), dim=-1).bfloat16().requires_grad_()  # noqa: E731
+    leaves = [unit(), unit(), torch.randn(T, H, 128, device=DEV).bfloat16().requires_grad_(), (-torch.rand(T, H, device=DEV)).requires_grad_(),
+              torch.rand(T, H, device=DEV).requires_grad_()]
+    do = torch.randn(T, H, 128, device=DEV).bfloat16()
+    plain = torch.autograd.grad(ops.gated_delta_rule_varlen(*leaves, cu, chunk=64), leaves, do)
+    grads = torch.autograd.grad(ops.gated_delta_rule_varlen(*leaves, cu, chunk=64), leaves, do, create_graph=True)
+    for a, b in zip(grads, plain):
+        assert a.requires_grad and a.dtype == b.dtype
+        _close(a.detach(), b, rtol=2.5e-2, atol=4e-3)
+    (some,) = torch.autograd.grad(ops.gated_delta_rule_varlen(*leaves, cu, chunk=64), leaves[2:3], do, create_graph=True)
+    assert some.requires_grad
+    x, s = torch.randn(5, 384, device=DEV).bfloat16().requires_grad_(), torch.ones((), device=DEV, requires_grad=True)
+    (dx,) = torch.autograd.grad((ops.delta_heads(x, 1, 1, 128, 128)[2].float() * s).sum(), [x], create_graph=True)
+    assert float(torch.autograd.grad(dx.float().sum(), [s])[0]) == 5 * 128
