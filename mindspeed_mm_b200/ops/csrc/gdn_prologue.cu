@@ -10,13 +10,13 @@
 // rows past the end of a sequence's last chunk are zero (beta = g = 0), so they leave T, U, W and the state untouched.
 // Outputs are bf16 [H, NC, 64, *] (what the tcgen05 state-pass kernel reads) and gamma fp32 [H, NC].
 //
-// Arithmetic is fp32 throughout (exponentials too: this file is built without fast math), on the tensor cores where that costs nothing: in every 64 x 64 x 128 product one operand is a
-// bf16 tensor as it is in memory (q, k, v, dVn, ...), and the other, if it is fp32 (T, dS, dP, with beta and the gates folded into
-// its columns), is split into three bf16 terms that hold all 24 bits of it; products of bf16 numbers are exact in the fp32
-// accumulator.  (mma.sync, not tcgen05: the operands are 64 rows high and come out of registers and shared memory in between
-// elementwise steps; the chain of small dependent steps, not the tensor pipe, sets the time.)  The triangular inverse goes by
-// 16 x 16 blocks: four diagonal blocks by substitution in registers, then three levels of block products with all threads,
-// instead of 64 dependent rows.
+// Arithmetic is fp32 throughout (exponentials too: this file is built without fast math), on the tensor cores where that costs
+// nothing: in every 64 x 64 x 128 product one operand is a bf16 tensor as it is in memory (q, k, v, dVn, ...), and the other, if it
+// is fp32 (T, dS, dP, with beta and the gates folded into its columns), is split into three bf16 terms that hold all 24 bits of it;
+// products of bf16 numbers are exact in the fp32 accumulator.  (mma.sync, not tcgen05: the operands are 64 rows high and come out of
+// registers and shared memory in between elementwise steps; the chain of small dependent steps, not the tensor pipe, sets the time.)
+// The triangular inverse goes by 16 x 16 blocks: four diagonal blocks by substitution in registers, then three levels of block
+// products with all threads, instead of 64 dependent rows.
 #include "common.cuh"
 
 namespace {

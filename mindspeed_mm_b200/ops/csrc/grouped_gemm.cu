@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(W * 32) moe_place_kernel(const long long* __re
         __syncwarp();
     }
     __syncthreads();
-    int start = 0;                                        // first row of the experts of this round
+    int start = 0;                                        // first row of the experts of this step
     for (int e0 = 0; e0 < E; e0 += W * 32) {
         const int e = e0 + threadIdx.x, count = e < E ? counts[e] : 0, padded = (count + 127) / 128 * 128;
         int total;

@@ -186,10 +186,11 @@ def test_decay_of_a_chunk_is_an_fp32_exponential():
     H, K, z = 64, 128, dict(dtype=torch.bfloat16, device=DEV)
     q = torch.nn.functional.normalize(torch.randn(64, H, K, device=DEV), dim=-1).bfloat16()
     g = (-torch.arange(1, H + 1, device=DEV, dtype=torch.float32) / 64).expand(64, H).contiguous()      # sums of -1 .. -64
+    beta, first, count = torch.ones_like(g), torch.tensor([0], dtype=torch.int32, device=DEV), torch.tensor([64], dtype=torch.int32, device=DEV)
     W, Qg, Kd, U, At = *(torch.empty(H, 1, 64, K, **z) for _ in range(4)), torch.empty(H, 1, 64, 64, **z)
-    gamma, at = torch.empty(H, 1, device=DEV), [torch.tensor([i], dtype=torch.int32, device=DEV) for i in (0, 64)]
-    assert native.lib().mm_gdn_prologue(q.data_ptr(), q.data_ptr(), q.data_ptr(), g.data_ptr(), torch.ones_like(g).data_ptr(), at[0].data_ptr(), at[1].data_ptr(),
-                                        W.data_ptr(), Qg.data_ptr(), Kd.data_ptr(), At.data_ptr(), U.data_ptr(), gamma.data_ptr(), H, 1, 1.0, native._st()) == 0
+    gamma = torch.empty(H, 1, device=DEV)
+    pointers = [t.data_ptr() for t in (q, q, q, g, beta, first, count, W, Qg, Kd, At, U, gamma)]
+    assert native.lib().mm_gdn_prologue(*pointers, H, 1, 1.0, native._st()) == 0
     want = (-torch.arange(1, H + 1, device=DEV, dtype=torch.float64)).exp()
     assert float((gamma[:, 0].double() / want - 1).abs().max()) <= 2.5 * 2 ** -23
 
