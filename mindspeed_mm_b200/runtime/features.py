@@ -46,6 +46,7 @@ class ActivationOffload:
             self.h2d.wait_event(ev)
             out = host.to(dev, non_blocking=True)
         torch.cuda.current_stream().wait_stream(self.h2d)
+        out.record_stream(torch.cuda.current_stream())       # its memory belongs to h2d, whose next copy would not wait for its readers
         return out
 
     def __enter__(self):

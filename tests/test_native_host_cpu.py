@@ -149,3 +149,21 @@ def test_backward_reads_the_layout_of_what_the_hooks_give_back(name, monkeypatch
         y.backward(torch.ones_like(y))
     pointer, pitch = ld(next(a for fn, a in calls.items() if "_bwd" in fn and not fn.endswith("_grid")))
     assert any(t.data_ptr() == pointer for t in back) and pitch == 512
+
+
+def test_a_tensor_brought_back_from_the_host_lives_until_its_readers_are_done(monkeypatch):
+    """It is allocated on the copy stream; the allocator has to know the stream that reads it, or the next copy takes its memory."""
+    import contextlib
+    from mindspeed_mm_b200.runtime.features import ActivationOffload
+
+    class Recorder:
+        def __init__(self):
+            self.calls = []
+
+        def __getattr__(self, name):
+            return lambda *a, **k: self.calls.append((name, a)) or self
+    reader, host, off = Recorder(), Recorder(), ActivationOffload(enabled=False)
+    off.h2d = Recorder()
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: reader)
+    assert off._unpack(("host", host, None, "cuda")) is host and ("record_stream", (reader,)) in host.calls
