@@ -9,14 +9,21 @@
 //    dgrad    dx = dy W      is (A_MN=0, B_MN=1) on (dy [T,N], W [N,K] read as [K'=N, N'=K]),
 //    wgrad    dW = dy^T x    is (A_MN=1, B_MN=1) on (dy [T,N] read as [K'=T, M'=N], x [T,K] read as [K'=T, N'=K]).
 //
-// One CTA per SM walks output tiles of 128 x BN.  Roles:
+// One CTA per SM, or a pair of CTAs on two SMs (cta_group::2), walks output tiles of 128, 256 or 512 rows x BN.  Roles:
 //   warp 0     : TMA producer  (cp.async.bulk.tensor into a multi-stage 128B-swizzled smem ring)
-//   warp 1     : MMA issuer    (one elected thread issues tcgen05.mma; tcgen05.commit frees ring slots)
-//   warps 2..5 : epilogue      (tcgen05.ld TMEM -> registers -> bf16 -> swizzled smem -> TMA store)
-// The accumulator is double-buffered in TMEM (2 x BN columns) so the epilogue of tile i overlaps the main
-// loop of tile i+1.  Tiles are visited in groups of 8 M-blocks per N sweep to keep A/B tiles L2-resident.
+//   warp 1     : MMA issuer    (one thread issues tcgen05.mma, of a pair one thread of its first CTA; tcgen05.commit frees ring slots)
+//   warps 4..11: epilogue      (tcgen05.ld TMEM -> registers -> bf16 -> swizzled smem -> TMA store), four warps per accumulator
+// Tensor memory holds two accumulators of 128 rows a CTA: of two tiles, so that the epilogue of tile i overlaps the main loop of tile
+// i + 1, or (512 rows) the two halves of one tile.  Tiles are visited in groups of 8 to 16 row blocks per N sweep to keep operands in L2.
 // All mbarrier waits are bounded (tc05::mbar_wait); a timeout is reported through `status` and the CTA
 // unwinds: it lets in-flight copies land, frees its TMEM and returns.
+//
+// What bounds a large product is the power cap: every tile size keeps the tensor pipe 90 to 96 % busy, at a clock that the energy of its
+// operand traffic sets.  A step of 64 of K brings a CTA 48 KB for 128 x 256 (one CTA), 32 KB for the same as half of a 256-row pair, and
+// 48 KB for 256 x 256 as half of a 512-row pair: 19.1 / 15.0 GB through L2 for 8192 x 37888 x 3584 with 256 / 512 rows.  Sustained, TFLOP/s, tiles
+// of 128 / 256 / 512 rows (cuBLAS): 8192 x 37888 x 3584 1202 / 1432 / 1430 (1416), 8192 x 3584 x 18944 1209 / 1291 / 1399 (1238), 32760 x 5120 x
+// 13824 1188 / 1274 / 1388 (1401), 8192 x 3840 x 1280 1104 / 1157 / 1107 (1130).  Groups of 4096 rows against 1024 / 2048 / 8192: 1432 against
+// 1292 / 1350 (256 rows), 1430 against 1421 / 1381 at 2048 / 8192 (512 rows, 8192 x 37888 x 3584); single tiles are used for few rows only.
 #include "tc05.cuh"
 
 namespace {
@@ -25,19 +32,27 @@ using namespace tc05;
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int kThreads = 192;
-constexpr int kEpiThreads = 128;
+constexpr int kGroupThreads = 128;                        // of an epilogue group
+constexpr int kThreads = 128 + 2 * kGroupThreads;
+// registers of a thread: 168 at launch; the epilogue holds a packed accumulator row, the issuing warps need few
+constexpr int kIssueRegs = 56, kEpiRegs = 224;
 constexpr int kSmemBudget = 227 * 1024;
 
-template <int BN>
+// TM: rows of a tile.  128: one CTA;  256 and 512: a pair of CTAs on two SMs, each with half of the rows and, for the operands, half of the
+// columns (cta_group::2).
+template <int BN, int TM>
 struct Cfg {
-    static constexpr int kABytes = BM * BK * 2;
-    static constexpr int kBBytes = BN * BK * 2;
+    static constexpr bool kPair = TM > BM;
+    static constexpr int kHalves = TM == 512 ? 2 : 1;    // accumulators of 128 rows that a tile has in a CTA's tensor memory
+    static constexpr int kBRows = kPair ? BN / 2 : BN;   // rows of B in a CTA's shared memory
+    static constexpr int kABytes = kHalves * BM * BK * 2;
+    static constexpr int kBBytes = kBRows * BK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
     static constexpr int kCBytes = 2 * BM * 64 * 2;  // two 128x64 bf16 staging slabs
     static constexpr int kAux = 1024;                // barriers etc.
     static constexpr int kStages = (kSmemBudget - kCBytes - kAux - 1024) / kStageBytes;
     static constexpr int kSmem = kStages * kStageBytes + kCBytes + kAux + 1024;
+    static constexpr int kAhead = kStages < 3 ? kStages : 3;
     static constexpr int kTmemCols = 2 * BN;
 };
 
@@ -95,11 +110,12 @@ __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks
 // SWIGLU (BN = 256, K-major operands, no bias): B is the fused [2F, K] gate/up weight, p.N = F.  A tile's accumulator holds
 // 128 gate columns (weight rows nb*128 ..) next to the 128 up columns of the same features (rows F + nb*128 ..); the
 // epilogue writes silu(gate) * up, so the [M, 2F] pre-activation never reaches memory.
-template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false>
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false, int TM = BM>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ TMapSet tmC, Params p) {
-    using C = Cfg<BN>;
+    using C = Cfg<BN, TM>;
+    constexpr bool PAIR = C::kPair;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sA = smem;
@@ -115,7 +131,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int m_blocks = (p.M + BM - 1) / BM;
+    // a worker: this CTA, or the pair that it belongs to
+    const int rank = PAIR ? (int)cluster_rank() : 0;
+    const int worker = PAIR ? blockIdx.x / 2 : blockIdx.x, n_workers = PAIR ? gridDim.x / 2 : gridDim.x;
+    const int m_blocks = (p.M + TM - 1) / TM;
     const int n_blocks = SWIGLU ? p.N / 128 : (p.N + BN - 1) / BN;
     const int n_tiles = m_blocks * n_blocks;
     const int k_blocks = (p.K + BK - 1) / BK;
@@ -128,7 +147,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&tfull[a], 1);
-            mbar_init(&tempty[a], kEpiThreads);
+            mbar_init(&tempty[a], (PAIR ? 2 : 1) * kGroupThreads / 32);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -137,21 +156,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         for (int d = 0; d < (p.mode ? p.world : 1); ++d) prefetch_tmap(&tmC.m[d]);
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, C::kTmemCols);
-        tmem_relinquish();
+        if constexpr (PAIR) {
+            tmem_alloc_pair(tmem_slot, C::kTmemCols);
+        } else {
+            tmem_alloc(tmem_slot, C::kTmemCols);
+            tmem_relinquish();
+        }
     }
     fence_before_sync();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();          // the other CTA's barriers are there, too
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+        if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
+            for (int i = worker; i < n_items && ok; i += n_workers) {
                 const Item item = item_at(p, i, n_tiles, k_blocks);
                 int mb, nb;
                 tile_coords(item.tile, m_blocks, n_blocks, p.group_m, mb, nb);
@@ -161,25 +187,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(&full[stage], C::kStageBytes);
                     uint8_t* a = sA + stage * C::kABytes;
                     uint8_t* b = sB + stage * C::kBBytes;
+                    const int m0 = mb * TM + rank * (TM / 2), n0 = nb * BN + rank * C::kBRows;
+                    const uint32_t bar = PAIR ? cluster_addr(&full[stage], 0) : 0;
+                    auto load = [&](uint8_t* dst, const CUtensorMap* m, int x, int y) {
+                        if constexpr (PAIR) tma_load_2d_pair(dst, m, bar, x, y);
+                        else tma_load_2d(dst, m, &full[stage], x, y);
+                    };
+                    // (a pair's copies are all counted in the CTA of rank 0, where the products are issued)
+                    if (rank == 0) mbar_expect_tx(&full[stage], C::kStageBytes * (PAIR ? 2 : 1));
                     if constexpr (!A_MN) {
-                        tma_load_2d(a, &tmA, &full[stage], kb * BK, mb * BM);
+                        load(a, &tmA, kb * BK, m0);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < BM / 64; ++j)
-                            tma_load_2d(a + j * (BK * 128), &tmA, &full[stage], mb * BM + j * 64, kb * BK);
+                        for (int j = 0; j < C::kHalves * BM / 64; ++j) load(a + j * (BK * 128), &tmA, m0 + j * 64, kb * BK);
                     }
-                    if constexpr (SWIGLU) {
-                        tma_load_2d(b, &tmB, &full[stage], kb * BK, nb * 128);
-                        tma_load_2d(b + 128 * 128, &tmB, &full[stage], kb * BK, p.N + nb * 128);
+                    if constexpr (SWIGLU && PAIR) {
+                        load(b, &tmB, kb * BK, rank * p.N + nb * 128);
+                    } else if constexpr (SWIGLU) {
+                        load(b, &tmB, kb * BK, nb * 128);
+                        load(b + 128 * 128, &tmB, kb * BK, p.N + nb * 128);
                     } else if constexpr (!B_MN) {
-                        tma_load_2d(b, &tmB, &full[stage], kb * BK, nb * BN);
+                        load(b, &tmB, kb * BK, n0);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < BN / 64; ++j)
-                            tma_load_2d(b + j * (BK * 128), &tmB, &full[stage], nb * BN + j * 64, kb * BK);
+                        for (int j = 0; j < C::kBRows / 64; ++j) load(b + j * (BK * 128), &tmB, n0 + j * 64, kb * BK);
                     }
                     if (++stage == C::kStages) {
                         stage = 0;
@@ -187,164 +220,247 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     }
                 }
             }
+            if constexpr (PAIR)                  // every slot's release, which comes from the other CTA, has arrived before this one ends
+                for (int s = 0; s < C::kStages && ok; ++s) {
+                    ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag);
+                    if (++stage == C::kStages) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
         }
-    } else if (warp == 1) {
+        } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = idesc_bf16(PAIR ? 2 * BM : BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
             int stage = 0;
             uint32_t phase = 0;
             int it = 0;
             bool ok = true;
-            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x, ++it) {
-                const Item item = item_at(p, i, n_tiles, k_blocks);
-                const int acc = it & 1;
-                if (!mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag)) {
-                    atomicExch(p.status, MM_TIMEOUT_MMA);
-                    break;
+            auto step = [](int& s, uint32_t& ph) {
+                if (++s == C::kStages) {
+                    s = 0;
+                    ph ^= 1;
                 }
-                fence_after_sync();
-                const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = item.kb0; kb < item.kb1; ++kb) {
-                    if (!mbar_wait(&full[stage], phase, abort_flag)) {
-                        atomicExch(p.status, MM_TIMEOUT_MMA);
-                        ok = false;
-                        break;
-                    }
+            };
+            auto arrived = [&](int s, uint32_t ph) {
+                if (mbar_wait(&full[s], ph, abort_flag)) return true;
+                atomicExch(p.status, MM_TIMEOUT_MMA);
+                return ok = false;
+            };
+            auto drained = [&](int acc) {
+                const uint32_t parity = ((it * C::kHalves / 2) & 1) ^ 1;
+                if (PAIR ? mbar_wait_cluster(&tempty[acc], parity, abort_flag) : mbar_wait(&tempty[acc], parity, abort_flag)) {
                     fence_after_sync();
-                    const uint32_t a0 = smem_u32(sA + stage * C::kABytes);
-                    const uint32_t b0 = smem_u32(sB + stage * C::kBBytes);
-#pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        // K-major: 16 elements of K = 32 bytes inside the swizzle atom.
-                        // MN-major: 16 rows of K = two 8-row groups = 2048 bytes.
-                        const uint64_t da = A_MN ? smem_desc_sw128(a0 + k * 2048, BK * 128, 1024)
-                                                 : smem_desc_sw128(a0 + k * 32, 16, 1024);
-                        const uint64_t db = B_MN ? smem_desc_sw128(b0 + k * 2048, BK * 128, 1024)
-                                                 : smem_desc_sw128(b0 + k * 32, 16, 1024);
-                        mma_ss(d_tmem, da, db, idesc, (kb != item.kb0 || k) ? 1u : 0u);
-                    }
-                    mma_commit(&empty[stage]);  // slot reusable once these MMAs have read it
-                    if (++stage == C::kStages) {
-                        stage = 0;
-                        phase ^= 1;
-                    }
+                    return true;
                 }
-                if (ok) mma_commit(&tfull[acc]);
+                atomicExch(p.status, MM_TIMEOUT_MMA);
+                return ok = false;
+            };
+            auto done = [&](uint64_t* bar) {
+                if constexpr (PAIR) mma_commit_pair(bar);
+                else mma_commit(bar);
+            };
+            // products of one slot's operands; h: which 128 rows of the CTA's A tile
+            auto products = [&](int s, int h, int acc, bool first) {
+                fence_after_sync();
+                const uint32_t a0 = smem_u32(sA + s * C::kABytes) + h * BM * BK * 2;
+                const uint32_t b0 = smem_u32(sB + s * C::kBBytes);
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) {
+                    // K-major: 16 elements of K = 32 bytes inside the swizzle atom.
+                    // MN-major: 16 rows of K = two 8-row groups = 2048 bytes.
+                    const uint64_t da = A_MN ? smem_desc_sw128(a0 + k * 2048, BK * 128, 1024)
+                                             : smem_desc_sw128(a0 + k * 32, 16, 1024);
+                    const uint64_t db = B_MN ? smem_desc_sw128(b0 + k * 2048, BK * 128, 1024)
+                                             : smem_desc_sw128(b0 + k * 32, 16, 1024);
+                    const uint32_t accum = !first || k ? 1u : 0u;
+                    if constexpr (PAIR) mma_ss_pair(tmem_base + acc * BN, da, db, idesc, accum);
+                    else mma_ss(tmem_base + acc * BN, da, db, idesc, accum);
+                }
+            };
+            for (int i = worker; i < n_items && ok; i += n_workers, ++it) {
+                const Item item = item_at(p, i, n_tiles, k_blocks);
+                if constexpr (C::kHalves == 1) {
+                    const int acc = it & 1;
+                    if (!drained(acc)) break;
+                    for (int kb = item.kb0; kb < item.kb1 && arrived(stage, phase); ++kb) {
+                        products(stage, 0, acc, kb == item.kb0);
+                        done(&empty[stage]);        // slot reusable once these MMAs have read it
+                        step(stage, phase);
+                    }
+                    if (ok) done(&tfull[acc]);
+                } else {
+                    // Tensor memory holds one tile, so its first accumulator runs ahead of the second at both ends, by up to kAhead
+                    // slots: it is complete, and drained, while the second one's last products run, and the next tile starts on it
+                    // while the second one is drained.
+                    const int n = item.kb1 - item.kb0, head = min(n, C::kAhead), tail = min(n - head, C::kAhead);
+                    auto ahead = [&](int count, bool first, bool last) {
+                        int s = stage;
+                        uint32_t ph = phase;
+                        if (first && !drained(0)) return;
+                        for (int k = 0; k < count; ++k) {
+                            if (!arrived(s, ph)) return;
+                            products(s, 0, 0, first && k == 0);
+                            step(s, ph);
+                        }
+                        if (last) done(&tfull[0]);
+                        if (first && !drained(1)) return;
+                        for (int k = 0; k < count; ++k) {
+                            products(stage, 1, 1, first && k == 0);
+                            done(&empty[stage]);
+                            step(stage, phase);
+                        }
+                        if (last) done(&tfull[1]);
+                    };
+                    ahead(head, true, head == n);
+                    for (int k = head; k < n - tail && ok && arrived(stage, phase); ++k) {
+                        products(stage, 0, 0, false);
+                        products(stage, 1, 1, false);
+                        done(&empty[stage]);
+                        step(stage, phase);
+                    }
+                    if (ok && tail) ahead(tail, false, true);
+                }
             }
         }
+        }
     } else {
-        // ------------------------------------------------------------------ epilogue (warps 2..5)
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+        // ------------------------------------------------------------------ epilogue
+        // Group g drains accumulator g.  A thread takes its whole row into registers, as bf16, before anything is stored: the products
+        // of the next tile wait for nothing but these reads.
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int row = q * 32 + lane;     // row inside the 128-row tile
-        const bool issuer = threadIdx.x == 64;
-        int it = 0;
-        int slab_count = 0;
-        for (int i = blockIdx.x; i < n_items; i += gridDim.x, ++it) {
+        const int group = (warp >> 2) - 1;
+        const bool issuer = threadIdx.x % kGroupThreads == 0;
+        uint8_t* buf = sC + group * (BM * 128);
+        auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+        auto drained = [&] {
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                if constexpr (PAIR) mbar_arrive_cluster(cluster_addr(&tempty[group], 0));
+                else mbar_arrive(&tempty[group]);
+            }
+        };
+        const uint32_t t_row = tmem_base + group * BN + ((uint32_t)(q * 32) << 16);
+        const bool wide_bias = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+        constexpr int kSlabs = SWIGLU ? 2 : BN / 64;         // of 64 output columns
+        int it = 0, use = 0;
+        for (int i = worker; i < n_items; i += n_workers, ++it) {
+            if (C::kHalves == 1 && (it & 1) != group) continue;
             const Item item = item_at(p, i, n_tiles, k_blocks);
             int mb, nb;
             tile_coords(item.tile, m_blocks, n_blocks, p.group_m, mb, nb);
-            const int acc = it & 1;
-            if (!mbar_wait(&tfull[acc], (it >> 1) & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
-            // make the go / no-go decision identical for all 128 epilogue threads before any bar.sync below
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (issuer) *epi_stop = *abort_flag;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (*epi_stop) break;
+            const int h = C::kHalves == 1 ? 0 : group, m0 = mb * TM + rank * (TM / 2) + h * BM;
+            if (!mbar_wait(&tfull[group], use++ & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
+            __syncwarp();
             fence_after_sync();
-            const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
-            constexpr int kSlabs = SWIGLU ? 2 : BN / 64;
+            uint32_t v[kSlabs * 32];
             if (!SWIGLU && item.slot >= 0) {
                 // [column / 4][row][4]: the lanes of a warp write neighbouring rows of a column group
-                float4* dst = reinterpret_cast<float4*>(p.ws) + (size_t)item.slot * (BM * BN / 4) + row;
+                float4* dst = reinterpret_cast<float4*>(p.ws) + (size_t)(item.slot * (TM / BM) + rank * C::kHalves + h) * (BM * BN / 4) + row;
 #pragma unroll 1
                 for (int slab = 0; slab < kSlabs; ++slab) {
                     uint32_t r[64];
                     tmem_ld_32x32(t_row + slab * 64, r);
                     tmem_ld_32x32(t_row + slab * 64 + 32, r + 32);
                     tmem_wait_ld();
+                    if (slab == kSlabs - 1) drained();
 #pragma unroll
                     for (int c = 0; c < 16; ++c)
                         dst[(slab * 16 + c) * BM] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
                                                                 __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
                 }
-                fence_before_sync();
-                mbar_arrive(&tempty[acc]);
-                continue;
-            }
-#pragma unroll 1
-            for (int slab = 0; slab < kSlabs; ++slab, ++slab_count) {
-                uint8_t* buf = sC + (slab_count & 1) * (BM * 128);
-                if (issuer) tma_wait_read<1>();  // the store that last read this buffer has drained
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                uint32_t r[64];
-                if constexpr (SWIGLU) {
+            } else {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        uint32_t u[32];
-                        tmem_ld_32x32(t_row + slab * 64 + h * 32, r + h * 32);
-                        tmem_ld_32x32(t_row + 128 + slab * 64 + h * 32, u);
+                for (int slab = 0; slab < kSlabs; ++slab) {
+                    uint32_t r[64];
+                    const int n0 = (SWIGLU ? nb * 128 : nb * BN) + slab * 64;
+                    if constexpr (SWIGLU) {
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            uint32_t u[32];
+                            tmem_ld_32x32(t_row + slab * 64 + half * 32, r + half * 32);
+                            tmem_ld_32x32(t_row + 128 + slab * 64 + half * 32, u);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int c = 0; c < 32; ++c) {
+                                const float g = __uint_as_float(r[half * 32 + c]);
+                                r[half * 32 + c] = __float_as_uint(__fdividef(g, 1.f + __expf(-g)) * __uint_as_float(u[c]));
+                            }
+                        }
+                    } else {
+                        tmem_ld_32x32(t_row + slab * 64, r);
+                        tmem_ld_32x32(t_row + slab * 64 + 32, r + 32);
                         tmem_wait_ld();
+                    }
+                    if (slab == kSlabs - 1) drained();
+                    if (!SWIGLU && p.bias != nullptr) {
+                        if (wide_bias && n0 + 64 <= p.N) {
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) {
-                            const float g = __uint_as_float(r[h * 32 + c]);
-                            r[h * 32 + c] = __float_as_uint(__fdividef(g, 1.f + __expf(-g)) * __uint_as_float(u[c]));
+                            for (int c = 0; c < 64; c += 8) {
+                                float b[8];
+                                unpack8(*reinterpret_cast<const Vec8*>(p.bias + n0 + c), b);
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) r[c + e] = __float_as_uint(__uint_as_float(r[c + e]) + b[e]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 64; ++c) {
+                                const int n = n0 + c;
+                                const float bv = n < p.N ? __bfloat162float(p.bias[n]) : 0.f;
+                                r[c] = __float_as_uint(__uint_as_float(r[c]) + bv);
+                            }
                         }
                     }
-                } else {
-                    tmem_ld_32x32(t_row + slab * 64, r);
-                    tmem_ld_32x32(t_row + slab * 64 + 32, r + 32);
-                    tmem_wait_ld();
+                    if (!SWIGLU && p.stats != nullptr) {
+                        float ss = 0.f;
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) {
+                            const float x = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[c])));
+                            ss += (n0 + c < p.N) ? x * x : 0.f;
+                        }
+                        const int m = m0 + row;
+                        if (m < p.M && n0 < p.N) atomicAdd(&p.stats[(size_t)m * p.n_slots + n0 / p.per_slot], ss);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) {
+                        const bf162 t = __floats2bfloat162_rn(__uint_as_float(r[2 * c]), __uint_as_float(r[2 * c + 1]));
+                        v[slab * 32 + c] = *reinterpret_cast<const uint32_t*>(&t);
+                    }
                 }
+            }
+            // one go / no-go decision for all threads of the group before its barriers below
+            group_sync();
+            if (issuer) epi_stop[group] = *abort_flag;
+            group_sync();
+            if (epi_stop[group]) break;
+            if (!SWIGLU && item.slot >= 0) continue;
+#pragma unroll
+            for (int slab = 0; slab < kSlabs; ++slab) {
                 const int n0 = (SWIGLU ? nb * 128 : nb * BN) + slab * 64;
-                if (!SWIGLU && p.bias != nullptr) {
+                if (issuer) tma_wait_read<0>();      // the store that last read this buffer has drained
+                group_sync();
 #pragma unroll
-                    for (int c = 0; c < 64; ++c) {
-                        const int n = n0 + c;
-                        const float bv = n < p.N ? __bfloat162float(p.bias[n]) : 0.f;
-                        r[c] = __float_as_uint(__uint_as_float(r[c]) + bv);
-                    }
-                }
-                if (!SWIGLU && p.stats != nullptr) {
-                    float ss = 0.f;
-#pragma unroll
-                    for (int c = 0; c < 64; ++c) {
-                        const float v = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[c])));
-                        ss += (n0 + c < p.N) ? v * v : 0.f;
-                    }
-                    const int m = mb * BM + row;
-                    if (m < p.M && n0 < p.N) atomicAdd(&p.stats[(size_t)m * p.n_slots + n0 / p.per_slot], ss);
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    uint4 v;
-                    bf162 t0 = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
-                    bf162 t1 = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
-                    bf162 t2 = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
-                    bf162 t3 = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-                    v.x = *reinterpret_cast<uint32_t*>(&t0);
-                    v.y = *reinterpret_cast<uint32_t*>(&t1);
-                    v.z = *reinterpret_cast<uint32_t*>(&t2);
-                    v.w = *reinterpret_cast<uint32_t*>(&t3);
-                    *reinterpret_cast<uint4*>(buf + row * 128 + ((j ^ (row & 7)) << 4)) = v;
-                }
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<uint4*>(buf + row * 128 + ((c ^ (row & 7)) << 4)) =
+                        make_uint4(v[slab * 32 + 4 * c], v[slab * 32 + 4 * c + 1], v[slab * 32 + 4 * c + 2], v[slab * 32 + 4 * c + 3]);
                 fence_proxy_async();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                group_sync();
                 if (issuer) {
                     if (p.mode == 0) {
-                        tma_store_2d(&tmC.m[0], buf, n0, mb * BM);
+                        if (m0 < p.M && n0 < p.N) tma_store_2d(&tmC.m[0], buf, n0, m0);
                     } else if (p.mode == 1) {
                         const int b = n0 / p.blk;
-                        tma_store_2d(&tmC.m[b % p.world], buf, (b / p.world) * p.blk + n0 % p.blk, p.row_off + mb * BM);
+                        tma_store_2d(&tmC.m[b % p.world], buf, (b / p.world) * p.blk + n0 % p.blk, p.row_off + m0);
                     } else {
-                        const int m0 = mb * BM;
                         tma_store_2d(&tmC.m[m0 / p.blk], buf, n0, p.rank * p.blk + m0 % p.blk);
                     }
                     tma_commit();
                 }
             }
-            fence_before_sync();
-            mbar_arrive(&tempty[acc]);
         }
         if (issuer) tma_wait_all<0>();
     }
@@ -356,44 +472,67 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
     fence_before_sync();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();          // nothing of the other CTA reaches for this one's memory from here on
     if (warp == 1) {
         fence_after_sync();
-        tmem_dealloc(tmem_base, C::kTmemCols);
+        if constexpr (PAIR) tmem_dealloc_pair(tmem_base, C::kTmemCols);
+        else tmem_dealloc(tmem_base, C::kTmemCols);
     }
 }
 
-// ---- split tail ----
+// ---- choice of the tile, and the split tail ----
 // 168 tiles on 148 SMs take two rounds, the second one with 20 CTAs at work.  The tiles behind the last whole round are therefore cut
-// along K into `parts` items each, so that ceil(rem * parts / 148) rounds of a 1 / parts tile follow; the items leave fp32 sums in a
-// workspace and a second kernel adds them in their order, adds the bias and rounds, exactly once, to bf16.  No CTA waits for another.
-struct SplitPlan {
-    int full, parts;
+// along K into `parts` items each, so that ceil(rem * parts / workers) rounds of a 1 / parts tile follow; the items leave fp32 sums in a
+// workspace and a second kernel adds them in their order, adds the bias and rounds, exactly once, to bf16.  No worker waits for another.
+struct Plan {
+    int rows;              // of a tile
+    int full, parts;       // tiles that are one item each; items that each of the others is cut into
 };
 
-// parts: the number that the estimate below makes fastest, 1 if the gain is under 4 us.  A 64-deep step of a 128 x 256 tile takes
-// 0.44 us (1.4 PFLOP/s over 148 SMs), and no product is over before its operands have come once at 6.2 TB/s: a single row of tiles
-// over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about 4 TB/s, a
-// further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
-// lost 2 us).
+// The tile size and the number of parts that the estimate below makes fastest; tiles stay whole for a gain under 4 us.  A 64-deep step of
+// a tile of 256 columns takes 0.45 / 0.415 / 0.79 us with 128 / 256 / 512 rows (rates of a burst; an SM, or a pair of them, works on it), a
+// 512-row tile has 1 us more for filling its ring anew, and no product is over before its operands have come once at 6.2 TB/s: a single
+// row of tiles over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about
+// 4 TB/s, a further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
+// lost 2 us).  A tile of which half the rows are empty is not taken.
 // Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 218 / 151 us, 405 x 3584 x 37888 (56) 216 / 122,
-// 8192 x 3584 x 18944 (896) 828 / 776, 8192 x 3584 x 152064 (7 rounds become 6 and a part) 6920 / 6210, 3840 x 1280 x 8192 (150)
-// 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands: 85 x 25368 x 27344 247 / 279, 126 x 26744 x 24168 251 / 271.
-inline SplitPlan split_plan(int M, int N, int K, int BN, int sms) {
-    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK, full = tiles / sms, rem = tiles % sms;
-    SplitPlan best{tiles, 1};
-    if (!rem) return best;
-    const double unit = kb * 0.44 * BN / 256, operands = 2.0 * K * ((double)M + N) / 6.2e6;
+// 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands: 85 x 25368 x 27344 247 / 279, 126 x 26744 x
+// 24168 251 / 271.
+inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool may_split) {
+    const int kb = (K + BK - 1) / BK;
+    const double operands = 2.0 * K * ((double)M + N) / 6.2e6;
     auto at_least = [&](double t) { return t > operands ? t : operands; };
-    double least = at_least(unit * (full + 1)) - 4.0;
-    for (int parts = 2; parts <= 16 && kb / parts >= 4; ++parts) {
-        const int rounds = (rem * parts + sms - 1) / sms;
-        const double t = at_least(unit * full + unit * rounds / parts) + 6.0 + rem * parts * (BM * BN * 8e-6 / 4.0);
+    Plan best{BM, 0, 1};
+    double least = 1e30;
+    for (int rows = BM; rows == BM || (may_pair && rows <= 4 * BM && M > rows / 2); rows *= 2) {
+        const int workers = rows > BM ? sms / 2 : sms;
+        const int tiles = ((M + rows - 1) / rows) * ((N + BN - 1) / BN), full = tiles / workers, rem = tiles % workers;
+        const double unit = (rows == BM ? kb * 0.45 : rows == 2 * BM ? kb * 0.415 : kb * 0.79 + 1.0) * BN / 256;
+        const double whole = at_least(unit * (full + (rem ? 1 : 0)));
+        double t = whole;
+        Plan p{rows, tiles, 1};
+        for (int parts = 2; may_split && rem && parts <= 16 && kb / parts >= 4; ++parts) {
+            const int rounds = (rem * parts + workers - 1) / workers;
+            const double s = at_least(unit * full + unit * rounds / parts) + 6.0 + rem * parts * (rows * BN * 8e-6 / 4.0);
+            if (s < t && s < whole - 4.0) {
+                t = s;
+                p.full = tiles - rem;
+                p.parts = parts;
+            }
+        }
         if (t < least) {
             least = t;
-            best = {tiles - rem, parts};
+            best = p;
         }
     }
     return best;
+}
+
+// bytes of the workspace that the plan's split tiles take (their fp32 sums)
+inline long long split_bytes(const Plan& p, int M, int N, int BN) {
+    if (p.parts == 1) return 0;
+    const long long tiles = (long long)((M + p.rows - 1) / p.rows) * ((N + BN - 1) / BN);
+    return (tiles - p.full) * p.parts * p.rows * BN * 4;
 }
 
 inline int sm_count() {
@@ -407,19 +546,19 @@ inline int sm_count() {
 }
 
 // C tile = bf16(sum over the parts of the workspace + bias); a thread makes 8 columns of a row
-template <int BN>
+template <int BN, int TM>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ ws, bf16* __restrict__ C, const bf16* __restrict__ bias,
                                                         int M, int N, long long ldc, int full, int parts, int group_m) {
-    const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM, t = blockIdx.y;      // cg: group of 8 columns
-    int mb, nb;
-    tile_coords(full + t, (M + BM - 1) / BM, (N + BN - 1) / BN, group_m, mb, nb);
-    const int m = mb * BM + row, n = nb * BN + cg * 8;
+    const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM % (BN / 8), half = i / (BM * BN / 8), t = blockIdx.y;
+    int mb, nb;                                                                                   // cg: group of 8 columns
+    tile_coords(full + t, (M + TM - 1) / TM, (N + BN - 1) / BN, group_m, mb, nb);
+    const int m = mb * TM + half * BM + row, n = nb * BN + cg * 8;
     if (m >= M || n >= N) return;
-    const float4* src = reinterpret_cast<const float4*>(ws) + (size_t)t * parts * (BM * BN / 4) + (size_t)(2 * cg) * BM + row;
+    const float4* src = reinterpret_cast<const float4*>(ws) + ((size_t)t * parts * (TM / BM) + half) * (BM * BN / 4) + (size_t)(2 * cg) * BM + row;
     float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
     for (int q = 0; q < parts; ++q) {
-        const float4 a = src[(size_t)q * (BM * BN / 4)], b = src[(size_t)q * (BM * BN / 4) + BM];
+        const float4 a = src[(size_t)q * (TM * BN / 4)], b = src[(size_t)q * (TM * BN / 4) + BM];
         f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
         f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
     }
@@ -442,20 +581,21 @@ struct Route {
     int n_slots = 1;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false>
-int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
-           long long ldc, int* status, cudaStream_t st, const Route& rt = Route(), float* ws = nullptr, long long ws_bytes = 0) {
-    using C = Cfg<BN>;
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU, int TM>
+int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
+                 long long ldc, int* status, cudaStream_t st, const Route& rt, const Plan& plan, float* ws) {
+    using C = Cfg<BN, TM>;
+    constexpr bool PAIR = C::kPair;
     CUtensorMap tA, tB;
     TMapSet tC;
     int r;
     // A_MN: memory is [K, M] -> rows=K, cols=M, box = 64 k-rows x 64 m ;  else rows=M, cols=K, box = 128 x 64
-    r = A_MN ? make_tmap_2d(&tA, A, K, M, lda, BK, 64) : make_tmap_2d(&tA, A, M, K, lda, BM, BK);
+    r = A_MN ? make_tmap_2d(&tA, A, K, M, lda, BK, 64) : make_tmap_2d(&tA, A, M, K, lda, C::kHalves * BM, BK);
     if (r) return 1000 + r;
     if (SWIGLU)
         r = make_tmap_2d(&tB, B, 2LL * N, K, ldb, 128, BK);      // gate and up halves are fetched as two 128-row boxes
     else
-        r = B_MN ? make_tmap_2d(&tB, B, K, N, ldb, BK, 64) : make_tmap_2d(&tB, B, N, K, ldb, BN, BK);
+        r = B_MN ? make_tmap_2d(&tB, B, K, N, ldb, BK, 64) : make_tmap_2d(&tB, B, N, K, ldb, C::kBRows, BK);
     if (r) return 2000 + r;
     if (rt.mode == 0) {
         r = make_tmap_2d(&tC.m[0], Cc, M, N, ldc, BM, 64);
@@ -474,32 +614,52 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
             if (r) return 3000 + r;
         }
     }
-    auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU>;
+    auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU, TM>;
     static bool done = false;
     if (!done) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
         if (e != cudaSuccess) return (int)e;
         done = true;
     }
-    const int m_blocks = (M + BM - 1) / BM, n_blocks = SWIGLU ? N / 128 : (N + BN - 1) / BN;
-    const int sms = sm_count(), tiles = m_blocks * n_blocks;
-    Params p{M, N, K, (const bf16*)bias, status, 8, rt.mode, rt.blk, rt.world, rt.rank, rt.mode == 1 ? 0 : rt.row_off,
+    Params p{M, N, K, (const bf16*)bias, status, (TM == BM ? 1024 : 4096) / TM, rt.mode, rt.blk, rt.world, rt.rank, rt.mode == 1 ? 0 : rt.row_off,
              rt.stats, rt.n_slots, rt.n_slots > 0 ? N / rt.n_slots : N};
-    const SplitPlan plan = !SWIGLU && ws && rt.mode == 0 ? split_plan(M, N, K, BN, sms) : SplitPlan{tiles, 1};
-    const int rem = tiles - plan.full;
-    if (plan.parts > 1 && (long long)rem * plan.parts * BM * BN * 4 <= ws_bytes) {
+    const int tiles = ((M + TM - 1) / TM) * (SWIGLU ? N / 128 : (N + BN - 1) / BN), rem = tiles - plan.full;
+    const int items = plan.full + rem * plan.parts, workers = PAIR ? sm_count() / 2 : sm_count();
+    if (rem) {
         p.full = plan.full;
         p.parts = plan.parts;
         p.ws = ws;
-        const int items = plan.full + rem * plan.parts;
-        kern<<<items < sms ? items : sms, kThreads, C::kSmem, st>>>(tA, tB, tC, p);
-        sum_parts_kernel<BN><<<dim3(BM * BN / 8 / 256, rem), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full, plan.parts,
-                                                                           p.group_m);
-        return (int)cudaGetLastError();
     }
-    const int grid = tiles < sms ? tiles : sms;
-    kern<<<grid, kThreads, C::kSmem, st>>>(tA, tB, tC, p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((items < workers ? items : workers) * (PAIR ? 2 : 1));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = C::kSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute pairs;
+    pairs.id = cudaLaunchAttributeClusterDimension;
+    pairs.val.clusterDim.x = 2;
+    pairs.val.clusterDim.y = pairs.val.clusterDim.z = 1;
+    cfg.attrs = &pairs;
+    cfg.numAttrs = PAIR ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tA, tB, tC, p);
+    if (e != cudaSuccess) return (int)e;
+    if (rem)
+        sum_parts_kernel<BN, TM><<<dim3(TM * BN / 8 / 256, rem), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full,
+                                                                                      plan.parts, p.group_m);
     return (int)cudaGetLastError();
+}
+
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false>
+int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
+           long long ldc, int* status, cudaStream_t st, const Route& rt = Route(), float* ws = nullptr, long long ws_bytes = 0) {
+    const bool may_pair = BN == 256 && rt.mode == 0, may_split = !SWIGLU && ws && rt.mode == 0;
+    Plan plan = make_plan(M, SWIGLU ? 2 * N : N, K, BN, sm_count(), may_pair, may_split);      // a tile of a SwiGLU product: 128 features
+    if (split_bytes(plan, M, N, BN) > ws_bytes) plan = make_plan(M, N, K, BN, sm_count(), may_pair, false);
+    if constexpr (BN == 256) {
+        if (plan.rows == 512) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 512>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
+        if (plan.rows == 256) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 256>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
+    }
+    return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
 }
 
 }  // namespace
@@ -519,13 +679,18 @@ bool skinny(int M, int rows, int K) {
 }
 }  // namespace
 
+// Rows of the tiles that mm_gemm_bf16_ws takes for this product (with its workspace): 128, 256 or 512.
+MM_API int mm_gemm_tile_rows(int M, int N, int K, int bn) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const int BN = bn == 128 ? 128 : 256;
+    return make_plan(M, N, K, BN, sm_count(), BN == 256, true).rows;
+}
+
 // Bytes of workspace with which mm_gemm_bf16_ws splits the tail of this product along K (0: it would not).
 MM_API long long mm_gemm_ws_bytes(int M, int N, int K, int a_mn, int b_mn, int bn) {
     if (M <= 0 || N <= 0 || K <= 0 || (!a_mn && !b_mn && skinny(M, N, K))) return 0;
     const int BN = bn == 128 ? 128 : 256;
-    const SplitPlan plan = split_plan(M, N, K, BN, sm_count());
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    return plan.parts > 1 ? (tiles - plan.full) * plan.parts * BM * BN * 4 : 0;
+    return split_bytes(make_plan(M, N, K, BN, sm_count(), BN == 256, true), M, N, BN);
 }
 
 // lda/ldb/ldc: elements between consecutive rows of the tensors as laid out in memory.

@@ -77,6 +77,7 @@ def _declare(L):
         "mm_adamw": [_p, _p, _p, _p, _i, _p, _ll, _ll, _f, _f, _f, _f, _f, _f, _f, _f, _p, _p],
         "mm_gemm_bf16_ws": [_p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _p, _p, _ll, _p],
         "mm_gemm_ws_bytes": [_i, _i, _i, _i, _i, _i],
+        "mm_gemm_tile_rows": [_i, _i, _i, _i],
         "mm_gemm_swiglu_bf16": [_p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _p, _p],
         "mm_gemv_bf16": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _ll, _ll, _ll, _ll, _f, _i, _p],
         "mm_rotary_tables": [_p, _p, _p, _i, _i, _i, _i, _i, C.c_double, _p],

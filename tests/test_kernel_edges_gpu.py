@@ -336,6 +336,28 @@ def test_products_with_a_split_tail(layout, M, N, K, splits):
     _close(got, want, rtol=4.5e-3, atol=2e-3 * K ** 0.5 / 100)
 
 
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K,rows", [(128, 256, 64, 128), (136, 264, 8, 256), (256, 1000, 72, 256), (264, 256, 200, 256), (384, 4096, 704, None),
+                                        (520, 9480, 4104, None), (1000, 9472, 2056, 512), (4600, 3840, 4104, 512), (4096, 4864, 2568, 512),
+                                        (2560, 3840, 18944, 512)])
+def test_products_on_pairs_of_sms(layout, M, N, K, rows):
+    """Tiles of one SM and of a pair, 256 and 512 rows: few rows, ragged rows, columns and depths, a main loop of fewer steps than the ring
+    has slots, several tiles a pair, whole and cut along K."""
+    torch.manual_seed(M + K)
+    a = torch.randn((K, M) if layout == "tn" else (M, K), device=DEV).bfloat16()
+    b = torch.randn((N, K) if layout == "nt" else (K, N), device=DEV).bfloat16()
+    bias = torch.randn(N + 1, device=DEV).bfloat16()[K // 64 % 2:][:N] if layout == "nt" else None     # aligned and not
+    if rows is not None:
+        assert native.lib().mm_gemm_tile_rows(M, N, K, 256) == rows
+    got = {"nt": lambda: native.gemm_nt(a, b, bias), "nn": lambda: native.gemm_nn(a, b), "tn": lambda: native.gemm_tn(a, b)}[layout]()
+    want = (a.float().t() if layout == "tn" else a.float()) @ (b.float().t() if layout == "nt" else b.float())
+    if bias is not None:
+        want += bias.float()
+    native.check_status()
+    # exact products, fp32 sums (of any order), one rounding to bf16: half an ulp, and the order's error
+    _close(got, want, rtol=4.5e-3, atol=2e-3 * K ** 0.5 / 100)
+
+
 @pytest.mark.parametrize("T,D,section,theta", [(1, 128, (16, 24, 24), 1e6), (77, 64, (8, 12, 12), 1e4), (3, 16, (2, 1, 1), 1e7), (5000, 128, (16, 24, 20), 1e6)])
 def test_rotary_tables(T, D, section, theta):
     """Positions up to 130 000: the table is that of a 64-bit angle, rounded once."""
