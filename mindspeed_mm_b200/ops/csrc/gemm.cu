@@ -76,7 +76,14 @@ struct Params {
     // split tail (see split_plan): tiles from `full` on are cut along K into `parts` items whose fp32 sums go to `ws`
     int full = 0, parts = 1;
     float* ws = nullptr;
+    // M (or, with `counts_depth`, K) is what `count` on the device says, less `count_base` and at most what is given here; the tail is then
+    // planned by the kernel, which leaves {full, parts} in front of the workspace
+    const int* count = nullptr;
+    int count_base = 0;
+    bool counts_depth = false;
 };
+constexpr int kPlanBytes = 256;        // in front of the sums in the workspace of such a product
+constexpr int kMostRounds = 8;         // of its split items, which the workspace (310 MB for tiles of 512 rows) is made for
 
 // One entry of a CTA's list: a tile and the part of K that it covers.
 struct Item {
@@ -107,6 +114,39 @@ __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks
     nb = r / gm;
 }
 
+// ---- split tail ----
+// 168 tiles on 148 SMs take two rounds, the second one with 20 CTAs at work.  The tiles behind the last whole round are therefore cut
+// along K into `parts` items each, so that ceil(rem * parts / workers) rounds of a 1 / parts tile follow; the items leave fp32 sums in a
+// workspace and a second kernel adds them in their order, adds the bias and rounds, exactly once, to bf16.  No worker waits for another.
+// Time of a product on tiles of `rows` rows, in us, and the number of parts that makes it shortest; tiles stay whole for a gain under 4 us.  A 64-deep step of
+// a tile of 256 columns takes 0.45 / 0.415 / 0.79 us with 128 / 256 / 512 rows (rates of a burst; an SM, or a pair of them, works on it), a
+// 512-row tile has 1 us more for filling its ring anew, and no product is over before its operands have come once at 6.2 TB/s: a single
+// row of tiles over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about
+// 4 TB/s, a further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
+// lost 2 us).
+// Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 218 / 151 us, 405 x 3584 x 37888 (56) 216 / 122,
+// 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands: 85 x 25368 x 27344 247 / 279, 126 x 26744 x
+// 24168 251 / 271.
+struct TailPlan {
+    float time;
+    int full, parts;
+};
+__host__ __device__ inline TailPlan plan_tail(int M, int N, int K, int BN, int rows, int workers, int most_parts, int most_items) {
+    const int kb = (K + BK - 1) / BK;
+    const float operands = 2.f * K * ((float)M + N) / 6.2e6f;
+    auto at_least = [&](float t) { return t > operands ? t : operands; };
+    const int tiles = ((M + rows - 1) / rows) * ((N + BN - 1) / BN), full = tiles / workers, rem = tiles % workers;
+    const float unit = (rows == BM ? kb * 0.45f : rows == 2 * BM ? kb * 0.415f : kb * 0.79f + 1.f) * BN / 256;
+    const float whole = at_least(unit * (full + (rem ? 1 : 0)));
+    TailPlan best{whole, tiles, 1};
+    for (int parts = 2; rem && parts <= most_parts && kb / parts >= 4 && rem * parts <= most_items; ++parts) {
+        const int rounds = (rem * parts + workers - 1) / workers;
+        const float t = at_least(unit * full + unit * rounds / parts) + 6.f + rem * parts * (rows * BN * 8e-6f / 4.f);
+        if (t < best.time && t < whole - 4.f) best = {t, tiles - rem, parts};
+    }
+    return best;
+}
+
 // SWIGLU (BN = 256, K-major operands, no bias): B is the fused [2F, K] gate/up weight, p.N = F.  A tile's accumulator holds
 // 128 gate columns (weight rows nb*128 ..) next to the 128 up columns of the same features (rows F + nb*128 ..); the
 // epilogue writes silu(gate) * up, so the [M, 2F] pre-activation never reaches memory.
@@ -134,6 +174,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // a worker: this CTA, or the pair that it belongs to
     const int rank = PAIR ? (int)cluster_rank() : 0;
     const int worker = PAIR ? blockIdx.x / 2 : blockIdx.x, n_workers = PAIR ? gridDim.x / 2 : gridDim.x;
+    if (p.count != nullptr) {
+        const int n = max(0, __ldg(p.count) - p.count_base);
+        if (p.counts_depth) p.K = min(p.K, n);
+        else p.M = min(p.M, n);
+        if (p.ws != nullptr && !p.counts_depth) {
+            int* plan = reinterpret_cast<int*>(tmem_slot + 4);
+            if (threadIdx.x == 0) {
+                const TailPlan t = plan_tail(p.M, p.N, p.K, BN, TM, n_workers, 16, kMostRounds * n_workers);
+                plan[0] = t.full;
+                plan[1] = t.parts;
+                if (blockIdx.x == 0) {
+                    reinterpret_cast<int*>(p.ws)[0] = t.full;
+                    reinterpret_cast<int*>(p.ws)[1] = t.parts;
+                }
+            }
+            __syncthreads();
+            p.full = plan[0];
+            p.parts = plan[1];
+            p.ws += kPlanBytes / 4;
+        }
+    }
     const int m_blocks = (p.M + TM - 1) / TM;
     const int n_blocks = SWIGLU ? p.N / 128 : (p.N + BN - 1) / BN;
     const int n_tiles = m_blocks * n_blocks;
@@ -357,6 +418,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (!mbar_wait(&tfull[group], use++ & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
             __syncwarp();
             fence_after_sync();
+            const bool none = item.kb0 == item.kb1;       // of a product without depth: nothing was accumulated
             uint32_t v[kSlabs * 32];
             if (!SWIGLU && item.slot >= 0) {
                 // [column / 4][row][4]: the lanes of a warp write neighbouring rows of a column group
@@ -368,6 +430,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     tmem_ld_32x32(t_row + slab * 64 + 32, r + 32);
                     tmem_wait_ld();
                     if (slab == kSlabs - 1) drained();
+                    if (none)
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) r[c] = 0;
 #pragma unroll
                     for (int c = 0; c < 16; ++c)
                         dst[(slab * 16 + c) * BM] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
@@ -397,6 +462,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         tmem_wait_ld();
                     }
                     if (slab == kSlabs - 1) drained();
+                    if (none)
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) r[c] = 0;
                     if (!SWIGLU && p.bias != nullptr) {
                         if (wide_bias && n0 + 64 <= p.N) {
 #pragma unroll
@@ -480,49 +548,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
 }
 
-// ---- choice of the tile, and the split tail ----
-// 168 tiles on 148 SMs take two rounds, the second one with 20 CTAs at work.  The tiles behind the last whole round are therefore cut
-// along K into `parts` items each, so that ceil(rem * parts / workers) rounds of a 1 / parts tile follow; the items leave fp32 sums in a
-// workspace and a second kernel adds them in their order, adds the bias and rounds, exactly once, to bf16.  No worker waits for another.
+// ---- choice of the tile ----
 struct Plan {
     int rows;              // of a tile
     int full, parts;       // tiles that are one item each; items that each of the others is cut into
 };
 
-// The tile size and the number of parts that the estimate below makes fastest; tiles stay whole for a gain under 4 us.  A 64-deep step of
-// a tile of 256 columns takes 0.45 / 0.415 / 0.79 us with 128 / 256 / 512 rows (rates of a burst; an SM, or a pair of them, works on it), a
-// 512-row tile has 1 us more for filling its ring anew, and no product is over before its operands have come once at 6.2 TB/s: a single
-// row of tiles over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about
-// 4 TB/s, a further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
-// lost 2 us).  A tile of which half the rows are empty is not taken.
-// Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 218 / 151 us, 405 x 3584 x 37888 (56) 216 / 122,
-// 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands: 85 x 25368 x 27344 247 / 279, 126 x 26744 x
-// 24168 251 / 271.
+// The tile size, of those that M fills more than half of, with the shortest estimate.
 inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool may_split) {
-    const int kb = (K + BK - 1) / BK;
-    const double operands = 2.0 * K * ((double)M + N) / 6.2e6;
-    auto at_least = [&](double t) { return t > operands ? t : operands; };
     Plan best{BM, 0, 1};
-    double least = 1e30;
+    float least = 1e30f;
     for (int rows = BM; rows == BM || (may_pair && rows <= 4 * BM && M > rows / 2); rows *= 2) {
-        const int workers = rows > BM ? sms / 2 : sms;
-        const int tiles = ((M + rows - 1) / rows) * ((N + BN - 1) / BN), full = tiles / workers, rem = tiles % workers;
-        const double unit = (rows == BM ? kb * 0.45 : rows == 2 * BM ? kb * 0.415 : kb * 0.79 + 1.0) * BN / 256;
-        const double whole = at_least(unit * (full + (rem ? 1 : 0)));
-        double t = whole;
-        Plan p{rows, tiles, 1};
-        for (int parts = 2; may_split && rem && parts <= 16 && kb / parts >= 4; ++parts) {
-            const int rounds = (rem * parts + workers - 1) / workers;
-            const double s = at_least(unit * full + unit * rounds / parts) + 6.0 + rem * parts * (rows * BN * 8e-6 / 4.0);
-            if (s < t && s < whole - 4.0) {
-                t = s;
-                p.full = tiles - rem;
-                p.parts = parts;
-            }
-        }
-        if (t < least) {
-            least = t;
-            best = p;
+        const TailPlan t = plan_tail(M, N, K, BN, rows, rows > BM ? sms / 2 : sms, may_split ? 16 : 1, 1 << 30);
+        if (t.time < least) {
+            least = t.time;
+            best = {rows, t.full, t.parts};
         }
     }
     return best;
@@ -548,9 +588,17 @@ inline int sm_count() {
 // C tile = bf16(sum over the parts of the workspace + bias); a thread makes 8 columns of a row
 template <int BN, int TM>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ ws, bf16* __restrict__ C, const bf16* __restrict__ bias,
-                                                        int M, int N, long long ldc, int full, int parts, int group_m) {
+                                                        int M, int N, long long ldc, int full, int parts, int group_m,
+                                                        const int* __restrict__ count, int count_base) {
     const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM % (BN / 8), half = i / (BM * BN / 8), t = blockIdx.y;
     int mb, nb;                                                                                   // cg: group of 8 columns
+    if (count != nullptr) {
+        M = min(M, max(0, __ldg(count) - count_base));
+        full = reinterpret_cast<const int*>(ws)[0];
+        parts = reinterpret_cast<const int*>(ws)[1];
+        ws += kPlanBytes / 4;
+        if (parts == 1 || full + t >= ((M + TM - 1) / TM) * ((N + BN - 1) / BN)) return;
+    }
     tile_coords(full + t, (M + TM - 1) / TM, (N + BN - 1) / BN, group_m, mb, nb);
     const int m = mb * TM + half * BM + row, n = nb * BN + cg * 8;
     if (m >= M || n >= N) return;
@@ -579,6 +627,9 @@ struct Route {
     long long dst_rows = 0, dst_cols = 0;
     float* stats = nullptr;         // see Params::stats
     int n_slots = 1;
+    const int* count = nullptr;     // see Params::count
+    int count_base = 0;
+    bool counts_depth = false;
 };
 
 template <int BN, bool A_MN, bool B_MN, bool SWIGLU, int TM>
@@ -617,35 +668,30 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
     auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU, TM>;
     static bool done = false;
     if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-        if (e != cudaSuccess) return (int)e;
+        r = opt_in(kern, C::kSmem, kThreads, (kIssueRegs + 2 * kEpiRegs) * 128);
+        if (r) return r;
         done = true;
     }
     Params p{M, N, K, (const bf16*)bias, status, (TM == BM ? 1024 : 4096) / TM, rt.mode, rt.blk, rt.world, rt.rank, rt.mode == 1 ? 0 : rt.row_off,
              rt.stats, rt.n_slots, rt.n_slots > 0 ? N / rt.n_slots : N};
     const int tiles = ((M + TM - 1) / TM) * (SWIGLU ? N / 128 : (N + BN - 1) / BN), rem = tiles - plan.full;
     const int items = plan.full + rem * plan.parts, workers = PAIR ? sm_count() / 2 : sm_count();
-    if (rem) {
+    const bool dynamic_rows = rt.count != nullptr && !rt.counts_depth;
+    if (rem || dynamic_rows) {
         p.full = plan.full;
         p.parts = plan.parts;
         p.ws = ws;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((items < workers ? items : workers) * (PAIR ? 2 : 1));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = C::kSmem;
-    cfg.stream = st;
-    cudaLaunchAttribute pairs;
-    pairs.id = cudaLaunchAttributeClusterDimension;
-    pairs.val.clusterDim.x = 2;
-    pairs.val.clusterDim.y = pairs.val.clusterDim.z = 1;
-    cfg.attrs = &pairs;
-    cfg.numAttrs = PAIR ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tA, tB, tC, p);
-    if (e != cudaSuccess) return (int)e;
-    if (rem)
-        sum_parts_kernel<BN, TM><<<dim3(TM * BN / 8 / 256, rem), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full,
-                                                                                      plan.parts, p.group_m);
+    p.count = rt.count;
+    p.count_base = rt.count_base;
+    p.counts_depth = rt.counts_depth;
+    r = launch_clusters(kern, PAIR ? 2 : 1, (items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1), kThreads, C::kSmem, st, tA, tB, tC, p);
+    if (r) return r;
+    const int may_split = dynamic_rows ? (ws ? workers - 1 : 0) : rem;       // tiles
+    if (may_split)
+        sum_parts_kernel<BN, TM><<<dim3(TM * BN / 8 / 256, may_split), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full,
+                                                                                     plan.parts, p.group_m, dynamic_rows ? rt.count : nullptr,
+                                                                                     rt.count_base);
     return (int)cudaGetLastError();
 }
 
@@ -654,6 +700,7 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
            long long ldc, int* status, cudaStream_t st, const Route& rt = Route(), float* ws = nullptr, long long ws_bytes = 0) {
     const bool may_pair = BN == 256 && rt.mode == 0, may_split = !SWIGLU && ws && rt.mode == 0;
     Plan plan = make_plan(M, SWIGLU ? 2 * N : N, K, BN, sm_count(), may_pair, may_split);      // a tile of a SwiGLU product: 128 features
+    if (rt.count != nullptr && !rt.counts_depth) plan.full = ((M + plan.rows - 1) / plan.rows) * ((N + BN - 1) / BN), plan.parts = 1;
     if (split_bytes(plan, M, N, BN) > ws_bytes) plan = make_plan(M, N, K, BN, sm_count(), may_pair, false);
     if constexpr (BN == 256) {
         if (plan.rows == 512) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 512>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
@@ -714,6 +761,33 @@ MM_API int mm_gemm_bf16_ws(const void* A, const void* B, void* C, const void* bi
     }
     MM_DISPATCH(256)
 #undef MM_DISPATCH
+}
+
+// Products over the rows in use of a buffer whose number only the device knows: `count` (device int), less `base`, at most M or, with
+// a_mn = b_mn = 1, K.
+//   NT / NN: C[:count] = op(A)[:count] op(B); rows of C behind them, up to a tile's end, are overwritten.
+//   TN:      C = A[:count]^T B[:count]; the operands' rows up to the next multiple of 64 have to be zero.
+// ws: workspace of mm_gemm_rows_ws_bytes (16-byte aligned).
+MM_API long long mm_gemm_rows_ws_bytes(int M, int N, int K, int a_mn, int b_mn) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const int sms = sm_count();
+    const Plan plan = make_plan(M, N, K, 256, sms, true, true);
+    if (a_mn && b_mn) return split_bytes(plan, M, N, 256);
+    return kPlanBytes + (long long)kMostRounds * (plan.rows > BM ? sms / 2 : sms) * plan.rows * 256 * 4;
+}
+MM_API int mm_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int a_mn,
+                             int b_mn, const int* count, int base, int* status, void* ws, long long ws_bytes, cudaStream_t st) {
+    if ((lda | ldb | ldc) % 8) return -1;
+    if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C | (uintptr_t)ws) & 15) return -2;
+    if (M <= 0 || N <= 0 || K <= 0 || (a_mn && !b_mn)) return -3;
+    if (ws_bytes < mm_gemm_rows_ws_bytes(M, N, K, a_mn, b_mn)) return -4;
+    Route rt;
+    rt.count = count;
+    rt.count_base = base;
+    rt.counts_depth = a_mn;
+    if (a_mn) return launch<256, true, true>(A, B, C, nullptr, M, N, K, lda, ldb, ldc, status, st, rt, (float*)ws, ws_bytes);
+    if (b_mn) return launch<256, false, true>(A, B, C, nullptr, M, N, K, lda, ldb, ldc, status, st, rt, (float*)ws, ws_bytes);
+    return launch<256, false, false>(A, B, C, nullptr, M, N, K, lda, ldb, ldc, status, st, rt, (float*)ws, ws_bytes);
 }
 
 // C[M, F] = silu(A W_gate^T) * (A W_up^T) with W = [W_gate; W_up] stored as one [2F, K] matrix.  F % 128 == 0.

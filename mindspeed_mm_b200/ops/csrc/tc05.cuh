@@ -284,6 +284,10 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
         ::"r"(smem_u32(dst)), "l"((uint64_t)m), "r"(bar), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
+// the same box into L2 only
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* m, int x, int y, int z) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"((uint64_t)m), "r"(x), "r"(y), "r"(z) : "memory");
+}
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)m),
                  "r"(smem_u32(src)), "r"(x), "r"(y)
@@ -490,5 +494,35 @@ inline int make_tmap_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t 
         return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     });
+}
+// ---- launch of kernels that run on pairs of CTAs, or split their registers between warpgroups
+// `regs`: what the warpgroups of a block claim by setmaxnreg, in all.  A claim above the launch's own would wait for good, so such a build
+// is refused here.
+template <class K>
+inline int opt_in(K kern, int smem, int threads, int regs) {
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e != cudaSuccess) return (int)e;
+    if (a.numRegs * threads < regs) return -101;
+    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}
+template <class K, class... Args>
+inline int launch_clusters(K kern, int cluster, int blocks, int threads, int smem, cudaStream_t st, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    return (int)cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <class K, class... Args>
+inline int launch_pairs(K kern, int pairs, int threads, int smem, cudaStream_t st, const Args&... args) {
+    return launch_clusters(kern, 2, 2 * pairs, threads, smem, st, args...);
 }
 }  // namespace tc05

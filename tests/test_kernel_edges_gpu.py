@@ -358,6 +358,33 @@ def test_products_on_pairs_of_sms(layout, M, N, K, rows):
     _close(got, want, rtol=4.5e-3, atol=2e-3 * K ** 0.5 / 100)
 
 
+@pytest.mark.parametrize("T,H,V,valid,chunk", [(512, 256, 512, 100, 8192), (513, 256, 512, 0, 8192), (513, 264, 520, 513, 8192), (600, 256, 1000, 1, 8192),
+                                               (700, 512, 4096, 64, 8192), (700, 512, 4096, 65, 256), (8300, 256, 512, 5000, 8192),
+                                               (8300, 256, 512, 130, 4096), (1600, 3584, 18944, 1421, 8192)])
+def test_loss_over_the_rows_with_a_target(T, H, V, valid, chunk):
+    """No target at all, one, all; lists that end at and behind a step of 64 and in the first of several chunks, and a tail that is cut
+    along K by the kernel's own plan.  Rows without a target get a gradient of exactly zero."""
+    torch.manual_seed(T + valid)
+    h = torch.randn(T, H, device=DEV).bfloat16().requires_grad_()
+    w = (0.02 * torch.randn(V, H, device=DEV)).bfloat16().requires_grad_()
+    lab = torch.full((T,), -100, device=DEV)
+    use = torch.randperm(T, device=DEV)[:valid]
+    lab[use] = torch.randint(0, V, (valid,), device=DEV)
+    poison = [torch.full((T, max(H, V)), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(3)]      # what the allocator hands out next
+    del poison
+    loss = native.linear_cross_entropy(h, w, lab, -100, chunk)[0]
+    dh, dw = torch.autograd.grad(loss, [h, w])
+    native.check_status()
+    hr, wr = h.detach().float().requires_grad_(), w.detach().float().requires_grad_()
+    want = torch.nn.functional.cross_entropy(hr @ wr.t(), lab, reduction="sum", ignore_index=-100)
+    eh, ew = torch.autograd.grad(want, [hr, wr])
+    assert abs(float(loss) - float(want)) <= 2e-3 * abs(float(want)) + 1e-6
+    assert not dh[lab == -100].any()
+    # logits and their gradient are rounded to bf16 (2^-9 of each term), the sums to bf16 once more
+    _close(dh, eh, rtol=2e-2, atol=1e-4)
+    _close(dw, ew, rtol=2e-2, atol=2e-3 * max(valid, 1) ** 0.5)
+
+
 @pytest.mark.parametrize("T,D,section,theta", [(1, 128, (16, 24, 24), 1e6), (77, 64, (8, 12, 12), 1e4), (3, 16, (2, 1, 1), 1e7), (5000, 128, (16, 24, 20), 1e6)])
 def test_rotary_tables(T, D, section, theta):
     """Positions up to 130 000: the table is that of a 64-bit angle, rounded once."""
