@@ -5,7 +5,7 @@
 //   fmha_bwd_dq_kernel   one CTA = one 128-row query tile of one head; walks the key tiles like the forward:
 //                           S = Q K_j^T, dP = dO V_j^T                       (tcgen05, accumulators in TMEM)
 //                           P = exp2(S c - lse), dS = P (dP - delta)          (one thread per query row)
-//                           dQ += dS K_j                                      (dS through swizzled smem)
+//                           dQ += dS K_j                                      (dS through tensor memory)
 //   fmha_bwd_dkv_kernel  one CTA = one 128-row key tile of one KV head; walks the query tiles (64 rows each) of
 //                        every query head that shares the KV head, computing the transposed products so that
 //                        the key index sits on the TMEM lanes:
@@ -47,27 +47,56 @@ struct BwdParams {
     int split;              // dK/dV kernel: 1 = one CTA per QUERY head writing partial dk / dv [Tk, Nq, 128]
 };
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h)
-__global__ void fmha_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dO, float* __restrict__ delta, int T,
-                                  int Nq, int D) {
-    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= (long long)T * Nq) return;
-    const int lane = threadIdx.x & 31;
-    uint2 a = make_uint2(0, 0), b = make_uint2(0, 0);
-    if (lane * 4 < D) {                     // D is a multiple of 8: a lane's four elements are all inside or all outside
-        a = reinterpret_cast<const uint2*>(o + row * D)[lane];
-        b = reinterpret_cast<const uint2*>(dO + row * D)[lane];
-    }
-    const bf162* pa = reinterpret_cast<const bf162*>(&a);
-    const bf162* pb = reinterpret_cast<const bf162*>(&b);
-    float s = 0.f;
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d].  Half a warp has a row (16 bytes a lane) and four rows in flight.
+// Bound by HBM.  8192 x 28 x 128: 42 us with a warp and 8 bytes a lane per row, 25 now.
+constexpr int kDeltaRows = 4;
+__global__ void __launch_bounds__(256) fmha_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dO, float* __restrict__ delta,
+                                                         int T, int Nq, int D) {
+    const long long rows = (long long)T * Nq, row0 = ((long long)blockIdx.x * 16 + (threadIdx.x >> 4)) * kDeltaRows;
+    const int l = threadIdx.x & 15;
+    uint4 a[kDeltaRows], b[kDeltaRows];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float2 x = __bfloat1622float2(pa[i]), y = __bfloat1622float2(pb[i]);
-        s += x.x * y.x + x.y * y.y;
+    for (int i = 0; i < kDeltaRows; ++i) {
+        a[i] = b[i] = make_uint4(0, 0, 0, 0);
+        if (row0 + i < rows && l * 8 < D) {
+            a[i] = reinterpret_cast<const uint4*>(o + (row0 + i) * D)[l];
+            b[i] = reinterpret_cast<const uint4*>(dO + (row0 + i) * D)[l];
+        }
     }
-    s = warp_sum(s);
-    if (lane == 0) delta[(size_t)(row % Nq) * T + row / Nq] = s;
+#pragma unroll
+    for (int i = 0; i < kDeltaRows; ++i) {
+        float x[8], y[8], s = 0.f;
+        unpack8(*reinterpret_cast<const Vec8*>(&a[i]), x);
+        unpack8(*reinterpret_cast<const Vec8*>(&b[i]), y);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += x[k] * y[k];
+#pragma unroll
+        for (int m = 8; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+        const long long row = row0 + i;
+        if (l == 0 && row < rows) delta[(size_t)(row % Nq) * T + row / Nq] = s;
+    }
+}
+
+// out[t, h, :] = sum over the G query heads of a group of part[t, h * G + g, :], for two tensors (y).  fp32 sums, in the heads' order.
+// 8192 x 28 -> 4 heads of 128, both: 72 us as torch.sum and conversions, 28 here.
+__global__ void __launch_bounds__(256) fmha_sum_heads_kernel(const bf16* __restrict__ part_k, const bf16* __restrict__ part_v,
+                                                             bf16* __restrict__ dk, bf16* __restrict__ dv, long long vecs, int G, int dvec) {
+    const bf16* part = blockIdx.y ? part_v : part_k;
+    bf16* out = blockIdx.y ? dv : dk;
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= vecs) return;
+    const long long th = i / dvec;
+    const uint4* src = reinterpret_cast<const uint4*>(part) + th * G * dvec + i % dvec;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+    for (int g = 0; g < G; ++g) {
+        const uint4 v = src[(long long)g * dvec];
+        float f[8];
+        unpack8(*reinterpret_cast<const Vec8*>(&v), f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += f[k];
+    }
+    reinterpret_cast<Vec8*>(out)[i] = pack8(acc);
 }
 
 struct PlanOut {
@@ -186,7 +215,8 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     } else if (warp == 1) {
         if (lane == 0 && n_kv > 0) {
             constexpr uint32_t idesc_kk = idesc_bf16(128, 128, 0, 0);     // both operands K-major
-            constexpr uint32_t idesc_kn = idesc_bf16(128, 128, 0, 1);     // B = K_j as [N = d, K = kv]: MN-major
+            const int dsteps = (p.D + 15) / 16;                           // a narrow head's zero columns are left out of all products
+            const uint32_t idesc_kn = idesc_bf16(128, dsteps * 16, 0, 1); // B = K_j as [N = d, K = kv]: MN-major
             bool ok = mbar_wait(q_full, 0, abort_flag);
             const uint32_t qa = smem_u32(sQ), doa = smem_u32(sdO);
             auto issue_s = [&](int j) -> bool {
@@ -198,8 +228,9 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k) {
                     const uint32_t off = (k >> 2) * kAtom + (k & 3) * 32;
-                    mma_ss(tS + st * 128, smem_desc_sw128(qa + off, 16, 1024), smem_desc_sw128(ka + off, 16, 1024), idesc_kk,
-                           k ? 1u : 0u);
+                    if (k < dsteps)
+                        mma_ss(tS + st * 128, smem_desc_sw128(qa + off, 16, 1024), smem_desc_sw128(ka + off, 16, 1024), idesc_kk,
+                               k ? 1u : 0u);
                 }
                 mma_commit(&s_full[st]);
                 return true;
@@ -213,7 +244,8 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k) {
                     const uint32_t off = (k >> 2) * kAtom + (k & 3) * 32;
-                    mma_ss(tdP, smem_desc_sw128(doa + off, 16, 1024), smem_desc_sw128(va + off, 16, 1024), idesc_kk, k ? 1u : 0u);
+                    if (k < dsteps)
+                        mma_ss(tdP, smem_desc_sw128(doa + off, 16, 1024), smem_desc_sw128(va + off, 16, 1024), idesc_kk, k ? 1u : 0u);
                 }
                 mma_commit(dp_full);
                 mma_commit(&v_empty[st]);
@@ -629,7 +661,7 @@ MM_API int mm_fmha_bwd(const void* q, const void* k, const void* v, const void* 
     int* k_nseq = q_nseq + mq;
     // short sequences share a tile when the mask allows it: non-causal, keys and queries the same packed sequences
     const int pack = !causal && cu_q == cu_k && T == Tk && variant != 0;
-    fmha_delta_kernel<<<(unsigned)(((long long)T * Nq + 7) / 8), 256, 0, st>>>((const bf16*)o, (const bf16*)dO, delta, T, Nq, D);
+    fmha_delta_kernel<<<(unsigned)(((long long)T * Nq + 16 * kDeltaRows - 1) / (16 * kDeltaRows)), 256, 0, st>>>((const bf16*)o, (const bf16*)dO, delta, T, Nq, D);
     fmha_bwd_plan_kernel<<<2, kPlanThreads, 0, st>>>(PlanOut{cu_q, q_seq, q_r0, q_n, q_nseq, mq}, PlanOut{cu_k, k_seq, k_r0, k_n, k_nseq, mk},
                                                      n_seqs, 128, pack);
     CUtensorMap tQ, tK, tV, tdO, tQ64, tdO64;
@@ -659,5 +691,15 @@ MM_API int mm_fmha_bwd(const void* q, const void* k, const void* v, const void* 
         return (int)cudaGetLastError();
     }
     fmha_bwd_dkv_kernel<<<k_grid, 320, kSmemDkv, st>>>(tQ64, tK, tV, tdO64, pk);
+    return (int)cudaGetLastError();
+}
+
+// dk, dv [Tk, Nkv, D] = sums over each group of the per-query-head partials [Tk, Nkv * G, D] of mm_fmha_bwd (split_heads = 1).
+MM_API int mm_fmha_sum_heads(const void* part_k, const void* part_v, void* dk, void* dv, int Tk, int Nkv, int G, int D, cudaStream_t st) {
+    if (D % 8 || G < 1) return -1;
+    const long long vecs = (long long)Tk * Nkv * (D / 8);
+    if (!vecs) return 0;
+    fmha_sum_heads_kernel<<<dim3((unsigned)((vecs + 255) / 256), 2), 256, 0, st>>>((const bf16*)part_k, (const bf16*)part_v, (bf16*)dk, (bf16*)dv,
+                                                                                  vecs, G, D / 8);
     return (int)cudaGetLastError();
 }

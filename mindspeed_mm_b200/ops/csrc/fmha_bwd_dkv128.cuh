@@ -138,7 +138,8 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // ------------------------------------------------------------------------------ MMA issuer
         if (lane == 0 && n_it > 0) {
             constexpr uint32_t idesc_t = idesc_bf16(128, 128, 0, 0);       // S^T, dP^T
-            constexpr uint32_t idesc_acc = idesc_bf16(128, 128, 0, 1);     // dV, dK: B = dO_i / Q_i read as [N = d, K = q]
+            const int dsteps = (p.D + 15) / 16;                            // a narrow head's zero columns are left out of all products
+            const uint32_t idesc_acc = idesc_bf16(128, dsteps * 16, 0, 1); // dV, dK: B = dO_i / Q_i read as [N = d, K = q]
             bool ok = mbar_wait(kv_full, 0, abort_flag);
             const uint32_t ka = smem_u32(sK), va = smem_u32(sV);
             auto issue_t = [&](int it, uint32_t a_base, const uint8_t* b_tiles, uint64_t* landed, int ring, uint32_t tdst,
@@ -150,7 +151,8 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k) {
                     const uint32_t off = (k >> 2) * kAtom + (k & 3) * 32;
-                    mma_ss(tdst, smem_desc_sw128(a_base + off, 16, 1024), smem_desc_sw128(ba + off, 16, 1024), idesc_t, k ? 1u : 0u);
+                    if (k < dsteps)
+                        mma_ss(tdst, smem_desc_sw128(a_base + off, 16, 1024), smem_desc_sw128(ba + off, 16, 1024), idesc_t, k ? 1u : 0u);
                 }
                 mma_commit(done);
                 return true;

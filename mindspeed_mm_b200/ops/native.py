@@ -90,6 +90,7 @@ def _declare(L):
         "mm_fmha_set_fwd_variant": [_i],
         "mm_fmha_fwd": [_p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _i, _f, _p, _p],
         "mm_fmha_bwd_max_tiles": [_i, _i],
+        "mm_fmha_sum_heads": [_p, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_fmha_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _i, _f,
                         _i, _i, _p, _p],
         "mm_grouped_gemm_bf16": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p],
@@ -822,8 +823,9 @@ def fmha_backward(do, q, k, v, out, lse, cu_q, cu_k, causal, scale):
     LAUNCHES += 4
     if split:
         G = Nq // Nkv
-        dk = torch.sum(dk.view(Tk, Nkv, G, D), 2, dtype=torch.float32).to(q.dtype)
-        dv = torch.sum(dv.view(Tk, Nkv, G, D), 2, dtype=torch.float32).to(q.dtype)
+        part_k, part_v = dk, dv
+        dk, dv = (torch.empty(Tk, Nkv, D, dtype=q.dtype, device=dev) for _ in range(2))
+        _check(L.mm_fmha_sum_heads(part_k.data_ptr(), part_v.data_ptr(), dk.data_ptr(), dv.data_ptr(), Tk, Nkv, G, D, _st()), "fmha_sum_heads")
     return dq, dk, dv
 
 

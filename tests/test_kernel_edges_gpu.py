@@ -313,6 +313,30 @@ def test_attention_tile_lists(lens, causal):
         _close(a, b, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("D", [8, 24, 40, 80, 88, 120, 128])
+@pytest.mark.parametrize("lens,nq,nkv,causal", [([1, 130, 257], 6, 2, True), ([300], 3, 3, False)])
+def test_attention_gradients_of_narrow_heads(D, lens, nq, nkv, causal):
+    """Depth steps of 16 that a head fills, half fills and does not have; row products and sums over a group's heads at odd row counts."""
+    torch.manual_seed(D)
+    T = sum(lens)
+    q, k, v = (torch.randn(T, n, D, device=DEV).bfloat16().requires_grad_() for n in (nq, nkv, nkv))
+    do = torch.randn(T, nq, D, device=DEV).bfloat16()
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    o = ops.attention_varlen(q, k, v, cu, cu, max(lens), max(lens), causal=causal)
+    got = torch.autograd.grad(o, [q, k, v], do)
+    leaf = [t.detach().float().requires_grad_() for t in (q, k, v)]
+    seq = torch.repeat_interleave(torch.arange(len(lens), device=DEV), torch.tensor(lens, device=DEV))
+    mask = seq[:, None] == seq[None]
+    if causal:
+        mask &= torch.arange(T, device=DEV)[:, None] >= torch.arange(T, device=DEV)[None]
+    kk, vv = (t.repeat_interleave(nq // nkv, 1) for t in leaf[1:])
+    s = (torch.einsum("qnd,knd->nqk", leaf[0], kk) * D ** -0.5).masked_fill(~mask, float("-inf"))
+    want = torch.einsum("nqk,knd->qnd", s.softmax(-1), vv)
+    _close(o.detach(), want.detach(), rtol=1e-2, atol=8e-3)
+    for a, b in zip(got, torch.autograd.grad(want, leaf, do.float())):
+        _close(a, b, rtol=2e-2, atol=2e-2)
+
+
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K,splits", [(1421, 3584, 3600, True), (1409, 3592, 4104, True), (1, 264, 18952, None), (5, 8, 18944, True), (136, 520, 8200, True),
                                           (128 * 148, 256, 8192, False), (128 * 149, 256, 8192, True), (128, 256, 256, False), (85, 25368, 8200, False)])
