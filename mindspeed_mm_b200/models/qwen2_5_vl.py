@@ -279,10 +279,7 @@ class VisionBlock(nn.Module):
 
     def forward(self, x, cos, sin, cu_seqlens, max_seqlen):
         T = x.shape[0]
-        # one unbind (a single stack in backward) instead of three selects (three zero-filled adds in backward)
-        q, k, v = self.attn_qkv(self.norm1(x)).view(T, 3, self.num_heads, self.head_dim).unbind(1)
-        q = ops.rope_rotate_half(q, cos, sin)
-        k = ops.rope_rotate_half(k, cos, sin)
+        q, k, v = ops.split_rope(self.attn_qkv(self.norm1(x)), self.num_heads, self.num_heads, cos, sin)
         o = ops.attention_varlen(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen, causal=False)
         x = x + self.attn_proj(o.reshape(T, -1))
         # the block's last product only feeds the residual add: its value is not needed when the block is recomputed
@@ -361,6 +358,7 @@ class VisionTransformer(nn.Module):
     def forward(self, pixel_values, grid_thw=None, plan=None):
         plan = plan or self.plan(grid_thw, pixel_values.device)
         x = self.embed(pixel_values, plan)
+        plan = dict(plan, cos=plan["cos"].to(x.dtype), sin=plan["sin"].to(x.dtype))        # once, not for each block
         for i in range(len(self.blocks)):
             x = self.run_block(i, x, plan)
         return self.finish(x, plan)
@@ -381,8 +379,8 @@ class DecoderLayer(nn.Module):
         """``cache`` (generation, one sequence): a dict that keeps this layer's rotated keys and the values of all
         tokens seen so far; the new tokens attend to them (causal mask aligned to the end of the key sequence)."""
         T = x.shape[0]
-        widths = [self.nq * self.hd, self.nkv * self.hd, self.nkv * self.hd]
         if cache is not None:
+            widths = [self.nq * self.hd, self.nkv * self.hd, self.nkv * self.hd]
             n1, n2, p_qkv, p_o, p_down = self.input_layernorm, self.post_attention_layernorm, self.qkv_proj, self.o_proj, self.down_proj
             # a wrapped or hooked projection (an adapter, an observer) is called as the module it is
             plain = _plain(n1, n2, p_qkv, p_o, p_down) and p_o.bias is None and p_down.bias is None
@@ -394,11 +392,7 @@ class DecoderLayer(nn.Module):
                 return ops.linear_add(ops.norm_linear_swiglu(x, n2.weight, n2.eps, self.gate_up_proj.weight), p_down.weight, x)
             x = x + p_o(o)
             return x + p_down(ops.linear_swiglu(n2(x), self.gate_up_proj.weight))
-        qkv = self.qkv_proj(self.input_layernorm(x))
-        q, k, v = qkv.split(widths, dim=-1)
-        q = ops.rope_rotate_half(q.view(T, self.nq, self.hd), cos, sin)
-        k = ops.rope_rotate_half(k.view(T, self.nkv, self.hd), cos, sin)
-        v = v.view(T, self.nkv, self.hd)
+        q, k, v = ops.split_rope(self.qkv_proj(self.input_layernorm(x)), self.nq, self.nkv, cos, sin)
         o = ops.attention_varlen(q, k, v, cu_seqlens, cu_seqlens,
                                  max_seqlen, max_seqlen, causal=True)
         x = x + self.o_proj(o.reshape(T, -1))

@@ -204,9 +204,7 @@ class Qwen3VisionBlock(nn.Module):
 
     def forward(self, x, cos, sin, cu_seqlens, max_seqlen):
         T = x.shape[0]
-        q, k, v = self.attn_qkv(self.norm1(x)).view(T, 3, self.num_heads, self.head_dim).unbind(1)
-        q = ops.rope_rotate_half(q, cos, sin)
-        k = ops.rope_rotate_half(k, cos, sin)
+        q, k, v = ops.split_rope(self.attn_qkv(self.norm1(x)), self.num_heads, self.num_heads, cos, sin)
         o = ops.attention_varlen(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen, causal=False)
         x = x + self.attn_proj(o.reshape(T, -1))
         return x + self.mlp_fc2(ops.gelu_tanh(self.mlp_fc1(self.norm2(x))), value_unused_in_backward=True)

@@ -140,6 +140,15 @@ def rope_rotate_half(x, cos, sin):
     return ref.rope_rotate_half(x, cos, sin)
 
 
+def split_rope(qkv, nq: int, nk: int, cos, sin):
+    """Queries and keys [T, heads, D], half-rotated, and values of a fused projection [T, (nq + 2 nk) D]."""
+    if _native(qkv) and _nat().split_rope_supported(qkv, nq, nk, cos, sin):
+        return _nat().split_rope(qkv, nq, nk, cos, sin)
+    T, D = qkv.shape[0], qkv.shape[-1] // (nq + 2 * nk)
+    q, k, v = (t.view(T, n, D) for t, n in zip(qkv.split([nq * D, nk * D, nk * D], dim=-1), (nq, nk, nk)))
+    return rope_rotate_half(q, cos, sin), rope_rotate_half(k, cos, sin), v
+
+
 def rope_interleaved(x, cos, sin):
     if _native(x) and x.dtype == torch.bfloat16:
         return _nat().rope(x, cos, sin, interleaved=True)
@@ -288,7 +297,10 @@ def attention_cached(q, k, v, cache: dict, cos=None, sin=None):
         o, cache["k"], cache["v"] = _nat().decode_attention(q, k, v, k_old, v_old, cos, sin)
         return o
     if cos is not None:
-        q, k = rope_rotate_half(q, cos, sin), rope_rotate_half(k, cos, sin)
+        if _native(q) and _nat().rope_pair_supported(q, k, cos, sin) and _nat()._keeps_no_graph((q, k, cos, sin)):
+            q, k = _nat().rope_pair(q, k, cos, sin)
+        else:
+            q, k = rope_rotate_half(q, cos, sin), rope_rotate_half(k, cos, sin)
     if k_old is not None:
         k, v = torch.cat([k_old, k]), torch.cat([v_old, v])
     cache["k"], cache["v"] = k, v

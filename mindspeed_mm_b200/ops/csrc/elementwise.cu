@@ -369,32 +369,58 @@ __global__ void gelu_bwd_kernel(const Vec8* __restrict__ in, const Vec8* __restr
 }
 
 // ------------------------------------------------------------------------------------------ RoPE
-// x: [T, N, D] with row stride `xs` elements between tokens (heads contiguous); out contiguous.
-// half-rotation: cos/sin [T, D] (bf16): o1 = x1*c1 - x2*s1 ; o2 = x2*c2 + x1*s2  (sign flips for bwd)
-__global__ void rope_half_kernel(const bf16* __restrict__ x, long long xs, const bf16* __restrict__ cosb,
-                                 const bf16* __restrict__ sinb, bf16* __restrict__ out, int T, int N, int D,
-                                 float sign) {
-    const int hv = D >> 4;  // vectors per half
-    const long long total = (long long)T * N * hv;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        int c = (int)(idx % hv);
-        long long tn = idx / hv;
-        int n = (int)(tn % N);
-        long long t = tn / N;
-        const bf16* xp = x + t * xs + (long long)n * D;
+// Half-rotation, cos / sin [T, D] (bf16): o1 = x1*c1 - x2*s1 ; o2 = x2*c2 + x1*s2  (the transpose for the backward), of up to two tensors
+// [T, N, D] (heads dense, any token stride), and a copy of a third: the queries, keys and values of a fused projection, or their
+// gradients on the way into that of the projection.  A thread has 8 elements of both halves of a head.
+// Bound by HBM.  8192 tokens of 16 + 16 heads of 80: 30 us as a launch for each tensor with 64-bit divisions of the index, 27 here; their
+// gradients with the values' into one buffer 34 against 49 as two rotations and a stack.
+struct RopePart {
+    const bf16* x;
+    bf16* out;
+    long long xs, os;            // elements between tokens
+    int heads;
+};
+struct RopeArgs {
+    RopePart part[3];            // rotated, rotated, copied
+    const bf16 *cosb, *sinb;
+    int T, D;
+};
+template <class Index, bool BACKWARD>
+__global__ void __launch_bounds__(256) rope_half_kernel(RopeArgs a) {
+    const Index hv = a.D >> 4, unit = (Index)(a.part[0].heads + a.part[1].heads + a.part[2].heads) * hv, total = (Index)a.T * unit;
+    for (Index idx = (Index)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (Index)gridDim.x * 256) {
+        const Index t = idx / unit;
+        const int u = (int)(idx - t * unit), c = u % (int)hv;
+        int n = u / (int)hv, w = 0;
+        if (n >= a.part[0].heads) {
+            n -= a.part[0].heads;
+            w = 1;
+            if (n >= a.part[1].heads) {
+                n -= a.part[1].heads;
+                w = 2;
+            }
+        }
+        const RopePart& p = w == 0 ? a.part[0] : w == 1 ? a.part[1] : a.part[2];
+        const bf16* xp = p.x + (long long)t * p.xs + (long long)n * a.D;
+        bf16* op = p.out + (long long)t * p.os + (long long)n * a.D;
+        const Vec8 v1 = reinterpret_cast<const Vec8*>(xp)[c], v2 = reinterpret_cast<const Vec8*>(xp + a.D / 2)[c];
+        if (w == 2) {
+            reinterpret_cast<Vec8*>(op)[c] = v1;
+            reinterpret_cast<Vec8*>(op + a.D / 2)[c] = v2;
+            continue;
+        }
         float x1[8], x2[8], c1[8], c2[8], s1[8], s2[8], o1[8], o2[8];
-        unpack8(reinterpret_cast<const Vec8*>(xp)[c], x1);
-        unpack8(reinterpret_cast<const Vec8*>(xp + D / 2)[c], x2);
-        const bf16* cp = cosb + t * D;
-        const bf16* sp = sinb + t * D;
+        unpack8(v1, x1);
+        unpack8(v2, x2);
+        const bf16* cp = a.cosb + (long long)t * a.D;
+        const bf16* sp = a.sinb + (long long)t * a.D;
         unpack8(reinterpret_cast<const Vec8*>(cp)[c], c1);
-        unpack8(reinterpret_cast<const Vec8*>(cp + D / 2)[c], c2);
+        unpack8(reinterpret_cast<const Vec8*>(cp + a.D / 2)[c], c2);
         unpack8(reinterpret_cast<const Vec8*>(sp)[c], s1);
-        unpack8(reinterpret_cast<const Vec8*>(sp + D / 2)[c], s2);
+        unpack8(reinterpret_cast<const Vec8*>(sp + a.D / 2)[c], s2);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            if (sign > 0.f) {
+            if (!BACKWARD) {
                 o1[k] = x1[k] * c1[k] - x2[k] * s1[k];
                 o2[k] = x2[k] * c2[k] + x1[k] * s2[k];
             } else {  // transpose of the rotation
@@ -402,10 +428,21 @@ __global__ void rope_half_kernel(const bf16* __restrict__ x, long long xs, const
                 o2[k] = x2[k] * c2[k] - x1[k] * s1[k];
             }
         }
-        bf16* op = out + (t * N + n) * (long long)D;
         reinterpret_cast<Vec8*>(op)[c] = pack8(o1);
-        reinterpret_cast<Vec8*>(op + D / 2)[c] = pack8(o2);
+        reinterpret_cast<Vec8*>(op + a.D / 2)[c] = pack8(o2);
     }
+}
+int rope_half(const RopeArgs& a, int backward, cudaStream_t st) {
+    const long long total = (long long)a.T * (a.part[0].heads + a.part[1].heads + a.part[2].heads) * (a.D / 16);
+    if (total <= 0) return 0;
+    const long long blocks = (total + 255) / 256;
+    const int grid = (int)(blocks < (1 << 20) ? blocks : (1 << 20));
+    const bool small = total < (1LL << 31) - (1LL << 28);            // the index and a grid's step fit 32 bits
+    if (small && backward) rope_half_kernel<unsigned, true><<<grid, 256, 0, st>>>(a);
+    else if (small) rope_half_kernel<unsigned, false><<<grid, 256, 0, st>>>(a);
+    else if (backward) rope_half_kernel<unsigned long long, true><<<grid, 256, 0, st>>>(a);
+    else rope_half_kernel<unsigned long long, false><<<grid, 256, 0, st>>>(a);
+    return (int)cudaGetLastError();
 }
 
 // the same rotation with 4-element (8-byte) accesses, for head dims whose half is a multiple of 4 but not of 8 (72, 88 ...)
@@ -458,18 +495,15 @@ __global__ void rope_half4_kernel(const bf16* __restrict__ x, long long xs, cons
     }
 }
 
-// interleaved pairs: cos/sin [T, D/2] fp32
+// interleaved pairs: cos/sin [T, D/2] fp32.  7800 tokens of 12 heads of 128: 11.7 us with 64-bit divisions of the index, 11.0 here
+template <class Index>
 __global__ void rope_inter_kernel(const bf16* __restrict__ x, long long xs, const float* __restrict__ cosf_,
                                   const float* __restrict__ sinf_, bf16* __restrict__ out, int T, int N, int D,
                                   float sign) {
-    const int dv = D >> 3;
-    const long long total = (long long)T * N * dv;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        int c = (int)(idx % dv);
-        long long tn = idx / dv;
-        int n = (int)(tn % N);
-        long long t = tn / N;
+    const Index dv = D >> 3, unit = dv * (Index)N, total = (Index)T * unit;
+    for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (Index)gridDim.x * blockDim.x) {
+        const long long t = idx / unit;
+        const int u = (int)(idx - (Index)t * unit), n = u / (int)dv, c = u % (int)dv;
         float f[8], o[8];
         unpack8(reinterpret_cast<const Vec8*>(x + t * xs + (long long)n * D)[c], f);
         const float4 cs = reinterpret_cast<const float4*>(cosf_ + t * (D / 2))[c];
@@ -967,16 +1001,43 @@ MM_API int mm_rope_half(const void* x, long long xs, const void* cosb, const voi
             (const bf16*)x, xs, (const bf16*)cosb, (const bf16*)sinb, (bf16*)out, T, N, D, backward ? -1.f : 1.f);
         return (int)cudaGetLastError();
     }
-    rope_half_kernel<<<grid_for((long long)T * N * (D / 16), 256), 256, 0, st>>>(
-        (const bf16*)x, xs, (const bf16*)cosb, (const bf16*)sinb, (bf16*)out, T, N, D, backward ? -1.f : 1.f);
-    return (int)cudaGetLastError();
+    RopeArgs a{};
+    a.part[0] = {(const bf16*)x, (bf16*)out, xs, (long long)N * D, N};
+    a.cosb = (const bf16*)cosb;
+    a.sinb = (const bf16*)sinb;
+    a.T = T;
+    a.D = D;
+    return rope_half(a, backward, st);
+}
+
+// Queries and keys rotated, values copied (nv = 0: left alone); strides in elements between tokens, heads dense.  D % 16 == 0, pointers
+// 16-byte aligned, strides multiples of 8.
+MM_API int mm_rope_qkv(const void* q, long long qs, const void* k, long long ks, const void* v, long long vs, const void* cosb, const void* sinb,
+                       void* qo, long long qos, void* ko, long long kos, void* vo, long long vos, int T, int nq, int nk, int nv, int D,
+                       int backward, cudaStream_t st) {
+    if (D % 16 || (qs | ks | vs | qos | kos | vos) % 8) return -1;
+    if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cosb | (uintptr_t)sinb | (uintptr_t)qo | (uintptr_t)ko | (uintptr_t)vo) & 15) return -2;
+    RopeArgs a{};
+    a.part[0] = {(const bf16*)q, (bf16*)qo, qs, qos, nq};
+    a.part[1] = {(const bf16*)k, (bf16*)ko, ks, kos, nk};
+    a.part[2] = {(const bf16*)v, (bf16*)vo, vs, vos, nv};
+    a.cosb = (const bf16*)cosb;
+    a.sinb = (const bf16*)sinb;
+    a.T = T;
+    a.D = D;
+    return rope_half(a, backward, st);
 }
 
 MM_API int mm_rope_interleaved(const void* x, long long xs, const float* cosf_, const float* sinf_, void* out, int T,
                                int N, int D, int backward, cudaStream_t st) {
     if (D % 8 || xs % 8) return -1;
-    rope_inter_kernel<<<grid_for((long long)T * N * (D / 8), 256), 256, 0, st>>>(
-        (const bf16*)x, xs, cosf_, sinf_, (bf16*)out, T, N, D, backward ? -1.f : 1.f);
+    const long long total = (long long)T * N * (D / 8), blocks = (total + 255) / 256;
+    if (total <= 0) return 0;
+    const int grid = (int)(blocks < (1 << 20) ? blocks : (1 << 20));
+    if (total < (1LL << 31) - (1LL << 28))                           // the index and a grid's step fit 32 bits
+        rope_inter_kernel<unsigned><<<grid, 256, 0, st>>>((const bf16*)x, xs, cosf_, sinf_, (bf16*)out, T, N, D, backward ? -1.f : 1.f);
+    else
+        rope_inter_kernel<unsigned long long><<<grid, 256, 0, st>>>((const bf16*)x, xs, cosf_, sinf_, (bf16*)out, T, N, D, backward ? -1.f : 1.f);
     return (int)cudaGetLastError();
 }
 

@@ -69,6 +69,7 @@ def _declare(L):
         "mm_gelu_fwd": [_p, _p, _ll, _i, _p],
         "mm_gelu_bwd": [_p, _p, _p, _ll, _i, _p],
         "mm_rope_half": [_p, _ll, _p, _p, _p, _i, _i, _i, _i, _p],
+        "mm_rope_qkv": [_p, _ll, _p, _ll, _p, _ll, _p, _p, _p, _ll, _p, _ll, _p, _ll, _i, _i, _i, _i, _i, _i, _p],
         "mm_rope_interleaved": [_p, _ll, _p, _p, _p, _i, _i, _i, _i, _p],
         "mm_ln_mod_fwd": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _f, _p],
         "mm_ln_mod_bwd_ctas": [_i, _i],
@@ -406,6 +407,74 @@ def rope(x, cos, sin, interleaved: bool):
             return reference.rope_rotate_half(x, cos, sin)
         cos, sin = cos.to(torch.bfloat16).contiguous(), sin.to(torch.bfloat16).contiguous()
     return _run(_Rope, x, cos, sin, interleaved)
+
+
+def _rope_parts(q, k, v, cos, sin, outs, backward):
+    """Rotates q and k into ``outs[:2]`` and copies v (None: left alone) into ``outs[2]``; all [T, N, D]."""
+    dense = lambda t: t if t is None else _dense(t) if t.data_ptr() % 16 else _dense_heads(t)  # noqa: E731
+    q, k, v = dense(q), dense(k), dense(v)
+    T, nq, D = q.shape
+    pointers = [a for t in (q, k, v) for a in ((None, 0) if t is None else (t.data_ptr(), t.stride(0)))]
+    targets = [a for t in outs for a in ((None, 0) if t is None else (t.data_ptr(), t.stride(0)))]
+    _check(lib().mm_rope_qkv(*pointers, cos.data_ptr(), sin.data_ptr(), *targets, T, nq, k.shape[1], 0 if v is None else v.shape[1], D,
+                             int(backward), _st()), "rope_qkv")
+
+
+def rope_pair_supported(q, k, cos, sin) -> bool:
+    """The queries and keys of the same tokens, heads of a multiple of 16, tables made for them."""
+    T, _, D = q.shape
+    return (q.dtype == torch.bfloat16 and k.dtype == q.dtype and D % 16 == 0 and k.shape[0] == T and k.shape[2] == D and q.device == k.device
+            and tuple(cos.shape) == (T, D) and tuple(sin.shape) == (T, D))
+
+
+def _tables(cos, sin):
+    return _dense(cos.to(torch.bfloat16)), _dense(sin.to(torch.bfloat16))
+
+
+def rope_pair(q, k, cos, sin):
+    """Both rotated by one kernel.  No autograd: for calls that keep no graph."""
+    cos, sin = _tables(cos, sin)
+    outs = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (q, k)]
+    _rope_parts(q, k, None, cos, sin, [*outs, None], False)
+    return outs
+
+
+class _SplitRope(torch.autograd.Function):
+    """Rotated queries and keys, and the values as they lie, of a fused projection [T, (nq + 2 nk) D]; its gradient is written whole by one
+    kernel (a rotation for each tensor and a stack or concatenation before)."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, nq, nk):
+        T, D = qkv.shape[0], qkv.shape[1] // (nq + 2 * nk)
+        ctx.save_for_backward(cos, sin)
+        ctx.heads = nq, nk, D
+        q, k, v = (t.view(T, -1, D) for t in qkv.split([nq * D, nk * D, nk * D], dim=1))
+        outs = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (q, k)]
+        _rope_parts(q, k, None, cos, sin, [*outs, None], False)
+        return (*outs, v)
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        cos, sin = ctx.saved_tensors
+        nq, nk, D = ctx.heads
+        T = dq.shape[0]
+        if torch.is_grad_enabled():          # create_graph: the values' part is differentiated
+            return torch.cat([_rope_call(t, cos, sin, False, True).view(T, -1) for t in (dq, dk)] + [dv.reshape(T, -1)], dim=1), None, None, None, None
+        dqkv = torch.empty(T, (nq + 2 * nk) * D, dtype=dq.dtype, device=dq.device)
+        _rope_parts(dq, dk, dv, cos, sin, [t.view(T, -1, D) for t in dqkv.split([nq * D, nk * D, nk * D], dim=1)], True)
+        return dqkv, None, None, None, None
+
+
+def split_rope_supported(qkv, nq, nk, cos, sin) -> bool:
+    heads = nq + 2 * nk
+    if qkv.dim() != 2 or qkv.dtype != torch.bfloat16 or qkv.shape[1] % heads or not _ok2d(qkv):
+        return False
+    T, D = qkv.shape[0], qkv.shape[1] // heads
+    return T > 0 and D % 16 == 0 and tuple(cos.shape) == (T, D) and tuple(sin.shape) == (T, D) and not (cos.requires_grad or sin.requires_grad)
+
+
+def split_rope(qkv, nq, nk, cos, sin):
+    return _run(_SplitRope, qkv, *_tables(cos, sin), nq, nk)
 
 
 # --------------------------------------------------------------------------- adaLN

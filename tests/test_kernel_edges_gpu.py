@@ -382,6 +382,45 @@ def test_products_on_pairs_of_sms(layout, M, N, K, rows):
     _close(got, want, rtol=4.5e-3, atol=2e-3 * K ** 0.5 / 100)
 
 
+@pytest.mark.parametrize("T,nq,nk,D,pitch", [(1, 1, 1, 16, 0), (37, 4, 2, 80, 0), (130, 28, 4, 128, 8), (257, 16, 16, 80, 0), (3, 5, 1, 48, 16), (33, 2, 2, 72, 0),
+                                             (65, 3, 3, 128, 4)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_rotation_of_a_fused_projection(T, nq, nk, D, pitch, graph):
+    """Heads whose half is a multiple of 8 and not, rows that lie apart (aligned and not), one token and one head: the separate
+    rotations to the bit, gradients too; create_graph keeps the values' part differentiable."""
+    torch.manual_seed(T)
+    wide = torch.randn(T, (nq + 2 * nk) * D + pitch, device=DEV).bfloat16()
+    qkv = wide[:, :(nq + 2 * nk) * D].detach().requires_grad_()
+    ang = torch.randn(T, D, device=DEV)
+    cos, sin = ang.cos().bfloat16(), ang.sin().bfloat16()
+    outs = ops.split_rope(qkv, nq, nk, cos, sin)
+    parts = [t.reshape(T, n, D) for t, n in zip(qkv.split([nq * D, nk * D, nk * D], 1), (nq, nk, nk))]
+    want = [ops.rope_rotate_half(parts[0].contiguous(), cos, sin), ops.rope_rotate_half(parts[1].contiguous(), cos, sin), parts[2]]
+    dys = [torch.randn_like(t).requires_grad_(graph) for t in want]
+    got_g = torch.autograd.grad(outs, qkv, dys, create_graph=graph)[0]
+    want_g = torch.autograd.grad(want, qkv, dys, create_graph=graph)[0]
+    for a, b in zip((*outs, got_g), (*want, want_g)):
+        assert torch.equal(a, b)
+    if graph:
+        assert torch.equal(torch.autograd.grad(got_g.float().sum(), dys[2])[0], torch.ones_like(dys[2]))
+    with torch.no_grad():
+        for a, b in zip(ops.split_rope(qkv, nq, nk, cos, sin), want):
+            assert torch.equal(a, b)
+    _close(outs[0].detach(), ref.rope_rotate_half(parts[0].detach(), cos, sin), rtol=4e-3, atol=1e-3)
+
+
+@pytest.mark.parametrize("T,N,D", [(1, 1, 8), (77, 12, 128), (33, 3, 24)])
+def test_interleaved_rotation(T, N, D):
+    x = torch.randn(T, N, D, device=DEV).bfloat16().requires_grad_()
+    ang = torch.randn(T, D // 2, device=DEV)
+    y = ops.rope_interleaved(x, ang.cos(), ang.sin())
+    dy = torch.randn_like(y)
+    xr = x.detach().float().requires_grad_()
+    yr = ref.rope_interleaved(xr, ang.cos(), ang.sin())
+    _close(y.detach(), yr.detach(), rtol=4e-3, atol=1e-3)
+    _close(torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(yr, xr, dy.float())[0], rtol=4e-3, atol=1e-3)
+
+
 @pytest.mark.parametrize("T,H,V,valid,chunk", [(512, 256, 512, 100, 8192), (513, 256, 512, 0, 8192), (513, 264, 520, 513, 8192), (600, 256, 1000, 1, 8192),
                                                (700, 512, 4096, 64, 8192), (700, 512, 4096, 65, 256), (8300, 256, 512, 5000, 8192),
                                                (8300, 256, 512, 130, 4096), (1600, 3584, 18944, 1421, 8192)])
