@@ -12,6 +12,32 @@ typedef __nv_bfloat162 bf162;
 // Status word written by kernels whose bounded waits ran out (read by the host; never traps).
 enum MmStatus : int { MM_OK = 0, MM_TIMEOUT_TMA = 1, MM_TIMEOUT_MMA = 2, MM_TIMEOUT_EPI = 3, MM_TIMEOUT_PEER = 4 };
 
+// ---- starting while the kernel in front drains (programmatic stream serialisation)
+// A kernel that is launched by launch_after() may start before its predecessor has ended: wait_for_predecessor() comes before its first
+// access to global memory, and the loads behind it are not marked as of constant memory (no __restrict__ const parameter, no __ldg: the
+// compiler may move those up past the wait).
+// let_successor_start() lets such a successor come up as soon as every block of this kernel has; it stands after the wait, never before, so
+// that a successor may rely on everything in front of this kernel being complete.
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline int launch_after(void (*kern)(P...), int cluster, dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 struct alignas(16) Vec8 {
     bf162 v[4];
 };

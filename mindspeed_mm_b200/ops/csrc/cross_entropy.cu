@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(kCEThreads) ce_fwd_bwd_kernel(bf16* __restrict
                                                                 const long long* __restrict__ labels,
                                                                 float* __restrict__ loss, int V, int ignore_index,
                                                                 const int* __restrict__ src, const int* __restrict__ count, int base) {
+    let_successor_start();
     __shared__ float red[72];
     const long long row = blockIdx.x;
     Vec8* zr = reinterpret_cast<Vec8*>(z + row * ld);
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kCEThreads) ce_fwd_bwd_kernel(bf16* __restrict
 constexpr int kListThreads = 1024, kListEach = 8;
 __global__ void __launch_bounds__(kListThreads) label_rows_kernel(const long long* __restrict__ labels, int T, int ignore_index,
                                                                  int* __restrict__ src, int* __restrict__ row, int* __restrict__ count) {
+    let_successor_start();
     __shared__ int sums[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int base = 0;

@@ -16,9 +16,6 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// After the wait, never before: a successor may then rely on everything in front of this kernel being complete.
-__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ uint4 ld_once(const uint4* p) {
@@ -31,24 +28,6 @@ __device__ __forceinline__ float2 bf2(uint32_t v) { return __bfloat1622float2(*r
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     bf162 t = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&t);
-}
-
-template <class... P, class... A>
-int launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, A... args) {
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // ------------------------------------------------------------------------------------------ skinny product
@@ -364,8 +343,8 @@ int run_gemv(const GemvParams& p, cudaStream_t st) {
         // 9.1 -> 5.1, 37888 x 3584 with norm and SwiGLU 48.2 -> 40.2 (6.8 TB/s), 152064 x 3584 165 -> 155, 3584 x 18944 37 -> 22
         const int pairs = SWIGLU ? p.N : p.N / 2;
         if (p.K <= kRowK)
-            return launch_pdl(gemv_rows_kernel<SWIGLU, NORM>, dim3(pairs < kRowBlocks ? pairs : kRowBlocks), kGemvWarps * 32, (size_t)0, 1, st, p);
-        if (!SWIGLU && !NORM) return launch_pdl(gemv_split_kernel, dim3(pairs), kGemvWarps * 32, (size_t)0, 1, st, p);
+            return launch_after(gemv_rows_kernel<SWIGLU, NORM>, 1, dim3(pairs < kRowBlocks ? pairs : kRowBlocks), kGemvWarps * 32, (size_t)0, st, p);
+        if (!SWIGLU && !NORM) return launch_after(gemv_split_kernel, 1, dim3(pairs), kGemvWarps * 32, (size_t)0, st, p);
     }
     auto kern = gemv_kernel<M, SWIGLU, NORM>;
     const size_t smem = (size_t)(M + NORM) * p.K * 2;
@@ -374,7 +353,7 @@ int run_gemv(const GemvParams& p, cudaStream_t st) {
         if (e != cudaSuccess) return (int)e;
     }
     const int units = SWIGLU ? p.N : p.N / 2;
-    return launch_pdl(kern, dim3((units + kGemvWarps - 1) / kGemvWarps), kGemvWarps * 32, smem, 1, st, p);
+    return launch_after(kern, 1, dim3((units + kGemvWarps - 1) / kGemvWarps), kGemvWarps * 32, smem, st, p);
 }
 
 template <int M>
@@ -758,5 +737,5 @@ MM_API int mm_decode_attention(const void* q, const void* k, const void* v, cons
     cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
-    return launch_pdl(decode_attention_kernel, dim3(splits, Nkv), kDecWarps * 32, (size_t)kDecSmem, splits, st, p);
+    return launch_after(decode_attention_kernel, splits, dim3(splits, Nkv), kDecWarps * 32, (size_t)kDecSmem, st, p);
 }

@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const bf16* __
                                                                    const bf16* __restrict__ w, bf16* __restrict__ y,
                                                                    float* __restrict__ rstd_out, int T, int H,
                                                                    long long ldx, float eps) {
+    let_successor_start();
     __shared__ float red[72];
     const int nvec = H >> 3;
     // a thread owns the same columns in every row: its slice of the weight is read once, not once per row (re-reading it
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_v16_kernel(const bf16
                                                                        const bf16* __restrict__ w, bf16* __restrict__ y,
                                                                        float* __restrict__ rstd_out, int T, int H,
                                                                        long long ldx, float eps) {
+    let_successor_start();
     __shared__ float red[72];
     const int nvec = H >> 4;
     Vec16 wc[NV], cache[NV];
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_bwd_kernel(const bf16* __rest
                                                                    const float* __restrict__ rstd_in,
                                                                    bf16* __restrict__ dx,
                                                                    float* __restrict__ dw_partial, int T, int H, long long ldx) {
+    let_successor_start();
     __shared__ float red[72];
     const int nvec = H >> 3;
     float dwacc[NV][8];
@@ -263,6 +266,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_bwd_kernel(const bf16* __rest
 // Folds [P, H] fp32 partials into bf16 [H]: one warp per 32 columns, lanes stride over P, then a
 // transposed shuffle-free reduction through shared memory.
 __global__ void fold_partials_kernel(const float* __restrict__ partial, bf16* __restrict__ out, int P, int H) {
+    let_successor_start();
     __shared__ float tile[8][33];
     const int c = blockIdx.x * 32 + threadIdx.x;  // blockDim = (32, 8)
     float s = 0.f;
@@ -281,6 +285,7 @@ __global__ void fold_partials_kernel(const float* __restrict__ partial, bf16* __
 // ------------------------------------------------------------------------------------------ SwiGLU
 // in: [T, 2F] = [gate | up];  out: [T, F] = silu(gate) * up
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, long long T, int F) {
+    let_successor_start();
     const int fv = F >> 3;
     const long long total = T * fv;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -299,6 +304,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ in, bf16* __restrict_
 
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ in, const bf16* __restrict__ dout, bf16* __restrict__ din,
                                   long long T, int F) {
+    let_successor_start();
     const int fv = F >> 3;
     const long long total = T * fv;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -346,6 +352,7 @@ __device__ __forceinline__ float gelu_df(float x) {
 
 template <bool TANH>
 __global__ void gelu_fwd_kernel(const Vec8* __restrict__ in, Vec8* __restrict__ out, long long nvec) {
+    let_successor_start();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
         float a[8];
         unpack8(in[i], a);
@@ -358,6 +365,7 @@ __global__ void gelu_fwd_kernel(const Vec8* __restrict__ in, Vec8* __restrict__ 
 template <bool TANH>
 __global__ void gelu_bwd_kernel(const Vec8* __restrict__ in, const Vec8* __restrict__ dout, Vec8* __restrict__ din,
                                 long long nvec) {
+    let_successor_start();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
         float a[8], g[8];
         unpack8(in[i], a);
@@ -387,6 +395,7 @@ struct RopeArgs {
 };
 template <class Index, bool BACKWARD>
 __global__ void __launch_bounds__(256) rope_half_kernel(RopeArgs a) {
+    let_successor_start();
     const Index hv = a.D >> 4, unit = (Index)(a.part[0].heads + a.part[1].heads + a.part[2].heads) * hv, total = (Index)a.T * unit;
     for (Index idx = (Index)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (Index)gridDim.x * 256) {
         const Index t = idx / unit;
@@ -461,6 +470,7 @@ __device__ __forceinline__ uint2 pack4(const float* f) {
 __global__ void rope_half4_kernel(const bf16* __restrict__ x, long long xs, const bf16* __restrict__ cosb,
                                   const bf16* __restrict__ sinb, bf16* __restrict__ out, int T, int N, int D,
                                   float sign) {
+    let_successor_start();
     const int hv = D >> 3;  // 4-element vectors per half
     const long long total = (long long)T * N * hv;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -500,6 +510,7 @@ template <class Index>
 __global__ void rope_inter_kernel(const bf16* __restrict__ x, long long xs, const float* __restrict__ cosf_,
                                   const float* __restrict__ sinf_, bf16* __restrict__ out, int T, int N, int D,
                                   float sign) {
+    let_successor_start();
     const Index dv = D >> 3, unit = dv * (Index)N, total = (Index)T * unit;
     for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (Index)gridDim.x * blockDim.x) {
         const long long t = idx / unit;
@@ -526,6 +537,7 @@ __global__ void __launch_bounds__(kThreads) ln_mod_fwd_kernel(const bf16* __rest
                                                               const bf16* __restrict__ shift, bf16* __restrict__ y,
                                                               float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                               int T, int S, int H, float eps) {
+    let_successor_start();
     __shared__ float red[72];
     const int nvec = H >> 3;
     // scale / shift of the batch entry the current row belongs to, kept (packed) in registers and re-read only when the
@@ -606,6 +618,7 @@ __global__ void __launch_bounds__(kThreads) ln_mod_fwd_v16_kernel(const bf16* __
                                                                   const bf16* __restrict__ shift, bf16* __restrict__ y,
                                                                   float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                                   int T, int S, int H, float eps) {
+    let_successor_start();
     __shared__ float red[72];
     const int nvec = H >> 4;
     Vec16 xc[NV], scv[NV], shv[NV];
@@ -688,6 +701,7 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
                                                               float* __restrict__ dscale_partial,
                                                               float* __restrict__ dshift_partial, int S, int H,
                                                               int ctas_per_batch) {
+    let_successor_start();
     __shared__ float red[72];
     const int nvec = H >> 3;
     const int b = blockIdx.x / ctas_per_batch, lane_cta = blockIdx.x % ctas_per_batch;
@@ -758,6 +772,7 @@ __global__ void __launch_bounds__(kThreads) ln_mod_bwd_kernel(const bf16* __rest
 // out[b, c] = sum over p of partial[b*P + p, c], for dscale (blockIdx.z = 0) and dshift; 32 lanes along c, 32 along p
 __global__ void __launch_bounds__(1024) fold_scale_shift_kernel(const float* __restrict__ p1, const float* __restrict__ p2,
                                                                bf16* __restrict__ out1, bf16* __restrict__ out2, int P, int H) {
+    let_successor_start();
     __shared__ float tile[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y;
     const float* partial = blockIdx.z ? p2 : p1;
@@ -779,6 +794,7 @@ __global__ void __launch_bounds__(1024) fold_scale_shift_kernel(const float* __r
 // block is faster: 1 x 7800 x 1536 44 us, 142 with a thread per column.
 __global__ void __launch_bounds__(256) fold_few_scale_shift_kernel(const float* __restrict__ p1, const float* __restrict__ p2,
                                                                    bf16* __restrict__ out1, bf16* __restrict__ out2, int P, int H) {
+    let_successor_start();
     const int c = blockIdx.x * 256 + threadIdx.x, b = blockIdx.y;
     if (c >= H) return;
     const float* partial = (blockIdx.z ? p2 : p1) + (size_t)b * P * H + c;
@@ -792,6 +808,7 @@ __global__ void __launch_bounds__(256) fold_few_scale_shift_kernel(const float* 
 __global__ void gated_residual_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y,
                                       const bf16* __restrict__ gate, bf16* __restrict__ out, long long T, int S,
                                       int H) {
+    let_successor_start();
     const int hv = H >> 3;
     const long long total = T * hv;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -817,6 +834,7 @@ __global__ void adamw_kernel(float* __restrict__ p, float* __restrict__ m, float
                              const G* __restrict__ g, bf16* __restrict__ p16, long long n, long long split, float lr,
                              float b1, float b2, float eps, float wd, float bc1, float bc2, float gscale,
                              const float* __restrict__ scale_ptr) {
+    let_successor_start();
     const float gs = scale_ptr ? gscale * (*scale_ptr) : gscale;
     const long long nv = n >> 2;
     const uint64_t pol = l2_evict_first_policy();      // 28 bytes per parameter, each touched once
@@ -869,6 +887,7 @@ inline int grid_for(long long work_items, int threads, int per_sm = 8) {
 constexpr int kSqNormBlocks = 128;
 
 __global__ void __launch_bounds__(256) sq_norm_kernel(const float* __restrict__ x, long long n, float* __restrict__ partials) {
+    let_successor_start();
     __shared__ float red[40];
     float acc = 0.f;
     const long long n4 = n >> 2;

@@ -52,6 +52,7 @@ struct BwdParams {
 constexpr int kDeltaRows = 4;
 __global__ void __launch_bounds__(256) fmha_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dO, float* __restrict__ delta,
                                                          int T, int Nq, int D) {
+    let_successor_start();
     const long long rows = (long long)T * Nq, row0 = ((long long)blockIdx.x * 16 + (threadIdx.x >> 4)) * kDeltaRows;
     const int l = threadIdx.x & 15;
     uint4 a[kDeltaRows], b[kDeltaRows];
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(256) fmha_delta_kernel(const bf16* __restrict_
 // 8192 x 28 -> 4 heads of 128, both: 72 us as torch.sum and conversions, 28 here.
 __global__ void __launch_bounds__(256) fmha_sum_heads_kernel(const bf16* __restrict__ part_k, const bf16* __restrict__ part_v,
                                                              bf16* __restrict__ dk, bf16* __restrict__ dv, long long vecs, int G, int dvec) {
+    let_successor_start();
     const bf16* part = blockIdx.y ? part_v : part_k;
     bf16* out = blockIdx.y ? dv : dk;
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -106,6 +108,7 @@ struct PlanOut {
 };
 // Block 0: query tiles, heavy ones first; block 1: key tiles (early ones see the most query tiles under a causal mask).
 __global__ void __launch_bounds__(kPlanThreads) fmha_bwd_plan_kernel(PlanOut q, PlanOut k, int n_seqs, int rows, int pack) {
+    let_successor_start();
     const PlanOut& o = blockIdx.x ? k : q;
     plan_tiles(o.cu, n_seqs, o.tile_seq, o.tile_r0, o.n_tiles, o.tile_nseq, o.max_tiles, rows, blockIdx.x == 0, pack);
 }
@@ -122,6 +125,8 @@ constexpr int kSmemDq = (2 + kRingK + 2) * kTile + 1024 + 1024;
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
+    wait_for_predecessor();
+    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;     // whole CTA leaves before any barrier or TMEM allocation
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -388,6 +393,8 @@ constexpr int kSmemDkv = 2 * kTile + 2 * kRing * kQTile + 2048 + 1024;
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
+    wait_for_predecessor();
+    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -683,15 +690,14 @@ MM_API int mm_fmha_bwd(const void* q, const void* k, const void* v, const void* 
     pk.n_tiles = k_n;
     pk.heads_first = heads_go_first(causal, mk);
     const dim3 k_grid = attention_grid(pk.heads_first, mk, split_heads ? Nq : Nkv);
-    fmha_bwd_dq_kernel<<<attention_grid(p.heads_first, mq, Nq), 320, kSmemDq, st>>>(tQ, tK, tV, tdO, p);
+    r = launch_after(fmha_bwd_dq_kernel, 1, attention_grid(p.heads_first, mq, Nq), 320, kSmemDq, st, tQ, tK, tV, tdO, p);
+    if (r) return r;
     if (variant != 0) {      // dK/dV over 128-row query steps: all four products at N = 128
         if (cudaFuncSetAttribute(fmha_bwd_dkv128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDkv128) != cudaSuccess)
             return -3;
-        fmha_bwd_dkv128_kernel<<<k_grid, 320, kSmemDkv128, st>>>(tQ, tK, tV, tdO, pk);
-        return (int)cudaGetLastError();
+        return launch_after(fmha_bwd_dkv128_kernel, 1, k_grid, 320, kSmemDkv128, st, tQ, tK, tV, tdO, pk);
     }
-    fmha_bwd_dkv_kernel<<<k_grid, 320, kSmemDkv, st>>>(tQ64, tK, tV, tdO64, pk);
-    return (int)cudaGetLastError();
+    return launch_after(fmha_bwd_dkv_kernel, 1, k_grid, 320, kSmemDkv, st, tQ64, tK, tV, tdO64, pk);
 }
 
 // dk, dv [Tk, Nkv, D] = sums over each group of the per-query-head partials [Tk, Nkv * G, D] of mm_fmha_bwd (split_heads = 1).

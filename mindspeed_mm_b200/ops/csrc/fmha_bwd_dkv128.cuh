@@ -35,6 +35,8 @@ static_assert(kSmemDkv128 <= 227 * 1024, "shared memory of a CTA");
 __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
+    wait_for_predecessor();
+    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     constexpr int BQ = 128;
     extern __shared__ uint8_t smem_raw[];

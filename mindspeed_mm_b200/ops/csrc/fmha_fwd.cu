@@ -50,12 +50,15 @@ struct FmhaParams {
 // Later query tiles of a causal sequence have more key tiles: emit them first so the tail of the grid is made of short work items.
 __global__ void __launch_bounds__(kPlanThreads) fmha_plan_kernel(const int* cu_q, int n_seqs, int* tile_seq, int* tile_q0, int* n_tiles,
                                                                 int* tile_nseq, int max_tiles, int pack) {
+    let_successor_start();
     plan_tiles(cu_q, n_seqs, tile_seq, tile_q0, n_tiles, tile_nseq, max_tiles, BQ, true, pack);
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaParams p) {
+    wait_for_predecessor();
+    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -369,11 +372,9 @@ MM_API int mm_fmha_fwd(const void* q, const void* k, const void* v, void* o, flo
     // 1 x 4096 182 / 156, 1 x 7800 461 / 388; 40 heads, 1 x 32760 24.3 / 20.2 ms.  Causal (half the tiles of a CTA on average):
     // 28 heads, 2048 312 / 314, 1 x 4096 247 / 223.
     const bool alternate = g_fwd_variant == 3 && Tk >= (causal ? 3072LL : 1024LL) * n_seqs;
-    if (alternate)
-        fmha_fwd_alt_kernel<<<grid, kAltThreads, kAltSmem, st>>>(tK, tV, p);
-    else if (g_fwd_variant == 0)      // fallback: one softmax warpgroup, O folded in registers
-        fmha_fwd_kernel<<<grid, kThreads, kSmem, st>>>(tQ, tK, tV, p);
-    else                         // default: split softmax, O accumulated in tensor memory with lazy rescaling
-        fmha_fwd_split_kernel<2, true><<<grid, 64 + 256, kSmem, st>>>(tQ, tK, tV, p);
-    return (int)cudaGetLastError();
+    if (alternate) return launch_after(fmha_fwd_alt_kernel, 1, grid, kAltThreads, kAltSmem, st, tK, tV, p);
+    if (g_fwd_variant == 0)           // fallback: one softmax warpgroup, O folded in registers
+        return launch_after(fmha_fwd_kernel, 1, grid, kThreads, kSmem, st, tQ, tK, tV, p);
+    // default: split softmax, O accumulated in tensor memory with lazy rescaling
+    return launch_after(fmha_fwd_split_kernel<2, true>, 1, grid, 64 + 256, kSmem, st, tQ, tK, tV, p);
 }

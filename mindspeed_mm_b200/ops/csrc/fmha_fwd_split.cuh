@@ -39,6 +39,8 @@ template <int PARTS, bool LAZY = false>
 __global__ void __launch_bounds__(64 + 128 * PARTS, 1)
 fmha_fwd_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaParams p) {
+    wait_for_predecessor();
+    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

@@ -51,6 +51,7 @@ struct GdnParams {
 __global__ void __launch_bounds__(192, 1)
 gdn_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmA, const GdnParams p) {
+    let_successor_start();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sStage = smem;                          // [2][W | Qg | Kd | At]

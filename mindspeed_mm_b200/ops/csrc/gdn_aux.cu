@@ -22,6 +22,7 @@ template <int K, bool SILU>
 __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w,
                                                          const int* __restrict__ seq_start, bf16* __restrict__ y, int T,
                                                          int D) {
+    let_successor_start();
     const int dv = D >> 3;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= dv) return;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps) conv1d_bwd_kernel(const bf16* 
                                                                     const int* __restrict__ seq_start, const int* __restrict__ seq_end,
                                                                     const bf16* __restrict__ dy, bf16* __restrict__ dx,
                                                                     float* __restrict__ dw, int T, int D) {
+    let_successor_start();
     constexpr int CH = 4;
     __shared__ uint2 stage[kBwdWarps][kBwdStages * kBwdChunk][2][32];       // x and dy of a token
     __shared__ int bounds[kBwdWarps][2][kStrip + kMaxK];                      // where the sequences of tokens t0, t0 + 1, ... start and end
@@ -240,6 +242,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps) conv1d_bwd_kernel(const bf16* 
 // ---- l2norm over the last dim (D <= 256, one warp per row)
 __global__ void l2norm_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, float* __restrict__ rnorm, long long rows,
                                   int D, float eps) {
+    let_successor_start();
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31;
@@ -257,6 +260,7 @@ __global__ void l2norm_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__
 
 __global__ void l2norm_bwd_kernel(const bf16* __restrict__ y, const bf16* __restrict__ dy, const float* __restrict__ rnorm,
                                   bf16* __restrict__ dx, long long rows, int D) {
+    let_successor_start();
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31;
@@ -289,6 +293,7 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 __global__ void __launch_bounds__(256) delta_heads_fwd_kernel(const Vec8* __restrict__ x, Vec8* __restrict__ q, Vec8* __restrict__ k,
                                                               Vec8* __restrict__ v, float* __restrict__ rnorm, int hk, int rep, int vvec,
                                                               float eps) {
+    let_successor_start();
     const size_t t = blockIdx.x;
     const int nn = 2 * hk * kHeadVec, W = nn + vvec;      // nn is a multiple of 32: a warp has rows to normalise or values, not both
     const Vec8* src = x + t * W;
@@ -318,6 +323,7 @@ __global__ void __launch_bounds__(256) delta_heads_bwd_kernel(const Vec8* __rest
                                                               const float* __restrict__ rnorm, const Vec8* __restrict__ dq,
                                                               const Vec8* __restrict__ dk, const Vec8* __restrict__ dv,
                                                               Vec8* __restrict__ dx, int hk, int rep, int vvec) {
+    let_successor_start();
     const size_t t = blockIdx.x;
     const int nn = 2 * hk * kHeadVec, W = nn + vvec;
     Vec8* dst = dx + t * W;

@@ -64,6 +64,7 @@ __device__ __forceinline__ void store_row_bf16(uint8_t* dst, int v, const float*
 __global__ void __launch_bounds__(192, 1)
 gdn_bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmA, const GdnBwdParams p) {
+    let_successor_start();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sStage = smem;                          // [2][W | Qg | Kd | At]

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prologue_kernel(
     const float* __restrict__ beta, const int* __restrict__ chunk_tok0, const int* __restrict__ chunk_len,
     bf16* __restrict__ W, bf16* __restrict__ Qg, bf16* __restrict__ Kd, bf16* __restrict__ At, bf16* __restrict__ U,
     float* __restrict__ gamma, int H, int NC, float scale) {
+    let_successor_start();
     extern __shared__ __align__(16) uint8_t sm[];
     bf16* sK = reinterpret_cast<bf16*>(sm);
     bf16* sV = reinterpret_cast<bf16*>(sm + kTile);
@@ -313,6 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_prologue_bwd_kernel(
     const bf16* __restrict__ dO, const bf16* __restrict__ Vn, const bf16* __restrict__ dVn, const bf16* __restrict__ SprevT,
     const bf16* __restrict__ GT, bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv, float* __restrict__ dg,
     float* __restrict__ dbeta, int H, int NC, float scale) {
+    let_successor_start();
     extern __shared__ __align__(16) uint8_t sm[];
     auto tile = [&](int i) { return reinterpret_cast<bf16*>(sm + i * kTile); };
     bf16 *sK = tile(0), *sQ = tile(1), *sV = tile(2), *sDU = tile(3), *sDW = tile(4), *sDO = tile(5), *sVN = tile(6), *sS = tile(7), *sG = tile(9);
@@ -541,6 +543,7 @@ template <bool PACK>
 __global__ void __launch_bounds__(kThreads) gdn_layout_kernel(const bf16* __restrict__ src, bf16* __restrict__ dst,
                                                               const int* __restrict__ chunk_tok0, const int* __restrict__ chunk_len, int H,
                                                               int NC) {
+    let_successor_start();
     const int c = blockIdx.x, head = blockIdx.y, len = chunk_len[c];
     const size_t slab = ((size_t)head * NC + c) * C * D;
     const long long tok0 = chunk_tok0[c];

@@ -174,33 +174,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // a worker: this CTA, or the pair that it belongs to
     const int rank = PAIR ? (int)cluster_rank() : 0;
     const int worker = PAIR ? blockIdx.x / 2 : blockIdx.x, n_workers = PAIR ? gridDim.x / 2 : gridDim.x;
-    if (p.count != nullptr) {
-        const int n = max(0, __ldg(p.count) - p.count_base);
-        if (p.counts_depth) p.K = min(p.K, n);
-        else p.M = min(p.M, n);
-        if (p.ws != nullptr && !p.counts_depth) {
-            int* plan = reinterpret_cast<int*>(tmem_slot + 4);
-            if (threadIdx.x == 0) {
-                const TailPlan t = plan_tail(p.M, p.N, p.K, BN, TM, n_workers, 16, kMostRounds * n_workers);
-                plan[0] = t.full;
-                plan[1] = t.parts;
-                if (blockIdx.x == 0) {
-                    reinterpret_cast<int*>(p.ws)[0] = t.full;
-                    reinterpret_cast<int*>(p.ws)[1] = t.parts;
-                }
-            }
-            __syncthreads();
-            p.full = plan[0];
-            p.parts = plan[1];
-            p.ws += kPlanBytes / 4;
-        }
-    }
-    const int m_blocks = (p.M + TM - 1) / TM;
-    const int n_blocks = SWIGLU ? p.N / 128 : (p.N + BN - 1) / BN;
-    const int n_tiles = m_blocks * n_blocks;
-    const int k_blocks = (p.K + BK - 1) / BK;
-    const int n_items = item_count(p, n_tiles);
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
             mbar_init(&full[s], 1);
@@ -229,6 +202,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     if constexpr (PAIR) cluster_sync();          // the other CTA's barriers are there, too
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    wait_for_predecessor();
+    let_successor_start();
+
+    if (p.count != nullptr) {
+        const int n = max(0, *p.count - p.count_base);
+        if (p.counts_depth) p.K = min(p.K, n);
+        else p.M = min(p.M, n);
+        if (p.ws != nullptr && !p.counts_depth) {
+            int* plan = reinterpret_cast<int*>(tmem_slot + 4);
+            if (threadIdx.x == 0) {
+                const TailPlan t = plan_tail(p.M, p.N, p.K, BN, TM, n_workers, 16, kMostRounds * n_workers);
+                plan[0] = t.full;
+                plan[1] = t.parts;
+                if (blockIdx.x == 0) {
+                    reinterpret_cast<int*>(p.ws)[0] = t.full;
+                    reinterpret_cast<int*>(p.ws)[1] = t.parts;
+                }
+            }
+            __syncthreads();
+            p.full = plan[0];
+            p.parts = plan[1];
+            p.ws += kPlanBytes / 4;
+        }
+    }
+    const int m_blocks = (p.M + TM - 1) / TM;
+    const int n_blocks = SWIGLU ? p.N / 128 : (p.N + BN - 1) / BN;
+    const int n_tiles = m_blocks * n_blocks;
+    const int k_blocks = (p.K + BK - 1) / BK;
+    const int n_items = item_count(p, n_tiles);
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
@@ -587,13 +589,15 @@ inline int sm_count() {
 
 // C tile = bf16(sum over the parts of the workspace + bias); a thread makes 8 columns of a row
 template <int BN, int TM>
-__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ ws, bf16* __restrict__ C, const bf16* __restrict__ bias,
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* ws, bf16* C, const bf16* bias,
                                                         int M, int N, long long ldc, int full, int parts, int group_m,
-                                                        const int* __restrict__ count, int count_base) {
+                                                        const int* count, int count_base) {
+    wait_for_predecessor();
+    let_successor_start();
     const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM % (BN / 8), half = i / (BM * BN / 8), t = blockIdx.y;
     int mb, nb;                                                                                   // cg: group of 8 columns
     if (count != nullptr) {
-        M = min(M, max(0, __ldg(count) - count_base));
+        M = min(M, max(0, *count - count_base));
         full = reinterpret_cast<const int*>(ws)[0];
         parts = reinterpret_cast<const int*>(ws)[1];
         ws += kPlanBytes / 4;
@@ -685,13 +689,11 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
     p.count = rt.count;
     p.count_base = rt.count_base;
     p.counts_depth = rt.counts_depth;
-    r = launch_clusters(kern, PAIR ? 2 : 1, (items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1), kThreads, C::kSmem, st, tA, tB, tC, p);
+    r = launch_after(kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
     if (r) return r;
     const int may_split = dynamic_rows ? (ws ? workers - 1 : 0) : rem;       // tiles
     if (may_split)
-        sum_parts_kernel<BN, TM><<<dim3(TM * BN / 8 / 256, may_split), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full,
-                                                                                     plan.parts, p.group_m, dynamic_rows ? rt.count : nullptr,
-                                                                                     rt.count_base);
+        return launch_after(sum_parts_kernel<BN, TM>, 1, dim3(TM * BN / 8 / 256, may_split), 256, 0, st, ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full, plan.parts, p.group_m, dynamic_rows ? rt.count : nullptr, rt.count_base);
     return (int)cudaGetLastError();
 }
 
@@ -855,6 +857,7 @@ MM_API int mm_gemm_bf16_routed(const void* A, const void* B, const void* bias, i
 namespace {
 __global__ void fold_slots_kernel(const bf16* __restrict__ slots, bf16* __restrict__ out, long long rows, int cols,
                                   long long pitch, int world) {
+    let_successor_start();
     const int cv = cols >> 3;
     const long long total = rows * cv;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {

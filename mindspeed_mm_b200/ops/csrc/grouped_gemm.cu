@@ -80,6 +80,7 @@ template <int MODE, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, GGParams p) {
+    let_successor_start();
     constexpr int kBBytes = Cfg<BN>::kBBytes, kStageBytes = Cfg<BN>::kStageBytes, kStages = Cfg<BN>::kStages;
     constexpr int kTmemCols = Cfg<BN>::kTmemCols;
     extern __shared__ uint8_t smem_raw[];
@@ -330,6 +331,7 @@ namespace {
 // dst_row[i] for every (token, slot) pair i = t * k + s, in the aligned expert-major layout; pad rows get -1 source.
 __global__ void moe_permute_kernel(const bf16* __restrict__ x, const int* __restrict__ src_of_row, bf16* __restrict__ out,
                                    int R, int H) {
+    let_successor_start();
     const int hv = H >> 3;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)R * hv;
          i += (long long)gridDim.x * blockDim.x) {
@@ -347,6 +349,7 @@ __global__ void moe_permute_kernel(const bf16* __restrict__ x, const int* __rest
 // out[t, :] = sum_s probs[t, s] * y[row_of_pair[t * k + s], :]   (probs null: all ones)
 __global__ void moe_unpermute_kernel(const bf16* __restrict__ y, const int* __restrict__ row_of_pair,
                                      const bf16* __restrict__ probs, bf16* __restrict__ out, int T, int k, int H) {
+    let_successor_start();
     const int hv = H >> 3;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)T * hv;
          i += (long long)gridDim.x * blockDim.x) {
@@ -372,6 +375,7 @@ __global__ void __launch_bounds__(256) moe_unpermute_bwd_kernel(
     const bf16* __restrict__ g, const bf16* __restrict__ y, const int* __restrict__ row_of_pair,
     const int* __restrict__ src_of_row, const bf16* __restrict__ probs, bf16* __restrict__ dy, bf16* __restrict__ dprobs,
     int pairs, int k, int R, int H) {
+    let_successor_start();
     const int lane = threadIdx.x & 31, hv = H >> 3;
     const long long warps = (long long)gridDim.x * 8, total = (long long)pairs + (src_of_row ? R : 0);
     for (long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); i < total; i += warps) {
@@ -417,6 +421,7 @@ constexpr int kRoutePairs = 128;                 // of a warp
 template <int W>
 __global__ void __launch_bounds__(W * 32) moe_count_kernel(const long long* __restrict__ ids, int n, int E, int chunks, int* __restrict__ hist,
                                                            int* __restrict__ bad) {
+    let_successor_start();
     extern __shared__ int route_smem[];
     for (int e = threadIdx.x; e < E; e += W * 32) route_smem[e] = 0;
     __syncthreads();
@@ -453,6 +458,7 @@ __device__ __forceinline__ int block_scan(int v, int* sums, int& total) {
 
 // One block per expert: counts by chunk -> pairs in the chunks before; counts[e]: all of them
 __global__ void __launch_bounds__(256) moe_scan_kernel(int* __restrict__ hist, int chunks, int* __restrict__ counts) {
+    let_successor_start();
     __shared__ int sums[8];
     int* h = hist + (size_t)blockIdx.x * chunks;
     int base = 0;
@@ -471,6 +477,7 @@ template <int W>
 __global__ void __launch_bounds__(W * 32) moe_place_kernel(const long long* __restrict__ ids, int n, int k, int E, int chunks,
                                                            const int* __restrict__ hist, const int* __restrict__ counts, int R,
                                                            int* __restrict__ off, int* __restrict__ row_of_pair, int* __restrict__ src_of_row) {
+    let_successor_start();
     extern __shared__ int route_smem[];
     __shared__ int sums[W];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

@@ -23,6 +23,7 @@ template <bool GATED>
 __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y,
                                                                 const bf16* __restrict__ gate, bf16* __restrict__ out,
                                                                 float* __restrict__ partial, int rows, int cols, long long ldx) {
+    let_successor_start();
     __shared__ float tile[kWarps][kCols + 4];
     const int groups = (cols + kCols - 1) / kCols, b = blockIdx.x / groups, c0 = (blockIdx.x - b * groups) * kCols;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per_row = lanes_per_row(cols), sub = lane / per_row, at_once = 32 / per_row;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_sum_kernel(const bf16* __r
 // for each batch and column group, 431 and 153 in PyTorch.
 __global__ void __launch_bounds__(256) gated_short_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ y, const bf16* __restrict__ gate,
                                                           bf16* __restrict__ dy, bf16* __restrict__ dgate, int batches, int rows, int cols) {
+    let_successor_start();
     const int vecs = cols >> 3;
     const long long total = (long long)batches * vecs;
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
@@ -111,6 +113,7 @@ __global__ void __launch_bounds__(256) gated_short_kernel(const bf16* __restrict
 
 // sums[b][c] = sum over the splits, in their order
 __global__ void __launch_bounds__(256) fold_splits_kernel(const float* __restrict__ partial, bf16* __restrict__ sums, int splits, int cols) {
+    let_successor_start();
     __shared__ float tile[8][33];
     const int groups = (cols + 31) / 32, b = blockIdx.x / groups, c = (blockIdx.x - b * groups) * 32 + threadIdx.x;
     float s = 0.f;
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(256) fold_splits_kernel(const float* __restric
 
 // x *= *scale in place; nothing is read when the scale is one
 __global__ void __launch_bounds__(256) scale_kernel(bf16* __restrict__ x, long long n, const float* __restrict__ scale) {
+    let_successor_start();
     const float s = *scale;
     if (s == 1.f) return;
     const long long stride = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kBlock) rownorm_fwd_kernel(const bf16* __restr
                                                             const bf16* __restrict__ b, bf16* __restrict__ y,
                                                             float* __restrict__ s0, float* __restrict__ s1,
                                                             long long rows, int S, int H, float eps) {
+    let_successor_start();
     constexpr int kRowsPerBlock = kBlock / G;
     const int nvec = H >> 3;
     const int gl = threadIdx.x % G;                     // lane inside the group
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(kBlock) gated_rms_fwd_kernel(const void* __res
                                                               const bf16* __restrict__ w, bf16* __restrict__ y,
                                                               float* __restrict__ rstd_out, long long rows, int H, int zh, long long ldz,
                                                               float eps) {
+    let_successor_start();
     constexpr int kRowsPerBlock = kBlock / G;
     const int nvec = H >> 3;
     const int gl = threadIdx.x % G;
@@ -213,6 +215,7 @@ __global__ void __launch_bounds__(kBlock) gated_rms_bwd_kernel(const void* __res
                                                               const float* __restrict__ rstd_in, void* __restrict__ dx,
                                                               bf16* __restrict__ dz, float* __restrict__ dw, long long rows,
                                                               int H, int zh, long long ldz) {
+    let_successor_start();
     constexpr int kRowsPerBlock = kBlock / G;
     __shared__ float sdw[256];
     const int nvec = H >> 3;

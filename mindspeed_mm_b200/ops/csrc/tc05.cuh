@@ -495,7 +495,7 @@ inline int make_tmap_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t 
                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     });
 }
-// ---- launch of kernels that run on pairs of CTAs, or split their registers between warpgroups
+// ---- kernels that split their registers between warpgroups
 // `regs`: what the warpgroups of a block claim by setmaxnreg, in all.  A claim above the launch's own would wait for good, so such a build
 // is refused here.
 template <class K>
@@ -505,24 +505,5 @@ inline int opt_in(K kern, int smem, int threads, int regs) {
     if (e != cudaSuccess) return (int)e;
     if (a.numRegs * threads < regs) return -101;
     return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-}
-template <class K, class... Args>
-inline int launch_clusters(K kern, int cluster, int blocks, int threads, int smem, cudaStream_t st, const Args&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = cluster;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = cluster > 1 ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, kern, args...);
-}
-template <class K, class... Args>
-inline int launch_pairs(K kern, int pairs, int threads, int smem, cudaStream_t st, const Args&... args) {
-    return launch_clusters(kern, 2, 2 * pairs, threads, smem, st, args...);
 }
 }  // namespace tc05
