@@ -20,7 +20,7 @@
 //
 // What bounds a large product is the power cap: every tile size keeps the tensor pipe 90 to 96 % busy, at a clock that the energy of its
 // operand traffic sets.  A step of 64 of K brings a CTA 48 KB for 128 x 256 (one CTA), 32 KB for the same as half of a 256-row pair, and
-// 48 KB for 256 x 256 as half of a 512-row pair: 19.1 / 15.0 GB through L2 for 8192 x 37888 x 3584 with 256 / 512 rows.  Sustained, TFLOP/s, tiles
+// 48 KB for 256 x 256 as half of a 512-row pair: 19.1 / 14.5 GB through L2 for 8192 x 37888 x 3584 with 256 / 512 rows.  Sustained, TFLOP/s, tiles
 // of 128 / 256 / 512 rows (cuBLAS): 8192 x 37888 x 3584 1202 / 1432 / 1430 (1416), 8192 x 3584 x 18944 1209 / 1291 / 1399 (1238), 32760 x 5120 x
 // 13824 1188 / 1274 / 1388 (1401), 8192 x 3840 x 1280 1104 / 1157 / 1107 (1130).  Groups of 4096 rows against 1024 / 2048 / 8192: 1432 against
 // 1292 / 1350 (256 rows), 1430 against 1421 / 1381 at 2048 / 8192 (512 rows, 8192 x 37888 x 3584); single tiles are used for few rows only.
@@ -73,7 +73,7 @@ struct Params {
     // the whole row can then be applied after the columns have been scattered to other GPUs)
     float* stats = nullptr;
     int n_slots = 1, per_slot = 0;
-    // split tail (see split_plan): tiles from `full` on are cut along K into `parts` items whose fp32 sums go to `ws`
+    // split tail (see plan_tail): tiles from `full` on are cut along K into `parts` items whose fp32 sums go to `ws`
     int full = 0, parts = 1;
     float* ws = nullptr;
     // M (or, with `counts_depth`, K) is what `count` on the device says, less `count_base` and at most what is given here; the tail is then
