@@ -144,9 +144,9 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint64_t* s_empty = v_full + 6;           // [2]
     uint64_t* dp_full = v_full + 8;
     uint64_t* dp_empty = v_full + 9;
-    uint64_t* ds_full = v_full + 10;
-    uint64_t* dq_full = v_full + 11;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_full + 12);
+    uint64_t* ds_full = v_full + 10;          // [2]  by tile: a warp may be done with tile j + 1 while another still works on tile j
+    uint64_t* dq_full = v_full + 12;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_full + 13);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -174,10 +174,10 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             mbar_init(&v_empty[i], 1);
             mbar_init(&s_full[i], 1);
             mbar_init(&s_empty[i], 8);                // one arrival per warp
+            mbar_init(&ds_full[i], 8);
         }
         mbar_init(dp_full, 1);
         mbar_init(dp_empty, 8);
-        mbar_init(ds_full, 8);
         mbar_init(dq_full, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -264,7 +264,7 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 // buffer is free as soon as the threads have pulled dP(j) into registers
                 if (j + 1 < n_kv && !(ok = issue_s(j + 1) && issue_dp(j + 1))) break;
                 // dQ += dS_j K_j
-                if (!mbar_wait(ds_full, j & 1, abort_flag)) { ok = false; break; }
+                if (!mbar_wait(&ds_full[st], (j >> 1) & 1, abort_flag)) { ok = false; break; }
                 fence_after_sync();
                 const int ks = j % kRingK;
                 const uint32_t ka = smem_u32(sK + ks * kTile);
@@ -342,7 +342,7 @@ fmha_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tmem_wait_st();
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ds_full);
+            if (lane == 0) mbar_arrive(&ds_full[st]);
         }
         bf16* dst = p.dq + ((size_t)(q_begin + qi) * p.Nq + head) * p.D + half * 64;
         if (ok && n_kv > 0) ok = __all_sync(0xffffffffu, mbar_wait(dq_full, 0, abort_flag));

@@ -421,6 +421,22 @@ def test_interleaved_rotation(T, N, D):
     _close(torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(yr, xr, dy.float())[0], rtol=4e-3, atol=1e-3)
 
 
+@pytest.mark.parametrize("lens,D", [([512] * 16, 80), ([1564, 1276, 2048], 80), ([512] * 16, 128)])
+def test_attention_backward_many_times_over(lens, D):
+    """Back to back, so that a CTA's warps fall out of step now and then: the same gradients to the bit, and no wait that gives up."""
+    torch.manual_seed(D)
+    T, N = sum(lens), 16
+    q, k, v, do = (torch.randn(T, N, D, device=DEV).bfloat16() for _ in range(4))
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    o, lse = native.fmha_forward(q, k, v, cu, cu, False, D ** -0.5)
+    want = [t.clone() for t in native.fmha_backward(do, q, k, v, o, lse, cu, cu, False, D ** -0.5)]
+    for _ in range(40):
+        for _ in range(30):
+            got = native.fmha_backward(do, q, k, v, o, lse, cu, cu, False, D ** -0.5)
+        native.check_status()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("T,H,V,valid,chunk", [(512, 256, 512, 100, 8192), (513, 256, 512, 0, 8192), (513, 264, 520, 513, 8192), (600, 256, 1000, 1, 8192),
                                                (700, 512, 4096, 64, 8192), (700, 512, 4096, 65, 256), (8300, 256, 512, 5000, 8192),
                                                (8300, 256, 512, 130, 4096), (1600, 3584, 18944, 1421, 8192)])
