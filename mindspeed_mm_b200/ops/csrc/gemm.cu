@@ -40,7 +40,11 @@ constexpr int kSmemBudget = 227 * 1024;
 
 // TM: rows of a tile.  128: one CTA;  256 and 512: a pair of CTAs on two SMs, each with half of the rows and, for the operands, half of the
 // columns (cta_group::2).
-template <int BN, int TM>
+// SHALLOW (depth up to kStaged): the stores take longer than the products, so each epilogue group has two staging slabs, for one operand
+// stage less: one store is under way while the next slab is written.  The gradient of a vocabulary's weight (152064 x 3584) over 256 rows,
+// behind the products that make its operand: 377 us with one slab a group, 336 with two; 310 rows 381, 372; 350 rows 408, 423: from there on
+// the fourth stage is worth more.
+template <int BN, int TM, bool SHALLOW = false>
 struct Cfg {
     static constexpr bool kPair = TM > BM;
     static constexpr int kHalves = TM == 512 ? 2 : 1;    // accumulators of 128 rows that a tile has in a CTA's tensor memory
@@ -48,7 +52,8 @@ struct Cfg {
     static constexpr int kABytes = kHalves * BM * BK * 2;
     static constexpr int kBBytes = kBRows * BK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kCBytes = 2 * BM * 64 * 2;  // two 128x64 bf16 staging slabs
+    static constexpr int kSlabBufs = SHALLOW ? 2 : 1;
+    static constexpr int kCBytes = 2 * kSlabBufs * BM * 64 * 2;  // 128x64 bf16 staging slabs of both epilogue groups
     static constexpr int kAux = 1024;                // barriers etc.
     static constexpr int kStages = (kSmemBudget - kCBytes - kAux - 1024) / kStageBytes;
     static constexpr int kSmem = kStages * kStageBytes + kCBytes + kAux + 1024;
@@ -150,11 +155,11 @@ __host__ __device__ inline TailPlan plan_tail(int M, int N, int K, int BN, int r
 // SWIGLU (BN = 256, K-major operands, no bias): B is the fused [2F, K] gate/up weight, p.N = F.  A tile's accumulator holds
 // 128 gate columns (weight rows nb*128 ..) next to the 128 up columns of the same features (rows F + nb*128 ..); the
 // epilogue writes silu(gate) * up, so the [M, 2F] pre-activation never reaches memory.
-template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false, int TM = BM>
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false, int TM = BM, bool SHALLOW = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ TMapSet tmC, Params p) {
-    using C = Cfg<BN, TM>;
+    using C = Cfg<BN, TM, SHALLOW>;
     constexpr bool PAIR = C::kPair;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -397,7 +402,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int row = q * 32 + lane;     // row inside the 128-row tile
         const int group = (warp >> 2) - 1;
         const bool issuer = threadIdx.x % kGroupThreads == 0;
-        uint8_t* buf = sC + group * (BM * 128);
+        uint8_t* bufs = sC + group * C::kSlabBufs * (BM * 128);
         auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
         auto drained = [&] {
             fence_before_sync();
@@ -511,7 +516,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
             for (int slab = 0; slab < kSlabs; ++slab) {
                 const int n0 = (SWIGLU ? nb * 128 : nb * BN) + slab * 64;
-                if (issuer) tma_wait_read<0>();      // the store that last read this buffer has drained
+                uint8_t* buf = bufs + slab % C::kSlabBufs * (BM * 128);
+                if (issuer) tma_wait_read<C::kSlabBufs - 1>();      // the store that last read this buffer has drained
                 group_sync();
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
@@ -556,11 +562,16 @@ struct Plan {
     int full, parts;       // tiles that are one item each; items that each of the others is cut into
 };
 
+// Depth up to which tiles are one CTA's: the accumulators are emptied and written as long as the next tile's products take, or longer, and
+// a CTA of a pair waits for both of its halves.  152064 x 3584, 128 / 256 / 512 rows: depth 256 299 / 339 / 342 us, 384 388 / 400 / 411,
+// 448 429 / 394 / 445; 8192 x 8192: 256 47 / 55 / 55, 384 53 / 57 / 61, 448 59 / 59 / 65; 3584 x 3584: 64 17 / 21 / 24, 384 21.5 / 23.5 / 27.
+constexpr int kShallow = 6 * BK, kStaged = 5 * BK;
+
 // The tile size, of those that M fills more than half of, with the shortest estimate.
 inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool may_split) {
     Plan best{BM, 0, 1};
     float least = 1e30f;
-    for (int rows = BM; rows == BM || (may_pair && rows <= 4 * BM && M > rows / 2); rows *= 2) {
+    for (int rows = BM; rows == BM || (may_pair && K > kShallow && rows <= 4 * BM && M > rows / 2); rows *= 2) {
         const TailPlan t = plan_tail(M, N, K, BN, rows, rows > BM ? sms / 2 : sms, may_split ? 16 : 1, 1 << 30);
         if (t.time < least) {
             least = t.time;
@@ -636,10 +647,10 @@ struct Route {
     bool counts_depth = false;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool SWIGLU, int TM>
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU, int TM, bool SHALLOW = false>
 int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
                  long long ldc, int* status, cudaStream_t st, const Route& rt, const Plan& plan, float* ws) {
-    using C = Cfg<BN, TM>;
+    using C = Cfg<BN, TM, SHALLOW>;
     constexpr bool PAIR = C::kPair;
     CUtensorMap tA, tB;
     TMapSet tC;
@@ -669,7 +680,7 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
             if (r) return 3000 + r;
         }
     }
-    auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU, TM>;
+    auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU, TM, SHALLOW>;
     static bool done = false;
     if (!done) {
         r = opt_in(kern, C::kSmem, kThreads, (kIssueRegs + 2 * kEpiRegs) * 128);
@@ -708,6 +719,8 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
         if (plan.rows == 512) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 512>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
         if (plan.rows == 256) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 256>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
     }
+    if constexpr (BN == 256 && !SWIGLU)
+        if (K <= kStaged) return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
     return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
 }
 

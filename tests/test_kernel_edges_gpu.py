@@ -361,12 +361,13 @@ def test_products_with_a_split_tail(layout, M, N, K, splits):
 
 
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
-@pytest.mark.parametrize("M,N,K,rows", [(128, 256, 64, 128), (136, 264, 8, 256), (256, 1000, 72, 256), (264, 256, 200, 256), (384, 4096, 704, None),
+@pytest.mark.parametrize("M,N,K,rows", [(128, 256, 64, 128), (136, 264, 8, 128), (256, 1000, 72, 128), (264, 9480, 320, 128), (4600, 3848, 328, 128),
+                                        (264, 256, 384, 128), (264, 256, 392, 256), (384, 4096, 704, None),
                                         (520, 9480, 4104, None), (1000, 9472, 2056, 512), (4600, 3840, 4104, 512), (4096, 4864, 2568, 512),
                                         (2560, 3840, 18944, 512)])
 def test_products_on_pairs_of_sms(layout, M, N, K, rows):
     """Tiles of one SM and of a pair, 256 and 512 rows: few rows, ragged rows, columns and depths, a main loop of fewer steps than the ring
-    has slots, several tiles a pair, whole and cut along K."""
+    has slots, several tiles a pair, whole and cut along K; shallow products, which stay on one SM, at the ends of their staging's range."""
     torch.manual_seed(M + K)
     a = torch.randn((K, M) if layout == "tn" else (M, K), device=DEV).bfloat16()
     b = torch.randn((N, K) if layout == "nt" else (K, N), device=DEV).bfloat16()
