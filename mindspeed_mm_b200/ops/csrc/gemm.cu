@@ -560,7 +560,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 struct Plan {
     int rows;              // of a tile
     int full, parts;       // tiles that are one item each; items that each of the others is cut into
+    float time;            // estimated, us
 };
+
+// A product that takes longer (us) starts when the kernel in front has ended: CTAs that come up one by one on SMs as these fall idle lose more
+// over its time than the gap that they save.  The three products of the vocabulary loss, behind one another, early / not: 256 rows
+// 840 / 825 us, 310 rows 1061 / 1034, 400 rows 1280 / 1187.
+constexpr float kLong = 100.f;
 
 // Depth up to which tiles are one CTA's: the accumulators are emptied and written as long as the next tile's products take, or longer, and
 // a CTA of a pair waits for both of its halves.  152064 x 3584, 128 / 256 / 512 rows: depth 256 299 / 339 / 342 us, 384 388 / 400 / 411,
@@ -569,13 +575,13 @@ constexpr int kShallow = 6 * BK, kStaged = 5 * BK;
 
 // The tile size, of those that M fills more than half of, with the shortest estimate.
 inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool may_split) {
-    Plan best{BM, 0, 1};
+    Plan best{BM, 0, 1, 0.f};
     float least = 1e30f;
     for (int rows = BM; rows == BM || (may_pair && K > kShallow && rows <= 4 * BM && M > rows / 2); rows *= 2) {
         const TailPlan t = plan_tail(M, N, K, BN, rows, rows > BM ? sms / 2 : sms, may_split ? 16 : 1, 1 << 30);
         if (t.time < least) {
             least = t.time;
-            best = {rows, t.full, t.parts};
+            best = {rows, t.full, t.parts, t.time};
         }
     }
     return best;
@@ -700,7 +706,7 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
     p.count = rt.count;
     p.count_base = rt.count_base;
     p.counts_depth = rt.counts_depth;
-    r = launch_after(kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
+    r = launch_after_if(plan.time < kLong, kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
     if (r) return r;
     const int may_split = dynamic_rows ? (ws ? workers - 1 : 0) : rem;       // tiles
     if (may_split)
