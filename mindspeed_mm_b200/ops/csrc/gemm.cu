@@ -61,11 +61,118 @@ struct Cfg {
     static constexpr int kTmemCols = 2 * BN;
 };
 
+// ---- which parts of a product are cut along K
+// The unit is a block of `rows` x BN outputs, counted in groups of `group` row blocks, column by column.  Blocks from `full` on are summed as
+// `parts` stretches of K each, all others in one go: this alone decides the order of an output's fp32 sum, and with it its bits, whatever
+// the tiles are that the work is done in.
+struct Cut {
+    int full = 0, parts = 1;
+    int rows = BM, group = 1024 / BM;
+};
+
+__host__ __device__ inline void tile_coords(int tile, int m_blocks, int n_blocks, int group_m, int& mb, int& nb) {
+    const int per_group = group_m * n_blocks;
+    const int g = tile / per_group;
+    const int first_m = g * group_m;
+    const int gm = group_m < m_blocks - first_m ? group_m : m_blocks - first_m;
+    const int r = tile - g * per_group;
+    mb = first_m + r % gm;
+    nb = r / gm;
+}
+__host__ __device__ inline int tile_index(int mb, int nb, int m_blocks, int n_blocks, int group_m) {
+    const int first_m = mb / group_m * group_m, gm = group_m < m_blocks - first_m ? group_m : m_blocks - first_m;
+    return first_m * n_blocks + nb * gm + mb - first_m;
+}
+
+// ---- a CTA's (or pair's) list of work
+// Tiles of TM rows.  First those that hold an uncut block, each over the whole of K, in groups of `group` row blocks; then, for each of the
+// `parts`, those that hold a cut one, in the cut's own order.  A tile with blocks of both kinds is in both lists, and each time only the
+// blocks that it is there for are stored.  The uncut blocks are all rows in front of the cut's first group, and that group's columns up to
+// where the cut begins: the last group of row blocks is lower from there on.
+struct TileList {
+    int n_blocks, k_blocks;                  // of tiles
+    int group, last, high, low, from;        // the last group starts at row block `last`; it has `high` row blocks up to column `from` and `low` behind
+    int head, tail, tail_group;              // row blocks in front of the cut's first group, row blocks from it on, and of a group of them
+    int whole, first, cut, parts;            // tiles in one go; first one with a cut block (of the tail's), and how many have one
+    int halves;                              // of the tiles in one go, the last ones that are two items of half their rows each (tiles of 512 rows)
+};
+// One entry of the list.
+struct Item {
+    int mb, nb;                              // tile
+    int kb0, kb1;
+    int part;                                // of K, or -1: in one go
+    int half;                                // of the rows, or -1: all
+};
+
+__host__ __device__ inline TileList make_list(int M, int N, int K, int TM, int BN, const Cut& c, int halves) {
+    TileList l;
+    const int m_blocks = (M + TM - 1) / TM;
+    l.n_blocks = l.from = (N + BN - 1) / BN;
+    l.k_blocks = (K + BK - 1) / BK;
+    l.group = (TM == BM ? 1024 : 4096) / TM;
+    l.head = m_blocks;
+    l.first = l.cut = l.tail = 0;
+    l.tail_group = c.group * c.rows / TM;
+    l.parts = c.parts;
+    l.halves = halves;
+    int row = 0, uncut = m_blocks;                                // row: where the cut begins in its first group, in units of the cut
+    if (c.parts > 1) {
+        tile_coords(c.full, (M + c.rows - 1) / c.rows, l.n_blocks, c.group, row, l.from);
+        l.head = row / c.group * c.group * c.rows / TM;
+        row %= c.group;
+        l.tail = m_blocks - l.head;
+        const int high = l.tail < l.tail_group ? l.tail : l.tail_group;
+        l.first = l.from * high + row * c.rows / TM;
+        l.cut = l.tail * l.n_blocks - l.first;
+        uncut = l.head + high;
+    }
+    l.last = uncut > 0 ? (uncut - 1) / l.group * l.group : 0;
+    l.high = uncut - l.last;
+    l.low = l.head - l.last;
+    l.whole = l.last * l.n_blocks + l.from * l.high + (l.n_blocks - l.from) * l.low + (row * c.rows + TM - 1) / TM;
+    return l;
+}
+__host__ __device__ inline int item_count(const TileList& l) { return l.whole + l.halves + l.cut * l.parts; }
+
+__host__ __device__ inline Item item_at(const TileList& l, int i) {
+    Item it{0, 0, 0, l.k_blocks, -1, -1};
+    if (i >= l.whole + l.halves) {
+        // neighbours in the list are neighbouring tiles over the same part of K, so that they share operand tiles in L2
+        const int j = i - l.whole;
+        it.part = j / l.cut;
+        it.kb0 = it.part * l.k_blocks / l.parts;
+        it.kb1 = (it.part + 1) * l.k_blocks / l.parts;
+        tile_coords(l.first + j - it.part * l.cut, l.tail, l.n_blocks, l.tail_group, it.mb, it.nb);
+        it.mb += l.head;
+        return it;
+    }
+    if (i >= l.whole - l.halves && l.halves) {
+        it.half = i >= l.whole;
+        i -= it.half * l.halves;
+    }
+    if (i < l.last * l.n_blocks) {
+        tile_coords(i, l.last, l.n_blocks, l.group, it.mb, it.nb);
+        return it;
+    }
+    i -= l.last * l.n_blocks;
+    if (i < l.from * l.high) {
+        it.nb = i / l.high;
+        it.mb = l.last + i - it.nb * l.high;
+    } else if ((i -= l.from * l.high) < (l.n_blocks - l.from) * l.low) {
+        it.nb = i / l.low;
+        it.mb = l.last + i - it.nb * l.low;
+        it.nb += l.from;
+    } else {
+        it.nb = l.from;
+        it.mb = l.head + i - (l.n_blocks - l.from) * l.low;
+    }
+    return it;
+}
+
 struct Params {
     int M, N, K;
     const bf16* bias;
     int* status;
-    int group_m;
     // output routing (fused all-to-all / reduce-scatter push): where a 128 x 64 output slab goes
     //   mode 0: C[m, n] of this GPU
     //   mode 1: column blocks of width `blk` are dealt round-robin to `world` destinations (Ulysses head scatter):
@@ -78,9 +185,10 @@ struct Params {
     // the whole row can then be applied after the columns have been scattered to other GPUs)
     float* stats = nullptr;
     int n_slots = 1, per_slot = 0;
-    // split tail (see plan_tail): tiles from `full` on are cut along K into `parts` items whose fp32 sums go to `ws`
-    int full = 0, parts = 1;
+    // split tail (see Cut): fp32 sums of the parts go to `ws`
+    Cut cut;
     float* ws = nullptr;
+    TileList list;                 // (made by the host unless the device counts: the index arithmetic takes 1 - 2 us, longer than a launch is worth)
     // M (or, with `counts_depth`, K) is what `count` on the device says, less `count_base` and at most what is given here; the tail is then
     // planned by the kernel, which leaves {full, parts} in front of the workspace
     const int* count = nullptr;
@@ -90,48 +198,53 @@ struct Params {
 constexpr int kPlanBytes = 256;        // in front of the sums in the workspace of such a product
 constexpr int kMostRounds = 8;         // of its split items, which the workspace (310 MB for tiles of 512 rows) is made for
 
-// One entry of a CTA's list: a tile and the part of K that it covers.
-struct Item {
-    int tile, kb0, kb1, slot;      // slot: tile-sized block of `ws`, or -1: the whole tile, stored as output
-};
-
-__device__ __forceinline__ int item_count(const Params& p, int n_tiles) { return p.ws ? p.full + (n_tiles - p.full) * p.parts : n_tiles; }
-
-__device__ __forceinline__ Item item_at(const Params& p, int i, int n_tiles, int k_blocks) {
-    if (!p.ws || i < p.full) return {i, 0, k_blocks, -1};
-    // neighbours in the list are neighbouring tiles over the same part of K, so that they share operand tiles in L2
-    const int rem = n_tiles - p.full, t = (i - p.full) % rem, part = (i - p.full) / rem;
-    return {p.full + t, part * k_blocks / p.parts, (part + 1) * k_blocks / p.parts, t * p.parts + part};
-}
-
 constexpr int kMaxDst = 8;
 struct TMapSet {
     CUtensorMap m[kMaxDst];
 };
 
-__device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks, int group_m, int& mb, int& nb) {
-    const int per_group = group_m * n_blocks;
-    const int g = tile / per_group;
-    const int first_m = g * group_m;
-    const int gm = min(group_m, m_blocks - first_m);
-    const int r = tile - g * per_group;
-    mb = first_m + r % gm;
-    nb = r / gm;
-}
-
 // ---- split tail ----
 // 168 tiles on 148 SMs take two rounds, the second one with 20 CTAs at work.  The tiles behind the last whole round are therefore cut
 // along K into `parts` items each, so that ceil(rem * parts / workers) rounds of a 1 / parts tile follow; the items leave fp32 sums in a
 // workspace and a second kernel adds them in their order, adds the bias and rounds, exactly once, to bf16.  No worker waits for another.
-// Time of a product on tiles of `rows` rows, in us, and the number of parts that makes it shortest; tiles stay whole for a gain under 4 us.  A 64-deep step of
-// a tile of 256 columns takes 0.45 / 0.415 / 0.79 us with 128 / 256 / 512 rows (rates of a burst; an SM, or a pair of them, works on it), a
-// 512-row tile has 1 us more for filling its ring anew, and no product is over before its operands have come once at 6.2 TB/s: a single
-// row of tiles over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about
-// 4 TB/s, a further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
+//
+// What is cut, and into how many parts, is what makes a product of 128-row tiles shortest on as many CTAs as there are SMs, 1 part if the gain
+// is under 4 us.  It holds for tiles of every size: another order of the fp32 sums is as exact, but its bits are others, and the layers of
+// a model carry them on (16 layers: 1.6 % of a prompt's logits).  A 64-deep step of a 128 x 256 tile takes
+// 0.44 us (1.4 PFLOP/s over 148 SMs), and no product is over before its operands have come once at 6.2 TB/s: a single row of tiles
+// over a large weight is bound by that, and cutting it only adds traffic.  An item's sums are written and read once at about 4 TB/s, a
+// further launch and the shorter main loops cost 6 us (fitted to the figures: at 3 us and 5 TB/s 7800 x 1536 x 4608 was split and
 // lost 2 us).
 // Measured, 128 x 256 tiles, L2 flushed, whole / split: 1421 x 3584 x 18944 (168 tiles) 218 / 151 us, 405 x 3584 x 37888 (56) 216 / 122,
-// 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands: 85 x 25368 x 27344 247 / 279, 126 x 26744 x
-// 24168 251 / 271.
+// 8192 x 3584 x 18944 (896) 828 / 776, 3840 x 1280 x 8192 (150) 132 / 91, 1421 x 3584 x 3584 50 / 46.  Left whole for its operands:
+// 85 x 25368 x 27344 247 / 279, 126 x 26744 x 24168 251 / 271.
+inline Cut split_plan(int M, int N, int K, int BN, int sms) {
+    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), kb = (K + BK - 1) / BK, full = tiles / sms, rem = tiles % sms;
+    Cut best;
+    best.full = tiles;
+    if (!rem) return best;
+    const double unit = kb * 0.44 * BN / 256, operands = 2.0 * K * ((double)M + N) / 6.2e6;
+    auto at_least = [&](double t) { return t > operands ? t : operands; };
+    double least = at_least(unit * (full + 1)) - 4.0;
+    for (int parts = 2; parts <= 16 && kb / parts >= 4; ++parts) {
+        const int rounds = (rem * parts + sms - 1) / sms;
+        const double t = at_least(unit * full + unit * rounds / parts) + 6.0 + rem * parts * (BM * BN * 8e-6 / 4.0);
+        if (t < least) {
+            least = t;
+            best.full = tiles - rem;
+            best.parts = parts;
+        }
+    }
+    return best;
+}
+
+// Time of a 64-deep step of a tile of 256 columns with 128 / 256 / 512 rows, in us: 0.45 / 0.415 / 0.79 (rates of a burst; an SM, or a pair of
+// them, works on it); a 512-row tile has 1 us more for filling its ring anew, and so have its halves, which run at the rate of 256 rows.
+__host__ __device__ inline float tile_time(int kb, int rows, int BN) {
+    return (rows == BM ? kb * 0.45f : rows == 2 * BM ? kb * 0.415f : kb * 0.79f + 1.f) * BN / 256;
+}
+
+// Cut and time of a product whose number of rows only the device knows: the tiles themselves are the units, and their own times decide.
 struct TailPlan {
     float time;
     int full, parts;
@@ -141,7 +254,7 @@ __host__ __device__ inline TailPlan plan_tail(int M, int N, int K, int BN, int r
     const float operands = 2.f * K * ((float)M + N) / 6.2e6f;
     auto at_least = [&](float t) { return t > operands ? t : operands; };
     const int tiles = ((M + rows - 1) / rows) * ((N + BN - 1) / BN), full = tiles / workers, rem = tiles % workers;
-    const float unit = (rows == BM ? kb * 0.45f : rows == 2 * BM ? kb * 0.415f : kb * 0.79f + 1.f) * BN / 256;
+    const float unit = tile_time(kb, rows, BN);
     const float whole = at_least(unit * (full + (rem ? 1 : 0)));
     TailPlan best{whole, tiles, 1};
     for (int parts = 2; rem && parts <= most_parts && kb / parts >= 4 && rem * parts <= most_items; ++parts) {
@@ -155,7 +268,8 @@ __host__ __device__ inline TailPlan plan_tail(int M, int N, int K, int BN, int r
 // SWIGLU (BN = 256, K-major operands, no bias): B is the fused [2F, K] gate/up weight, p.N = F.  A tile's accumulator holds
 // 128 gate columns (weight rows nb*128 ..) next to the 128 up columns of the same features (rows F + nb*128 ..); the
 // epilogue writes silu(gate) * up, so the [M, 2F] pre-activation never reaches memory.
-template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false, int TM = BM, bool SHALLOW = false>
+// COUNTED: M, or the depth, is what Params::count says.
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false, int TM = BM, bool SHALLOW = false, bool COUNTED = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ TMapSet tmC, Params p) {
@@ -210,7 +324,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     wait_for_predecessor();
     let_successor_start();
 
-    if (p.count != nullptr) {
+    TileList counted;
+    if constexpr (COUNTED) {
         const int n = max(0, *p.count - p.count_base);
         if (p.counts_depth) p.K = min(p.K, n);
         else p.M = min(p.M, n);
@@ -226,16 +341,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 }
             }
             __syncthreads();
-            p.full = plan[0];
-            p.parts = plan[1];
+            p.cut.full = plan[0];
+            p.cut.parts = plan[1];
             p.ws += kPlanBytes / 4;
         }
+        counted = make_list(p.M, p.N, p.K, TM, BN, p.cut, 0);
     }
-    const int m_blocks = (p.M + TM - 1) / TM;
-    const int n_blocks = SWIGLU ? p.N / 128 : (p.N + BN - 1) / BN;
-    const int n_tiles = m_blocks * n_blocks;
-    const int k_blocks = (p.K + BK - 1) / BK;
-    const int n_items = item_count(p, n_tiles);
+    const TileList& list = COUNTED ? counted : p.list;
+    const int n_items = item_count(list);
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
@@ -246,9 +359,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             uint32_t phase = 0;
             bool ok = true;
             for (int i = worker; i < n_items && ok; i += n_workers) {
-                const Item item = item_at(p, i, n_tiles, k_blocks);
-                int mb, nb;
-                tile_coords(item.tile, m_blocks, n_blocks, p.group_m, mb, nb);
+                const Item item = item_at(list, i);
+                const int mb = item.mb, nb = item.nb;
                 for (int kb = item.kb0; kb < item.kb1; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
                         atomicExch(p.status, MM_TIMEOUT_TMA);
@@ -303,7 +415,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             constexpr uint32_t idesc = idesc_bf16(PAIR ? 2 * BM : BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
             int stage = 0;
             uint32_t phase = 0;
-            int it = 0;
+            int used0 = 0, used1 = 0;               // items that each accumulator has had
             bool ok = true;
             auto step = [](int& s, uint32_t& ph) {
                 if (++s == C::kStages) {
@@ -317,7 +429,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 return ok = false;
             };
             auto drained = [&](int acc) {
-                const uint32_t parity = ((it * C::kHalves / 2) & 1) ^ 1;
+                const uint32_t parity = ((acc ? used1 : used0) & 1) ^ 1;
+                ++(acc ? used1 : used0);
                 if (PAIR ? mbar_wait_cluster(&tempty[acc], parity, abort_flag) : mbar_wait(&tempty[acc], parity, abort_flag)) {
                     fence_after_sync();
                     return true;
@@ -347,17 +460,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     else mma_ss(tmem_base + acc * BN, da, db, idesc, accum);
                 }
             };
+            int it = 0;
             for (int i = worker; i < n_items && ok; i += n_workers, ++it) {
-                const Item item = item_at(p, i, n_tiles, k_blocks);
-                if constexpr (C::kHalves == 1) {
-                    const int acc = it & 1;
-                    if (!drained(acc)) break;
+                const Item item = item_at(list, i);
+                auto alone = [&](int h, int acc) {           // an item with one accumulator
+                    if (!drained(acc)) return;
                     for (int kb = item.kb0; kb < item.kb1 && arrived(stage, phase); ++kb) {
-                        products(stage, 0, acc, kb == item.kb0);
+                        products(stage, h, acc, kb == item.kb0);
                         done(&empty[stage]);        // slot reusable once these MMAs have read it
                         step(stage, phase);
                     }
                     if (ok) done(&tfull[acc]);
+                };
+                if constexpr (C::kHalves == 1) {
+                    alone(0, it & 1);
+                } else if (item.half >= 0) {
+                    alone(item.half, item.half);
                 } else {
                     // Tensor memory holds one tile, so its first accumulator runs ahead of the second at both ends, by up to kAhead
                     // slots: it is complete, and drained, while the second one's last products run, and the next tile starts on it
@@ -418,18 +536,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         int it = 0, use = 0;
         for (int i = worker; i < n_items; i += n_workers, ++it) {
             if (C::kHalves == 1 && (it & 1) != group) continue;
-            const Item item = item_at(p, i, n_tiles, k_blocks);
-            int mb, nb;
-            tile_coords(item.tile, m_blocks, n_blocks, p.group_m, mb, nb);
+            const Item item = item_at(list, i);
+            if (C::kHalves == 2 && item.half >= 0 && item.half != group) continue;
+            const int mb = item.mb, nb = item.nb;
             const int h = C::kHalves == 1 ? 0 : group, m0 = mb * TM + rank * (TM / 2) + h * BM;
+            bool mine = m0 < p.M;                         // these 128 rows are what the item is there for
+            size_t slot = 0;                              // of the workspace, in blocks of 128 rows
+            if (!SWIGLU && list.cut > 0 && mine) {
+                const int c = tile_index(m0 / p.cut.rows, nb, (p.M + p.cut.rows - 1) / p.cut.rows, list.n_blocks, p.cut.group) - p.cut.full;
+                mine = (item.part >= 0) == (c >= 0);
+                if (item.part >= 0 && mine) slot = (size_t)(c * p.cut.parts + item.part) * (p.cut.rows / BM) + m0 % p.cut.rows / BM;
+            }
             if (!mbar_wait(&tfull[group], use++ & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
             __syncwarp();
             fence_after_sync();
             const bool none = item.kb0 == item.kb1;       // of a product without depth: nothing was accumulated
             uint32_t v[kSlabs * 32];
-            if (!SWIGLU && item.slot >= 0) {
+            if (!SWIGLU && item.part >= 0) {
                 // [column / 4][row][4]: the lanes of a warp write neighbouring rows of a column group
-                float4* dst = reinterpret_cast<float4*>(p.ws) + (size_t)(item.slot * (TM / BM) + rank * C::kHalves + h) * (BM * BN / 4) + row;
+                float4* dst = reinterpret_cast<float4*>(p.ws) + slot * (BM * BN / 4) + row;
 #pragma unroll 1
                 for (int slab = 0; slab < kSlabs; ++slab) {
                     uint32_t r[64];
@@ -440,10 +565,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     if (none)
 #pragma unroll
                         for (int c = 0; c < 64; ++c) r[c] = 0;
+                    if (mine)
 #pragma unroll
-                    for (int c = 0; c < 16; ++c)
-                        dst[(slab * 16 + c) * BM] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
-                                                                __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
+                        for (int c = 0; c < 16; ++c)
+                            dst[(slab * 16 + c) * BM] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
+                                                                    __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
                 }
             } else {
 #pragma unroll
@@ -512,7 +638,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (issuer) epi_stop[group] = *abort_flag;
             group_sync();
             if (epi_stop[group]) break;
-            if (!SWIGLU && item.slot >= 0) continue;
+            if (!SWIGLU && item.part >= 0) continue;
 #pragma unroll
             for (int slab = 0; slab < kSlabs; ++slab) {
                 const int n0 = (SWIGLU ? nb * 128 : nb * BN) + slab * 64;
@@ -527,7 +653,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 group_sync();
                 if (issuer) {
                     if (p.mode == 0) {
-                        if (m0 < p.M && n0 < p.N) tma_store_2d(&tmC.m[0], buf, n0, m0);
+                        if (mine && n0 < p.N) tma_store_2d(&tmC.m[0], buf, n0, m0);
                     } else if (p.mode == 1) {
                         const int b = n0 / p.blk;
                         tma_store_2d(&tmC.m[b % p.world], buf, (b / p.world) * p.blk + n0 % p.blk, p.row_off + m0);
@@ -559,7 +685,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 // ---- choice of the tile ----
 struct Plan {
     int rows;              // of a tile
-    int full, parts;       // tiles that are one item each; items that each of the others is cut into
+    Cut cut;
+    int halves;            // see TileList::halves
     float time;            // estimated, us
 };
 
@@ -573,15 +700,52 @@ constexpr float kLong = 100.f;
 // 448 429 / 394 / 445; 8192 x 8192: 256 47 / 55 / 55, 384 53 / 57 / 61, 448 59 / 59 / 65; 3584 x 3584: 64 17 / 21 / 24, 384 21.5 / 23.5 / 27.
 constexpr int kShallow = 6 * BK, kStaged = 5 * BK;
 
-// The tile size, of those that M fills more than half of, with the shortest estimate.
-inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool may_split) {
-    Plan best{BM, 0, 1, 0.f};
+// Time of a product on tiles of `rows` rows, in us.  The list is dealt out one by one: the CTA
+// with the most work has the last tile in one go, or is the first behind it.
+inline Plan plan_tiles(int M, int N, int K, int BN, int rows, int workers, const Cut& cut) {
+    const int kb = (K + BK - 1) / BK;
+    const float unit = tile_time(kb, rows, BN), operands = 2.f * K * ((float)M + N) / 6.2e6f;
+    const TileList l = make_list(M, N, K, rows, BN, cut, 0);
+    const int q = l.whole / workers, r = l.whole % workers, parts = l.cut * l.parts;
+    Plan p{rows, cut, 0, 0.f};
+    if (l.cut) {
+        const int each = parts / workers, more = parts % workers;        // parts go to the CTAs from number r on
+        const float first = r ? q + 1 + (float)(each + (more > workers - r)) / l.parts : 0.f;
+        const float other = q + (float)(each + (more > 0)) / l.parts;
+        p.time = unit * (first > other ? first : other);
+    } else {
+        p.time = unit * (q + (r > 0));
+        // 512 rows: the last tiles as two halves each, where these fit one round.  152 tiles on 74 pairs (4096 x 4864 x 2568) 101.4 us whole,
+        // 99.3 with halves, 101.4 on tiles of 256 rows; behind one round only 256 rows are faster: 96 tiles (3626 x 2992 x 3880) 93.2, 91.5, 89.1.
+        if (rows == 4 * BM && q >= 2 && r && 2 * r <= workers) {
+            p.halves = r;
+            p.time = unit * q + tile_time(kb, 2 * BM, BN) + 1.f;
+        }
+    }
+    if (p.time < operands) p.time = operands;
+    if (l.cut) p.time += 6.f + (((M + BM - 1) / BM) * l.n_blocks - cut.full) * l.parts * (BM * BN * 8e-6f / 4.f);      // the sums
+    return p;
+}
+
+// The tile size, of those that M fills more than half of, with the shortest estimate.  device_rows: the device counts the rows, M at most.
+inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool may_split, bool device_rows = false) {
+    Cut cut;
+    if (may_split) cut = split_plan(M, N, K, BN, sms);
+    Plan best{BM, cut, 0, 0.f};
     float least = 1e30f;
     for (int rows = BM; rows == BM || (may_pair && K > kShallow && rows <= 4 * BM && M > rows / 2); rows *= 2) {
-        const TailPlan t = plan_tail(M, N, K, BN, rows, rows > BM ? sms / 2 : sms, may_split ? 16 : 1, 1 << 30);
-        if (t.time < least) {
-            least = t.time;
-            best = {rows, t.full, t.parts, t.time};
+        const int workers = rows > BM ? sms / 2 : sms;
+        Plan p = plan_tiles(M, N, K, BN, rows, workers, cut);
+        if (device_rows) {
+            p.cut.rows = rows;
+            p.cut.group = (rows == BM ? 1024 : 4096) / rows;
+            p.cut.parts = 1;                                    // the device's plan takes its place
+            p.halves = 0;
+            p.time = plan_tail(M, N, K, BN, rows, workers, 16, 1 << 30).time;
+        }
+        if (p.time < least) {
+            least = p.time;
+            best = p;
         }
     }
     return best;
@@ -589,9 +753,9 @@ inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool 
 
 // bytes of the workspace that the plan's split tiles take (their fp32 sums)
 inline long long split_bytes(const Plan& p, int M, int N, int BN) {
-    if (p.parts == 1) return 0;
-    const long long tiles = (long long)((M + p.rows - 1) / p.rows) * ((N + BN - 1) / BN);
-    return (tiles - p.full) * p.parts * p.rows * BN * 4;
+    if (p.cut.parts == 1) return 0;
+    const long long tiles = (long long)((M + p.cut.rows - 1) / p.cut.rows) * ((N + BN - 1) / BN);
+    return (tiles - p.cut.full) * p.cut.parts * p.cut.rows * BN * 4;
 }
 
 inline int sm_count() {
@@ -604,30 +768,30 @@ inline int sm_count() {
     return sms;
 }
 
-// C tile = bf16(sum over the parts of the workspace + bias); a thread makes 8 columns of a row
-template <int BN, int TM>
-__global__ void __launch_bounds__(256) sum_parts_kernel(const float* ws, bf16* C, const bf16* bias,
-                                                        int M, int N, long long ldc, int full, int parts, int group_m,
+// Cut block of C = bf16(sum over the parts of the workspace + bias); a thread makes 8 columns of a row
+template <int BN>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* ws, bf16* C, const bf16* bias, int M, int N, long long ldc, Cut cut,
                                                         const int* count, int count_base) {
     wait_for_predecessor();
     let_successor_start();
-    const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM % (BN / 8), half = i / (BM * BN / 8), t = blockIdx.y;
+    const int i = blockIdx.x * 256 + threadIdx.x, row = i % BM, cg = i / BM % (BN / 8), sub = i / (BM * BN / 8), t = blockIdx.y;
     int mb, nb;                                                                                   // cg: group of 8 columns
     if (count != nullptr) {
         M = min(M, max(0, *count - count_base));
-        full = reinterpret_cast<const int*>(ws)[0];
-        parts = reinterpret_cast<const int*>(ws)[1];
+        cut.full = reinterpret_cast<const int*>(ws)[0];
+        cut.parts = reinterpret_cast<const int*>(ws)[1];
         ws += kPlanBytes / 4;
-        if (parts == 1 || full + t >= ((M + TM - 1) / TM) * ((N + BN - 1) / BN)) return;
+        if (cut.parts == 1 || cut.full + t >= ((M + cut.rows - 1) / cut.rows) * ((N + BN - 1) / BN)) return;
     }
-    tile_coords(full + t, (M + TM - 1) / TM, (N + BN - 1) / BN, group_m, mb, nb);
-    const int m = mb * TM + half * BM + row, n = nb * BN + cg * 8;
+    tile_coords(cut.full + t, (M + cut.rows - 1) / cut.rows, (N + BN - 1) / BN, cut.group, mb, nb);
+    const int m = mb * cut.rows + sub * BM + row, n = nb * BN + cg * 8, parts = cut.parts;
     if (m >= M || n >= N) return;
-    const float4* src = reinterpret_cast<const float4*>(ws) + ((size_t)t * parts * (TM / BM) + half) * (BM * BN / 4) + (size_t)(2 * cg) * BM + row;
+    const size_t step = (size_t)cut.rows * BN / 4;               // between the parts of a block, in float4
+    const float4* src = reinterpret_cast<const float4*>(ws) + t * parts * step + (size_t)sub * (BM * BN / 4) + (size_t)(2 * cg) * BM + row;
     float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
     for (int q = 0; q < parts; ++q) {
-        const float4 a = src[(size_t)q * (TM * BN / 4)], b = src[(size_t)q * (TM * BN / 4) + BM];
+        const float4 a = src[q * step], b = src[q * step + BM];
         f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
         f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
     }
@@ -653,7 +817,7 @@ struct Route {
     bool counts_depth = false;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool SWIGLU, int TM, bool SHALLOW = false>
+template <int BN, bool A_MN, bool B_MN, bool SWIGLU, int TM, bool SHALLOW = false, bool COUNTED = false>
 int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
                  long long ldc, int* status, cudaStream_t st, const Route& rt, const Plan& plan, float* ws) {
     using C = Cfg<BN, TM, SHALLOW>;
@@ -686,31 +850,31 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
             if (r) return 3000 + r;
         }
     }
-    auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU, TM, SHALLOW>;
+    auto kern = gemm_kernel<BN, A_MN, B_MN, SWIGLU, TM, SHALLOW, COUNTED>;
     static bool done = false;
     if (!done) {
         r = opt_in(kern, C::kSmem, kThreads, (kIssueRegs + 2 * kEpiRegs) * 128);
         if (r) return r;
         done = true;
     }
-    Params p{M, N, K, (const bf16*)bias, status, (TM == BM ? 1024 : 4096) / TM, rt.mode, rt.blk, rt.world, rt.rank, rt.mode == 1 ? 0 : rt.row_off,
+    Params p{M, N, K, (const bf16*)bias, status, rt.mode, rt.blk, rt.world, rt.rank, rt.mode == 1 ? 0 : rt.row_off,
              rt.stats, rt.n_slots, rt.n_slots > 0 ? N / rt.n_slots : N};
-    const int tiles = ((M + TM - 1) / TM) * (SWIGLU ? N / 128 : (N + BN - 1) / BN), rem = tiles - plan.full;
-    const int items = plan.full + rem * plan.parts, workers = PAIR ? sm_count() / 2 : sm_count();
+    const int workers = PAIR ? sm_count() / 2 : sm_count();
     const bool dynamic_rows = rt.count != nullptr && !rt.counts_depth;
-    if (rem || dynamic_rows) {
-        p.full = plan.full;
-        p.parts = plan.parts;
-        p.ws = ws;
-    }
+    p.cut = plan.cut;
+    p.list = make_list(M, SWIGLU ? 2 * N : N, K, TM, BN, plan.cut, plan.halves);
+    const int items = item_count(p.list);
+    if (plan.cut.parts > 1 || dynamic_rows) p.ws = ws;
     p.count = rt.count;
     p.count_base = rt.count_base;
     p.counts_depth = rt.counts_depth;
     r = launch_after_if(plan.time < kLong, kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
     if (r) return r;
-    const int may_split = dynamic_rows ? (ws ? workers - 1 : 0) : rem;       // tiles
-    if (may_split)
-        return launch_after(sum_parts_kernel<BN, TM>, 1, dim3(TM * BN / 8 / 256, may_split), 256, 0, st, ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.full, plan.parts, p.group_m, dynamic_rows ? rt.count : nullptr, rt.count_base);
+    const int cut = dynamic_rows ? (ws ? workers - 1 : 0)                    // blocks, at most
+                    : plan.cut.parts > 1 ? ((M + plan.cut.rows - 1) / plan.cut.rows) * ((N + BN - 1) / BN) - plan.cut.full : 0;
+    if (cut)
+        return launch_after(sum_parts_kernel<BN>, 1, dim3(plan.cut.rows * BN / 8 / 256, cut), 256, 0, st, ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc,
+                            plan.cut, dynamic_rows ? rt.count : nullptr, rt.count_base);
     return (int)cudaGetLastError();
 }
 
@@ -718,9 +882,17 @@ template <int BN, bool A_MN, bool B_MN, bool SWIGLU = false>
 int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int N, int K, long long lda, long long ldb,
            long long ldc, int* status, cudaStream_t st, const Route& rt = Route(), float* ws = nullptr, long long ws_bytes = 0) {
     const bool may_pair = BN == 256 && rt.mode == 0, may_split = !SWIGLU && ws && rt.mode == 0;
-    Plan plan = make_plan(M, SWIGLU ? 2 * N : N, K, BN, sm_count(), may_pair, may_split);      // a tile of a SwiGLU product: 128 features
-    if (rt.count != nullptr && !rt.counts_depth) plan.full = ((M + plan.rows - 1) / plan.rows) * ((N + BN - 1) / BN), plan.parts = 1;
-    if (split_bytes(plan, M, N, BN) > ws_bytes) plan = make_plan(M, N, K, BN, sm_count(), may_pair, false);
+    const int cols = SWIGLU ? 2 * N : N;                  // a tile of a SwiGLU product: 128 features
+    const bool device_rows = rt.count != nullptr && !rt.counts_depth;
+    Plan plan = make_plan(M, cols, K, BN, sm_count(), may_pair, may_split, device_rows);
+    if (split_bytes(plan, M, cols, BN) > ws_bytes) plan = make_plan(M, cols, K, BN, sm_count(), may_pair, false, device_rows);
+    if constexpr (BN == 256 && !SWIGLU && (!A_MN || B_MN))
+        if (rt.count != nullptr) {
+            plan.halves = 0;
+            if (plan.rows == 512) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 512, false, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
+            if (plan.rows == 256) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 256, false, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
+            return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM, false, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
+        }
     if constexpr (BN == 256) {
         if (plan.rows == 512) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 512>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
         if (plan.rows == 256) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 256>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
@@ -792,7 +964,7 @@ MM_API int mm_gemm_bf16_ws(const void* A, const void* B, void* C, const void* bi
 MM_API long long mm_gemm_rows_ws_bytes(int M, int N, int K, int a_mn, int b_mn) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     const int sms = sm_count();
-    const Plan plan = make_plan(M, N, K, 256, sms, true, true);
+    const Plan plan = make_plan(M, N, K, 256, sms, true, true, !(a_mn && b_mn));
     if (a_mn && b_mn) return split_bytes(plan, M, N, 256);
     return kPlanBytes + (long long)kMostRounds * (plan.rows > BM ? sms / 2 : sms) * plan.rows * 256 * 4;
 }

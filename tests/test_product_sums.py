@@ -1,0 +1,65 @@
+"""Which blocks of a product are cut along K, and into how many parts: this is the order of an output's fp32 sum, and with it its bits."""
+import os
+
+import pytest
+import torch
+
+from mindspeed_mm_b200.ops import build, native
+
+DEV = "cuda"
+
+
+def _cut(M, N, K, bn, sms=148):
+    """(blocks of 128 x bn in one go, parts of each of the others): what is shortest on tiles of 128 rows, one for each SM."""
+    tiles, kb = -(-M // 128) * -(-N // bn), -(-K // 64)
+    full, rem = divmod(tiles, sms)
+    best, unit, operands = (tiles, 1), kb * 0.44 * bn / 256, 2.0 * K * (M + N) / 6.2e6
+    least = max(unit * (full + 1), operands) - 4.0
+    for parts in range(2, 17):
+        if not rem or kb // parts < 4:
+            break
+        t = max(unit * full + unit * -(-rem * parts // sms) / parts, operands) + 6.0 + rem * parts * (128 * bn * 8e-6 / 4.0)
+        if t < least:
+            least, best = t, (tiles - rem, parts)
+    return best
+
+
+@pytest.mark.skipif(not os.path.exists(build.lib_path()), reason="the library is not built")
+@pytest.mark.parametrize("N,K", [(4608, 3584), (3584, 3584), (37888, 3584), (3584, 18944), (3840, 1280), (1280, 3456), (6912, 1280), (1536, 8960), (200, 8192)])
+def test_what_is_cut_depends_on_128_row_tiles_alone(N, K):
+    """Rows from 5 to 9000, products of several models' layers: a prompt's logits move by more than a bf16 rounding where another rule cuts."""
+    bn = 256 if N >= 256 else 128
+    for M in [*range(5, 600, 7), *range(600, 4000, 31), *range(4000, 9000, 127)]:
+        full, parts = _cut(M, N, K, bn)
+        want = (-(-M // 128) * -(-N // bn) - full) * parts * 128 * bn * 4 if parts > 1 else 0
+        assert native.lib().mm_gemm_ws_bytes(M, N, K, 0, 0, bn) == want, (M, N, K)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K", [(136, 200, 8200), (405, 3584, 37888), (1421, 3584, 3600), (520, 9480, 4104), (2533, 5752, 6480), (2400, 32008, 5208), (4096, 4864, 2568),
+                                   (3118, 3304, 3760), (2560, 3840, 18944), (17232, 4608, 18192), (1100, 3584, 3584)])
+def test_blocks_are_cut_as_the_rule_says_on_every_tile(layout, M, N, K):
+    """2^30 first, then ones, then -2^30: a sum in one go loses the ones (32 for 16 of K is under half an ulp at 2^30); in parts, each but the
+    first keeps its own.  Tiles of 128, 256 and 512 rows, halves of the last, tiles with blocks of both kinds; all sums are exact."""
+    kb = -(-K // 64)
+    row = torch.zeros(K)
+    row[0], row[64:(kb - 1) * 64], row[K - 1] = 2.0 ** 15, 1.0, -(2.0 ** 15)
+    col = torch.zeros(K)
+    col[0], col[64:(kb - 1) * 64], col[K - 1] = 2.0 ** 15, 2.0, 2.0 ** 15
+    a, col_of_a = row.bfloat16().to(DEV).expand(M, K).contiguous(), row.bfloat16().to(DEV)[:, None]
+    b = col.bfloat16().to(DEV).expand(N, K).contiguous()
+    got = {"nt": lambda: native.gemm_nt(a, b), "nn": lambda: native.gemm_nn(a, b.t().contiguous()),
+           "tn": lambda: native.gemm_tn(col_of_a.expand(K, -(-M // 8) * 8).contiguous()[:, :M], b.t().contiguous())}[layout]()
+    native.check_status()
+    bn = 256 if N >= 256 else 128
+    full, parts = _cut(M, N, K, bn)
+    m_blocks, n_blocks = -(-M // 128), -(-N // bn)
+    want = torch.zeros(m_blocks, n_blocks)
+    kept = 128.0 * (kb - 1 - kb // parts) if parts > 1 else 0.0
+    for t in range(full, m_blocks * n_blocks):             # groups of 8 row blocks, column by column
+        first = t // (8 * n_blocks) * 8
+        rows, at = min(8, m_blocks - first), t - first * n_blocks
+        want[first + at % rows, at // rows] = kept
+    want = want.bfloat16().to(DEV).repeat_interleave(128, 0)[:M].repeat_interleave(bn, 1)[:, :N]
+    assert torch.equal(got, want)
