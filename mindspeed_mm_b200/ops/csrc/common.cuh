@@ -20,7 +20,7 @@ enum MmStatus : int { MM_OK = 0, MM_TIMEOUT_TMA = 1, MM_TIMEOUT_MMA = 2, MM_TIME
 // that a successor may rely on everything in front of this kernel being complete.
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Products, their split tails' sums and attention are launched so: between dependent kernels lay 2.5 us.  A decoder layer on 1421 tokens
+// Products and attention are launched so: between dependent kernels lay 2.5 us.  A decoder layer on 1421 tokens
 // took 2.05 ms, 1.99 then; a vision block on 8192 patches 1.43, 1.40.  Row kernels and grouped products gained nothing or lost (an expert
 // layer 1.71, 1.80): blocks that come up beside the predecessor's last ones are spread unevenly over the SMs.
 template <class... P, class... A>
