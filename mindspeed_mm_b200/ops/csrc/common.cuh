@@ -16,8 +16,12 @@ enum MmStatus : int { MM_OK = 0, MM_TIMEOUT_TMA = 1, MM_TIMEOUT_MMA = 2, MM_TIME
 // A kernel that is launched by launch_after() may start before its predecessor has ended: wait_for_predecessor() comes before its first
 // access to global memory, and the loads behind it are not marked as of constant memory (no __restrict__ const parameter, no __ldg: the
 // compiler may move those up past the wait).
-// let_successor_start() lets such a successor come up as soon as every block of this kernel has; it stands after the wait, never before, so
-// that a successor may rely on everything in front of this kernel being complete.
+// let_successor_start() lets such a successor come up as soon as every block of this kernel has called it or ended.
+//  - In a kernel launched by launch_after() it stands behind the wait: a successor may rely on everything in front of this kernel being
+//    complete.  One launched in the ordinary way starts when all in front of it is complete, so it may call it at once; such a kernel must never
+//    be launched by launch_after() as it is.
+//  - Behind the allocation of tensor memory: a successor allocates before its own wait, and could otherwise hold the columns of an SM that a
+//    block of this kernel, which it waits for, still needs.
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Products and attention are launched so: between dependent kernels lay 2.5 us.  A decoder layer on 1421 tokens

@@ -36,7 +36,6 @@ __global__ void __launch_bounds__(320, 1)
 fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
     wait_for_predecessor();
-    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     constexpr int BQ = 128;
     extern __shared__ uint8_t smem_raw[];
@@ -111,6 +110,7 @@ fmha_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    let_successor_start();           // behind the allocation, see common.cuh
     const uint32_t tST = tmem_base, tdPT = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
 
     if (warp == 0) {

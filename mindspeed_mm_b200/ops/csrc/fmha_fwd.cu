@@ -58,7 +58,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaParams p) {
     wait_for_predecessor();
-    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -123,6 +122,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    let_successor_start();           // behind the allocation, see common.cuh
     const uint32_t tS = tmem_base, tO = tmem_base + 256;
 
     if (warp == 0) {

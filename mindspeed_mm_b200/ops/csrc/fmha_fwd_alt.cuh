@@ -30,7 +30,6 @@ constexpr int kAltSmem = (kAltK + kAltV) * kTileBytes + 256 + 4 * 128 * 4 + 1024
 __global__ void __launch_bounds__(kAltThreads, 1)
 fmha_fwd_alt_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, FmhaParams p) {
     wait_for_predecessor();
-    let_successor_start();
     if ((int)tile_of(p.heads_first) >= *p.n_tiles) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -87,6 +86,7 @@ fmha_fwd_alt_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    let_successor_start();           // behind the allocation, see common.cuh
     const uint32_t tS = tmem_base, tO = tmem_base + 256, tQ = tmem_base + 384, tP = tmem_base + 448;
 
     if (warp < 4) {

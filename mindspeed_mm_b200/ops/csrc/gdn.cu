@@ -51,7 +51,6 @@ struct GdnParams {
 __global__ void __launch_bounds__(192, 1)
 gdn_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmA, const GdnParams p) {
-    let_successor_start();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sStage = smem;                          // [2][W | Qg | Kd | At]
@@ -95,6 +94,7 @@ gdn_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    let_successor_start();           // behind the allocation, see common.cuh
     const uint32_t tS = tmem_base, tD1 = tmem_base + 128, tD2 = tmem_base + 192;
 
     if (warp == 0) {

@@ -64,7 +64,6 @@ __device__ __forceinline__ void store_row_bf16(uint8_t* dst, int v, const float*
 __global__ void __launch_bounds__(192, 1)
 gdn_bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmA, const GdnBwdParams p) {
-    let_successor_start();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sStage = smem;                          // [2][W | Qg | Kd | At]
@@ -109,6 +108,7 @@ gdn_bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    let_successor_start();           // behind the allocation, see common.cuh
     const uint32_t tG = tmem_base, tE = tmem_base + 128;
 
     if (warp == 0) {

@@ -80,7 +80,6 @@ template <int MODE, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, GGParams p) {
-    let_successor_start();
     constexpr int kBBytes = Cfg<BN>::kBBytes, kStageBytes = Cfg<BN>::kStageBytes, kStages = Cfg<BN>::kStages;
     constexpr int kTmemCols = Cfg<BN>::kTmemCols;
     extern __shared__ uint8_t smem_raw[];
@@ -123,6 +122,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    let_successor_start();           // behind the allocation, see common.cuh
 
     if (warp == 0) {
         if (lane == 0) {
