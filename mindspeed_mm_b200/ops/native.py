@@ -380,16 +380,18 @@ def _rope_call(x, cos, sin, interleaved, backward):
 
 
 class _Rope(torch.autograd.Function):
+    """The rotation or, with ``back``, its transpose: each is the other's gradient, which can so be differentiated in its turn."""
+
     @staticmethod
-    def forward(ctx, x, cos, sin, interleaved):
+    def forward(ctx, x, cos, sin, interleaved, back):
         ctx.save_for_backward(cos, sin)
-        ctx.interleaved = interleaved
-        return _rope_call(x, cos, sin, interleaved, False)
+        ctx.meta = interleaved, back
+        return _rope_call(x, cos, sin, interleaved, back)
 
     @staticmethod
     def backward(ctx, dy):
-        cos, sin = ctx.saved_tensors
-        return _rope_call(dy, cos, sin, ctx.interleaved, True), None, None, None
+        interleaved, back = ctx.meta
+        return _run(_Rope, dy, *ctx.saved_tensors, interleaved, not back), None, None, None, None
 
 
 def rope(x, cos, sin, interleaved: bool):
@@ -406,7 +408,7 @@ def rope(x, cos, sin, interleaved: bool):
             _eager("rope_rotate_half", x, f"D={D}")
             return reference.rope_rotate_half(x, cos, sin)
         cos, sin = cos.to(torch.bfloat16).contiguous(), sin.to(torch.bfloat16).contiguous()
-    return _run(_Rope, x, cos, sin, interleaved)
+    return _run(_Rope, x, cos, sin, interleaved, False)
 
 
 def _rope_parts(q, k, v, cos, sin, outs, backward):
@@ -458,8 +460,8 @@ class _SplitRope(torch.autograd.Function):
         cos, sin = ctx.saved_tensors
         nq, nk, D = ctx.heads
         T = dq.shape[0]
-        if torch.is_grad_enabled():          # create_graph: the values' part is differentiated
-            return torch.cat([_rope_call(t, cos, sin, False, True).view(T, -1) for t in (dq, dk)] + [dv.reshape(T, -1)], dim=1), None, None, None, None
+        if torch.is_grad_enabled():          # create_graph: all three parts are differentiated
+            return torch.cat([*(_run(_Rope, t, cos, sin, False, True).view(T, -1) for t in (dq, dk)), dv.reshape(T, -1)], dim=1), None, None, None, None
         dqkv = torch.empty(T, (nq + 2 * nk) * D, dtype=dq.dtype, device=dq.device)
         _rope_parts(dq, dk, dv, cos, sin, [t.view(T, -1, D) for t in dqkv.split([nq * D, nk * D, nk * D], dim=1)], True)
         return dqkv, None, None, None, None

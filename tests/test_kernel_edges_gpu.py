@@ -693,3 +693,25 @@ def test_delta_rule_gradients_keep_a_graph_where_they_had_one():
     x, s = torch.randn(5, 384, device=DEV).bfloat16().requires_grad_(), torch.ones((), device=DEV, requires_grad=True)
     (dx,) = torch.autograd.grad((ops.delta_heads(x, 1, 1, 128, 128)[2].float() * s).sum(), [x], create_graph=True)
     assert float(torch.autograd.grad(dx.float().sum(), [s])[0]) == 5 * 128
+
+
+@pytest.mark.parametrize("T,nq,nk,D", [(1, 1, 1, 16), (37, 4, 2, 80), (33, 2, 2, 72), (65, 3, 3, 128)])
+def test_gradients_of_a_rotation_can_be_differentiated(T, nq, nk, D):
+    """create_graph: a rotation's gradient is linear in the incoming one, so its derivative by that is the rotation itself, to the bit; the
+    derivative after that is the gradient again."""
+    torch.manual_seed(T)
+    ang = torch.randn(T, D, device=DEV)
+    cos, sin, half_cos, half_sin = ang.cos().bfloat16(), ang.sin().bfloat16(), ang[:, :D // 2].cos().contiguous(), ang[:, :D // 2].sin().contiguous()
+    bf = lambda *s: torch.randn(*s, device=DEV).bfloat16()  # noqa: E731
+    width = (nq + 2 * nk) * D
+    for op, shape in ((lambda t: ops.split_rope(t, nq, nk, cos, sin), (T, width)), (lambda t: (ops.rope_rotate_half(t, cos, sin),), (T, nq, D)),
+                      (lambda t: (ops.rope_interleaved(t, half_cos, half_sin),), (T, nq, D))):
+        x, r = bf(*shape).requires_grad_(), bf(*shape)
+        outs = op(x)
+        dys = [bf(*o.shape).requires_grad_() for o in outs]
+        (g,) = torch.autograd.grad(outs, x, dys, create_graph=True)
+        seconds = torch.autograd.grad(g, dys, r.requires_grad_(), create_graph=True)
+        for a, b in zip(seconds, op(r.detach())):
+            assert torch.equal(a, b)
+        (third,) = torch.autograd.grad(seconds, r, [d.detach() for d in dys])
+        assert torch.equal(third, g)
