@@ -194,9 +194,10 @@ struct Params {
     const int* count = nullptr;
     int count_base = 0;
     bool counts_depth = false;
+    int most_items = 0;            // of the cut blocks, that the workspace has room for
 };
 constexpr int kPlanBytes = 256;        // in front of the sums in the workspace of such a product
-constexpr int kMostRounds = 8;         // of its split items, which the workspace (310 MB for tiles of 512 rows) is made for
+constexpr int kMostRounds = 8;         // of its split items
 
 constexpr int kMaxDst = 8;
 struct TMapSet {
@@ -244,16 +245,17 @@ __host__ __device__ inline float tile_time(int kb, int rows, int BN) {
     return (rows == BM ? kb * 0.45f : rows == 2 * BM ? kb * 0.415f : kb * 0.79f + 1.f) * BN / 256;
 }
 
-// Cut and time of a product whose number of rows only the device knows: the tiles themselves are the units, and their own times decide.
+// Cut and time of a product whose number of rows only the device knows: the tiles themselves are the units, and their own times decide.  Whole
+// tiles are counted, so that there is one cut for each number of row blocks.
 struct TailPlan {
     float time;
     int full, parts;
 };
 __host__ __device__ inline TailPlan plan_tail(int M, int N, int K, int BN, int rows, int workers, int most_parts, int most_items) {
-    const int kb = (K + BK - 1) / BK;
-    const float operands = 2.f * K * ((float)M + N) / 6.2e6f;
+    const int kb = (K + BK - 1) / BK, m_blocks = (M + rows - 1) / rows;
+    const float operands = 2.f * K * ((float)m_blocks * rows + N) / 6.2e6f;
     auto at_least = [&](float t) { return t > operands ? t : operands; };
-    const int tiles = ((M + rows - 1) / rows) * ((N + BN - 1) / BN), full = tiles / workers, rem = tiles % workers;
+    const int tiles = m_blocks * ((N + BN - 1) / BN), full = tiles / workers, rem = tiles % workers;
     const float unit = tile_time(kb, rows, BN);
     const float whole = at_least(unit * (full + (rem ? 1 : 0)));
     TailPlan best{whole, tiles, 1};
@@ -332,7 +334,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (p.ws != nullptr && !p.counts_depth) {
             int* plan = reinterpret_cast<int*>(tmem_slot + 4);
             if (threadIdx.x == 0) {
-                const TailPlan t = plan_tail(p.M, p.N, p.K, BN, TM, n_workers, 16, kMostRounds * n_workers);
+                const TailPlan t = plan_tail(p.M, p.N, p.K, BN, TM, n_workers, 16, p.most_items);
                 plan[0] = t.full;
                 plan[1] = t.parts;
                 if (blockIdx.x == 0) {
@@ -688,6 +690,7 @@ struct Plan {
     Cut cut;
     int halves;            // see TileList::halves
     float time;            // estimated, us
+    int most_items = 0;    // see Params::most_items
 };
 
 // A product that takes longer (us) starts when the kernel in front has ended: CTAs that come up one by one on SMs as these fall idle lose more
@@ -870,9 +873,10 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
     p.count = rt.count;
     p.count_base = rt.count_base;
     p.counts_depth = rt.counts_depth;
+    p.most_items = plan.most_items;
     r = launch_after_if(plan.time < kLong, kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
     if (r) return r;
-    const int cut = dynamic_rows ? (ws ? workers - 1 : 0)                    // blocks, at most
+    const int cut = dynamic_rows ? (plan.most_items / 2 < workers ? plan.most_items / 2 : workers - 1)           // blocks, at most
                     : plan.cut.parts > 1 ? ((M + plan.cut.rows - 1) / plan.cut.rows) * ((N + BN - 1) / BN) - plan.cut.full : 0;
     if (cut)
         sum_parts_kernel<BN><<<dim3(plan.cut.rows * BN / 8 / 256, cut), 256, 0, st>>>(ws, (bf16*)Cc, (const bf16*)bias, M, N, ldc, plan.cut,
@@ -891,6 +895,7 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
     if constexpr (BN == 256 && !SWIGLU && (!A_MN || B_MN))
         if (rt.count != nullptr) {
             plan.halves = 0;
+            if (device_rows) plan.most_items = (int)((ws_bytes - kPlanBytes) / (plan.rows * BN * 4));
             if (plan.rows == 512) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 512, false, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
             if (plan.rows == 256) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 256, false, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
             return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM, false, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
@@ -968,7 +973,15 @@ MM_API long long mm_gemm_rows_ws_bytes(int M, int N, int K, int a_mn, int b_mn) 
     const int sms = sm_count();
     const Plan plan = make_plan(M, N, K, 256, sms, true, true, !(a_mn && b_mn));
     if (a_mn && b_mn) return split_bytes(plan, M, N, 256);
-    return kPlanBytes + (long long)kMostRounds * (plan.rows > BM ? sms / 2 : sms) * plan.rows * 256 * 4;
+    // what the most that any number of rows is cut into takes.  The device is told the room, not the count: its divisions may round otherwise
+    const int workers = plan.rows > BM ? sms / 2 : sms;
+    int most = 0;
+    for (int m = 1; m <= (M + plan.rows - 1) / plan.rows; ++m) {
+        const TailPlan t = plan_tail(m * plan.rows, N, K, 256, plan.rows, workers, 16, kMostRounds * workers);
+        const int items = t.parts > 1 ? (m * ((N + 255) / 256) - t.full) * t.parts : 0;
+        if (items > most) most = items;
+    }
+    return kPlanBytes + (long long)most * plan.rows * 256 * 4;
 }
 MM_API int mm_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int a_mn,
                              int b_mn, const int* count, int base, int* status, void* ws, long long ws_bytes, cudaStream_t st) {

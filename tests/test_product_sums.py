@@ -35,6 +35,18 @@ def test_what_is_cut_depends_on_128_row_tiles_alone(N, K):
         assert native.lib().mm_gemm_ws_bytes(M, N, K, 0, 0, bn) == want, (M, N, K)
 
 
+@pytest.mark.skipif(not os.path.exists(build.lib_path()), reason="the library is not built")
+@pytest.mark.parametrize("T,V,H", [(513, 512, 256), (600, 152064, 3584), (2048, 152064, 3584), (8192, 152064, 3584), (1, 256, 256)])
+def test_the_workspace_of_a_loss_is_bounded_by_its_products(T, V, H):
+    """fp32 sums of 16 parts for each tile of 512 rows (256 columns), of at most eight rounds on half of the SMs; short main loops have fewer."""
+    for M, N, K, b_mn in ((T, V, H, 0), (T, H, V, 1)):
+        got = native.lib().mm_gemm_rows_ws_bytes(M, N, K, 0, b_mn)
+        tiles, parts = -(-M // 512) * -(-N // 256), min(16, -(-K // 64) // 4)
+        assert got <= 256 + 512 * 256 * 4 * (min(8 * 74, min(73, tiles) * parts) if parts > 1 else 0), (M, N, K)
+        if T == 600:                        # (they are held one after the other) no more than a quarter of the logits, which are 182 MB
+            assert got <= T * V * 2 // 4
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K", [(136, 200, 8200), (405, 3584, 37888), (1421, 3584, 3600), (520, 9480, 4104), (2533, 5752, 6480), (2400, 32008, 5208), (4096, 4864, 2568),
