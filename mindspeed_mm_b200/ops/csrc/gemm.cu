@@ -35,7 +35,7 @@ constexpr int BK = 64;
 constexpr int kGroupThreads = 128;                        // of an epilogue group
 constexpr int kThreads = 128 + 2 * kGroupThreads;
 // registers of a thread: 168 at launch; the epilogue holds a packed accumulator row, the issuing warps need few
-constexpr int kIssueRegs = 56, kEpiRegs = 224;
+constexpr int kIssueRegs = 72, kEpiRegs = 216;
 constexpr int kSmemBudget = 227 * 1024;
 
 // TM: rows of a tile.  128: one CTA;  256 and 512: a pair of CTAs on two SMs, each with half of the rows and, for the operands, half of the
@@ -169,6 +169,12 @@ __host__ __device__ inline Item item_at(const TileList& l, int i) {
     return it;
 }
 
+struct Work {
+    TileList list;
+    Cut cut;
+    int M;
+};
+
 struct Params {
     int M, N, K;
     const bf16* bias;
@@ -186,9 +192,8 @@ struct Params {
     float* stats = nullptr;
     int n_slots = 1, per_slot = 0;
     // split tail (see Cut): fp32 sums of the parts go to `ws`
-    Cut cut;
     float* ws = nullptr;
-    TileList list;                 // (made by the host unless the device counts: the index arithmetic takes 1 - 2 us, longer than a launch is worth)
+    Work work;                     // (made by the host unless the device counts: the index arithmetic takes 1 - 2 us, longer than a launch is worth)
     // M (or, with `counts_depth`, K) is what `count` on the device says, less `count_base` and at most what is given here; the tail is then
     // planned by the kernel, which leaves {full, parts} in front of the workspace
     const int* count = nullptr;
@@ -326,30 +331,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     wait_for_predecessor();
     let_successor_start();
 
-    TileList counted;
+    Work& counted = *reinterpret_cast<Work*>(tmem_slot + 4);
     if constexpr (COUNTED) {
-        const int n = max(0, *p.count - p.count_base);
-        if (p.counts_depth) p.K = min(p.K, n);
-        else p.M = min(p.M, n);
-        if (p.ws != nullptr && !p.counts_depth) {
-            int* plan = reinterpret_cast<int*>(tmem_slot + 4);
-            if (threadIdx.x == 0) {
-                const TailPlan t = plan_tail(p.M, p.N, p.K, BN, TM, n_workers, 16, p.most_items);
-                plan[0] = t.full;
-                plan[1] = t.parts;
+        if (threadIdx.x == 0) {
+            const int n = max(0, *p.count - p.count_base);
+            Work w = p.work;
+            if (p.counts_depth) p.K = min(p.K, n);
+            else w.M = min(p.M, n);
+            if (p.ws != nullptr && !p.counts_depth) {
+                const TailPlan t = plan_tail(w.M, p.N, p.K, BN, TM, n_workers, 16, p.most_items);
+                w.cut.full = t.full;
+                w.cut.parts = t.parts;
                 if (blockIdx.x == 0) {
-                    reinterpret_cast<int*>(p.ws)[0] = t.full;
-                    reinterpret_cast<int*>(p.ws)[1] = t.parts;
+                    int* plan = reinterpret_cast<int*>(p.ws - kPlanBytes / 4);
+                    plan[0] = t.full;
+                    plan[1] = t.parts;
                 }
             }
-            __syncthreads();
-            p.cut.full = plan[0];
-            p.cut.parts = plan[1];
-            p.ws += kPlanBytes / 4;
+            w.list = make_list(w.M, p.N, p.K, TM, BN, w.cut, 0);
+            counted = w;
         }
-        counted = make_list(p.M, p.N, p.K, TM, BN, p.cut, 0);
+        __syncthreads();
     }
-    const TileList& list = COUNTED ? counted : p.list;
+    const Work& work = COUNTED ? counted : p.work;          // (in shared memory: registers for it would be spilled)
+    const TileList& list = work.list;
     const int n_items = item_count(list);
 
     if (warp < 4) {
@@ -542,12 +547,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (C::kHalves == 2 && item.half >= 0 && item.half != group) continue;
             const int mb = item.mb, nb = item.nb;
             const int h = C::kHalves == 1 ? 0 : group, m0 = mb * TM + rank * (TM / 2) + h * BM;
-            bool mine = m0 < p.M;                         // these 128 rows are what the item is there for
+            bool mine = m0 < work.M;                      // these 128 rows are what the item is there for
             size_t slot = 0;                              // of the workspace, in blocks of 128 rows
             if (!SWIGLU && list.cut > 0 && mine) {
-                const int c = tile_index(m0 / p.cut.rows, nb, (p.M + p.cut.rows - 1) / p.cut.rows, list.n_blocks, p.cut.group) - p.cut.full;
+                const Cut& cut = work.cut;
+                const int c = tile_index(m0 / cut.rows, nb, (work.M + cut.rows - 1) / cut.rows, list.n_blocks, cut.group) - cut.full;
                 mine = (item.part >= 0) == (c >= 0);
-                if (item.part >= 0 && mine) slot = (size_t)(c * p.cut.parts + item.part) * (p.cut.rows / BM) + m0 % p.cut.rows / BM;
+                if (item.part >= 0 && mine) slot = (size_t)(c * cut.parts + item.part) * (cut.rows / BM) + m0 % cut.rows / BM;
             }
             if (!mbar_wait(&tfull[group], use++ & 1, abort_flag) && lane == 0) atomicExch(p.status, MM_TIMEOUT_EPI);
             __syncwarp();
@@ -866,10 +872,10 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
              rt.stats, rt.n_slots, rt.n_slots > 0 ? N / rt.n_slots : N};
     const int workers = PAIR ? sm_count() / 2 : sm_count();
     const bool dynamic_rows = rt.count != nullptr && !rt.counts_depth;
-    p.cut = plan.cut;
-    p.list = make_list(M, SWIGLU ? 2 * N : N, K, TM, BN, plan.cut, plan.halves);
-    const int items = item_count(p.list);
-    if (plan.cut.parts > 1 || dynamic_rows) p.ws = ws;
+    p.work = {make_list(M, SWIGLU ? 2 * N : N, K, TM, BN, plan.cut, plan.halves), plan.cut, M};
+    const int items = item_count(p.work.list);
+    if (dynamic_rows) p.ws = ws + kPlanBytes / 4;
+    else if (plan.cut.parts > 1) p.ws = ws;
     p.count = rt.count;
     p.count_base = rt.count_base;
     p.counts_depth = rt.counts_depth;
