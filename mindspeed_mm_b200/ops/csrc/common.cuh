@@ -28,10 +28,10 @@ __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcon
 // took 2.05 ms, 1.99 then; a vision block on 8192 patches 1.43, 1.40.  Row kernels and grouped products gained nothing or lost (an expert
 // layer 1.71, 1.80): blocks that come up beside the predecessor's last ones are spread unevenly over the SMs.
 template <class... P, class... A>
-inline int launch_after_if(bool early, void (*kern)(P...), int cluster, dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+inline int launch_after(void (*kern)(P...), int cluster, dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = early;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = cluster;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
@@ -43,10 +43,6 @@ inline int launch_after_if(bool early, void (*kern)(P...), int cluster, dim3 gri
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-template <class... P, class... A>
-inline int launch_after(void (*kern)(P...), int cluster, dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
-    return launch_after_if(true, kern, cluster, grid, threads, smem, st, args...);
 }
 
 struct alignas(16) Vec8 {

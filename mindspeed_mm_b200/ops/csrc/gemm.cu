@@ -699,11 +699,6 @@ struct Plan {
     int most_items = 0;    // see Params::most_items
 };
 
-// A product that takes longer (us) starts when the kernel in front has ended: CTAs that come up one by one on SMs as these fall idle lose more
-// over its time than the gap that they save.  The three products of the vocabulary loss, behind one another, early / not: 256 rows
-// 840 / 825 us, 310 rows 1061 / 1034, 400 rows 1280 / 1187.
-constexpr float kLong = 100.f;
-
 // Depth up to which tiles are one CTA's: the accumulators are emptied and written as long as the next tile's products take, or longer, and
 // a CTA of a pair waits for both of its halves.  152064 x 3584, 128 / 256 / 512 rows: depth 256 299 / 339 / 342 us, 384 388 / 400 / 411,
 // 448 429 / 394 / 445; 8192 x 8192: 256 47 / 55 / 55, 384 53 / 57 / 61, 448 59 / 59 / 65; 3584 x 3584: 64 17 / 21 / 24, 384 21.5 / 23.5 / 27.
@@ -880,7 +875,7 @@ int launch_tiles(const void* A, const void* B, void* Cc, const void* bias, int M
     p.count_base = rt.count_base;
     p.counts_depth = rt.counts_depth;
     p.most_items = plan.most_items;
-    r = launch_after_if(plan.time < kLong, kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
+    r = launch_after(kern, PAIR ? 2 : 1, dim3((items < workers && !dynamic_rows ? items : workers) * (PAIR ? 2 : 1)), kThreads, C::kSmem, st, tA, tB, tC, p);
     if (r) return r;
     const int cut = dynamic_rows ? (plan.most_items / 2 < workers ? plan.most_items / 2 : workers - 1)           // blocks, at most
                     : plan.cut.parts > 1 ? ((M + plan.cut.rows - 1) / plan.cut.rows) * ((N + BN - 1) / BN) - plan.cut.full : 0;
