@@ -697,6 +697,7 @@ struct Plan {
     int halves;            // see TileList::halves
     float time;            // estimated, us
     int most_items = 0;    // see Params::most_items
+    bool staged = false;   // two staging slabs an epilogue group, see Cfg
 };
 
 // Depth up to which tiles are one CTA's: the accumulators are emptied and written as long as the next tile's products take, or longer, and
@@ -752,6 +753,7 @@ inline Plan make_plan(int M, int N, int K, int BN, int sms, bool may_pair, bool 
             best = p;
         }
     }
+    best.staged = best.rows == BM && BN == 256 && K <= kStaged;
     return best;
 }
 
@@ -906,7 +908,7 @@ int launch(const void* A, const void* B, void* Cc, const void* bias, int M, int 
         if (plan.rows == 256) return launch_tiles<BN, A_MN, B_MN, SWIGLU, 256>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
     }
     if constexpr (BN == 256 && !SWIGLU)
-        if (K <= kStaged) return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
+        if (plan.staged) return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM, true>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
     return launch_tiles<BN, A_MN, B_MN, SWIGLU, BM>(A, B, Cc, bias, M, N, K, lda, ldb, ldc, status, st, rt, plan, ws);
 }
 
