@@ -75,3 +75,52 @@ def test_blocks_are_cut_as_the_rule_says_on_every_tile(layout, M, N, K):
         want[first + at % rows, at // rows] = kept
     want = want.bfloat16().to(DEV).repeat_interleave(128, 0)[:M].repeat_interleave(bn, 1)[:, :N]
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,widths", [(1421, (3584, 3584, 4096, 3584)), (405, (3584, 4608, 3584, 1536)), (3118, (3760, 3304, 3760, 1024)), (2560, (8192, 3840, 1280, 3840))])
+def test_products_behind_one_another_repeat_to_the_bit(T, widths):
+    """Each starts while the one in front drains and reads what that one, or the sums of its split tail, has written: the same results as with a wait
+    between them.  Tiles of 128, 256 and 512 rows, cut and not."""
+    torch.manual_seed(T)
+    x = torch.randn(T, widths[0], device=DEV).bfloat16()
+    weights = [(torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16() for k, n in zip(widths, widths[1:])]
+    want = [x]
+    for w in weights:
+        want.append(native.gemm_nt(want[-1], w))
+        torch.cuda.synchronize()
+    same = torch.ones((), dtype=torch.bool, device=DEV)
+    for _ in range(60):
+        rows = [x]
+        for w in weights:
+            rows.append(native.gemm_nt(rows[-1], w))
+        back = native.gemm_nn(native.gemm_nn(rows[-1], weights[-1]), weights[-2])
+        for a, b in zip(rows, want):
+            same &= (a == b).all()
+        del rows, back
+    native.check_status()
+    assert bool(same)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,H,V,valid,chunk", [(1600, 1024, 18944, 1421, 8192), (700, 512, 4096, 65, 256), (513, 256, 512, 0, 8192), (300, 1024, 8192, 200, 8192)])
+def test_a_loss_repeats_to_the_bit(T, H, V, valid, chunk):
+    """Its chain of products over counted rows, softmax, gathers and sums, many times without a wait."""
+    torch.manual_seed(T)
+    h = torch.randn(T, H, device=DEV).bfloat16().requires_grad_()
+    w = (0.02 * torch.randn(V, H, device=DEV)).bfloat16().requires_grad_()
+    lab = torch.full((T,), -100, device=DEV)
+    lab[torch.randperm(T, device=DEV)[:valid]] = torch.randint(0, V, (valid,), device=DEV)
+
+    def once():
+        loss = native.linear_cross_entropy(h, w, lab, -100, chunk)[0]
+        return (loss.detach(), *torch.autograd.grad(loss, [h, w]))
+
+    torch.cuda.synchronize()
+    want = [t.clone() for t in once()]
+    same = torch.ones((), dtype=torch.bool, device=DEV)
+    for _ in range(40):
+        for a, b in zip(once(), want):
+            same &= (a == b).all()
+    native.check_status()
+    assert bool(same)
