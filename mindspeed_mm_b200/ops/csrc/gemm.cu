@@ -18,12 +18,12 @@
 // All mbarrier waits are bounded (tc05::mbar_wait); a timeout is reported through `status` and the CTA
 // unwinds: it lets in-flight copies land, frees its TMEM and returns.
 //
-// What bounds a large product is the power cap: every tile size keeps the tensor pipe 90 to 96 % busy, at a clock that the energy of its
-// operand traffic sets.  A step of 64 of K brings a CTA 48 KB for 128 x 256 (one CTA), 32 KB for the same as half of a 256-row pair, and
-// 48 KB for 256 x 256 as half of a 512-row pair: 19.1 / 14.5 GB through L2 for 8192 x 37888 x 3584 with 256 / 512 rows.  Sustained, TFLOP/s, tiles
-// of 128 / 256 / 512 rows (cuBLAS): 8192 x 37888 x 3584 1202 / 1432 / 1430 (1416), 8192 x 3584 x 18944 1209 / 1291 / 1399 (1238), 32760 x 5120 x
-// 13824 1188 / 1274 / 1388 (1401), 8192 x 3840 x 1280 1104 / 1157 / 1107 (1130).  Groups of 4096 rows against 1024 / 2048 / 8192: 1432 against
-// 1292 / 1350 (256 rows), 1430 against 1421 / 1381 at 2048 / 8192 (512 rows, 8192 x 37888 x 3584); single tiles are used for few rows only.
+// What bounds a large product with a long main loop is the power cap: every tile size keeps the tensor pipe 90 to 96 % busy, at a clock that the
+// energy of its operand traffic sets.  A step of 64 of K brings a CTA 48 KB for 128 x 256 (one CTA), 32 KB for the same as half of a 256-row pair,
+// and 48 KB for 256 x 256 as half of a 512-row pair: 19.1 / 14.5 GB through L2 for 8192 x 37888 x 3584 with 256 / 512 rows.  Sustained, TFLOP/s, tiles
+// of 128 / 256 / 512 rows (cuBLAS): 8192 x 37888 x 3584 1198 / 1350 / 1388 (1356), 8192 x 3584 x 18944 1224 / 1278 / 1344 (1216), 32760 x 5120 x
+// 13824 1161 / 1198 / 1309 (1376), 8192 x 3840 x 1280 1075 / 1149 / 1126 (1108).  Groups of 1024 / 2048 / 8192 rows reach 0.90 / 0.94 / - of the rate
+// of groups of 4096 on tiles of 256 rows, - / 0.99 / 0.97 on 512 (8192 x 37888 x 3584); single tiles are used for few rows only.
 #include "tc05.cuh"
 
 namespace {
@@ -41,9 +41,10 @@ constexpr int kSmemBudget = 227 * 1024;
 // TM: rows of a tile.  128: one CTA;  256 and 512: a pair of CTAs on two SMs, each with half of the rows and, for the operands, half of the
 // columns (cta_group::2).
 // SHALLOW (depth up to kStaged): the stores take longer than the products, so each epilogue group has two staging slabs, for one operand
-// stage less: one store is under way while the next slab is written.  The gradient of a vocabulary's weight (152064 x 3584) over 256 rows,
-// behind the products that make its operand: 377 us with one slab a group, 336 with two; 310 rows 381, 372; 350 rows 408, 423: from there on
-// the fourth stage is worth more.
+// stage less: one store is under way while the next slab is written.  One slab a group / two, us: 152064 x 3584 at depth 128 311 / 227, at 256
+// 328 / 320, at 384 419 / 453; 37888 x 3584 at 64 118 / 88, 256 111 / 103, 320 112 / 114; 8192 x 8192 at 64 52 / 40, 256 51 / 49, 320 52 / 54; 3584 x 3584 at
+// 64 12.8 / 10.8, 320 15.9 / 15.4.  The gradient of a vocabulary's weight over 310 rows, behind the products that make its operand, is what the
+// line at 320 is for: 381 / 372, 350 rows 408 / 423.
 template <int BN, int TM, bool SHALLOW = false>
 struct Cfg {
     static constexpr bool kPair = TM > BM;

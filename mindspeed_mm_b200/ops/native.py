@@ -948,7 +948,8 @@ def lce_supported(h, w) -> bool:
 
 
 # Up to here a vocabulary product costs little less for fewer rows (its weight's bytes): with 70 % of the rows in use, 256 / 512 / 1024 / 8192
-# rows took 974 / 1497 / 2774 / 20566 us over all of them and 989 / 1491 / 2583 / 15249 over those.
+# rows take 928 / 1451 / 2695 / 19980 us over all of them and 1027 / 1460 / 2498 / 14990 over those.  Where all rows have a target the list is what
+# it costs: 1024 / 2048 / 8192 rows 2764 / 5222 / 20490 us without it, 2819 / 5366 / 20460 with it.
 _LIST_ROWS = 512
 
 
@@ -973,7 +974,7 @@ class _LinearCE(torch.autograd.Function):
 
     Rows without a target (prompts, images, padding) have neither loss nor gradient: the others are listed on the device, gathered,
     and the three products run over as many rows as the list has (which the host is not told).  8192 rows of which 70 % have
-    a target, vocabulary 152064: 20.6 -> 15.2 ms; where all of 2048 have one, the list costs 5.24 -> 5.43 ms."""
+    a target, vocabulary 152064: 20.0 -> 15.0 ms; where all of 2048 have one, the list costs 5.22 -> 5.37 ms."""
 
     @staticmethod
     def forward(ctx, h, w, labels, ignore_index, chunk):
